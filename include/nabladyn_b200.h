@@ -191,6 +191,19 @@ typedef struct nd_lj_batch_args {
 /* E, F, W of every frame. */
 int nd_lj_batch_forward(const nd_lj_batch_args* args, nd_stream_t stream);
 
+/* E, F, W of every frame over a caller-owned workspace of nd_lj_workspace_bytes bytes
+ * (256-byte aligned): packed atoms and forces, which the kernels gather and add 16 bytes at a
+ * time. Unlike nd_lj_batch_forward's, `energy` [F] and `virial` [F, 3, 3] point to values of the
+ * frames' dtype (their sums are float64 all the same); with `wrap` nonzero the positions may
+ * lie anywhere. */
+int64_t nd_lj_workspace_bytes(int dtype, int64_t frames, int64_t num_atoms);
+int nd_lj_frames(const nd_lj_batch_args* args, int32_t wrap, void* workspace, nd_stream_t stream);
+
+/* Positions [F, N, 3] wrapped into [0, L) by cells [F, 3] (src/nabladyn/space.py:22-38 without
+ * the crossings). `wrapped` may be `positions`. */
+int nd_wrap(int dtype, const void* positions, const void* cells, int64_t frames,
+            int64_t num_atoms, void* wrapped, nd_stream_t stream);
+
 /* The hand-written parameter backward: dLoss/dsigma and dLoss/depsilon from the gradients of
  * the loss with respect to every frame's E, F and W (the reference takes it by torch.func
  * double backward). */

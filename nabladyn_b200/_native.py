@@ -7,6 +7,7 @@ the torch.library layer and returns ``torch.ops.nabladyn_neighbors``. Both raise
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 from pathlib import Path
 from threading import RLock
@@ -314,6 +315,10 @@ _SIGNATURES = {
     "nd_lj_energy_force_virial": [ctypes.POINTER(LJPairsArgs), ctypes.c_void_p],
     "nd_lj_batch_forward": [ctypes.POINTER(LJBatchArgs), ctypes.c_void_p],
     "nd_lj_batch_parameter_backward": [ctypes.POINTER(LJBatchArgs), ctypes.c_void_p],
+    "nd_lj_frames": [ctypes.POINTER(LJBatchArgs), ctypes.c_int32, ctypes.c_void_p,
+                     ctypes.c_void_p],
+    "nd_wrap": [ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64,
+                ctypes.c_void_p, ctypes.c_void_p],
     "nd_md_import": [
         ctypes.POINTER(MDSystem), ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
         ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
@@ -352,6 +357,7 @@ _SIGNATURES = {
 
 # name -> (argument types) of the entry points that return a byte count (int64, -1 on error).
 _SIZES = {
+    "nd_lj_workspace_bytes": [ctypes.c_int, ctypes.c_int64, ctypes.c_int64],
     "nd_schnet_weight_bytes": [ctypes.c_int32, ctypes.c_int32],
     "nd_schnet_workspace_bytes": [ctypes.c_int64, ctypes.c_int64, ctypes.c_int32],
     "nd_schnet_atom_parameter_floats": [ctypes.c_int32, ctypes.c_int32],
@@ -423,6 +429,16 @@ def call(name: str, *args) -> None:
 def stream_handle(device: torch.device) -> int:
     """The raw cudaStream_t of torch's current stream on ``device``."""
     return torch.cuda.current_stream(device).cuda_stream
+
+
+_NOTHING = contextlib.nullcontext()
+
+
+def on_device(device: torch.device):
+    """``torch.cuda.device(device)``, or nothing to enter when it is the current device."""
+    if device.index is None or device.index == torch.cuda.current_device():
+        return _NOTHING
+    return torch.cuda.device(device)
 
 
 def dtype_code(dtype: torch.dtype) -> int:

@@ -57,4 +57,18 @@ __device__ __forceinline__ T wrap_axis(T x, T length, long long& crossings)
     return wrapped;
 }
 
+__device__ __forceinline__ float multiply(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double multiply(double a, double b) { return __dmul_rn(a, b); }
+
+// x wrapped into [0, L) in the rounding of separate elementwise operations, as
+// nabladyn_b200/space.py computes it on tensors: the product is rounded before it is
+// subtracted (wrap_axis above leaves the contraction to the compiler).
+template <typename T>
+__device__ __forceinline__ T wrap_separately(T x, T length)
+{
+    T wrapped = x - multiply(floor(x / length), length);
+    wrapped = wrapped < T(0) ? wrapped + length : wrapped;
+    return wrapped >= length ? wrapped - length : wrapped;
+}
+
 }  // namespace nd

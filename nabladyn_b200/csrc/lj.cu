@@ -19,9 +19,11 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "common.cuh"
+#include "geometry.cuh"
 
 namespace nd {
 
@@ -40,6 +42,20 @@ __device__ __forceinline__ T displacement(T left, T right, T length)
     return (left - left_shift) - (right - right_shift);
 }
 
+// Positions [F, N, 3] wrapped into [0, L) by their frame's cell, in one pass instead of the
+// dozen elementwise ones of space.wrap.
+template <typename T>
+__global__ void __launch_bounds__(kThreads) wrap_kernel(
+    const T* __restrict__ positions, const T* __restrict__ cells, std::int64_t num_atoms,
+    std::int64_t values, T* __restrict__ wrapped)
+{
+    const std::int64_t k = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (k < values)
+    {
+        wrapped[k] = wrap_separately(positions[k], cells[k / (3 * num_atoms) * 3 + k % 3]);
+    }
+}
+
 __device__ __forceinline__ int pair_row(int a, int b, int num_types)
 {
     const int low = a < b ? a : b;
@@ -54,6 +70,40 @@ struct LJAccumulators
     T w[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};  // row-major W
 };
 
+// Block sums of `count` per-thread values in float64, one atomic per block into out[k].
+template <int kCount>
+__device__ __forceinline__ void add_block_sums(double (&values)[kCount], double* const (&out)[kCount])
+{
+    __shared__ double partial[kCount][kLJThreads / kWarp];
+    const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
+#pragma unroll
+    for (int k = 0; k < kCount; ++k)
+    {
+        values[k] = warp_sum(values[k]);
+        if (lane == 0)
+        {
+            partial[k][warp] = values[k];
+        }
+    }
+    __syncthreads();
+    if (warp == 0)
+    {
+#pragma unroll
+        for (int k = 0; k < kCount; ++k)
+        {
+            double v = lane < kLJThreads / kWarp ? partial[k][lane] : 0.0;
+            v = warp_sum(v);
+            if (lane == 0)
+            {
+                atomicAdd(out[k], v);
+            }
+        }
+    }
+}
+
+// One frame with a strain, or with the energy's parameter gradients (the model's own energy
+// under autograd): one column per thread, scalar atomics. Calls without either run
+// lj_frames_kernel below.
 template <typename T, bool kParameterGrads, bool kStrained>
 __global__ void __launch_bounds__(kLJThreads) lj_pairs_kernel(
     const T* __restrict__ positions,
@@ -74,14 +124,6 @@ __global__ void __launch_bounds__(kLJThreads) lj_pairs_kernel(
     double* __restrict__ epsilon_grad
 )
 {
-    // Frame blockIdx.y of a batch of frames with the same atoms and capacity.
-    const std::int64_t frame = blockIdx.y;
-    positions += frame * 3 * num_atoms;
-    cell += frame * 3;
-    pairs += frame * 2 * capacity;
-    energy += frame;
-    forces += frame * 3 * num_atoms;
-    virial += frame * 9;
     const int rows = num_types * (num_types + 1) / 2;
     __shared__ double row_grads[2 * kMaxRows];
     if (kParameterGrads)
@@ -194,8 +236,6 @@ __global__ void __launch_bounds__(kLJThreads) lj_pairs_kernel(
         acc.w[6] = acc.w[2];
         acc.w[7] = acc.w[5];
     }
-    __shared__ double partial[10][kLJThreads / kWarp];
-    const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
     double values[10];
     values[0] = double(acc.energy);
 #pragma unroll
@@ -203,29 +243,9 @@ __global__ void __launch_bounds__(kLJThreads) lj_pairs_kernel(
     {
         values[k + 1] = double(acc.w[k]);
     }
-#pragma unroll
-    for (int k = 0; k < 10; ++k)
-    {
-        values[k] = warp_sum(values[k]);
-        if (lane == 0)
-        {
-            partial[k][warp] = values[k];
-        }
-    }
-    __syncthreads();
-    if (warp == 0)
-    {
-#pragma unroll
-        for (int k = 0; k < 10; ++k)
-        {
-            double v = lane < kLJThreads / kWarp ? partial[k][lane] : 0.0;
-            v = warp_sum(v);
-            if (lane == 0)
-            {
-                atomicAdd(k == 0 ? energy : virial + (k - 1), v);
-            }
-        }
-    }
+    double* const out[10] = {energy, virial, virial + 1, virial + 2, virial + 3, virial + 4,
+                             virial + 5, virial + 6, virial + 7, virial + 8};
+    add_block_sums(values, out);
     if (kParameterGrads)
     {
         __syncthreads();
@@ -237,58 +257,612 @@ __global__ void __launch_bounds__(kLJThreads) lj_pairs_kernel(
     }
 }
 
+// ---------------------------------------------------------------------------------------
+// E, F and W of F frames of one system, without strain or parameter gradients: the path of
+// quantity.energy_force_virial and of the training predictions.
+//
+// What bounds it is the force scatter and the position gathers through L2, not the index
+// stream: one column costs two gathered atoms and two scattered forces, 48 B of L2 traffic
+// each way against 8 B of index. So:
+//   * atoms are gathered as packed (x, y, z, type) slots, one 16-B load each instead of three
+//     scalar ones and a type load; the pass that packs them wraps them too;
+//   * float32 forces are summed into packed [N, 4] slots, one 16-B vector atomic per atom
+//     instead of three scalar ones, and unpacked by the closing pass (float64 has no vector
+//     atomic and adds its three components in place);
+//   * a warp takes 128 consecutive columns, four per lane. The list groups its columns by
+//     first atom (about 60 columns each in a liquid), so a lane sums its first atom's force
+//     in registers, the lanes that end on the same first atom meet in a segmented warp sum,
+//     and a first atom costs two or three atomics instead of one per column. An index in any
+//     other order gives the same sums with more atomics.
+
+// Blocks an SM holds: the registers of four columns in flight, 80 (float32) or 124 (float64).
+template <typename T>
+constexpr int kFrameBlocksPerSM = sizeof(T) == 4 ? 3 : 2;
+
+constexpr int kLaneColumns = 4;                          // consecutive columns per lane
+constexpr int kWarpColumns = kWarp * kLaneColumns;
+
+// An atom as the kernels gather it; w holds the type's bits. 16-B aligned: float64 slots are
+// two 16-B words.
+template <typename T>
+struct alignas(16) PackedAtom
+{
+    T x, y, z, w;
+};
+
+__device__ __forceinline__ float type_word(float, index_t type) { return __int_as_float(type); }
+__device__ __forceinline__ double type_word(double, index_t type)
+{
+    return __longlong_as_double(static_cast<long long>(type));
+}
+__device__ __forceinline__ int word_type(float w) { return __float_as_int(w); }
+__device__ __forceinline__ int word_type(double w)
+{
+    return static_cast<int>(__double_as_longlong(w));
+}
+
+constexpr int kFrameSums = 7;  // E, W xx yy zz xy xz yz
+constexpr int kFrameSlots = 8;
+
+// The workspace of a batch: float64 sums per frame, packed atoms, and (float32) packed forces.
+template <typename T>
+struct FrameWorkspace
+{
+    std::int64_t sums, atoms, forces, total;
+
+    FrameWorkspace(std::int64_t frames, std::int64_t num_atoms)
+    {
+        const std::int64_t slots = frames * num_atoms;
+        sums = 0;
+        atoms = (frames * kFrameSlots * 8 + 255) / 256 * 256;
+        forces = atoms + (slots * static_cast<std::int64_t>(sizeof(PackedAtom<T>)) + 255) / 256 * 256;
+        total = forces + (sizeof(T) == 4 ? slots * 16 : 0);
+    }
+};
+
+// Packs the atoms (wrapped into the cell first when kWrap, in space.wrap's rounding) and sets
+// the sums and the forces to zero. One thread per atom of the batch.
+template <typename T, bool kWrap>
+__global__ void __launch_bounds__(kThreads) pack_atoms_kernel(
+    const T* __restrict__ positions, const T* __restrict__ cells,
+    const index_t* __restrict__ atom_types, index_t num_atoms, std::int64_t slots,
+    std::int64_t frames, PackedAtom<T>* __restrict__ atoms, float4* __restrict__ packed_forces,
+    T* __restrict__ forces, double* __restrict__ sums)
+{
+    const std::int64_t slot = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    for (std::int64_t k = slot; k < frames * kFrameSlots;
+         k += static_cast<std::int64_t>(gridDim.x) * blockDim.x)
+    {
+        sums[k] = 0.0;
+    }
+    if (slot >= slots)
+    {
+        return;
+    }
+    const std::int64_t frame = slot / num_atoms;
+    const index_t atom = static_cast<index_t>(slot - frame * num_atoms);
+    const T* cell = cells + 3 * frame;
+    PackedAtom<T> p;
+    p.x = positions[3 * slot];
+    p.y = positions[3 * slot + 1];
+    p.z = positions[3 * slot + 2];
+    if (kWrap)
+    {
+        p.x = wrap_separately(p.x, cell[0]);
+        p.y = wrap_separately(p.y, cell[1]);
+        p.z = wrap_separately(p.z, cell[2]);
+    }
+    p.w = type_word(T(0), atom_types == nullptr ? 0 : atom_types[atom]);
+    atoms[slot] = p;
+    if (packed_forces != nullptr)
+    {
+        packed_forces[slot] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    else
+    {
+        forces[3 * slot] = T(0);
+        forces[3 * slot + 1] = T(0);
+        forces[3 * slot + 2] = T(0);
+    }
+}
+
+// Unpacks the forces (float32) and casts the sums: E [F] and W [F, 3, 3] in the frames' dtype.
+template <typename T>
+__global__ void __launch_bounds__(kThreads) unpack_frames_kernel(
+    const float4* __restrict__ packed_forces, std::int64_t slots, std::int64_t frames,
+    const double* __restrict__ sums, float* __restrict__ forces, T* __restrict__ energy,
+    T* __restrict__ virial)
+{
+    const std::int64_t slot = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    for (std::int64_t k = slot; k < frames * 10;
+         k += static_cast<std::int64_t>(gridDim.x) * blockDim.x)
+    {
+        constexpr int place[10] = {0, 1, 4, 5, 4, 2, 6, 5, 6, 3};  // E, then W row-major
+        const std::int64_t frame = k / 10;
+        const int entry = static_cast<int>(k - 10 * frame);
+        int from = 0;
+#pragma unroll
+        for (int e = 0; e < 10; ++e)
+        {
+            from = entry == e ? place[e] : from;
+        }
+        const double value = sums[kFrameSlots * frame + from];
+        if (entry == 0)
+        {
+            energy[frame] = static_cast<T>(value);
+        }
+        else
+        {
+            virial[9 * frame + entry - 1] = static_cast<T>(value);
+        }
+    }
+    if (packed_forces != nullptr && slot < slots)
+    {
+        const float4 f = packed_forces[slot];
+        forces[3 * slot] = f.x;
+        forces[3 * slot + 1] = f.y;
+        forces[3 * slot + 2] = f.z;
+    }
+}
+
+// Four consecutive ints of a row from element c; elements at or past `end` read as `fill`.
+// `skew` is the row's offset from a 16-B boundary, in ints (the same for every thread): an
+// interior lane reads whole aligned words and takes its four from them, so an odd capacity
+// (whose second row starts anywhere) costs one more word, not four scalar loads.
+__device__ __forceinline__ void load_columns(const index_t* __restrict__ row, std::int64_t c,
+                                             std::int64_t end, int skew, index_t fill,
+                                             index_t (&out)[kLaneColumns])
+{
+    const std::int64_t from = c - skew;
+    if (from >= 0 && from + (skew == 0 ? 4 : 8) <= end)
+    {
+        const int4 a = *reinterpret_cast<const int4*>(row + from);
+        if (skew == 0)
+        {
+            out[0] = a.x;
+            out[1] = a.y;
+            out[2] = a.z;
+            out[3] = a.w;
+            return;
+        }
+        const int4 b = *reinterpret_cast<const int4*>(row + from + 4);
+        out[0] = skew == 1 ? a.y : (skew == 2 ? a.z : a.w);
+        out[1] = skew == 1 ? a.z : (skew == 2 ? a.w : b.x);
+        out[2] = skew == 1 ? a.w : (skew == 2 ? b.x : b.y);
+        out[3] = skew == 1 ? b.x : (skew == 2 ? b.y : b.z);
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < kLaneColumns; ++k)
+    {
+        out[k] = c + k < end ? row[c + k] : fill;
+    }
+}
+
+__device__ __forceinline__ int row_skew(const index_t* row)
+{
+    return static_cast<int>((reinterpret_cast<std::uintptr_t>(row) / sizeof(index_t)) % 4);
+}
+
+// The four columns from element c: first and second atoms, -1 past the capacity.
+__device__ __forceinline__ void load_pairs(const index_t* __restrict__ pairs,
+                                           std::int64_t capacity, std::int64_t c, int skew_first,
+                                           int skew_second, index_t (&i)[kLaneColumns],
+                                           index_t (&j)[kLaneColumns])
+{
+    load_columns(pairs, c, capacity, skew_first, -1, i);
+    load_columns(pairs + capacity, c, capacity, skew_second, -1, j);
+}
+
+// A column counts when its atoms differ and both lie in [0, N): self-pairs are padding, an
+// index outside is skipped and never read.
+__device__ __forceinline__ bool counts(index_t i, index_t j, index_t num_atoms)
+{
+    return i != j && static_cast<unsigned>(i) < static_cast<unsigned>(num_atoms) &&
+           static_cast<unsigned>(j) < static_cast<unsigned>(num_atoms);
+}
+
+// One type-pair row's constants, in the pair arithmetic's dtype.
+template <typename T>
+struct RowConstants
+{
+    T s2, eps4, eps24, shift;
+};
+
+template <typename T>
+struct FramesPass
+{
+    const PackedAtom<T>* atoms;   // packed, or null: positions and types below
+    const T* positions;
+    const index_t* atom_types;    // null: one type
+    const T* cells;
+    const index_t* pairs;
+    std::int64_t capacity;
+    index_t num_atoms;
+    int num_types;
+    const T* sigma;
+    const T* epsilon;
+    T cutoff_squared;
+    float4* packed_forces;        // float32 with a workspace; else the forces below
+    T* forces;
+    double* sums;                 // packed: [F][8]; else null and the two below
+    double* energy;
+    double* virial;
+};
+
+template <typename T, bool kPacked>
+__device__ __forceinline__ void add_force(const FramesPass<T>& a, index_t atom, T x, T y, T z)
+{
+    if constexpr (kPacked && sizeof(T) == 4)
+    {
+        atomicAdd(a.packed_forces + atom, make_float4(x, y, z, 0.f));
+    }
+    else
+    {
+        T* f = a.forces + 3LL * atom;
+        atomicAdd(f, x);
+        atomicAdd(f + 1, y);
+        atomicAdd(f + 2, z);
+    }
+}
+
+template <typename T, bool kPacked>
+__device__ __forceinline__ PackedAtom<T> gather(const FramesPass<T>& a, index_t atom)
+{
+    if constexpr (kPacked)
+    {
+        return a.atoms[atom];
+    }
+    else
+    {
+        const T* p = a.positions + 3LL * atom;
+        return {p[0], p[1], p[2],
+                type_word(T(0), a.atom_types == nullptr ? 0 : a.atom_types[atom])};
+    }
+}
+
+// Frame blockIdx.y; its warps take runs of 128 columns in turn.
+template <typename T, bool kPacked, bool kTypes>
+__global__ void __launch_bounds__(kLJThreads, kFrameBlocksPerSM<T>)
+lj_frames_kernel(FramesPass<T> a)
+{
+    const std::int64_t frame = blockIdx.y;
+    if (kPacked)
+    {
+        a.atoms += frame * a.num_atoms;
+        a.packed_forces += sizeof(T) == 4 ? frame * a.num_atoms : 0;
+    }
+    else
+    {
+        a.positions += 3 * frame * a.num_atoms;
+    }
+    if (!(kPacked && sizeof(T) == 4))
+    {
+        a.forces += 3 * frame * a.num_atoms;
+    }
+    a.cells += 3 * frame;
+    a.pairs += 2 * frame * a.capacity;
+    __shared__ RowConstants<T> rows[kTypes ? kMaxRows : 1];
+    const int row_count = kTypes ? a.num_types * (a.num_types + 1) / 2 : 1;
+    if (threadIdx.x < row_count)
+    {
+        const T s = a.sigma[threadIdx.x], eps = a.epsilon[threadIdx.x];
+        const T qc = s * s / a.cutoff_squared;
+        const T pc6 = qc * qc * qc;
+        rows[threadIdx.x] = {s * s, T(4) * eps, T(24) * eps, T(4) * eps * (pc6 * pc6 - pc6)};
+    }
+    __syncthreads();
+    const T lx = a.cells[0], ly = a.cells[1], lz = a.cells[2];
+    const int lane = threadIdx.x % kWarp;
+    const int skew_first = row_skew(a.pairs), skew_second = row_skew(a.pairs + a.capacity);
+    T energy = 0, wxx = 0, wyy = 0, wzz = 0, wxy = 0, wxz = 0, wyz = 0;
+    const std::int64_t warps = static_cast<std::int64_t>(gridDim.x) * (kLJThreads / kWarp);
+    std::int64_t base = (static_cast<std::int64_t>(blockIdx.x) * (kLJThreads / kWarp) +
+                         threadIdx.x / kWarp) * kWarpColumns;
+    index_t i[kLaneColumns], j[kLaneColumns];
+    if (base < a.capacity)
+    {
+        load_pairs(a.pairs, a.capacity, base + kLaneColumns * lane, skew_first, skew_second, i, j);
+    }
+    while (base < a.capacity)
+    {
+        // All gathers of the four columns before any is used.
+        PackedAtom<T> left[kLaneColumns], right[kLaneColumns];
+        bool live[kLaneColumns];
+#pragma unroll
+        for (int k = 0; k < kLaneColumns; ++k)
+        {
+            live[k] = counts(i[k], j[k], a.num_atoms);
+            right[k] = gather<T, kPacked>(a, live[k] ? j[k] : 0);
+            if (k > 0 && i[k] == i[k - 1])
+            {
+                left[k] = left[k - 1];
+            }
+            else
+            {
+                const bool inside = static_cast<unsigned>(i[k]) <
+                                    static_cast<unsigned>(a.num_atoms);
+                left[k] = gather<T, kPacked>(a, inside ? i[k] : 0);
+            }
+        }
+        index_t first[kLaneColumns], second[kLaneColumns];
+#pragma unroll
+        for (int k = 0; k < kLaneColumns; ++k)
+        {
+            first[k] = i[k];
+            second[k] = j[k];
+        }
+        // The next run's columns, loaded behind this run's arithmetic.
+        base += warps * kWarpColumns;
+        if (base < a.capacity)
+        {
+            load_pairs(a.pairs, a.capacity, base + kLaneColumns * lane, skew_first, skew_second,
+                       i, j);
+        }
+        index_t key = -1;
+        T fx = 0, fy = 0, fz = 0;  // the force on `key` from this lane's columns
+#pragma unroll
+        for (int k = 0; k < kLaneColumns; ++k)
+        {
+            const T dx = displacement(left[k].x, right[k].x, lx);
+            const T dy = displacement(left[k].y, right[k].y, ly);
+            const T dz = displacement(left[k].z, right[k].z, lz);
+            const T r2 = dx * dx + dy * dy + dz * dz;
+            if (!(live[k] && r2 < a.cutoff_squared))
+            {
+                continue;
+            }
+            const RowConstants<T> c =
+                rows[kTypes ? pair_row(word_type(left[k].w), word_type(right[k].w), a.num_types)
+                            : 0];
+            const T inv_r2 = T(1) / r2;
+            const T q = c.s2 * inv_r2;
+            const T p6 = q * q * q;
+            energy += c.eps4 * (p6 * p6 - p6) - c.shift;
+            const T fs = c.eps24 * (T(2) * p6 * p6 - p6) * inv_r2;
+            const T px = fs * dx, py = fs * dy, pz = fs * dz;
+            wxx += px * dx;
+            wyy += py * dy;
+            wzz += pz * dz;
+            wxy += px * dy;
+            wxz += px * dz;
+            wyz += py * dz;
+            add_force<T, kPacked>(a, second[k], -px, -py, -pz);
+            if (first[k] != key)
+            {
+                if (key >= 0)
+                {
+                    add_force<T, kPacked>(a, key, fx, fy, fz);
+                }
+                key = first[k];
+                fx = fy = fz = T(0);
+            }
+            fx += px;
+            fy += py;
+            fz += pz;
+        }
+        // Lanes in a row that end on the same first atom sum into their first lane.
+        __syncwarp();
+        const index_t before = __shfl_up_sync(kFullMask, key, 1);
+        const bool head = lane == 0 || before != key;
+        const unsigned heads = __ballot_sync(kFullMask, head);
+        const unsigned later = lane == kWarp - 1 ? 0u : heads >> (lane + 1);
+        const int reach = later == 0 ? kWarp - 1 - lane : __ffs(later) - 1;  // lanes after mine
+#pragma unroll
+        for (int offset = 1; offset < kWarp; offset *= 2)
+        {
+            const T ox = __shfl_down_sync(kFullMask, fx, offset);
+            const T oy = __shfl_down_sync(kFullMask, fy, offset);
+            const T oz = __shfl_down_sync(kFullMask, fz, offset);
+            if (offset <= reach)
+            {
+                fx += ox;
+                fy += oy;
+                fz += oz;
+            }
+        }
+        if (head && key >= 0)
+        {
+            add_force<T, kPacked>(a, key, fx, fy, fz);
+        }
+    }
+    double values[kFrameSums] = {double(energy), double(wxx), double(wyy), double(wzz),
+                                 double(wxy), double(wxz), double(wyz)};
+    if (kPacked)
+    {
+        double* s = a.sums + kFrameSlots * frame;
+        double* const out[kFrameSums] = {s, s + 1, s + 2, s + 3, s + 4, s + 5, s + 6};
+        add_block_sums(values, out);
+    }
+    else
+    {
+        double all[10] = {values[0], values[1], values[4], values[5], values[4], values[2],
+                          values[6], values[5], values[6], values[3]};
+        double* w = a.virial + 9 * frame;
+        double* const out[10] = {a.energy + frame, w, w + 1, w + 2, w + 3, w + 4, w + 5, w + 6,
+                                 w + 7, w + 8};
+        add_block_sums(all, out);
+    }
+}
+
+// Blocks per frame, each taking kColumns columns at a time: as many as the columns fill, up to
+// `per_sm` blocks per SM over all frames, then several turns per block.
+template <int kColumns>
+int frame_blocks(std::int64_t capacity, std::int64_t frames, int per_sm, unsigned* blocks)
+{
+    int sms = 148;
+    ND_CUDA_TRY(multiprocessors(&sms));
+    const std::int64_t wanted = (capacity + kColumns - 1) / kColumns;
+    const std::int64_t most = std::max<std::int64_t>(1, static_cast<std::int64_t>(sms) * per_sm /
+                                                            std::max<std::int64_t>(1, frames));
+    *blocks = static_cast<unsigned>(std::max<std::int64_t>(1, std::min(wanted, most)));
+    return ND_OK;
+}
+
+template <typename T, bool kPacked>
+int launch_frames(const FramesPass<T>& pass, std::int64_t frames, cudaStream_t stream)
+{
+    unsigned blocks = 1;
+    const int rc = frame_blocks<kLJThreads * kLaneColumns>(
+        pass.capacity, frames, frames == 1 ? kFrameBlocksPerSM<T> : 4 * kFrameBlocksPerSM<T>,
+        &blocks);
+    if (rc != ND_OK)
+    {
+        return rc;
+    }
+    const dim3 grid(blocks, static_cast<unsigned>(frames));
+    if (pass.num_types > 1)
+    {
+        lj_frames_kernel<T, kPacked, true><<<grid, kLJThreads, 0, stream>>>(pass);
+    }
+    else
+    {
+        lj_frames_kernel<T, kPacked, false><<<grid, kLJThreads, 0, stream>>>(pass);
+    }
+    ND_LAUNCH_CHECK();
+    return ND_OK;
+}
+
+// The frames with a workspace: pack (and wrap), pairs, unpack.
+template <typename T>
+int lj_frames(const nd_lj_batch_args* a, bool wrap, void* workspace, cudaStream_t stream)
+{
+    const std::int64_t n = a->num_atoms, frames = a->frames, slots = n * frames;
+    const FrameWorkspace<T> ws(frames, n);
+    auto* base = static_cast<unsigned char*>(workspace);
+    auto* sums = reinterpret_cast<double*>(base + ws.sums);
+    auto* atoms = reinterpret_cast<PackedAtom<T>*>(base + ws.atoms);
+    auto* packed = sizeof(T) == 4 ? reinterpret_cast<float4*>(base + ws.forces) : nullptr;
+    const auto* types = a->num_types > 1 ? a->atom_types : nullptr;
+    auto* forces = static_cast<T*>(a->forces);
+    const auto* positions = static_cast<const T*>(a->positions);
+    const auto* cells = static_cast<const T*>(a->cells);
+    const auto atoms_n = static_cast<index_t>(n);
+    if (wrap)
+    {
+        pack_atoms_kernel<T, true><<<blocks_for(slots), kThreads, 0, stream>>>(
+            positions, cells, types, atoms_n, slots, frames, atoms, packed, forces, sums);
+    }
+    else
+    {
+        pack_atoms_kernel<T, false><<<blocks_for(slots), kThreads, 0, stream>>>(
+            positions, cells, types, atoms_n, slots, frames, atoms, packed, forces, sums);
+    }
+    ND_LAUNCH_CHECK();
+    const T rc = static_cast<T>(a->cutoff);
+    FramesPass<T> pass{};
+    pass.atoms = atoms;
+    pass.cells = cells;
+    pass.pairs = a->pairs;
+    pass.capacity = a->capacity;
+    pass.num_atoms = atoms_n;
+    pass.num_types = a->num_types;
+    pass.sigma = static_cast<const T*>(a->sigma);
+    pass.epsilon = static_cast<const T*>(a->epsilon);
+    pass.cutoff_squared = rc * rc;
+    pass.packed_forces = packed;
+    pass.forces = forces;
+    pass.sums = sums;
+    const int launched = launch_frames<T, true>(pass, frames, stream);
+    if (launched != ND_OK)
+    {
+        return launched;
+    }
+    const std::int64_t items = sizeof(T) == 4 ? slots : frames * 10;
+    unpack_frames_kernel<T><<<blocks_for(items), kThreads, 0, stream>>>(
+        packed, slots, frames, sums, sizeof(T) == 4 ? reinterpret_cast<float*>(forces) : nullptr,
+        reinterpret_cast<T*>(a->energy), reinterpret_cast<T*>(a->virial));
+    ND_LAUNCH_CHECK();
+    return ND_OK;
+}
+
+// The frames without a workspace: float64 sums and scalar force atomics in place.
+template <typename T>
+int lj_frames_in_place(std::int64_t frames, const nd_lj_batch_args* a, cudaStream_t stream)
+{
+    const std::int64_t n = a->num_atoms;
+    ND_CUDA_TRY(cudaMemsetAsync(a->forces, 0, sizeof(T) * 3 * n * frames, stream));
+    ND_CUDA_TRY(cudaMemsetAsync(a->energy, 0, sizeof(double) * frames, stream));
+    ND_CUDA_TRY(cudaMemsetAsync(a->virial, 0, sizeof(double) * 9 * frames, stream));
+    const T rc = static_cast<T>(a->cutoff);
+    FramesPass<T> pass{};
+    pass.positions = static_cast<const T*>(a->positions);
+    pass.atom_types = a->num_types > 1 ? a->atom_types : nullptr;
+    pass.cells = static_cast<const T*>(a->cells);
+    pass.pairs = a->pairs;
+    pass.capacity = a->capacity;
+    pass.num_atoms = static_cast<index_t>(n);
+    pass.num_types = a->num_types;
+    pass.sigma = static_cast<const T*>(a->sigma);
+    pass.epsilon = static_cast<const T*>(a->epsilon);
+    pass.cutoff_squared = rc * rc;
+    pass.forces = static_cast<T*>(a->forces);
+    pass.energy = a->energy;
+    pass.virial = a->virial;
+    return launch_frames<T, false>(pass, frames, stream);
+}
+
 template <typename T>
 int lj_pairs(const nd_lj_pairs_args* a, cudaStream_t stream)
 {
+    const bool grads = a->sigma_grad != nullptr;
+    if (!grads && a->strain == nullptr)
+    {
+        nd_lj_batch_args frame{};
+        frame.frames = 1;
+        frame.positions = a->positions;
+        frame.cells = a->cell;
+        frame.num_atoms = a->num_atoms;
+        frame.pairs = a->pairs;
+        frame.capacity = a->capacity;
+        frame.atom_types = a->atom_types;
+        frame.num_types = a->num_types;
+        frame.sigma = a->sigma;
+        frame.epsilon = a->epsilon;
+        frame.cutoff = a->cutoff;
+        frame.energy = a->energy;
+        frame.forces = a->forces;
+        frame.virial = a->virial;
+        return lj_frames_in_place<T>(1, &frame, stream);
+    }
     const std::int64_t n = a->num_atoms;
     ND_CUDA_TRY(cudaMemsetAsync(a->forces, 0, sizeof(T) * 3 * n, stream));
     ND_CUDA_TRY(cudaMemsetAsync(a->energy, 0, sizeof(double), stream));
     ND_CUDA_TRY(cudaMemsetAsync(a->virial, 0, sizeof(double) * 9, stream));
     const int rows = a->num_types * (a->num_types + 1) / 2;
-    const bool grads = a->sigma_grad != nullptr;
     if (grads)
     {
         ND_CUDA_TRY(cudaMemsetAsync(a->sigma_grad, 0, sizeof(double) * rows, stream));
         ND_CUDA_TRY(cudaMemsetAsync(a->epsilon_grad, 0, sizeof(double) * rows, stream));
     }
-    int device = 0, sms = 148;
-    ND_CUDA_TRY(cudaGetDevice(&device));
-    ND_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    const std::int64_t wanted = (a->capacity + kLJThreads - 1) / kLJThreads;
-    const std::int64_t most = static_cast<std::int64_t>(sms) * 8;
-    const auto blocks = static_cast<unsigned>(wanted < most ? (wanted > 0 ? wanted : 1) : most);
+    unsigned blocks = 1;
+    const int counted = frame_blocks<kLJThreads>(a->capacity, 1, 8, &blocks);
+    if (counted != ND_OK)
+    {
+        return counted;
+    }
     const T rc = static_cast<T>(a->cutoff);
     const auto* types = a->num_types > 1 ? a->atom_types : nullptr;
     const auto* strain = static_cast<const T*>(a->strain);
-#define ND_LJ_LAUNCH(GRADS, STRAINED)                                                         \
-    lj_pairs_kernel<T, GRADS, STRAINED><<<blocks, kLJThreads, 0, stream>>>(                  \
-        static_cast<const T*>(a->positions), static_cast<const T*>(a->cell), a->pairs,       \
-        a->capacity, static_cast<index_t>(a->num_atoms), types, a->num_types, static_cast<const T*>(a->sigma),                   \
-        static_cast<const T*>(a->epsilon), strain, rc * rc, a->energy,                        \
-        static_cast<T*>(a->forces), a->virial, a->sigma_grad, a->epsilon_grad)
-    if (grads)
+    auto launch = [&](auto kernel) {
+        kernel<<<blocks, kLJThreads, 0, stream>>>(
+            static_cast<const T*>(a->positions), static_cast<const T*>(a->cell), a->pairs,
+            a->capacity, static_cast<index_t>(a->num_atoms), types, a->num_types,
+            static_cast<const T*>(a->sigma), static_cast<const T*>(a->epsilon), strain, rc * rc,
+            a->energy, static_cast<T*>(a->forces), a->virial, a->sigma_grad, a->epsilon_grad);
+    };
+    if (grads && strain)
     {
-        if (strain)
-        {
-            ND_LJ_LAUNCH(true, true);
-        }
-        else
-        {
-            ND_LJ_LAUNCH(true, false);
-        }
+        launch(lj_pairs_kernel<T, true, true>);
+    }
+    else if (grads)
+    {
+        launch(lj_pairs_kernel<T, true, false>);
     }
     else
     {
-        if (strain)
-        {
-            ND_LJ_LAUNCH(false, true);
-        }
-        else
-        {
-            ND_LJ_LAUNCH(false, false);
-        }
+        launch(lj_pairs_kernel<T, false, true>);
     }
-#undef ND_LJ_LAUNCH
     ND_LAUNCH_CHECK();
     return ND_OK;
 }
@@ -392,36 +966,6 @@ __global__ void __launch_bounds__(kLJThreads) lj_parameter_backward_kernel(
     }
 }
 
-unsigned pair_blocks(std::int64_t capacity, std::int64_t frames)
-{
-    int device = 0, sms = 148;
-    cudaGetDevice(&device);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    const std::int64_t wanted = (capacity + kLJThreads - 1) / kLJThreads;
-    std::int64_t most = static_cast<std::int64_t>(sms) * 8 / (frames > 0 ? frames : 1);
-    most = most < 1 ? 1 : most;
-    return static_cast<unsigned>(wanted < most ? (wanted > 0 ? wanted : 1) : most);
-}
-
-template <typename T>
-int lj_batch_forward(const nd_lj_batch_args* a, cudaStream_t stream)
-{
-    const std::int64_t n = a->num_atoms, frames = a->frames;
-    ND_CUDA_TRY(cudaMemsetAsync(a->forces, 0, sizeof(T) * 3 * n * frames, stream));
-    ND_CUDA_TRY(cudaMemsetAsync(a->energy, 0, sizeof(double) * frames, stream));
-    ND_CUDA_TRY(cudaMemsetAsync(a->virial, 0, sizeof(double) * 9 * frames, stream));
-    const T rc = static_cast<T>(a->cutoff);
-    const auto* types = a->num_types > 1 ? a->atom_types : nullptr;
-    const dim3 grid(pair_blocks(a->capacity, frames), static_cast<unsigned>(frames));
-    lj_pairs_kernel<T, false, false><<<grid, kLJThreads, 0, stream>>>(
-        static_cast<const T*>(a->positions), static_cast<const T*>(a->cells), a->pairs,
-        a->capacity, static_cast<index_t>(n), types, a->num_types,
-        static_cast<const T*>(a->sigma), static_cast<const T*>(a->epsilon), nullptr, rc * rc,
-        a->energy, static_cast<T*>(a->forces), a->virial, nullptr, nullptr);
-    ND_LAUNCH_CHECK();
-    return ND_OK;
-}
-
 template <typename T>
 int lj_batch_parameter_backward(const nd_lj_batch_args* a, cudaStream_t stream)
 {
@@ -430,7 +974,13 @@ int lj_batch_parameter_backward(const nd_lj_batch_args* a, cudaStream_t stream)
     ND_CUDA_TRY(cudaMemsetAsync(a->epsilon_grad, 0, sizeof(double) * rows, stream));
     const T rc = static_cast<T>(a->cutoff);
     const auto* types = a->num_types > 1 ? a->atom_types : nullptr;
-    const dim3 grid(pair_blocks(a->capacity, a->frames), static_cast<unsigned>(a->frames));
+    unsigned blocks = 1;
+    const int counted = frame_blocks<kLJThreads>(a->capacity, a->frames, 8, &blocks);
+    if (counted != ND_OK)
+    {
+        return counted;
+    }
+    const dim3 grid(blocks, static_cast<unsigned>(a->frames));
     lj_parameter_backward_kernel<T><<<grid, kLJThreads, 0, stream>>>(
         static_cast<const T*>(a->positions), static_cast<const T*>(a->cells), a->pairs,
         a->capacity, static_cast<index_t>(a->num_atoms), types, a->num_types,
@@ -476,8 +1026,64 @@ extern "C" int nd_lj_batch_forward(const nd_lj_batch_args* args, nd_stream_t str
         return rc;
     }
     auto s = static_cast<cudaStream_t>(stream);
-    return args->dtype == ND_FLOAT32 ? nd::lj_batch_forward<float>(args, s)
-                                     : nd::lj_batch_forward<double>(args, s);
+    return args->dtype == ND_FLOAT32 ? nd::lj_frames_in_place<float>(args->frames, args, s)
+                                     : nd::lj_frames_in_place<double>(args->frames, args, s);
+}
+
+extern "C" int64_t nd_lj_workspace_bytes(int dtype, int64_t frames, int64_t num_atoms)
+{
+    if ((dtype != ND_FLOAT32 && dtype != ND_FLOAT64) || frames < 1 || num_atoms < 1)
+    {
+        return -1;
+    }
+    return dtype == ND_FLOAT32 ? nd::FrameWorkspace<float>(frames, num_atoms).total
+                               : nd::FrameWorkspace<double>(frames, num_atoms).total;
+}
+
+extern "C" int nd_lj_frames(const nd_lj_batch_args* args, int32_t wrap, void* workspace,
+                            nd_stream_t stream)
+{
+    const int rc = nd::check_batch(args, false);
+    if (rc != ND_OK)
+    {
+        return rc;
+    }
+    ND_REQUIRE(workspace != nullptr, "the workspace is null");
+    ND_REQUIRE(reinterpret_cast<std::uintptr_t>(workspace) % 256 == 0,
+               "the workspace must be 256-byte aligned");
+    auto s = static_cast<cudaStream_t>(stream);
+    return args->dtype == ND_FLOAT32 ? nd::lj_frames<float>(args, wrap != 0, workspace, s)
+                                     : nd::lj_frames<double>(args, wrap != 0, workspace, s);
+}
+
+extern "C" int nd_wrap(int dtype, const void* positions, const void* cells, int64_t frames,
+                       int64_t num_atoms, void* wrapped, nd_stream_t stream)
+{
+    ND_REQUIRE(dtype == ND_FLOAT32 || dtype == ND_FLOAT64, "positions must be float32 or float64");
+    ND_REQUIRE(frames >= 0 && num_atoms >= 0 && frames <= INT32_MAX && num_atoms <= INT32_MAX &&
+                   frames * num_atoms <= INT64_C(1) << 38,
+               "too many atoms");
+    if (frames * num_atoms == 0)
+    {
+        return ND_OK;
+    }
+    ND_REQUIRE(positions && cells && wrapped, "a required pointer is null");
+    auto s = static_cast<cudaStream_t>(stream);
+    const int64_t values = 3 * frames * num_atoms;
+    if (dtype == ND_FLOAT32)
+    {
+        nd::wrap_kernel<float><<<nd::blocks_for(values), nd::kThreads, 0, s>>>(
+            static_cast<const float*>(positions), static_cast<const float*>(cells), num_atoms,
+            values, static_cast<float*>(wrapped));
+    }
+    else
+    {
+        nd::wrap_kernel<double><<<nd::blocks_for(values), nd::kThreads, 0, s>>>(
+            static_cast<const double*>(positions), static_cast<const double*>(cells), num_atoms,
+            values, static_cast<double*>(wrapped));
+    }
+    ND_LAUNCH_CHECK();
+    return ND_OK;
 }
 
 extern "C" int nd_lj_batch_parameter_backward(const nd_lj_batch_args* args, nd_stream_t stream)

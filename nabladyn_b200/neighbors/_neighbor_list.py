@@ -204,7 +204,7 @@ class NeighborList:
         scan_bytes = max(ops.scan_temp_bytes(positions, math.prod(dims) + 1),
                          ops.scan_temp_bytes(positions, n))
         device = _DeviceList(n, dims, lengths, scan_bytes, positions.dtype, positions.device)
-        frame, _ = space.wrap(positions.detach(), cell.detach())
+        frame = space.wrapped_only(positions, cell)
         box = cell.detach().contiguous()
         ops.count_first_frame(frame, box, self.radius, *device.build_args())
         # The pairs of the frame: the last atom's offset plus its count.
@@ -243,7 +243,7 @@ class NeighborList:
         if (positions.shape, positions.dtype, positions.device) != (like.shape, like.dtype,
                                                                     like.device):
             raise ValueError("positions must match the allocated shape, dtype and device")
-        frame, _ = space.wrap(positions.detach(), cell.detach())
+        frame = space.wrapped_only(positions, cell)
         self._update_wrapped(frame, cell.detach().contiguous())
         self._check_status()
 

@@ -58,6 +58,10 @@ class Potential(nn.Module, ABC):
     def device(self) -> torch.device:
         """The device the model computes on."""
 
+    # Whether the fused kernels of a model that has them can wrap the positions themselves
+    # (``_energy_force_virial(..., wrap=True)``).
+    _fused_wraps = False
+
     @property
     def _list_cutoffs(self) -> tuple[float, ...]:
         return (self.cutoff,)

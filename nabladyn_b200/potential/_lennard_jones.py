@@ -3,8 +3,10 @@
 Mirrors src/nabladyn/potential/_lennard_jones/_potential.py (LennardJones :113-237,
 pair_index :143-151) and the constructor src/nabladyn/potential/_api.py:18-57. The energy and
 all its first derivatives (forces, virial, parameter gradients) come from one pass of the
-CUDA pair kernel (nd_lj_energy_force_virial); ``_LJEnergy`` exposes them to autograd and
-torch.func, so ``quantity``'s generic path and plain ``.backward()`` work on the model.
+CUDA pair kernels: nd_lj_frames for E, F and W alone (``quantity``, training, sums), and
+nd_lj_energy_force_virial where autograd asks for a strain or parameter gradients too;
+``_LJEnergy`` exposes the latter to autograd and torch.func, so ``quantity``'s generic path and
+plain ``.backward()`` work on the model.
 """
 
 from __future__ import annotations
@@ -17,7 +19,8 @@ import torch
 from torch import Tensor, nn
 
 from .. import _native
-from .._native import LJPairsArgs, call, dtype_code, ptr, stream_handle
+from .._native import (LJBatchArgs, LJPairsArgs, call, dtype_code, lib, on_device, ptr,
+                       stream_handle)
 from ..neighbors import NeighborPairs
 from ._base import Potential
 
@@ -167,6 +170,32 @@ def evaluate_pairs(
     )
 
 
+def evaluate_frames(positions: Tensor, cells: Tensor, index: Tensor, kernel_types: Tensor | None,
+                    num_types: int, sigma: Tensor, epsilon: Tensor, cutoff: float,
+                    wrap: bool):
+    """(E [F], F [F, N, 3], W [F, 3, 3]) of frames [F, N, 3] in the positions' dtype, from
+    nd_lj_frames: cells [F, 3], index int32 [F, 2, C] (all contiguous), the parameters in the
+    positions' dtype; ``wrap`` for positions that may lie outside the cell. No host sync."""
+    device, dtype = positions.device, positions.dtype
+    frames, atoms = positions.shape[0], positions.shape[1]
+    code = dtype_code(dtype)
+    workspace = torch.empty(int(lib().nd_lj_workspace_bytes(code, frames, atoms)),
+                            dtype=torch.uint8, device=device)
+    energy = torch.empty(frames, dtype=dtype, device=device)
+    virial = torch.empty((frames, 3, 3), dtype=dtype, device=device)
+    forces = torch.empty((frames, atoms, 3), dtype=dtype, device=device)
+    args = LJBatchArgs(
+        dtype=code, frames=frames, positions=ptr(positions), cells=ptr(cells), num_atoms=atoms,
+        pairs=ptr(index), capacity=index.shape[2],
+        atom_types=ptr(kernel_types) if num_types > 1 else None, num_types=num_types,
+        sigma=ptr(sigma), epsilon=ptr(epsilon), cutoff=float(cutoff), energy=ptr(energy),
+        forces=ptr(forces), virial=ptr(virial),
+    )
+    with on_device(device):
+        call("nd_lj_frames", args, int(wrap), ptr(workspace), stream_handle(device))
+    return energy, forces, virial
+
+
 class _LJEnergy(torch.autograd.Function):
     """E of the pair kernel, with its saved first derivatives as the backward.
 
@@ -276,14 +305,23 @@ class LennardJones(Potential):
         )
         return energy
 
-    def _energy_force_virial(self, positions: Tensor, cell: Tensor, pairs: NeighborPairs):
-        """(E, F, W) of wrapped positions in one kernel pass, in the model's dtype."""
-        energy, forces, virial, _, _ = evaluate_pairs(
-            positions, cell, pairs.index, self._kernel_types, self._num_types, self.sigma,
-            self.epsilon, self._cutoff,
-        )
+    _fused_wraps = True
+
+    def _energy_force_virial(self, positions: Tensor, cell: Tensor, pairs: NeighborPairs,
+                             wrap: bool = False):
+        """(E, F, W) in one kernel pass, in the positions' dtype; positions wrapped, or with
+        ``wrap`` anywhere."""
         dtype = positions.dtype
-        return energy.to(dtype), forces, virial.to(dtype)
+        index = pairs.index.detach()
+        if index.dtype != torch.int32:
+            index = index.to(torch.int32)
+        energy, forces, virial = evaluate_frames(
+            positions.detach().contiguous()[None], cell.detach().contiguous()[None],
+            index.contiguous()[None], self._kernel_types, self._num_types,
+            self.sigma.detach().to(dtype).contiguous(),
+            self.epsilon.detach().to(dtype).contiguous(), self._cutoff, wrap,
+        )
+        return energy[0], forces[0], virial[0]
 
 
 def lennard_jones(*, atom_types: Tensor, sigma: Tensor, epsilon: Tensor, cutoff: Real,

@@ -43,7 +43,9 @@ def _fused_evaluate(model: Potential, wraps: bool):
             _check_tensor("positions", positions, (model.num_atoms, 3), model.dtype, model.device)
             _check_tensor("cell", cell, (3,), model.dtype, model.device)
             _check_pairs(pairs, model.num_atoms, model.cutoff, model.device)
-            positions = space.wrap(positions, cell)[0]
+            if model._fused_wraps:
+                return model._energy_force_virial(positions, cell, pairs, wrap=True)
+            positions = space.wrapped_only(positions, cell)
         return model._energy_force_virial(positions, cell, pairs)
 
     return evaluate

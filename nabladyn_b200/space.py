@@ -7,6 +7,8 @@ wrapping inside its kernels; these serve the host-side API (allocation, checks, 
 import torch
 from torch import Tensor
 
+from . import _native
+
 
 def _displacement_wrapped(left: Tensor, right: Tensor, cell: Tensor) -> Tensor:
     """The minimum-image vector ``left - right`` for coordinates already in [0, L).
@@ -36,6 +38,26 @@ def wrap(positions: Tensor, cell: Tensor) -> tuple[Tensor, Tensor]:
     wrapped = torch.where(above, wrapped - cell, wrapped)
     crossings = torch.where(above, crossings + 1, crossings)
     return wrapped, crossings.to(torch.int64)
+
+
+def wrapped_only(positions: Tensor, cell: Tensor) -> Tensor:
+    """``wrap(positions, cell)[0]`` of a frame [N, 3] and cell [3], or of frames [F, N, 3] and
+    their cells [F, 3], without autograd and contiguous. CUDA frames take one kernel (nd_wrap,
+    the same rounding) instead of ``wrap``'s dozen elementwise ones."""
+    positions, cell = positions.detach(), cell.detach()
+    if not (positions.is_cuda and positions.dtype in (torch.float32, torch.float64)
+            and cell.dtype == positions.dtype and cell.device == positions.device
+            and positions.shape[-1:] == (3,) and positions.ndim in (2, 3)
+            and cell.shape == (*positions.shape[:-2], 3)):
+        return wrap(positions, cell if cell.ndim == 1 else cell[:, None])[0].contiguous()
+    positions, cell = positions.contiguous(), cell.contiguous()
+    out = torch.empty_like(positions)
+    frames = 1 if positions.ndim == 2 else positions.shape[0]
+    with _native.on_device(positions.device):
+        _native.call("nd_wrap", _native.dtype_code(positions.dtype), positions.data_ptr(),
+                     cell.data_ptr(), frames, positions.shape[-2], out.data_ptr(),
+                     _native.stream_handle(positions.device))
+    return out
 
 
 def shift(positions: Tensor, delta: Tensor, cell: Tensor) -> tuple[Tensor, Tensor]:

@@ -1,7 +1,7 @@
 """Batched Lennard-Jones predictions with a hand-written parameter backward.
 
 ``predict`` gives the energy, forces and virial of F frames in one kernel launch
-(nd_lj_batch_forward); its autograd backward is nd_lj_batch_parameter_backward, which turns the
+(nd_lj_frames); its autograd backward is nd_lj_batch_parameter_backward, which turns the
 loss's gradients with respect to E, F and W into dLoss/dsigma and dLoss/depsilon in one pass
 over the pairs. The reference gets the same numbers by a torch.func double backward through
 vmapped forces (src/nabladyn/training/_loss.py:71-102, _fit.py:245-271).
@@ -16,7 +16,7 @@ from torch import Tensor
 
 from .. import space
 from .._native import LJBatchArgs, call, dtype_code, ptr, stream_handle
-from ..potential._lennard_jones import LennardJones
+from ..potential._lennard_jones import LennardJones, evaluate_frames
 
 CHANNELS = ("energy", "forces", "virial")
 
@@ -44,21 +44,15 @@ class _BatchLJ(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, sigma, epsilon, positions, cells, stacks, kernel_types, num_types, cutoff):
-        dtype, device = positions.dtype, positions.device
-        frames, atoms = positions.shape[:2]
+        dtype = positions.dtype
         sigma_c = sigma.detach().to(dtype).contiguous()
         epsilon_c = epsilon.detach().to(dtype).contiguous()
-        energy = torch.empty(frames, dtype=torch.float64, device=device)
-        forces = torch.empty((frames, atoms, 3), dtype=dtype, device=device)
-        virial = torch.empty((frames, 3, 3), dtype=torch.float64, device=device)
-        args = _args(positions, cells, stacks, kernel_types, num_types, sigma_c, epsilon_c, cutoff)
-        args.energy, args.forces, args.virial = ptr(energy), ptr(forces), ptr(virial)
-        with torch.cuda.device(device):
-            call("nd_lj_batch_forward", args, stream_handle(device))
+        energy, forces, virial = evaluate_frames(positions, cells, stacks, kernel_types,
+                                                 num_types, sigma_c, epsilon_c, cutoff, False)
         ctx.save_for_backward(sigma_c, epsilon_c, positions, cells, stacks, kernel_types)
         ctx.num_types, ctx.cutoff = num_types, cutoff
         ctx.parameter_dtype = sigma.dtype
-        return energy.to(dtype), forces, virial.to(dtype)
+        return energy, forces, virial
 
     @staticmethod
     def backward(ctx, grad_energy, grad_forces, grad_virial):
@@ -104,7 +98,7 @@ def predict(model: LennardJones, parameters: Mapping[str, Tensor], positions: Te
         raise ValueError(f"channels must be a nonempty subsequence of {CHANNELS}")
     sigma = parameters.get("sigma", model.sigma)
     epsilon = parameters.get("epsilon", model.epsilon)
-    wrapped = space.wrap(positions.detach(), cells.detach()[:, None])[0].contiguous()
+    wrapped = space.wrapped_only(positions, cells)
     stack = stacks[-1]
     if stack.dtype != torch.int32:
         stack = stack.to(torch.int32)

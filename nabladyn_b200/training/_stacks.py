@@ -33,7 +33,7 @@ def pair_stack(positions: Tensor, cells: Tensor, cutoff: float) -> Tensor:
     """
     frames, atoms = positions.shape[:2]
     device = positions.device
-    wrapped = space.wrap(positions.detach(), cells.detach()[:, None])[0].contiguous()
+    wrapped = space.wrapped_only(positions, cells)
     cells = cells.detach().contiguous()
 
     # Counting: every frame rebuilt into a list sized for frame 0; totals and error flags
