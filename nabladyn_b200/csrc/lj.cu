@@ -269,17 +269,18 @@ __global__ void __launch_bounds__(kLJThreads) lj_pairs_kernel(
 //   * float32 forces are summed into packed [N, 4] slots, one 16-B vector atomic per atom
 //     instead of three scalar ones, and unpacked by the closing pass (float64 has no vector
 //     atomic and adds its three components in place);
-//   * a warp takes 128 consecutive columns, four per lane. The list groups its columns by
-//     first atom (about 60 columns each in a liquid), so a lane sums its first atom's force
-//     in registers, the lanes that end on the same first atom meet in a segmented warp sum,
-//     and a first atom costs two or three atomics instead of one per column. An index in any
-//     other order gives the same sums with more atomics.
+//   * a warp takes 128 consecutive columns. The list groups its columns by first atom (about
+//     60 columns each in a liquid), so the pair forces pass through shared memory into four
+//     consecutive columns per lane, a lane sums its first atom's force in registers, the
+//     lanes that end on the same first atom meet in a segmented warp sum, and a first atom
+//     costs two or three atomics instead of one per column. An index in any other order gives
+//     the same sums with more atomics.
 
 // Blocks an SM holds: the registers of four columns in flight, 80 (float32) or 124 (float64).
 template <typename T>
 constexpr int kFrameBlocksPerSM = sizeof(T) == 4 ? 3 : 2;
 
-constexpr int kLaneColumns = 4;                          // consecutive columns per lane
+constexpr int kLaneColumns = 4;  // columns a lane has in flight
 constexpr int kWarpColumns = kWarp * kLaneColumns;
 
 // An atom as the kernels gather it; w holds the type's bits. 16-B aligned: float64 slots are
@@ -405,55 +406,6 @@ __global__ void __launch_bounds__(kThreads) unpack_frames_kernel(
     }
 }
 
-// Four consecutive ints of a row from element c; elements at or past `end` read as `fill`.
-// `skew` is the row's offset from a 16-B boundary, in ints (the same for every thread): an
-// interior lane reads whole aligned words and takes its four from them, so an odd capacity
-// (whose second row starts anywhere) costs one more word, not four scalar loads.
-__device__ __forceinline__ void load_columns(const index_t* __restrict__ row, std::int64_t c,
-                                             std::int64_t end, int skew, index_t fill,
-                                             index_t (&out)[kLaneColumns])
-{
-    const std::int64_t from = c - skew;
-    if (from >= 0 && from + (skew == 0 ? 4 : 8) <= end)
-    {
-        const int4 a = *reinterpret_cast<const int4*>(row + from);
-        if (skew == 0)
-        {
-            out[0] = a.x;
-            out[1] = a.y;
-            out[2] = a.z;
-            out[3] = a.w;
-            return;
-        }
-        const int4 b = *reinterpret_cast<const int4*>(row + from + 4);
-        out[0] = skew == 1 ? a.y : (skew == 2 ? a.z : a.w);
-        out[1] = skew == 1 ? a.z : (skew == 2 ? a.w : b.x);
-        out[2] = skew == 1 ? a.w : (skew == 2 ? b.x : b.y);
-        out[3] = skew == 1 ? b.x : (skew == 2 ? b.y : b.z);
-        return;
-    }
-#pragma unroll
-    for (int k = 0; k < kLaneColumns; ++k)
-    {
-        out[k] = c + k < end ? row[c + k] : fill;
-    }
-}
-
-__device__ __forceinline__ int row_skew(const index_t* row)
-{
-    return static_cast<int>((reinterpret_cast<std::uintptr_t>(row) / sizeof(index_t)) % 4);
-}
-
-// The four columns from element c: first and second atoms, -1 past the capacity.
-__device__ __forceinline__ void load_pairs(const index_t* __restrict__ pairs,
-                                           std::int64_t capacity, std::int64_t c, int skew_first,
-                                           int skew_second, index_t (&i)[kLaneColumns],
-                                           index_t (&j)[kLaneColumns])
-{
-    load_columns(pairs, c, capacity, skew_first, -1, i);
-    load_columns(pairs + capacity, c, capacity, skew_second, -1, j);
-}
-
 // A column counts when its atoms differ and both lie in [0, N): self-pairs are padding, an
 // index outside is skipped and never read.
 __device__ __forceinline__ bool counts(index_t i, index_t j, index_t num_atoms)
@@ -467,6 +419,25 @@ template <typename T>
 struct RowConstants
 {
     T s2, eps4, eps24, shift;
+};
+
+// 1 / x: a hardware estimate and one Newton step in float32 (within an ulp of the rounded
+// quotient), the division in float64.
+__device__ __forceinline__ float reciprocal(float x)
+{
+    float y;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return fmaf(y, fmaf(-x, y, 1.0f), y);
+}
+__device__ __forceinline__ double reciprocal(double x) { return 1.0 / x; }
+
+// A warp's 128 pair forces and first atoms (-1: no pair), written a column per lane and read
+// four consecutive columns per lane.
+template <typename T>
+struct alignas(16) PairStage
+{
+    T x[kWarpColumns], y[kWarpColumns], z[kWarpColumns];
+    index_t key[kWarpColumns];
 };
 
 template <typename T>
@@ -553,96 +524,111 @@ lj_frames_kernel(FramesPass<T> a)
     }
     __syncthreads();
     const T lx = a.cells[0], ly = a.cells[1], lz = a.cells[2];
+    const T hx = T(0.5) * lx, hy = T(0.5) * ly, hz = T(0.5) * lz;
     const int lane = threadIdx.x % kWarp;
-    const int skew_first = row_skew(a.pairs), skew_second = row_skew(a.pairs + a.capacity);
+    __shared__ PairStage<T> stages[kLJThreads / kWarp];
+    PairStage<T>& stage = stages[threadIdx.x / kWarp];
     T energy = 0, wxx = 0, wyy = 0, wzz = 0, wxy = 0, wxz = 0, wyz = 0;
     const std::int64_t warps = static_cast<std::int64_t>(gridDim.x) * (kLJThreads / kWarp);
     std::int64_t base = (static_cast<std::int64_t>(blockIdx.x) * (kLJThreads / kWarp) +
                          threadIdx.x / kWarp) * kWarpColumns;
     index_t i[kLaneColumns], j[kLaneColumns];
-    if (base < a.capacity)
-    {
-        load_pairs(a.pairs, a.capacity, base + kLaneColumns * lane, skew_first, skew_second, i, j);
-    }
+    auto load_columns = [&](std::int64_t from) {
+#pragma unroll
+        for (int k = 0; k < kLaneColumns; ++k)
+        {
+            const std::int64_t column = from + kWarp * k + lane;
+            i[k] = column < a.capacity ? a.pairs[column] : -1;
+            j[k] = column < a.capacity ? a.pairs[a.capacity + column] : -1;
+        }
+    };
+    load_columns(base);
     while (base < a.capacity)
     {
         // All gathers of the four columns before any is used.
         PackedAtom<T> left[kLaneColumns], right[kLaneColumns];
-        bool live[kLaneColumns];
-#pragma unroll
-        for (int k = 0; k < kLaneColumns; ++k)
-        {
-            live[k] = counts(i[k], j[k], a.num_atoms);
-            right[k] = gather<T, kPacked>(a, live[k] ? j[k] : 0);
-            if (k > 0 && i[k] == i[k - 1])
-            {
-                left[k] = left[k - 1];
-            }
-            else
-            {
-                const bool inside = static_cast<unsigned>(i[k]) <
-                                    static_cast<unsigned>(a.num_atoms);
-                left[k] = gather<T, kPacked>(a, inside ? i[k] : 0);
-            }
-        }
         index_t first[kLaneColumns], second[kLaneColumns];
 #pragma unroll
         for (int k = 0; k < kLaneColumns; ++k)
         {
-            first[k] = i[k];
-            second[k] = j[k];
+            const bool live = counts(i[k], j[k], a.num_atoms);
+            first[k] = live ? i[k] : -1;
+            second[k] = live ? j[k] : 0;
+            left[k] = gather<T, kPacked>(a, live ? i[k] : 0);
+            right[k] = gather<T, kPacked>(a, second[k]);
         }
         // The next run's columns, loaded behind this run's arithmetic.
         base += warps * kWarpColumns;
-        if (base < a.capacity)
-        {
-            load_pairs(a.pairs, a.capacity, base + kLaneColumns * lane, skew_first, skew_second,
-                       i, j);
-        }
-        index_t key = -1;
-        T fx = 0, fy = 0, fz = 0;  // the force on `key` from this lane's columns
+        load_columns(base);
 #pragma unroll
         for (int k = 0; k < kLaneColumns; ++k)
         {
-            const T dx = displacement(left[k].x, right[k].x, lx);
-            const T dy = displacement(left[k].y, right[k].y, ly);
-            const T dz = displacement(left[k].z, right[k].z, lz);
-            const T r2 = dx * dx + dy * dy + dz * dz;
-            if (!(live[k] && r2 < a.cutoff_squared))
+            T dx = left[k].x - right[k].x;
+            T dy = left[k].y - right[k].y;
+            T dz = left[k].z - right[k].z;
+            // Few pairs cross a face: a warp without one takes the plain differences.
+            if (fabs(dx) > hx || fabs(dy) > hy || fabs(dz) > hz)
             {
-                continue;
+                dx = displacement(left[k].x, right[k].x, lx);
+                dy = displacement(left[k].y, right[k].y, ly);
+                dz = displacement(left[k].z, right[k].z, lz);
             }
-            const RowConstants<T> c =
-                rows[kTypes ? pair_row(word_type(left[k].w), word_type(right[k].w), a.num_types)
-                            : 0];
-            const T inv_r2 = T(1) / r2;
-            const T q = c.s2 * inv_r2;
-            const T p6 = q * q * q;
-            energy += c.eps4 * (p6 * p6 - p6) - c.shift;
-            const T fs = c.eps24 * (T(2) * p6 * p6 - p6) * inv_r2;
-            const T px = fs * dx, py = fs * dy, pz = fs * dz;
-            wxx += px * dx;
-            wyy += py * dy;
-            wzz += pz * dz;
-            wxy += px * dy;
-            wxz += px * dz;
-            wyz += py * dz;
-            add_force<T, kPacked>(a, second[k], -px, -py, -pz);
-            if (first[k] != key)
+            const T r2 = dx * dx + dy * dy + dz * dz;
+            const bool hit = first[k] >= 0 && r2 < a.cutoff_squared;
+            T px = 0, py = 0, pz = 0;
+            if (hit)
+            {
+                const RowConstants<T> c =
+                    rows[kTypes ? pair_row(word_type(left[k].w), word_type(right[k].w),
+                                           a.num_types)
+                                : 0];
+                const T inv_r2 = reciprocal(r2);
+                const T q = c.s2 * inv_r2;
+                const T p6 = q * q * q;
+                energy += c.eps4 * (p6 * p6 - p6) - c.shift;
+                const T fs = c.eps24 * (T(2) * p6 * p6 - p6) * inv_r2;
+                px = fs * dx;
+                py = fs * dy;
+                pz = fs * dz;
+                wxx += px * dx;
+                wyy += py * dy;
+                wzz += pz * dz;
+                wxy += px * dy;
+                wxz += px * dz;
+                wyz += py * dz;
+                add_force<T, kPacked>(a, second[k], -px, -py, -pz);
+            }
+            const int at = kWarp * k + lane;
+            stage.x[at] = px;
+            stage.y[at] = py;
+            stage.z[at] = pz;
+            stage.key[at] = hit ? first[k] : -1;
+        }
+        __syncwarp();
+        // The first atoms' side: the lane's four consecutive columns, summed while the atom
+        // stays the same.
+        index_t key = -1;
+        T fx = 0, fy = 0, fz = 0;
+#pragma unroll
+        for (int k = 0; k < kLaneColumns; ++k)
+        {
+            const int at = kLaneColumns * lane + k;
+            const index_t atom = stage.key[at];
+            if (atom >= 0 && atom != key)
             {
                 if (key >= 0)
                 {
                     add_force<T, kPacked>(a, key, fx, fy, fz);
                 }
-                key = first[k];
+                key = atom;
                 fx = fy = fz = T(0);
             }
-            fx += px;
-            fy += py;
-            fz += pz;
+            fx += stage.x[at];
+            fy += stage.y[at];
+            fz += stage.z[at];
         }
-        // Lanes in a row that end on the same first atom sum into their first lane.
         __syncwarp();
+        // Lanes in a row that end on the same first atom sum into their first lane.
         const index_t before = __shfl_up_sync(kFullMask, key, 1);
         const bool head = lane == 0 || before != key;
         const unsigned heads = __ballot_sync(kFullMask, head);
