@@ -440,6 +440,20 @@ struct alignas(16) PairStage
     index_t key[kWarpColumns];
 };
 
+// Four consecutive staged values, read 16 bytes at a time (scalar reads 16 bytes apart would
+// meet in the same banks four at a time).
+template <typename T>
+struct alignas(16) Four
+{
+    T v[4];
+};
+
+template <typename T>
+__device__ __forceinline__ Four<T> load4(const T* staged)
+{
+    return *reinterpret_cast<const Four<T>*>(staged);
+}
+
 template <typename T>
 struct FramesPass
 {
@@ -529,37 +543,54 @@ lj_frames_kernel(FramesPass<T> a)
     __shared__ PairStage<T> stages[kLJThreads / kWarp];
     PairStage<T>& stage = stages[threadIdx.x / kWarp];
     T energy = 0, wxx = 0, wyy = 0, wzz = 0, wxy = 0, wxz = 0, wyz = 0;
-    const std::int64_t warps = static_cast<std::int64_t>(gridDim.x) * (kLJThreads / kWarp);
-    std::int64_t base = (static_cast<std::int64_t>(blockIdx.x) * (kLJThreads / kWarp) +
-                         threadIdx.x / kWarp) * kWarpColumns;
+    // Columns are below 2^31 and the grid below 2^20 columns, so 32 bits hold every step.
+    const auto capacity = static_cast<unsigned>(a.capacity);
+    const index_t* firsts = a.pairs;
+    const index_t* seconds = a.pairs + a.capacity;
+    const unsigned stride = gridDim.x * (kLJThreads / kWarp) * kWarpColumns;
+    unsigned base = (blockIdx.x * (kLJThreads / kWarp) + threadIdx.x / kWarp) * kWarpColumns;
     index_t i[kLaneColumns], j[kLaneColumns];
-    auto load_columns = [&](std::int64_t from) {
+    auto load_columns = [&](unsigned from) {
 #pragma unroll
         for (int k = 0; k < kLaneColumns; ++k)
         {
-            const std::int64_t column = from + kWarp * k + lane;
-            i[k] = column < a.capacity ? a.pairs[column] : -1;
-            j[k] = column < a.capacity ? a.pairs[a.capacity + column] : -1;
+            const unsigned column = from + kWarp * k + lane;
+            i[k] = column < capacity ? firsts[column] : -1;
+            j[k] = column < capacity ? seconds[column] : -1;
         }
     };
     load_columns(base);
-    while (base < a.capacity)
+    while (base < capacity)
     {
         // All gathers of the four columns before any is used.
         PackedAtom<T> left[kLaneColumns], right[kLaneColumns];
         index_t first[kLaneColumns], second[kLaneColumns];
+        bool any = false;
 #pragma unroll
         for (int k = 0; k < kLaneColumns; ++k)
         {
             const bool live = counts(i[k], j[k], a.num_atoms);
+            any = any || live;
             first[k] = live ? i[k] : -1;
             second[k] = live ? j[k] : 0;
-            left[k] = gather<T, kPacked>(a, live ? i[k] : 0);
-            right[k] = gather<T, kPacked>(a, second[k]);
+        }
+        const bool padding = !__any_sync(kFullMask, any);  // a fifth of a list's columns
+        if (!padding)
+        {
+#pragma unroll
+            for (int k = 0; k < kLaneColumns; ++k)
+            {
+                left[k] = gather<T, kPacked>(a, first[k] < 0 ? 0 : first[k]);
+                right[k] = gather<T, kPacked>(a, second[k]);
+            }
         }
         // The next run's columns, loaded behind this run's arithmetic.
-        base += warps * kWarpColumns;
+        base += stride;
         load_columns(base);
+        if (padding)
+        {
+            continue;
+        }
 #pragma unroll
         for (int k = 0; k < kLaneColumns; ++k)
         {
@@ -609,11 +640,14 @@ lj_frames_kernel(FramesPass<T> a)
         // stays the same.
         index_t key = -1;
         T fx = 0, fy = 0, fz = 0;
+        const Four<T> sx = load4(stage.x + kLaneColumns * lane);
+        const Four<T> sy = load4(stage.y + kLaneColumns * lane);
+        const Four<T> sz = load4(stage.z + kLaneColumns * lane);
+        const Four<index_t> keys = load4(stage.key + kLaneColumns * lane);
 #pragma unroll
         for (int k = 0; k < kLaneColumns; ++k)
         {
-            const int at = kLaneColumns * lane + k;
-            const index_t atom = stage.key[at];
+            const index_t atom = keys.v[k];
             if (atom >= 0 && atom != key)
             {
                 if (key >= 0)
@@ -623,9 +657,9 @@ lj_frames_kernel(FramesPass<T> a)
                 key = atom;
                 fx = fy = fz = T(0);
             }
-            fx += stage.x[at];
-            fy += stage.y[at];
-            fz += stage.z[at];
+            fx += sx.v[k];
+            fy += sy.v[k];
+            fz += sz.v[k];
         }
         __syncwarp();
         // Lanes in a row that end on the same first atom sum into their first lane.
