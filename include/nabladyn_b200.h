@@ -199,6 +199,13 @@ int nd_lj_batch_forward(const nd_lj_batch_args* args, nd_stream_t stream);
 int64_t nd_lj_workspace_bytes(int dtype, int64_t frames, int64_t num_atoms);
 int nd_lj_frames(const nd_lj_batch_args* args, int32_t wrap, void* workspace, nd_stream_t stream);
 
+/* nd_lj_batch_parameter_backward of the frames of an nd_lj_frames call: `positions` is that
+ * call's workspace (its packed atoms are read, nothing of it is written), `workspace` another of
+ * the same size; `energy_grad`, `virial_grad`, `sigma_grad` and `epsilon_grad` point to values
+ * of the frames' dtype. */
+int nd_lj_frames_parameter_backward(const nd_lj_batch_args* args, void* workspace,
+                                    nd_stream_t stream);
+
 /* Positions [F, N, 3] wrapped into [0, L) by cells [F, 3] (src/nabladyn/space.py:22-38 without
  * the crossings). `wrapped` may be `positions`. */
 int nd_wrap(int dtype, const void* positions, const void* cells, int64_t frames,

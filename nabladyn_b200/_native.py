@@ -317,6 +317,8 @@ _SIGNATURES = {
     "nd_lj_batch_parameter_backward": [ctypes.POINTER(LJBatchArgs), ctypes.c_void_p],
     "nd_lj_frames": [ctypes.POINTER(LJBatchArgs), ctypes.c_int32, ctypes.c_void_p,
                      ctypes.c_void_p],
+    "nd_lj_frames_parameter_backward": [ctypes.POINTER(LJBatchArgs), ctypes.c_void_p,
+                                        ctypes.c_void_p],
     "nd_wrap": [ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64,
                 ctypes.c_void_p, ctypes.c_void_p],
     "nd_md_import": [

@@ -305,7 +305,8 @@ __device__ __forceinline__ int word_type(double w)
 constexpr int kFrameSums = 7;  // E, W xx yy zz xy xz yz
 constexpr int kFrameSlots = 8;
 
-// The workspace of a batch: float64 sums per frame, packed atoms, and (float32) packed forces.
+// The workspace of a batch: float64 sums (per frame, or of the parameter rows), packed atoms,
+// and packed forces (the forward's in float32, the loss's force gradients in the backward).
 template <typename T>
 struct FrameWorkspace
 {
@@ -313,13 +314,29 @@ struct FrameWorkspace
 
     FrameWorkspace(std::int64_t frames, std::int64_t num_atoms)
     {
-        const std::int64_t slots = frames * num_atoms;
+        const std::int64_t bytes =
+            (frames * num_atoms * static_cast<std::int64_t>(sizeof(PackedAtom<T>)) + 255) / 256 * 256;
         sums = 0;
-        atoms = (frames * kFrameSlots * 8 + 255) / 256 * 256;
-        forces = atoms + (slots * static_cast<std::int64_t>(sizeof(PackedAtom<T>)) + 255) / 256 * 256;
-        total = forces + (sizeof(T) == 4 ? slots * 16 : 0);
+        atoms = (std::max<std::int64_t>(frames * kFrameSlots, 2 * kMaxRows) * 8 + 255) / 256 * 256;
+        forces = atoms + bytes;
+        total = forces + bytes;
     }
 };
+
+template <typename T, bool kWrap>
+__device__ __forceinline__ PackedAtom<T> packed_atom(const T* position, const T* cell,
+                                                     const index_t* atom_types, index_t atom)
+{
+    PackedAtom<T> p{position[0], position[1], position[2],
+                    type_word(T(0), atom_types == nullptr ? 0 : atom_types[atom])};
+    if (kWrap)
+    {
+        p.x = wrap_separately(p.x, cell[0]);
+        p.y = wrap_separately(p.y, cell[1]);
+        p.z = wrap_separately(p.z, cell[2]);
+    }
+    return p;
+}
 
 // Packs the atoms (wrapped into the cell first when kWrap, in space.wrap's rounding) and sets
 // the sums and the forces to zero. One thread per atom of the batch.
@@ -341,20 +358,8 @@ __global__ void __launch_bounds__(kThreads) pack_atoms_kernel(
         return;
     }
     const std::int64_t frame = slot / num_atoms;
-    const index_t atom = static_cast<index_t>(slot - frame * num_atoms);
-    const T* cell = cells + 3 * frame;
-    PackedAtom<T> p;
-    p.x = positions[3 * slot];
-    p.y = positions[3 * slot + 1];
-    p.z = positions[3 * slot + 2];
-    if (kWrap)
-    {
-        p.x = wrap_separately(p.x, cell[0]);
-        p.y = wrap_separately(p.y, cell[1]);
-        p.z = wrap_separately(p.z, cell[2]);
-    }
-    p.w = type_word(T(0), atom_types == nullptr ? 0 : atom_types[atom]);
-    atoms[slot] = p;
+    atoms[slot] = packed_atom<T, kWrap>(positions + 3 * slot, cells + 3 * frame, atom_types,
+                                        static_cast<index_t>(slot - frame * num_atoms));
     if (packed_forces != nullptr)
     {
         packed_forces[slot] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -887,6 +892,7 @@ int lj_pairs(const nd_lj_pairs_args* a, cudaStream_t stream)
     return ND_OK;
 }
 
+// ---------------------------------------------------------------------------------------
 // The parameter backward of a batch: given the loss's gradients with respect to each frame's
 // energy, forces and virial, accumulates dLoss/dsigma and dLoss/depsilon per type-pair row.
 // For a valid column with d = x_i - x_j and f_s = 24 eps (2 p6^2 - p6) / r^2 (so F_i = f_s d,
@@ -896,117 +902,301 @@ int lj_pairs(const nd_lj_pairs_args* a, cudaStream_t stream)
 // 2 pc6^2 + pc6), df_s/deps = f_s / eps and df_s/dsigma = 144 eps p6 (4 p6 - 1) / (sigma r^2).
 // This is the double backward the reference takes through torch.func
 // (src/nabladyn/training/_fit.py:245-271), written out. Per-row sums are float64.
-template <typename T>
-__global__ void __launch_bounds__(kLJThreads) lj_parameter_backward_kernel(
-    const T* __restrict__ positions,
-    const T* __restrict__ cell,
-    const index_t* __restrict__ pairs,
-    std::int64_t capacity,
-    index_t num_atoms,
-    const index_t* __restrict__ atom_types,
-    int num_types,
-    const T* __restrict__ sigma,
-    const T* __restrict__ epsilon,
-    T cutoff_squared,
-    const double* __restrict__ energy_grad,
-    const T* __restrict__ forces_grad,
-    const double* __restrict__ virial_grad,
-    double* __restrict__ sigma_grad,
-    double* __restrict__ epsilon_grad
-)
+//
+// A column gathers two atoms and two force gradients and scatters nothing, so with packed
+// slots it is bound by the float64 arithmetic: the row's constants are worked out once per
+// block, and a thread keeps its rows' sums to itself (in registers for one row, else in its own
+// column of shared memory), since float64 atomics on a few shared words serialise the block.
+
+// One type-pair row's float64 constants.
+struct RowGradients
 {
+    double s2, eps24_s, eps144_s, pc_deps, pc_dsigma;
+};
+
+template <typename T>
+struct BackwardPass
+{
+    FramesPass<T> frames;             // atoms, cells, pairs, parameters
+    const PackedAtom<T>* force_slots; // packed force gradients, or null:
+    const T* force_grads;             // [F, N, 3]
+    const T* energy_grad;             // packed: [F] and [F, 9] in the frames' dtype
+    const T* virial_grad;
+    const double* energy_grad64;      // else float64
+    const double* virial_grad64;
+    double* row_sums;                 // sigma rows, then epsilon rows
+    double* epsilon_sums;
+};
+
+template <typename T, bool kPacked>
+__device__ __forceinline__ PackedAtom<T> gather_gradient(const BackwardPass<T>& a, index_t atom)
+{
+    if constexpr (kPacked)
+    {
+        return a.force_slots[atom];
+    }
+    else
+    {
+        const T* g = a.force_grads + 3LL * atom;
+        return {g[0], g[1], g[2], T(0)};
+    }
+}
+
+// 1 / x in float64. A float32 x starts from the hardware estimate (23 bits), doubled twice.
+__device__ __forceinline__ double reciprocal64(float x)
+{
+    float estimate;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(estimate) : "f"(x));
+    double y = estimate;
+    const double d = x;
+    y = fma(y, fma(-d, y, 1.0), y);
+    return fma(y, fma(-d, y, 1.0), y);
+}
+__device__ __forceinline__ double reciprocal64(double x) { return 1.0 / x; }
+
+template <typename T, bool kPacked, bool kTypes>
+__global__ void __launch_bounds__(kLJThreads) lj_parameter_backward_kernel(BackwardPass<T> a)
+{
+    extern __shared__ double own_sums[];  // [2 rows][kLJThreads] with several types
     const std::int64_t frame = blockIdx.y;
-    positions += frame * 3 * num_atoms;
-    cell += frame * 3;
-    pairs += frame * 2 * capacity;
-    forces_grad += frame * 3 * num_atoms;
-    const double ge = energy_grad[frame];
+    FramesPass<T>& f = a.frames;
+    if (kPacked)
+    {
+        f.atoms += frame * f.num_atoms;
+        a.force_slots += frame * f.num_atoms;
+    }
+    else
+    {
+        f.positions += 3 * frame * f.num_atoms;
+        a.force_grads += 3 * frame * f.num_atoms;
+    }
+    f.cells += 3 * frame;
+    f.pairs += 2 * frame * f.capacity;
+    const double ge = kPacked ? static_cast<double>(a.energy_grad[frame]) : a.energy_grad64[frame];
     double gw[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k)
     {
-        gw[k] = virial_grad[frame * 9 + k];
+        gw[k] = kPacked ? static_cast<double>(a.virial_grad[9 * frame + k])
+                        : a.virial_grad64[9 * frame + k];
     }
-    const int rows = num_types * (num_types + 1) / 2;
-    __shared__ double row_grads[2 * kMaxRows];
-    for (int k = threadIdx.x; k < 2 * rows; k += blockDim.x)
+    // d^T g_W d takes the sums of mirrored entries.
+    const double gxy = gw[1] + gw[3], gxz = gw[2] + gw[6], gyz = gw[5] + gw[7];
+    __shared__ RowGradients rows[kTypes ? kMaxRows : 1];
+    const int row_count = kTypes ? f.num_types * (f.num_types + 1) / 2 : 1;
+    if (threadIdx.x < row_count)
     {
-        row_grads[k] = 0.0;
-    }
-    __syncthreads();
-    const T lx = cell[0], ly = cell[1], lz = cell[2];
-    const std::int64_t stride = static_cast<std::int64_t>(gridDim.x) * blockDim.x;
-    for (std::int64_t column = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-         column < capacity; column += stride)
-    {
-        const index_t i = pairs[column];
-        const index_t j = pairs[capacity + column];
-        if (i == j || static_cast<unsigned>(i) >= static_cast<unsigned>(num_atoms) ||
-            static_cast<unsigned>(j) >= static_cast<unsigned>(num_atoms))
-        {
-            continue;
-        }
-        const T dx = displacement(positions[3LL * i], positions[3LL * j], lx);
-        const T dy = displacement(positions[3LL * i + 1], positions[3LL * j + 1], ly);
-        const T dz = displacement(positions[3LL * i + 2], positions[3LL * j + 2], lz);
-        const T r2 = dx * dx + dy * dy + dz * dz;
-        if (!(r2 < cutoff_squared))
-        {
-            continue;
-        }
-        const int row = atom_types == nullptr ? 0 : pair_row(atom_types[i], atom_types[j], num_types);
-        const double s = sigma[row];
-        const double eps = epsilon[row];
-        const double inv_r2 = 1.0 / double(r2);
-        const double q = s * s * inv_r2;
-        const double p6 = q * q * q;
-        const double qc = s * s / double(cutoff_squared);
+        const double s = f.sigma[threadIdx.x], eps = f.epsilon[threadIdx.x];
+        const double qc = s * s / static_cast<double>(f.cutoff_squared);
         const double pc6 = qc * qc * qc;
-        const double fs = 24.0 * eps * (2.0 * p6 * p6 - p6) * inv_r2;
-        const double x = dx, y = dy, z = dz;
-        const double dgx = double(forces_grad[3LL * i]) - double(forces_grad[3LL * j]);
-        const double dgy = double(forces_grad[3LL * i + 1]) - double(forces_grad[3LL * j + 1]);
-        const double dgz = double(forces_grad[3LL * i + 2]) - double(forces_grad[3LL * j + 2]);
-        const double g = x * dgx + y * dgy + z * dgz +
-                         x * (gw[0] * x + gw[1] * y + gw[2] * z) +
-                         y * (gw[3] * x + gw[4] * y + gw[5] * z) +
-                         z * (gw[6] * x + gw[7] * y + gw[8] * z);
-        const double du_deps = 4.0 * (p6 * p6 - p6) - 4.0 * (pc6 * pc6 - pc6);
-        const double du_dsigma = 24.0 * eps / s * (2.0 * p6 * p6 - p6 - 2.0 * pc6 * pc6 + pc6);
-        const double dfs_deps = fs / eps;
-        const double dfs_dsigma = 144.0 * eps * p6 * (4.0 * p6 - 1.0) * inv_r2 / s;
-        atomicAdd(row_grads + row, ge * du_dsigma + g * dfs_dsigma);
-        atomicAdd(row_grads + rows + row, ge * du_deps + g * dfs_deps);
+        rows[threadIdx.x] = {s * s, 24.0 * eps / s, 144.0 * eps / s, 4.0 * (pc6 * pc6 - pc6),
+                             2.0 * pc6 * pc6 - pc6};
+    }
+    if (kTypes)
+    {
+        for (int r = 0; r < 2 * row_count; ++r)
+        {
+            own_sums[r * kLJThreads + threadIdx.x] = 0.0;
+        }
     }
     __syncthreads();
-    for (int k = threadIdx.x; k < rows; k += blockDim.x)
+    double sigma_sum = 0.0, epsilon_sum = 0.0;  // one type
+    const T lx = f.cells[0], ly = f.cells[1], lz = f.cells[2];
+    const auto capacity = static_cast<unsigned>(f.capacity);
+    const index_t* firsts = f.pairs;
+    const index_t* seconds = f.pairs + f.capacity;
+    const unsigned stride = gridDim.x * kLJThreads;
+    for (unsigned column = blockIdx.x * kLJThreads + threadIdx.x; column < capacity;
+         column += stride)
     {
-        atomicAdd(sigma_grad + k, row_grads[k]);
-        atomicAdd(epsilon_grad + k, row_grads[rows + k]);
+        const index_t i = firsts[column], j = seconds[column];
+        if (!counts(i, j, f.num_atoms))
+        {
+            continue;
+        }
+        const PackedAtom<T> left = gather<T, kPacked>(f, i), right = gather<T, kPacked>(f, j);
+        const T tx = displacement(left.x, right.x, lx);
+        const T ty = displacement(left.y, right.y, ly);
+        const T tz = displacement(left.z, right.z, lz);
+        const T r2 = tx * tx + ty * ty + tz * tz;
+        if (!(r2 < f.cutoff_squared))
+        {
+            continue;
+        }
+        const PackedAtom<T> gi = gather_gradient<T, kPacked>(a, i);
+        const PackedAtom<T> gj = gather_gradient<T, kPacked>(a, j);
+        const int row =
+            kTypes ? pair_row(word_type(left.w), word_type(right.w), f.num_types) : 0;
+        const RowGradients c = rows[row];
+        const double inv_r2 = reciprocal64(r2);
+        const double q = c.s2 * inv_r2;
+        const double p6 = q * q * q;
+        const double x = tx, y = ty, z = tz;
+        const double dgx = static_cast<double>(gi.x) - static_cast<double>(gj.x);
+        const double dgy = static_cast<double>(gi.y) - static_cast<double>(gj.y);
+        const double dgz = static_cast<double>(gi.z) - static_cast<double>(gj.z);
+        const double g = x * (dgx + gw[0] * x + gxy * y + gxz * z) +
+                         y * (dgy + gw[4] * y + gyz * z) + z * (dgz + gw[8] * z);
+        const double slope = p6 * (2.0 * p6 - 1.0);  // 2 p6^2 - p6
+        const double pull = g * inv_r2;
+        const double dsigma = c.eps24_s * (ge * (slope - c.pc_dsigma)) +
+                              c.eps144_s * (pull * (p6 * (4.0 * p6 - 1.0)));
+        const double depsilon = ge * (4.0 * (p6 * (p6 - 1.0)) - c.pc_deps) + 24.0 * (pull * slope);
+        if (kTypes)
+        {
+            own_sums[row * kLJThreads + threadIdx.x] += dsigma;
+            own_sums[(row_count + row) * kLJThreads + threadIdx.x] += depsilon;
+        }
+        else
+        {
+            sigma_sum += dsigma;
+            epsilon_sum += depsilon;
+        }
+    }
+    if (!kTypes)
+    {
+        double values[2] = {sigma_sum, epsilon_sum};
+        double* const out[2] = {a.row_sums, a.epsilon_sums};
+        add_block_sums(values, out);
+        return;
+    }
+    __syncthreads();
+    const int lane = threadIdx.x % kWarp;
+    for (int r = threadIdx.x / kWarp; r < 2 * row_count; r += kLJThreads / kWarp)
+    {
+        double sum = 0.0;
+#pragma unroll
+        for (int k = 0; k < kLJThreads; k += kWarp)
+        {
+            sum += own_sums[r * kLJThreads + k + lane];
+        }
+        sum = warp_sum(sum);
+        if (lane == 0)
+        {
+            atomicAdd(r < row_count ? a.row_sums + r : a.epsilon_sums + (r - row_count), sum);
+        }
     }
 }
 
+template <typename T, bool kPacked>
+int launch_backward(const BackwardPass<T>& pass, std::int64_t frames, cudaStream_t stream)
+{
+    unsigned blocks = 1;
+    const int counted = frame_blocks<kLJThreads>(pass.frames.capacity, frames, 8, &blocks);
+    if (counted != ND_OK)
+    {
+        return counted;
+    }
+    const dim3 grid(blocks, static_cast<unsigned>(frames));
+    if (pass.frames.num_types == 1)
+    {
+        lj_parameter_backward_kernel<T, kPacked, false><<<grid, kLJThreads, 0, stream>>>(pass);
+    }
+    else
+    {
+        const int rows = pass.frames.num_types * (pass.frames.num_types + 1) / 2;
+        const std::size_t bytes = 2 * rows * kLJThreads * sizeof(double);
+        static DeviceGrant grant;
+        ND_CUDA_TRY(grant.allow(lj_parameter_backward_kernel<T, kPacked, true>, bytes));
+        lj_parameter_backward_kernel<T, kPacked, true><<<grid, kLJThreads, bytes, stream>>>(pass);
+    }
+    ND_LAUNCH_CHECK();
+    return ND_OK;
+}
+
+template <typename T>
+FramesPass<T> backward_frames(const nd_lj_batch_args* a)
+{
+    const T rc = static_cast<T>(a->cutoff);
+    FramesPass<T> frames{};
+    frames.positions = static_cast<const T*>(a->positions);
+    frames.atom_types = a->num_types > 1 ? a->atom_types : nullptr;
+    frames.cells = static_cast<const T*>(a->cells);
+    frames.pairs = a->pairs;
+    frames.capacity = a->capacity;
+    frames.num_atoms = static_cast<index_t>(a->num_atoms);
+    frames.num_types = a->num_types;
+    frames.sigma = static_cast<const T*>(a->sigma);
+    frames.epsilon = static_cast<const T*>(a->epsilon);
+    frames.cutoff_squared = rc * rc;
+    return frames;
+}
+
+// Without a workspace: the caller's arrays as they are.
 template <typename T>
 int lj_batch_parameter_backward(const nd_lj_batch_args* a, cudaStream_t stream)
 {
     const int rows = a->num_types * (a->num_types + 1) / 2;
     ND_CUDA_TRY(cudaMemsetAsync(a->sigma_grad, 0, sizeof(double) * rows, stream));
     ND_CUDA_TRY(cudaMemsetAsync(a->epsilon_grad, 0, sizeof(double) * rows, stream));
-    const T rc = static_cast<T>(a->cutoff);
-    const auto* types = a->num_types > 1 ? a->atom_types : nullptr;
-    unsigned blocks = 1;
-    const int counted = frame_blocks<kLJThreads>(a->capacity, a->frames, 8, &blocks);
-    if (counted != ND_OK)
+    BackwardPass<T> pass{};
+    pass.frames = backward_frames<T>(a);
+    pass.force_grads = static_cast<const T*>(a->forces_grad);
+    pass.energy_grad64 = a->energy_grad;
+    pass.virial_grad64 = a->virial_grad;
+    pass.row_sums = a->sigma_grad;
+    pass.epsilon_sums = a->epsilon_grad;
+    return launch_backward<T, false>(pass, a->frames, stream);
+}
+
+// Packs the force gradients and sets the row sums to zero.
+template <typename T>
+__global__ void __launch_bounds__(kThreads) pack_gradients_kernel(
+    const T* __restrict__ force_grads, std::int64_t slots, PackedAtom<T>* __restrict__ gradients,
+    double* __restrict__ sums)
+{
+    const std::int64_t slot = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (blockIdx.x == 0 && threadIdx.x < 2 * kMaxRows)
     {
-        return counted;
+        sums[threadIdx.x] = 0.0;
     }
-    const dim3 grid(blocks, static_cast<unsigned>(a->frames));
-    lj_parameter_backward_kernel<T><<<grid, kLJThreads, 0, stream>>>(
-        static_cast<const T*>(a->positions), static_cast<const T*>(a->cells), a->pairs,
-        a->capacity, static_cast<index_t>(a->num_atoms), types, a->num_types,
-        static_cast<const T*>(a->sigma), static_cast<const T*>(a->epsilon), rc * rc,
-        a->energy_grad, static_cast<const T*>(a->forces_grad), a->virial_grad, a->sigma_grad,
-        a->epsilon_grad);
+    if (slot < slots)
+    {
+        const T* g = force_grads + 3 * slot;
+        gradients[slot] = {g[0], g[1], g[2], T(0)};
+    }
+}
+
+// The row sums in the parameters' dtype.
+template <typename T>
+__global__ void cast_rows_kernel(const double* __restrict__ sums, int rows,
+                                 T* __restrict__ sigma_grad, T* __restrict__ epsilon_grad)
+{
+    if (threadIdx.x < rows)
+    {
+        sigma_grad[threadIdx.x] = static_cast<T>(sums[threadIdx.x]);
+        epsilon_grad[threadIdx.x] = static_cast<T>(sums[kMaxRows + threadIdx.x]);
+    }
+}
+
+template <typename T>
+int lj_frames_parameter_backward(const nd_lj_batch_args* a, void* workspace, cudaStream_t stream)
+{
+    const std::int64_t n = a->num_atoms, slots = n * a->frames;
+    const FrameWorkspace<T> ws(a->frames, n);
+    auto* base = static_cast<unsigned char*>(workspace);
+    auto* sums = reinterpret_cast<double*>(base + ws.sums);
+    auto* gradients = reinterpret_cast<PackedAtom<T>*>(base + ws.forces);
+    pack_gradients_kernel<T><<<blocks_for(slots), kThreads, 0, stream>>>(
+        static_cast<const T*>(a->forces_grad), slots, gradients, sums);
+    ND_LAUNCH_CHECK();
+    BackwardPass<T> pass{};
+    pass.frames = backward_frames<T>(a);
+    pass.frames.atoms = reinterpret_cast<const PackedAtom<T>*>(
+        static_cast<const unsigned char*>(a->positions) + ws.atoms);
+    pass.force_slots = gradients;
+    pass.energy_grad = reinterpret_cast<const T*>(a->energy_grad);
+    pass.virial_grad = reinterpret_cast<const T*>(a->virial_grad);
+    pass.row_sums = sums;
+    pass.epsilon_sums = sums + kMaxRows;
+    const int launched = launch_backward<T, true>(pass, a->frames, stream);
+    if (launched != ND_OK)
+    {
+        return launched;
+    }
+    cast_rows_kernel<T><<<1, 64, 0, stream>>>(
+        sums, a->num_types * (a->num_types + 1) / 2, reinterpret_cast<T*>(a->sigma_grad),
+        reinterpret_cast<T*>(a->epsilon_grad));
     ND_LAUNCH_CHECK();
     return ND_OK;
 }
@@ -1074,6 +1264,24 @@ extern "C" int nd_lj_frames(const nd_lj_batch_args* args, int32_t wrap, void* wo
     auto s = static_cast<cudaStream_t>(stream);
     return args->dtype == ND_FLOAT32 ? nd::lj_frames<float>(args, wrap != 0, workspace, s)
                                      : nd::lj_frames<double>(args, wrap != 0, workspace, s);
+}
+
+extern "C" int nd_lj_frames_parameter_backward(const nd_lj_batch_args* args, void* workspace,
+                                               nd_stream_t stream)
+{
+    const int rc = nd::check_batch(args, true);
+    if (rc != ND_OK)
+    {
+        return rc;
+    }
+    ND_REQUIRE(workspace != nullptr, "the workspace is null");
+    ND_REQUIRE(reinterpret_cast<std::uintptr_t>(workspace) % 256 == 0 &&
+                   reinterpret_cast<std::uintptr_t>(args->positions) % 256 == 0,
+               "the workspaces must be 256-byte aligned");
+    auto s = static_cast<cudaStream_t>(stream);
+    return args->dtype == ND_FLOAT32
+               ? nd::lj_frames_parameter_backward<float>(args, workspace, s)
+               : nd::lj_frames_parameter_backward<double>(args, workspace, s);
 }
 
 extern "C" int nd_wrap(int dtype, const void* positions, const void* cells, int64_t frames,

@@ -174,8 +174,9 @@ def evaluate_frames(positions: Tensor, cells: Tensor, index: Tensor, kernel_type
                     num_types: int, sigma: Tensor, epsilon: Tensor, cutoff: float,
                     wrap: bool):
     """(E [F], F [F, N, 3], W [F, 3, 3]) of frames [F, N, 3] in the positions' dtype, from
-    nd_lj_frames: cells [F, 3], index int32 [F, 2, C] (all contiguous), the parameters in the
-    positions' dtype; ``wrap`` for positions that may lie outside the cell. No host sync."""
+    nd_lj_frames, and its workspace, which holds the packed frames: cells [F, 3], index int32
+    [F, 2, C] (all contiguous), the parameters in the positions' dtype; ``wrap`` for positions
+    that may lie outside the cell. No host sync."""
     device, dtype = positions.device, positions.dtype
     frames, atoms = positions.shape[0], positions.shape[1]
     code = dtype_code(dtype)
@@ -193,7 +194,7 @@ def evaluate_frames(positions: Tensor, cells: Tensor, index: Tensor, kernel_type
     )
     with on_device(device):
         call("nd_lj_frames", args, int(wrap), ptr(workspace), stream_handle(device))
-    return energy, forces, virial
+    return energy, forces, virial, workspace
 
 
 class _LJEnergy(torch.autograd.Function):
@@ -315,7 +316,7 @@ class LennardJones(Potential):
         index = pairs.index.detach()
         if index.dtype != torch.int32:
             index = index.to(torch.int32)
-        energy, forces, virial = evaluate_frames(
+        energy, forces, virial, _ = evaluate_frames(
             positions.detach().contiguous()[None], cell.detach().contiguous()[None],
             index.contiguous()[None], self._kernel_types, self._num_types,
             self.sigma.detach().to(dtype).contiguous(),

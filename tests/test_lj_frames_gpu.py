@@ -1,4 +1,4 @@
-"""nd_lj_frames and nd_wrap against plain torch float64 on the same inputs, where the kernels can
+"""nd_lj_frames, its parameter backward and nd_wrap against plain torch float64 on the same inputs, where the kernels can
 go wrong: capacities around the 4 columns of a lane and the 128 of a warp (so the second row
 starts at every offset from a 16-byte boundary), columns in any order, self-pairs and indices
 outside the atoms between live ones, one to three frames and types, positions outside the cell.
@@ -15,6 +15,7 @@ import torch
 
 from nabladyn_b200 import space
 from nabladyn_b200.potential._lennard_jones import evaluate_frames, pair_index
+from nabladyn_b200.training._predict import _BatchLJ
 
 pytestmark = pytest.mark.gpu
 
@@ -82,10 +83,10 @@ def test_frames_match_float64(cuda, dtype, frames, atoms, capacity, types, group
     x, cells, index, kinds, sigma, epsilon = system(frames, atoms, capacity, types, dtype, cuda,
                                                     grouped)
     got = evaluate_frames(x, cells, index, kinds.to(torch.int32), types, sigma, epsilon, CUTOFF,
-                          True)
+                          True)[:3]
     wrapped = space.wrapped_only(x, cells)
     again = evaluate_frames(wrapped, cells, index, kinds.to(torch.int32), types, sigma, epsilon,
-                            CUTOFF, False)
+                            CUTOFF, False)[:3]
     want = reference(wrapped, cells, index, kinds, types, sigma, epsilon)
     tolerance = 1e-12 if dtype == torch.float64 else 1e-5
     for values in (got, again):
@@ -93,6 +94,36 @@ def test_frames_match_float64(cuda, dtype, frames, atoms, capacity, types, group
             assert value.dtype == dtype and value.shape == exact.shape
             scale = float(exact.abs().max()) + 1.0
             assert float((value.double() - exact).abs().max()) <= tolerance * scale
+
+
+@pytest.mark.parametrize("dtype", (torch.float32, torch.float64))
+@pytest.mark.parametrize("frames, atoms, capacity, types, grouped", [
+    (1, 2, 1, 1, True), (2, 9, 5, 2, False), (3, 40, 255, 1, True), (2, 65, 257, 3, True),
+    (1, 130, 70001, 8, False),
+])
+def test_parameter_gradients_match_float64(cuda, dtype, frames, atoms, capacity, types, grouped):
+    """The backward of arbitrary adjoints of E, F and W, one to thirty-six parameter rows. The
+    rows' sums are float64; the float32 inputs' geometry carries float32 roundings."""
+    x, cells, index, kinds, sigma, epsilon = system(frames, atoms, capacity, types, dtype, cuda,
+                                                    grouped)
+    generator = torch.Generator().manual_seed(capacity)
+    adjoints = [torch.randn(shape, generator=generator, dtype=torch.float64).to(dtype).to(cuda)
+                for shape in ((frames,), (frames, atoms, 3), (frames, 3, 3))]
+    parameters = [p.clone().requires_grad_(True) for p in (sigma, epsilon)]
+    values = _BatchLJ.apply(*parameters, x, cells, index, kinds.to(torch.int32), types, CUTOFF)
+    got = torch.autograd.grad(values, parameters, adjoints, retain_graph=True)
+    again = torch.autograd.grad(values, parameters, adjoints)
+    exact_parameters = [p.double().requires_grad_(True) for p in (sigma, epsilon)]
+    exact = reference(space.wrapped_only(x, cells), cells, index, kinds, types,
+                      *exact_parameters)
+    want = torch.autograd.grad(exact, exact_parameters, [a.double() for a in adjoints])
+    # A row's terms may cancel: the scale is their size, about that of the largest row.
+    tolerance = 1e-11 if dtype == torch.float64 else 1e-4
+    for value, second, exact_value in zip(got, again, want):
+        assert value.dtype == dtype
+        scale = float(exact_value.abs().max()) + 1.0
+        assert float((value.double() - exact_value).abs().max()) <= tolerance * scale
+        assert float((second.double() - exact_value).abs().max()) <= tolerance * scale
 
 
 @pytest.mark.parametrize("dtype", (torch.float32, torch.float64))
