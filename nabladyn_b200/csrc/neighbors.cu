@@ -13,13 +13,12 @@
 // How the GPU builds it is this file's own design:
 //   * binning takes each atom's in-bin slot from the counting atomic, and one warp per bin
 //     orders the bin by id with shuffles while gathering the sorted positions;
-//   * the pairs are built per HOME BIN, one warp each. Every candidate of a home bin's atoms
+//   * the pairs are built per HOME BIN, one CTA each. Every candidate of a home bin's atoms
 //     sits in the home bin itself (after the atom) or in a stencil bin that comes later in bin
-//     order; the warp stages exactly those bins into shared memory as 16-B (x, y, z, id) slots,
-//     each bin's coordinates already moved by its image where the move is exact. The lanes are
-//     the home bin's atoms: each staged candidate is read once (a broadcast) and tested against
-//     all of them, and a lane sets one bit per hit in a word of 32 candidates, so the count is
-//     a popcount per word and only the fill's writes diverge;
+//     order; the CTA stages exactly those bins into shared memory as (x, y, z, id) slots, each
+//     bin's coordinates already moved by its image where the move is exact, tests each staged
+//     candidate against 32 of the bin's atoms at a time into words of hit bits, and either
+//     counts the bits or turns them into columns in shared memory that leave in whole lines;
 //   * small boxes (at most three bins per axis) keep a word-major bit matrix: one thread per
 //     (center, 32-candidate word) with the word's candidates staged in shared memory, so
 //     threads of a block store consecutive words;
@@ -30,6 +29,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdint>
@@ -163,20 +163,23 @@ __global__ void order_bins_kernel(
 }
 
 // ---------------------------------------------------------------------------------------
-// Pairs on the grid path: one warp per home bin.
+// Pairs on the grid path: one CTA per home bin.
+//
+// What bounds a build is the distance tests (about 410 candidates for each of a bin's 30 atoms
+// in a liquid, 15 % of them hits) and, in the fill, the appends. So a candidate is read once
+// from shared memory for 32 centers: a lane holds two centers, the two halves of a warp take
+// alternate words of 32 candidates, and in float32 the two centers are the halves of packed
+// f32x2 instructions whose sign bits a funnel shift collects. The four warps share a bin's
+// words, so the few bins of a small system still fill a CTA, and the hits of a word are
+// appended by a thread of their own: a center's words find their columns by a 16-lane scan.
+// A bin's columns are one contiguous range, so entries go to shared memory first and leave in
+// whole lines.
 
-constexpr int kHoodWarps = 4;                 // bins per CTA, one per warp
-constexpr int kHoodThreads = kHoodWarps * kWarp;
-constexpr int kHoodBins = 27;                 // the home bin and its stencil, at most
-
-// Shared-memory slots of one warp's neighborhood: 8 KB in either dtype (512 float32 or 256
-// float64 candidates; a liquid at 21 atoms/nm^3 with 1.1 nm bins needs about 410). A larger
-// neighborhood is read from global memory instead, with the same arithmetic.
-template <typename T>
-struct HoodSlots
-{
-    static constexpr int value = 8192 / static_cast<int>(sizeof(Slot<T>));
-};
+constexpr int kHoodThreads = 128;
+constexpr int kHoodBins = 27;      // the home bin and its stencil, at most
+constexpr int kHoodSlots = 512;    // candidates staged at once (a liquid needs about 410)
+constexpr int kHoodWords = kHoodSlots / kWarp;
+constexpr int kHoodEntries = 3072;  // pairs of 32 centers staged at once (a liquid: 2,000)
 
 // The part of a home bin's stencil that holds candidates: the home bin (its atoms after the
 // center) and each stencil bin that comes later in bin order (all its atoms). With three or
@@ -193,6 +196,7 @@ struct Hood
     int slot[kHoodBins + 1];      // first slot of each bin in the staged list
     unsigned char ahead[kHoodBins];
     unsigned char behind[kHoodBins];
+    int any_ahead;
 };
 
 // One warp lists the home bin's stencil. Lane s takes stencil bin s; the kept bins follow the
@@ -242,6 +246,7 @@ __device__ __forceinline__ void plan_hood(
         keep = bin > home;
     }
     const unsigned kept = __ballot_sync(kFullMask, keep);
+    const unsigned ahead_lanes = __ballot_sync(kFullMask, keep && ahead != 0);
     const int count = 1 + __popc(kept);
     if (keep)
     {
@@ -260,6 +265,7 @@ __device__ __forceinline__ void plan_hood(
         hood.ahead[0] = 0;
         hood.behind[0] = 0;
         hood.count = count;
+        hood.any_ahead = ahead_lanes != 0;
     }
     __syncwarp();
     // Slots: an exclusive scan of the kept bins' sizes, in their order.
@@ -304,136 +310,102 @@ __device__ __forceinline__ Slot<T> hood_candidate(
     return out;
 }
 
-// One word of the lane's center against 32 consecutive candidates of kept bin `g` (each read
-// once for the whole warp): bit j is set when candidate base + j is closer than the radius.
-template <typename T, bool kFixed, bool kStaged>
-__device__ __forceinline__ unsigned hit_word(
-    const Hood& hood, const Slot<T>* __restrict__ staged,
-    const T* __restrict__ sorted_positions, const index_t* __restrict__ sorted_ids,
-    int g, int base, int size, const Slot<T>& c, T ax, T ay, T az, T lx, T ly, T lz,
-    T radius_squared)
+// How a home bin's displacements are taken (one choice per CTA).
+enum HoodImages : int
 {
-    auto test = [&](int j) {
-        const int k = base + j;
-        const Slot<T> p = kStaged ? staged[hood.slot[g] + k]
-                                  : hood_candidate(hood, g, k, sorted_positions, sorted_ids,
-                                                   lx, ly, lz);
-        T dx, dy, dz;
-        if (kFixed)
+    kPlain,    // fixed images, no kept bin past an upper face: center - candidate
+    kAhead,    // fixed images: the center moves by -L towards bins past an upper face
+    kMinimum,  // an axis of fewer than three bins: the minimum image per candidate
+};
+
+// A lane's two centers. For kAhead also the centers moved by -L, rounded once.
+template <typename T>
+struct CenterPair
+{
+    T x0, y0, z0, x1, y1, z1;
+};
+
+// Shifts into the bits of two centers from the right: set when the candidate lies closer than
+// the radius (r^2 - R^2 is negative exactly when r^2 < R^2).
+template <typename T>
+__device__ __forceinline__ void shift_in_hits(T x0, T y0, T z0, T x1, T y1, T z1,
+                                              const Slot<T>& p, T radius_squared,
+                                              unsigned& bits0, unsigned& bits1)
+{
+    const T r0 = squared_norm(x0 - p.x, y0 - p.y, z0 - p.z);
+    const T r1 = squared_norm(x1 - p.x, y1 - p.y, z1 - p.z);
+    bits0 = (bits0 << 1) | static_cast<unsigned>(r0 < radius_squared);
+    bits1 = (bits1 << 1) | static_cast<unsigned>(r1 < radius_squared);
+}
+
+// The two centers as the halves of packed f32x2 instructions: each half rounds as the scalar
+// test, p - x being the exact negative of x - p.
+__device__ __forceinline__ void shift_in_hits(float x0, float y0, float z0, float x1, float y1,
+                                              float z1, const Slot<float>& p,
+                                              float radius_squared, unsigned& bits0,
+                                              unsigned& bits1)
+{
+    const float2 dx = __fadd2_rn(make_float2(p.x, p.x), make_float2(-x0, -x1));
+    const float2 dy = __fadd2_rn(make_float2(p.y, p.y), make_float2(-y0, -y1));
+    const float2 dz = __fadd2_rn(make_float2(p.z, p.z), make_float2(-z0, -z1));
+    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dx, dx, __fmul2_rn(dy, dy)));
+    const float2 d = __fadd2_rn(r2, make_float2(-radius_squared, -radius_squared));
+    bits0 = __funnelshift_l(__float_as_uint(d.x), bits0, 1);
+    bits1 = __funnelshift_l(__float_as_uint(d.y), bits1, 1);
+}
+
+// The hits of a lane's two centers among the 32 staged candidates from slot `base`: bit j for
+// candidate base + j.
+template <typename T, int kImages>
+__device__ __forceinline__ void hit_words(
+    const Slot<T>* __restrict__ staged, const unsigned char* __restrict__ ahead, int base,
+    const CenterPair<T>& c, T lx, T ly, T lz, T radius_squared, unsigned& hits0, unsigned& hits1)
+{
+    hits0 = hits1 = 0;
+#pragma unroll 8
+    for (int j = kWarp - 1; j >= 0; --j)
+    {
+        const Slot<T> p = staged[base + j];
+        if (kImages == kMinimum)
         {
-            dx = ax - p.x;
-            dy = ay - p.y;
-            dz = az - p.z;
+            const T r0 = squared_norm(min_image(c.x0, p.x, lx), min_image(c.y0, p.y, ly),
+                                      min_image(c.z0, p.z, lz));
+            const T r1 = squared_norm(min_image(c.x1, p.x, lx), min_image(c.y1, p.y, ly),
+                                      min_image(c.z1, p.z, lz));
+            hits0 = (hits0 << 1) | static_cast<unsigned>(r0 < radius_squared);
+            hits1 = (hits1 << 1) | static_cast<unsigned>(r1 < radius_squared);
+        }
+        else if (kImages == kAhead)
+        {
+            const unsigned moved = ahead[base + j];
+            const T sx = (moved & 1u) ? lx : T(0), sy = (moved & 2u) ? ly : T(0),
+                    sz = (moved & 4u) ? lz : T(0);
+            shift_in_hits(c.x0 - sx, c.y0 - sy, c.z0 - sz, c.x1 - sx, c.y1 - sy, c.z1 - sz, p,
+                          radius_squared, hits0, hits1);
         }
         else
         {
-            dx = min_image(c.x, p.x, lx);
-            dy = min_image(c.y, p.y, ly);
-            dz = min_image(c.z, p.z, lz);
-        }
-        return squared_norm(dx, dy, dz) < radius_squared;
-    };
-    unsigned hits = 0;
-    if (size == kWarp)
-    {
-#pragma unroll
-        for (int j = 0; j < kWarp; ++j)
-        {
-            hits |= test(j) ? 1u << j : 0u;
+            shift_in_hits(c.x0, c.y0, c.z0, c.x1, c.y1, c.z1, p, radius_squared, hits0, hits1);
         }
     }
-    else
-    {
-        for (int j = 0; j < size; ++j)
-        {
-            hits |= test(j) ? 1u << j : 0u;
-        }
-    }
-    return hits;
 }
 
-// One warp, one home bin: the lanes are the bin's atoms (32 at a time), every candidate is
-// read once per warp and tested against all of them. Each lane keeps a word of hits per 32
-// candidates: the count adds its popcount; the fill writes its set bits from the lane's next
-// column (only the writes diverge).
-template <typename T, bool kFill, bool kFixed, bool kStaged>
-__device__ __forceinline__ void hood_lanes(
-    const Hood& hood, const Slot<T>* __restrict__ staged,
-    const T* __restrict__ sorted_positions, const index_t* __restrict__ sorted_ids,
-    T lx, T ly, T lz, T radius_squared,
-    index_t* __restrict__ pair_counts, const index_t* __restrict__ pair_offsets,
-    std::int64_t capacity, index_t* __restrict__ pairs)
+// Bits of a word from slot `first` on whose candidates come after center `h` (slots and
+// centers count from the home bin's first atom) and before slot `end`.
+__device__ __forceinline__ unsigned word_mask(int first, int h, int end)
 {
-    const int lane = threadIdx.x % kWarp;
-    const int homes = hood.size[0];
-    for (int group = 0; group < homes; group += kWarp)
-    {
-        const int h = group + lane;
-        const bool active = h < homes;
-        const Slot<T> c = !active ? Slot<T>{T(0), T(0), T(0), T(0)}
-                          : kStaged ? staged[h]
-                                    : hood_candidate(hood, 0, h, sorted_positions, sorted_ids,
-                                                     lx, ly, lz);
-        // The center past the lower face of a later bin's image: center - L, rounded once.
-        const T cx_ahead = c.x - lx, cy_ahead = c.y - ly, cz_ahead = c.z - lz;
-        const index_t center = hood.first[0] + h;
-        index_t count = 0;
-        std::int64_t column = kFill && active ? pair_offsets[center] : 0;
-        const index_t center_id = kFill && active ? sorted_ids[center] : 0;
-        // The home bin's candidates start after the group's first center.
-        for (int g = 0; g < hood.count; ++g)
-        {
-            const unsigned ahead = hood.ahead[g];
-            const T ax = (ahead & 1u) ? cx_ahead : c.x;
-            const T ay = (ahead & 2u) ? cy_ahead : c.y;
-            const T az = (ahead & 4u) ? cz_ahead : c.z;
-            const int end = hood.size[g];
-            for (int base = g == 0 ? group + 1 : 0; base < end; base += kWarp)
-            {
-                const int size = end - base < kWarp ? end - base : kWarp;
-                unsigned hits = hit_word<T, kFixed, kStaged>(hood, staged, sorted_positions,
-                                                             sorted_ids, g, base, size, c, ax,
-                                                             ay, az, lx, ly, lz, radius_squared);
-                if (g == 0)
-                {
-                    // Only candidates after the lane's own center: bits above h - base.
-                    const int above = h - base + 1;
-                    hits &= above <= 0 ? ~0u : (above >= kWarp ? 0u : ~0u << above);
-                }
-                hits = active ? hits : 0u;
-                if (kFill)
-                {
-                    while (hits != 0)
-                    {
-                        const int j = __ffs(hits) - 1;
-                        hits &= hits - 1;
-                        if (column < capacity)
-                        {
-                            const index_t other =
-                                kStaged ? word_id(staged[hood.slot[g] + base + j].w)
-                                        : sorted_ids[hood.first[g] + base + j];
-                            pairs[column] = center_id;
-                            pairs[capacity + column] = other;
-                        }
-                        ++column;
-                    }
-                }
-                else
-                {
-                    count += __popc(hits);
-                }
-            }
-        }
-        if (!kFill && active)
-        {
-            pair_counts[center] = count;
-        }
-    }
+    const int above = h + 1 - first, size = end - first;
+    const unsigned after = above <= 0 ? ~0u : (above >= kWarp ? 0u : ~0u << above);
+    const unsigned before = size >= kWarp ? ~0u : (size <= 0 ? 0u : (1u << size) - 1u);
+    return after & before;
 }
 
-// Counts (kFill false) or writes (kFill true) the pairs of one home bin per warp. The fill of
-// an update also stores the frame it was built from: each warp its home atoms' positions, the
-// first warp the cell and the rebuild count.
+// Counts (kFill false) or writes (kFill true) the pairs of one home bin. The fill of an update
+// also stores the frame it was built from: each CTA its home atoms' positions, the first the
+// cell and the rebuild count.
+//
+// The candidates, home bin first, are staged kHoodSlots at a time (once, in all but very dense
+// bins) and tested against the bin's atoms 32 at a time.
 template <typename T, bool kFill>
 __global__ void __launch_bounds__(kHoodThreads) hood_pairs_kernel(
     const T* __restrict__ sorted_positions,
@@ -442,7 +414,6 @@ __global__ void __launch_bounds__(kHoodThreads) hood_pairs_kernel(
     const index_t* __restrict__ dims,
     const T* __restrict__ cell,
     T radius_squared,
-    std::int64_t num_bins,
     index_t* __restrict__ pair_counts,
     const index_t* __restrict__ pair_offsets,
     index_t capacity,
@@ -455,71 +426,231 @@ __global__ void __launch_bounds__(kHoodThreads) hood_pairs_kernel(
     const index_t* __restrict__ status
 )
 {
-    const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
-    const std::int64_t home = static_cast<std::int64_t>(blockIdx.x) * kHoodWarps + warp;
-    if (home >= num_bins || !rebuilding(rebuild, status))
+    if (!rebuilding(rebuild, status))
     {
-        return;  // whole warps; no block barrier follows
+        return;
     }
-    __shared__ Hood hoods[kHoodWarps];
-    __shared__ Slot<T> tiles[kHoodWarps][HoodSlots<T>::value];
-    Hood& hood = hoods[warp];
-    Slot<T>* staged = tiles[warp];
-    const bool fixed = dims[0] >= 3 && dims[1] >= 3 && dims[2] >= 3;
-    const T lx = cell[0], ly = cell[1], lz = cell[2];
-    plan_hood(hood, static_cast<index_t>(home), dims, bin_offsets, fixed);
-    const int homes = hood.size[0];
+    const index_t home = static_cast<index_t>(blockIdx.x);
+    const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
+    const index_t begin = bin_offsets[home];
+    const int homes = bin_offsets[home + 1] - begin;
     if (kFill && reference_positions != nullptr)
     {
-        for (int k = lane; k < 3 * homes; k += kWarp)
+        for (int k = threadIdx.x; k < 3 * homes; k += kHoodThreads)
         {
-            const std::int64_t id = sorted_ids[hood.first[0] + k / 3];
+            const std::int64_t id = sorted_ids[begin + k / 3];
             reference_positions[3 * id + k % 3] = positions[3 * id + k % 3];
         }
-        if (home == 0 && lane < 3)
+        if (home == 0 && threadIdx.x < 3)
         {
-            reference_cell[lane] = cell[lane];
+            reference_cell[threadIdx.x] = cell[threadIdx.x];
         }
-        if (home == 0 && lane == 0)
+        if (home == 0 && threadIdx.x == 0)
         {
             ++rebuild_count[0];
         }
     }
     if (homes == 0)
     {
-        return;
+        return;  // the whole CTA
     }
-    const bool stage = hood.total <= HoodSlots<T>::value;
-    if (stage)
+    __shared__ Hood hood;
+    __shared__ Slot<T> staged[kHoodSlots];
+    __shared__ unsigned char ahead[kHoodSlots];
+    __shared__ unsigned words[kFill ? kHoodWords : 1][kWarp + 1];  // one center apart: no conflicts
+    __shared__ std::uint16_t entries[kFill ? kHoodEntries : 1];    // center << 9 | slot
+    __shared__ int cursors[kWarp];                                 // fill: each center's next column
+    __shared__ int warp_counts[kHoodThreads / kWarp][kWarp];
+    const T lx = cell[0], ly = cell[1], lz = cell[2];
+    const bool fixed = dims[0] >= 3 && dims[1] >= 3 && dims[2] >= 3;
+    if (warp == 0)
     {
-        for (int g = 0; g < hood.count; ++g)
+        plan_hood(hood, home, dims, bin_offsets, fixed);
+    }
+    __syncthreads();
+    const int images = !fixed ? kMinimum : (hood.any_ahead ? kAhead : kPlain);
+    const int total = hood.total;
+    const bool once = total <= kHoodSlots;
+    const int half = lane / 16, q = lane % 16;
+    for (int group = 0; group < homes; group += kWarp)
+    {
+        const int centers = homes - group < kWarp ? homes - group : kWarp;
+        const int h0 = group + 2 * q, h1 = h0 + 1;
+        CenterPair<T> c;
         {
-            for (int k = lane; k < hood.size[g]; k += kWarp)
+            const T* p0 = sorted_positions + 3LL * (begin + (h0 < homes ? h0 : group));
+            const T* p1 = sorted_positions + 3LL * (begin + (h1 < homes ? h1 : group));
+            c = {p0[0], p0[1], p0[2], p1[0], p1[1], p1[2]};
+        }
+        int count0 = 0, count1 = 0;
+        index_t region = 0;
+        int region_size = 0;
+        if (kFill)
+        {
+            // The group's columns are one range: its centers follow one another.
+            region = pair_offsets[begin + group];
+            const index_t last = begin + group + centers - 1;
+            region_size = pair_offsets[last] + pair_counts[last] - region;
+            if (threadIdx.x < centers)
             {
-                staged[hood.slot[g] + k] =
-                    hood_candidate(hood, g, k, sorted_positions, sorted_ids, lx, ly, lz);
+                cursors[threadIdx.x] = pair_offsets[begin + group + threadIdx.x];
             }
         }
-        __syncwarp();
-    }
-    const std::int64_t cap = capacity;
-    if (fixed)
-    {
-        stage ? hood_lanes<T, kFill, true, true>(hood, staged, sorted_positions, sorted_ids, lx,
-                                                 ly, lz, radius_squared, pair_counts,
-                                                 pair_offsets, cap, pairs)
-              : hood_lanes<T, kFill, true, false>(hood, staged, sorted_positions, sorted_ids, lx,
-                                                  ly, lz, radius_squared, pair_counts,
-                                                  pair_offsets, cap, pairs);
-    }
-    else
-    {
-        stage ? hood_lanes<T, kFill, false, true>(hood, staged, sorted_positions, sorted_ids, lx,
-                                                  ly, lz, radius_squared, pair_counts,
-                                                  pair_offsets, cap, pairs)
-              : hood_lanes<T, kFill, false, false>(hood, staged, sorted_positions, sorted_ids,
-                                                   lx, ly, lz, radius_squared, pair_counts,
-                                                   pair_offsets, cap, pairs);
+        const bool packed = kFill && once && region_size <= kHoodEntries;
+        for (int chunk = 0; chunk < total; chunk += kHoodSlots)
+        {
+            const int size = total - chunk < kHoodSlots ? total - chunk : kHoodSlots;
+            if (group == 0 || !once)
+            {
+                __syncthreads();  // the last chunk's readers are done
+                for (int g = warp; g < hood.count; g += kHoodThreads / kWarp)
+                {
+                    const int from = hood.slot[g] - chunk;  // the bin's first slot
+                    int k = lane;
+                    if (from < 0)
+                    {
+                        k += -from / kWarp * kWarp;
+                    }
+                    for (; k < hood.size[g] && from + k < size; k += kWarp)
+                    {
+                        if (from + k >= 0)
+                        {
+                            staged[from + k] = hood_candidate(hood, g, k, sorted_positions,
+                                                              sorted_ids, lx, ly, lz);
+                            ahead[from + k] = hood.ahead[g];
+                        }
+                    }
+                }
+                __syncthreads();
+            }
+            const int used = (size + kWarp - 1) / kWarp;
+            for (int pair = warp; 2 * pair < used; pair += kHoodThreads / kWarp)
+            {
+                const int w = 2 * pair + half;  // at most kHoodWords - 1
+                unsigned hits0, hits1;
+                if (images == kPlain)
+                {
+                    hit_words<T, kPlain>(staged, ahead, kWarp * w, c, lx, ly, lz, radius_squared,
+                                         hits0, hits1);
+                }
+                else if (images == kAhead)
+                {
+                    hit_words<T, kAhead>(staged, ahead, kWarp * w, c, lx, ly, lz, radius_squared,
+                                         hits0, hits1);
+                }
+                else
+                {
+                    hit_words<T, kMinimum>(staged, ahead, kWarp * w, c, lx, ly, lz,
+                                           radius_squared, hits0, hits1);
+                }
+                const int slot = chunk + kWarp * w;
+                hits0 &= h0 < homes ? word_mask(slot, h0, chunk + size) : 0u;
+                hits1 &= h1 < homes ? word_mask(slot, h1, chunk + size) : 0u;
+                if (kFill)
+                {
+                    words[w][2 * q] = hits0;
+                    words[w][2 * q + 1] = hits1;
+                }
+                else
+                {
+                    count0 += __popc(hits0);
+                    count1 += __popc(hits1);
+                }
+            }
+            if (!kFill)
+            {
+                continue;
+            }
+            __syncthreads();
+            // A lane per (center, word): its hits follow those of the center's earlier words.
+            for (int pair = warp; 2 * pair < centers; pair += kHoodThreads / kWarp)
+            {
+                const int center = 2 * pair + half, w = q;
+                unsigned hits = center < centers && w < used ? words[w][center] : 0u;
+                const int count = __popc(hits);
+                int inclusive = count;
+#pragma unroll
+                for (int offset = 1; offset < 16; offset *= 2)
+                {
+                    const int up = __shfl_up_sync(kFullMask, inclusive, offset, 16);
+                    inclusive += w >= offset ? up : 0;
+                }
+                index_t column = (center < centers ? cursors[center] : 0) + inclusive - count;
+                __syncwarp();
+                if (w == 15 && center < centers)
+                {
+                    cursors[center] += inclusive;
+                }
+                if (packed)
+                {
+                    int at = column - region;
+                    while (hits != 0)
+                    {
+                        const int j = __ffs(hits) - 1;
+                        hits &= hits - 1;
+                        if (static_cast<unsigned>(at) < static_cast<unsigned>(kHoodEntries))
+                        {
+                            entries[at] =
+                                static_cast<std::uint16_t>(center << 9 | (kWarp * w + j));
+                        }
+                        ++at;
+                    }
+                }
+                else
+                {
+                    const index_t id = hits != 0 ? sorted_ids[begin + group + center] : 0;
+                    while (hits != 0)
+                    {
+                        const int j = __ffs(hits) - 1;
+                        hits &= hits - 1;
+                        if (static_cast<unsigned>(column) < static_cast<unsigned>(capacity))
+                        {
+                            pairs[column] = id;
+                            pairs[static_cast<std::int64_t>(capacity) + column] =
+                                word_id(staged[kWarp * w + j].w);
+                        }
+                        ++column;
+                    }
+                }
+            }
+            __syncthreads();
+            if (packed)
+            {
+                for (int e = threadIdx.x; e < region_size; e += kHoodThreads)
+                {
+                    const index_t column = region + e;
+                    const unsigned entry = entries[e];
+                    if (static_cast<unsigned>(column) < static_cast<unsigned>(capacity))
+                    {
+                        pairs[column] = word_id(staged[group + (entry >> 9)].w);
+                        pairs[static_cast<std::int64_t>(capacity) + column] =
+                            word_id(staged[entry & 511u].w);
+                    }
+                }
+            }
+        }
+        if (!kFill)
+        {
+            count0 += __shfl_xor_sync(kFullMask, count0, 16);
+            count1 += __shfl_xor_sync(kFullMask, count1, 16);
+            if (half == 0)
+            {
+                warp_counts[warp][2 * q] = count0;
+                warp_counts[warp][2 * q + 1] = count1;
+            }
+            __syncthreads();
+            if (threadIdx.x < centers)
+            {
+                index_t sum = 0;
+#pragma unroll
+                for (int w = 0; w < kHoodThreads / kWarp; ++w)
+                {
+                    sum += warp_counts[w][threadIdx.x];
+                }
+                pair_counts[begin + group + threadIdx.x] = sum;
+            }
+        }
+        __syncthreads();  // the next group's cursors, words and counts
     }
 }
 
@@ -673,9 +804,11 @@ __global__ void row_fill_kernel(
 // Total, overflow and padding, in one launch over the capacity.
 
 // Every thread derives the total from the last count and offset. Column k at or past the
-// total holds the self-pair (k mod N, k mod N), spreading their zero gradients over the atoms.
-// Thread 0 stores the total and, above the capacity, the overflow bit and the pairs needed;
-// with an overflow there is no padding column, so the gate's read of the status cannot race.
+// total holds the self-pair (k mod N, k mod N), spreading their zero gradients over the atoms;
+// the threads start at the total and step by the grid, so each takes one remainder and the
+// stores are whole lines. The first thread stores the total and, above the capacity, the
+// overflow bit and the pairs needed; with an overflow there is no padding column, so the gate's
+// read of the status cannot race.
 __global__ void total_and_pad_kernel(
     const index_t* __restrict__ pair_counts,
     const index_t* __restrict__ pair_offsets,
@@ -687,13 +820,13 @@ __global__ void total_and_pad_kernel(
     const index_t* __restrict__ rebuild
 )
 {
-    const std::int64_t column = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (!rebuilding(rebuild, status))
     {
         return;
     }
     const index_t total = pair_offsets[num_atoms - 1] + pair_counts[num_atoms - 1];
-    if (column == 0)
+    const unsigned thread = blockIdx.x * blockDim.x + threadIdx.x;
+    if (thread == 0)
     {
         pair_total[0] = total;
         if (total > capacity)
@@ -702,13 +835,25 @@ __global__ void total_and_pad_kernel(
             status[1] = total > status[1] ? total : status[1];
         }
     }
-    if (column < capacity && column >= total)
+    if (total >= capacity)
     {
-        const index_t atom = static_cast<index_t>(column % num_atoms);
-        pairs[column] = atom;
-        pairs[capacity + column] = atom;
+        return;
+    }
+    const unsigned n = static_cast<unsigned>(num_atoms);
+    const unsigned end = static_cast<unsigned>(capacity);
+    const unsigned stride = gridDim.x * blockDim.x, step = stride % n;
+    unsigned column = static_cast<unsigned>(total) + thread;  // below 2^32: the grid is bounded
+    unsigned atom = column % n;
+    for (; column < end; column += stride)
+    {
+        pairs[column] = static_cast<index_t>(atom);
+        pairs[static_cast<std::int64_t>(capacity) + column] = static_cast<index_t>(atom);
+        atom += step;
+        atom -= atom >= n ? n : 0u;
     }
 }
+
+constexpr std::int64_t kPadBlocks = 148 * 8;  // every SM full; more columns take more steps
 
 // ---------------------------------------------------------------------------------------
 // The update's gate (the rule of src/nabladyn/neighbors/csrc/update/update.cuh:13-20).
@@ -886,10 +1031,9 @@ void launch_hood(const T* cell, double radius, const List& list, const Commit<T>
     const nd_neighbor_buffers& b = *list.b;
     const T r = static_cast<T>(radius);
     const std::int64_t bins = b.num_bin_slots - 1;
-    hood_pairs_kernel<T, kFill><<<static_cast<unsigned>((bins + kHoodWarps - 1) / kHoodWarps),
-                                  kHoodThreads, 0, stream>>>(
+    hood_pairs_kernel<T, kFill><<<static_cast<unsigned>(bins), kHoodThreads, 0, stream>>>(
         static_cast<const T*>(b.sorted_positions), b.sorted_ids, b.bin_offsets, b.dims, cell,
-        r * r, bins, b.pair_counts, b.pair_offsets, static_cast<index_t>(b.capacity), b.pairs,
+        r * r, b.pair_counts, b.pair_offsets, static_cast<index_t>(b.capacity), b.pairs,
         commit.positions, commit.reference_positions, commit.reference_cell,
         commit.rebuild_count, list.rebuild, b.status);
 }
@@ -941,7 +1085,9 @@ int launch_fill(const T* cell, std::int64_t n, double radius, const List& list,
         launch_hood<T, true>(cell, radius, list, commit, stream);
     }
     ND_LAUNCH_CHECK();
-    total_and_pad_kernel<<<blocks_for(b.capacity), kThreads, 0, stream>>>(
+    const auto pad_blocks = static_cast<unsigned>(
+        std::min<std::int64_t>(blocks_for(b.capacity), kPadBlocks));
+    total_and_pad_kernel<<<pad_blocks, kThreads, 0, stream>>>(
         b.pair_counts, b.pair_offsets, num_atoms, capacity, b.pair_total, b.pairs, b.status,
         list.rebuild);
     ND_LAUNCH_CHECK();

@@ -1,0 +1,49 @@
+"""The grid path's pair build where a home bin does not fit its staging: more than 32 atoms per
+bin, more than 512 candidates (several chunks), more than 3,072 pairs of 32 atoms, a short axis
+(minimum images) with dense bins, atoms past every face. Pair sets, counts and order against the
+oracle: sets bit for bit, each first atom's columns together and in ascending list order twice."""
+
+import numpy as np
+import pytest
+import torch
+
+from nabladyn_b200 import space
+from nabladyn_b200.neighbors import NeighborList
+from oracle import neighbors as on
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", (torch.float32, torch.float64))
+@pytest.mark.parametrize("lengths, radius, background, cluster", [
+    ((4.5, 4.5, 4.5), 1.1, 1300, 0),      # ordinary bins, 4 per axis
+    ((4.5, 4.5, 4.5), 1.1, 3000, 0),      # 47 atoms per bin, some 600 candidates
+    ((4.5, 4.5, 4.5), 1.1, 200, 1200),    # one bin of over a thousand atoms
+    ((5.7, 2.6, 3.4), 1.1, 2200, 300),    # two bins on an axis, dense
+    ((9.0, 4.6, 4.6), 0.5, 900, 5),       # many nearly empty bins
+])
+def test_dense_and_short_grids_match_the_oracle(cuda, dtype, lengths, radius, background,
+                                                cluster):
+    rng = np.random.default_rng(background + cluster)
+    box = np.asarray(lengths)
+    positions = rng.uniform(-0.2, 1.2, (background, 3)) * box
+    dense = 0.05 * box + rng.uniform(0.0, 0.6, (cluster, 3))
+    positions = np.concatenate([positions, dense])
+    x = torch.tensor(positions, dtype=dtype, device=cuda)
+    cell = torch.tensor(box, dtype=dtype, device=cuda)
+    listed = NeighborList(radius, skin=0.0)
+    listed.allocate(x, cell)
+    index = listed.tensors().index.cpu().numpy()
+    total = listed.num_pairs
+    first, second, path = on.pairs(space.wrap(x, cell)[0].cpu().numpy(), cell.cpu().numpy(), radius)
+    assert path == "grid" and total == len(first)
+    np.testing.assert_array_equal(on.pair_set(index[0, :total], index[1, :total]),
+                                  on.pair_set(first, second))
+    runs = np.flatnonzero(np.diff(index[0, :total])) + 1
+    starts = index[0, np.concatenate([[0], runs])]
+    assert len(np.unique(starts)) == len(starts)  # each first atom's columns are together
+    # An update that rebuilds (another frame, then this one again) gives the same columns.
+    listed.update(x + 0.3, cell)
+    listed.update(x, cell)
+    assert listed._rebuild_count == 3
+    np.testing.assert_array_equal(listed.tensors().index.cpu().numpy(), index)
