@@ -354,8 +354,8 @@ __device__ __forceinline__ void shift_in_hits(float x0, float y0, float z0, floa
     bits1 = __funnelshift_l(__float_as_uint(d.y), bits1, 1);
 }
 
-// The hits of a lane's two centers among the 32 staged candidates from slot `base`: bit j for
-// candidate base + j.
+// The hits of a lane's two centers among the 32 staged candidates from slot `base`: bit 31 - j
+// for candidate base + j, so the first candidate is the highest bit (one instruction finds it).
 template <typename T, int kImages>
 __device__ __forceinline__ void hit_words(
     const Slot<T>* __restrict__ staged, const unsigned char* __restrict__ ahead, int base,
@@ -363,7 +363,7 @@ __device__ __forceinline__ void hit_words(
 {
     hits0 = hits1 = 0;
 #pragma unroll 8
-    for (int j = kWarp - 1; j >= 0; --j)
+    for (int j = 0; j < kWarp; ++j)
     {
         const Slot<T> p = staged[base + j];
         if (kImages == kMinimum)
@@ -395,9 +395,17 @@ __device__ __forceinline__ void hit_words(
 __device__ __forceinline__ unsigned word_mask(int first, int h, int end)
 {
     const int above = h + 1 - first, size = end - first;
-    const unsigned after = above <= 0 ? ~0u : (above >= kWarp ? 0u : ~0u << above);
-    const unsigned before = size >= kWarp ? ~0u : (size <= 0 ? 0u : (1u << size) - 1u);
+    const unsigned after = above <= 0 ? ~0u : (above >= kWarp ? 0u : ~0u >> above);
+    const unsigned before = size >= kWarp ? ~0u : (size <= 0 ? 0u : ~(~0u >> size));
     return after & before;
+}
+
+// Takes the first candidate's position out of a word.
+__device__ __forceinline__ int next_hit(unsigned& hits)
+{
+    const int j = __clz(static_cast<int>(hits));
+    hits &= ~(0x80000000u >> j);
+    return j;
 }
 
 // Counts (kFill false) or writes (kFill true) the pairs of one home bin. The fill of an update
@@ -584,14 +592,13 @@ __global__ void __launch_bounds__(kHoodThreads) hood_pairs_kernel(
                 if (packed)
                 {
                     int at = column - region;
+                    const int tag = center << 9 | (kWarp * w);
                     while (hits != 0)
                     {
-                        const int j = __ffs(hits) - 1;
-                        hits &= hits - 1;
+                        const int j = next_hit(hits);
                         if (static_cast<unsigned>(at) < static_cast<unsigned>(kHoodEntries))
                         {
-                            entries[at] =
-                                static_cast<std::uint16_t>(center << 9 | (kWarp * w + j));
+                            entries[at] = static_cast<std::uint16_t>(tag + j);
                         }
                         ++at;
                     }
@@ -601,8 +608,7 @@ __global__ void __launch_bounds__(kHoodThreads) hood_pairs_kernel(
                     const index_t id = hits != 0 ? sorted_ids[begin + group + center] : 0;
                     while (hits != 0)
                     {
-                        const int j = __ffs(hits) - 1;
-                        hits &= hits - 1;
+                        const int j = next_hit(hits);
                         if (static_cast<unsigned>(column) < static_cast<unsigned>(capacity))
                         {
                             pairs[column] = id;
