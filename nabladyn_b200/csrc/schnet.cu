@@ -225,311 +225,320 @@ struct PairPass
     float phase;              // pi / r_c
     int gaussians;
     int first;                // reverse: the first pass (last block) starts dE/dr
-    int last;                 // reverse: the last pass (block 0) applies forces and virial
 };
 
-// Shared memory of the pair passes: weight images, one row tile (each product's operand
-// replaces the last once that product completed), biases, barrier and tensor-memory slot. The
-// reverse pass's 16 KB run stage overlays its B1 and B1^T images, which only the first and
-// the last product of a tile read; they are copied in again (from L2) after the stage was used,
-// so four CTAs fit an SM.
-constexpr int kPairForwardShared = 2 * umma::kImageBytes + umma::kTileBytes + 2 * 256 + 64;
-constexpr int kPairReverseShared = 4 * umma::kImageBytes + umma::kTileBytes + 2 * 256 + 64;
+// Shared memory of the pair passes: the filter layers' two weight images (the reverse pass
+// reads them both ways), one row tile (each product's operand replaces the last once that
+// product completed), in the reverse pass the FP32 filter's stage (the forward pass stages it
+// in the row tile, free by then), biases, the pairs' atoms and envelopes, barrier and
+// tensor-memory slot.
+constexpr int kPairTail = 2 * 256 + 4 * kTile * 4 + 64;
+constexpr int kPairForwardShared = 2 * umma::kImageBytes + umma::kTileBytes + kPairTail;
+constexpr int kPairReverseShared = 2 * umma::kImageBytes + 2 * umma::kTileBytes + kPairTail;
+
+struct PairShared
+{
+    unsigned char* image_b1;
+    unsigned char* image_b2;
+    unsigned char* work;
+    float* stage;
+    float* bias1;
+    float* bias2;
+    int* first;       // -1: a dead row
+    int* second;
+    float* envelope;  // reverse
+    float* along;     // reverse
+    std::uint64_t* barrier;
+    std::uint32_t* slot;
+
+    __device__ PairShared(unsigned char* shared, bool own_stage)
+    {
+        image_b1 = shared;
+        image_b2 = image_b1 + umma::kImageBytes;
+        work = image_b2 + umma::kImageBytes;
+        unsigned char* after = work + umma::kTileBytes;
+        stage = reinterpret_cast<float*>(own_stage ? after : work);
+        bias1 = reinterpret_cast<float*>(own_stage ? after + umma::kTileBytes : after);
+        bias2 = bias1 + kFeatures;
+        first = reinterpret_cast<int*>(bias2 + kFeatures);
+        second = first + kTile;
+        envelope = reinterpret_cast<float*>(second + kTile);
+        along = envelope + kTile;
+        barrier = reinterpret_cast<std::uint64_t*>(along + kTile);
+        slot = reinterpret_cast<std::uint32_t*>(barrier + 1);
+    }
+
+    __device__ void load(const PairPass& a)
+    {
+        copy_bytes(image_b1, a.images + kB1 * umma::kImageBytes, umma::kImageBytes);
+        copy_bytes(image_b2, a.images + kB2 * umma::kImageBytes, umma::kImageBytes);
+        if (threadIdx.x < kFeatures)
+        {
+            bias1[threadIdx.x] = a.b1[threadIdx.x];
+            bias2[threadIdx.x] = a.b2[threadIdx.x];
+        }
+    }
+};
+
+// ssp(z + b1) of this thread's row, from tensor-memory columns 0-63, into the row tile.
+__device__ __forceinline__ void store_softplus(std::uint32_t tmem, const float* bias1,
+                                               unsigned char* tile)
+{
+#pragma unroll 1  // the unrolled kernel overflows the instruction cache
+    for (int half = 0; half < 2; ++half)
+    {
+        float z[32];
+        umma::load32(tmem + 32 * half, z);
+        umma::wait_loads();
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+        {
+            float s[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+            {
+                s[e] = softplus_shifted(z[8 * c + e] + bias1[32 * half + 8 * c + e]);
+            }
+            umma::store8(tile, threadIdx.x, 4 * half + c, s);
+        }
+    }
+}
+
+// A half (32 columns) of this thread's FP32 row, (value + bias) * scale, into the stage.
+__device__ __forceinline__ void stage_half(std::uint32_t tmem, const float* bias, float scale,
+                                           float* stage)
+{
+    float f[32];
+    umma::load32(tmem, f);
+    umma::wait_loads();
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+    {
+        put_run_part(stage, q,
+                     make_float4((f[4 * q] + bias[4 * q]) * scale,
+                                 (f[4 * q + 1] + bias[4 * q + 1]) * scale,
+                                 (f[4 * q + 2] + bias[4 * q + 2]) * scale,
+                                 (f[4 * q + 3] + bias[4 * q + 3]) * scale));
+    }
+}
 
 __global__ void __launch_bounds__(kTile, 6) pair_forward_kernel(PairPass a)
 {
     extern __shared__ __align__(1024) unsigned char shared[];
-    unsigned char* image_b1 = shared;
-    unsigned char* image_b2 = image_b1 + umma::kImageBytes;
-    unsigned char* basis = image_b2 + umma::kImageBytes;
-    unsigned char* work = basis;  // the basis is dead once the first product completed
-    float* bias1 = reinterpret_cast<float*>(work + umma::kTileBytes);
-    float* bias2 = bias1 + kFeatures;
-    auto* barrier = reinterpret_cast<std::uint64_t*>(bias2 + kFeatures);
-    auto* slot = reinterpret_cast<std::uint32_t*>(barrier + 1);
-
-    copy_bytes(image_b1, a.images + kB1 * umma::kImageBytes, umma::kImageBytes);
-    copy_bytes(image_b2, a.images + kB2 * umma::kImageBytes, umma::kImageBytes);
-    if (threadIdx.x < kFeatures)
-    {
-        bias1[threadIdx.x] = a.b1[threadIdx.x];
-        bias2[threadIdx.x] = a.b2[threadIdx.x];
-    }
+    PairShared sh(shared, false);
+    sh.load(a);
     Cores cores;
-    cores.open(barrier, slot, 64, a.counters, 1);
+    cores.open(sh.barrier, sh.slot, 64, a.counters, 1);
     const int count = *reinterpret_cast<volatile int*>(a.counters);
-    const uint4* v8 = reinterpret_cast<const uint4*>(a.v);
-    float4* m4 = reinterpret_cast<float4*>(a.m);
-    __shared__ int tile_first[kTile];
+    const auto* v = reinterpret_cast<const uint2*>(a.v);
+    float4* const m4 = reinterpret_cast<float4*>(a.m);
+    const FeatureLane at;
 
     // Each tile's pair records are loaded one tile ahead, so their latency hides behind the
     // previous tile's products.
     int2 next_ab = make_int2(0, 0);
-    float4 next_g = make_float4(0.f, 0.f, 0.f, 1.f);
-    if (blockIdx.x * kTile + static_cast<int>(threadIdx.x) < count)
-    {
-        next_ab = a.pairs[blockIdx.x * kTile + threadIdx.x];
-        next_g = a.geometry[blockIdx.x * kTile + threadIdx.x];
-    }
+    float next_r = 1.0f;
+    auto load_ahead = [&](int p) {
+        const bool live = p < count;
+        next_ab = live ? a.pairs[p] : make_int2(-1, 0);
+        next_r = live ? a.geometry[p].w : 1.0f;
+    };
+    load_ahead(blockIdx.x * kTile + threadIdx.x);
     for (int tile = blockIdx.x; tile * kTile < count; tile += gridDim.x)
     {
-        const int p = tile * kTile + threadIdx.x;
-        const bool live = p < count;
-        const int2 ab = next_ab;
-        const float4 g = next_g;
-        const int ahead = p + gridDim.x * kTile;
-        next_ab = ahead < count ? a.pairs[ahead] : make_int2(0, 0);
-        next_g = ahead < count ? a.geometry[ahead] : make_float4(0.f, 0.f, 0.f, 1.f);
-        const float envelope = live ? 0.5f * (__cosf(g.w * a.phase) + 1.0f) : 0.0f;
-        tile_first[threadIdx.x] = live ? ab.x : -1;
+        const float r = next_r;
+        const float envelope = 0.5f * (__cosf(r * a.phase) + 1.0f);
+        sh.first[threadIdx.x] = next_ab.x;
+        sh.second[threadIdx.x] = next_ab.y;
+        load_ahead((tile + gridDim.x) * kTile + threadIdx.x);
         cores.tile_index = tile;
-        store_basis(basis, g.w / a.width, a.gaussians, live);
-        if (!cores.run(0, basis, image_b1, 1))
+        store_basis(sh.work, r / a.width, a.gaussians);
+        if (!cores.run(0, sh.work, sh.image_b1, 1))
         {
             break;
         }
-#pragma unroll
-        for (int half = 0; half < 2; ++half)
-        {
-            float z[32];
-            umma::load32(cores.tmem + 32 * half, z);
-            umma::wait_loads();
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-            {
-                float s[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e)
-                {
-                    s[e] = softplus_shifted(z[8 * c + e] + bias1[32 * half + 8 * c + e]);
-                }
-                umma::store8(work, threadIdx.x, 4 * half + c, s);
-            }
-        }
-        if (!cores.run(0, work, image_b2, 2))
+        store_softplus(cores.tmem, sh.bias1, sh.work);
+        if (!cores.run(0, sh.work, sh.image_b2, 2))
         {
             break;
         }
-        float* stage = reinterpret_cast<float*>(work);  // free once the second product is done
-#pragma unroll
+        // Messages: m_a += f v_b along the lane's runs, m_b += f v_a pair by pair.
+#pragma unroll 1
         for (int half = 0; half < 2; ++half)
         {
+            uint2 vb[kLaneRows];
 #pragma unroll
-            for (int batch = 0; batch < 4; batch += kGatherBatch)
+            for (int i = 0; i < kLaneRows; ++i)
             {
-                // The batch's gathers first, so their latencies overlap; dead rows read atom 0
-                // and contribute zeros (their envelope is zero).
-                uint4 raw[kGatherBatch][2];
+                vb[i] = __ldg(v + at.word(sh.second[at.row(i)], half));
+            }
+            stage_half(cores.tmem + 32 * half, sh.bias2 + 32 * half, envelope, sh.stage);
+            __syncwarp();
+            RunSums<1> run;
+            float4* const targets[1] = {m4};
+            float4 va = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                for (int i = 0; i < kGatherBatch; ++i)
+            for (int i = 0; i < kLaneRows; ++i)
+            {
+                const int row = at.row(i);
+                const int first = sh.first[row];
+                if (first != run.atom)
                 {
-                    const int k = 32 * half + 8 * (batch + i);
-                    raw[i][0] = __ldg(v8 + 8 * static_cast<std::int64_t>(ab.x) + k / 8);
-                    raw[i][1] = __ldg(v8 + 8 * static_cast<std::int64_t>(ab.y) + k / 8);
+                    run.flush(targets, at.word(0, half));
+                    run.start(first);
+                    va = widen4(__ldg(v + at.word(first < 0 ? 0 : first, half)));
                 }
-#pragma unroll
-                for (int i = 0; i < kGatherBatch; ++i)
+                if (first >= 0)
                 {
-                    const int c = batch + i;
-                    const int k = 32 * half + 8 * c;
-                    float f[8];
-                    umma::load8(cores.tmem + k, f);
-                    umma::wait_loads();
-                    float va[8], vb[8], filter[8];
-                    widen8(raw[i][0], va);
-                    widen8(raw[i][1], vb);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                    {
-                        filter[j] = (f[j] + bias2[k + j]) * envelope;
-                    }
-                    if (live)
-                    {
-                        const std::int64_t gb = 8 * static_cast<std::int64_t>(ab.y) + k / 8;
-                        atomicAdd(m4 + 2 * gb, make_float4(filter[0] * va[0], filter[1] * va[1],
-                                                           filter[2] * va[2], filter[3] * va[3]));
-                        atomicAdd(m4 + 2 * gb + 1,
-                                  make_float4(filter[4] * va[4], filter[5] * va[5],
-                                              filter[6] * va[6], filter[7] * va[7]));
-                    }
-                    put_run_part(stage, 2 * c, make_float4(filter[0] * vb[0], filter[1] * vb[1],
-                                                           filter[2] * vb[2], filter[3] * vb[3]));
-                    put_run_part(stage, 2 * c + 1,
-                                 make_float4(filter[4] * vb[4], filter[5] * vb[5],
-                                             filter[6] * vb[6], filter[7] * vb[7]));
+                    const float4 f = staged4(sh.stage, row, at.lane);
+                    atomicAdd(m4 + at.word(sh.second[row], half), f * va);
+                    run.sums[0] = run.sums[0] + f * widen4(vb[i]);
                 }
             }
-            sum_runs(stage, tile_first, a.m, half, half == 1);  // the next basis overwrites it
+            run.flush(targets, at.word(0, half));
+            __syncwarp();  // the stage's rows are this warp's own: its next writes come after
         }
     }
     cores.close(64);
 }
 
+// Eight values per lane, summed over the eight lanes of each group: lane l returns the sum of
+// value l.
+__device__ __forceinline__ float sum_across(const float (&values)[8], int lane)
+{
+    float four[4], two[2];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+    {
+        const float keep = (lane & 4) ? values[k + 4] : values[k];
+        const float give = (lane & 4) ? values[k] : values[k + 4];
+        four[k] = keep + __shfl_xor_sync(kFullMask, give, 4);
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+    {
+        const float keep = (lane & 2) ? four[k + 2] : four[k];
+        const float give = (lane & 2) ? four[k] : four[k + 2];
+        two[k] = keep + __shfl_xor_sync(kFullMask, give, 2);
+    }
+    const float keep = (lane & 1) ? two[1] : two[0];
+    const float give = (lane & 1) ? two[0] : two[1];
+    return keep + __shfl_xor_sync(kFullMask, give, 1);
+}
+
+// kLast: the last pass (block 0) has no Gv to scatter and applies forces and virial.
+template <bool kLast>
 __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
 {
     extern __shared__ __align__(1024) unsigned char shared[];
-    unsigned char* image_b1 = shared;
-    unsigned char* image_b1t = image_b1 + umma::kImageBytes;
-    unsigned char* image_b2 = image_b1t + umma::kImageBytes;
-    unsigned char* image_b2t = image_b2 + umma::kImageBytes;
-    unsigned char* basis = image_b2t + umma::kImageBytes;
-    unsigned char* work = basis;  // each operand replaces the last once its product completed
-    float* stage = reinterpret_cast<float*>(image_b1);  // Gv runs, 16 KB over B1 and B1^T
-    float* bias1 = reinterpret_cast<float*>(work + umma::kTileBytes);
-    float* bias2 = bias1 + kFeatures;
-    auto* barrier = reinterpret_cast<std::uint64_t*>(bias2 + kFeatures);
-    auto* slot = reinterpret_cast<std::uint32_t*>(barrier + 1);
-
-    copy_bytes(image_b1, a.images + kB1 * umma::kImageBytes, umma::kImageBytes);
-    copy_bytes(image_b2, a.images + kB2 * umma::kImageBytes, umma::kImageBytes);
-    copy_bytes(image_b2t, a.images + kB2T * umma::kImageBytes, umma::kImageBytes);
-    copy_bytes(image_b1t, a.images + kB1T * umma::kImageBytes, umma::kImageBytes);
-    if (threadIdx.x < kFeatures)
-    {
-        bias1[threadIdx.x] = a.b1[threadIdx.x];
-        bias2[threadIdx.x] = a.b2[threadIdx.x];
-    }
+    PairShared sh(shared, true);
+    sh.load(a);
     // Columns 0-63 keep z1 - b1 for the whole tile; 64-127 take the other products in turn.
     Cores cores;
-    cores.open(barrier, slot, 128, a.counters, 2);
+    cores.open(sh.barrier, sh.slot, 128, a.counters, 2);
     const int count = *reinterpret_cast<volatile int*>(a.counters);
-    const uint4* v8 = reinterpret_cast<const uint4*>(a.v);
-    const uint4* gm8 = reinterpret_cast<const uint4*>(a.grad_m);
-    float4* gv4 = reinterpret_cast<float4*>(a.grad_v);
-    __shared__ int tile_first[kTile];
+    const auto* v = reinterpret_cast<const uint2*>(a.v);
+    const auto* gm = reinterpret_cast<const uint2*>(a.grad_m);
+    float4* const gv4 = reinterpret_cast<float4*>(a.grad_v);
+    const FeatureLane at;
     double w[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // xx yy zz xy xz yz
 
     // Each tile's pair records are loaded one tile ahead (see pair_forward_kernel).
-    int2 next_ab = make_int2(0, 0);
+    int2 next_ab = make_int2(-1, 0);
     float4 next_g = make_float4(0.f, 0.f, 0.f, 1.f);
-    if (blockIdx.x * kTile + static_cast<int>(threadIdx.x) < count)
-    {
-        next_ab = a.pairs[blockIdx.x * kTile + threadIdx.x];
-        next_g = a.geometry[blockIdx.x * kTile + threadIdx.x];
-    }
+    auto load_ahead = [&](int p) {
+        const bool live = p < count;
+        next_ab = live ? a.pairs[p] : make_int2(-1, 0);
+        next_g = live ? a.geometry[p] : make_float4(0.f, 0.f, 0.f, 1.f);
+    };
+    load_ahead(blockIdx.x * kTile + threadIdx.x);
     for (int tile = blockIdx.x; tile * kTile < count; tile += gridDim.x)
     {
         const int p = tile * kTile + threadIdx.x;
-        const bool live = p < count;
         const int2 ab = next_ab;
         const float4 g = next_g;
-        const int ahead = p + gridDim.x * kTile;
-        next_ab = ahead < count ? a.pairs[ahead] : make_int2(0, 0);
-        next_g = ahead < count ? a.geometry[ahead] : make_float4(0.f, 0.f, 0.f, 1.f);
+        load_ahead((tile + gridDim.x) * kTile + threadIdx.x);
         float sine, cosine;
         __sincosf(g.w * a.phase, &sine, &cosine);
-        const float envelope = live ? 0.5f * (cosine + 1.0f) : 0.0f;
-        const float slope = live ? -0.5f * a.phase * sine : 0.0f;
         const float t = g.w / a.width;
-        tile_first[threadIdx.x] = live ? ab.x : -1;
+        sh.first[threadIdx.x] = ab.x;
+        sh.second[threadIdx.x] = ab.y;
+        sh.envelope[threadIdx.x] = 0.5f * (cosine + 1.0f);
         cores.tile_index = tile;
-        if (gv4 != nullptr && tile != blockIdx.x)
-        {
-            // the previous tile's run stage overwrote B1
-            copy_bytes(image_b1, a.images + kB1 * umma::kImageBytes, umma::kImageBytes);
-        }
-        store_basis(basis, t, a.gaussians, live);
-        if (!cores.run(0, basis, image_b1, 1))
+        store_basis(sh.work, t, a.gaussians);
+        if (!cores.run(0, sh.work, sh.image_b1, 1))
         {
             break;
         }
         // ssp(z1) into the work tile; z1 - b1 stays in columns 0-63.
-#pragma unroll
-        for (int half = 0; half < 2; ++half)
-        {
-            float z[32];
-            umma::load32(cores.tmem + 32 * half, z);
-            umma::wait_loads();
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-            {
-                float s[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e)
-                {
-                    s[e] = softplus_shifted(z[8 * c + e] + bias1[32 * half + 8 * c + e]);
-                }
-                umma::store8(work, threadIdx.x, 4 * half + c, s);
-            }
-        }
-        if (!cores.run(64, work, image_b2, 2))
+        store_softplus(cores.tmem, sh.bias1, sh.work);
+        if (!cores.run(64, sh.work, sh.image_b2, 2))
         {
             break;
         }
-        // f_raw, Gf = Gm_a v_b + Gm_b v_a, C' Gf . f_raw, Gv, and Gf C into the work tile.
-        float along = 0.0f;
-#pragma unroll
+        // f_raw, Gf = Gm_a v_b + Gm_b v_a, Gf . f_raw, Gv, and Gf C into the work tile.
+        float along[kLaneRows] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
         for (int half = 0; half < 2; ++half)
         {
+            uint2 vb[kLaneRows], mb[kLaneRows];
 #pragma unroll
-            for (int batch = 0; batch < 4; batch += kGatherBatch)
+            for (int i = 0; i < kLaneRows; ++i)
             {
-                // The batch's gathers first; dead rows read atom 0 and contribute zeros.
-                uint4 raw[kGatherBatch][4];
-#pragma unroll
-                for (int i = 0; i < kGatherBatch; ++i)
-                {
-                    const int k = 32 * half + 8 * (batch + i);
-                    const std::int64_t ga = 8 * static_cast<std::int64_t>(ab.x) + k / 8;
-                    const std::int64_t gb = 8 * static_cast<std::int64_t>(ab.y) + k / 8;
-                    raw[i][0] = __ldg(v8 + ga);
-                    raw[i][1] = __ldg(v8 + gb);
-                    raw[i][2] = __ldg(gm8 + ga);
-                    raw[i][3] = __ldg(gm8 + gb);
-                }
-#pragma unroll
-                for (int i = 0; i < kGatherBatch; ++i)
-                {
-                    const int c = batch + i;
-                    const int k = 32 * half + 8 * c;
-                    float f[8];
-                    umma::load8(cores.tmem + 64 + k, f);
-                    umma::wait_loads();
-                    float va[8], vb[8], ma[8], mb[8];
-                    widen8(raw[i][0], va);
-                    widen8(raw[i][1], vb);
-                    widen8(raw[i][2], ma);
-                    widen8(raw[i][3], mb);
-                    float scaled[8], to_first[8], to_second[8];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                    {
-                        const float gf = ma[j] * vb[j] + mb[j] * va[j];
-                        const float raw_filter = f[j] + bias2[k + j];
-                        along += gf * raw_filter;
-                        to_second[j] = raw_filter * envelope * ma[j];
-                        to_first[j] = raw_filter * envelope * mb[j];
-                        scaled[j] = gf * envelope;
-                    }
-                    if (gv4 != nullptr)
-                    {
-                        if (live)
-                        {
-                            const std::int64_t gb = 8 * static_cast<std::int64_t>(ab.y) + k / 8;
-                            atomicAdd(gv4 + 2 * gb, make_float4(to_second[0], to_second[1],
-                                                                to_second[2], to_second[3]));
-                            atomicAdd(gv4 + 2 * gb + 1, make_float4(to_second[4], to_second[5],
-                                                                    to_second[6], to_second[7]));
-                        }
-                        put_run_part(stage, 2 * c, make_float4(to_first[0], to_first[1],
-                                                               to_first[2], to_first[3]));
-                        put_run_part(stage, 2 * c + 1, make_float4(to_first[4], to_first[5],
-                                                                   to_first[6], to_first[7]));
-                    }
-                    umma::store8(work, threadIdx.x, 4 * half + c, scaled);
-                }
+                const std::int64_t word = at.word(sh.second[at.row(i)], half);
+                vb[i] = __ldg(v + word);
+                mb[i] = __ldg(gm + word);
             }
-            if (gv4 != nullptr)
+            stage_half(cores.tmem + 64 + 32 * half, sh.bias2 + 32 * half, 1.0f, sh.stage);
+            __syncwarp();
+            RunSums<1> run;
+            float4* const targets[1] = {gv4};
+            float4 va = make_float4(0.f, 0.f, 0.f, 0.f), ma = va;
+#pragma unroll
+            for (int i = 0; i < kLaneRows; ++i)
             {
-                sum_runs(stage, tile_first, a.grad_v, half, half == 1);  // B1^T is copied over it
+                const int row = at.row(i);
+                const int first = sh.first[row];
+                if (first != run.atom)
+                {
+                    if (!kLast)
+                    {
+                        run.flush(targets, at.word(0, half));
+                    }
+                    run.start(first);
+                    const std::int64_t word = at.word(first < 0 ? 0 : first, half);
+                    va = widen4(__ldg(v + word));
+                    ma = widen4(__ldg(gm + word));
+                }
+                const float envelope = sh.envelope[row];
+                const float4 raw = staged4(sh.stage, row, at.lane);
+                const float4 right = widen4(vb[i]), right_gm = widen4(mb[i]);
+                const float4 gf = ma * right + right_gm * va;
+                along[i] += sum4(gf * raw);
+                if (!kLast && first >= 0)
+                {
+                    const float4 scaled = raw * envelope;
+                    atomicAdd(gv4 + at.word(sh.second[row], half), scaled * ma);
+                    run.sums[0] = run.sums[0] + scaled * right_gm;
+                }
+                *reinterpret_cast<uint2*>(sh.work +
+                                          umma::image_offset(row, 32 * half + 4 * at.lane)) =
+                    make_uint2(pack2(gf.x * envelope, gf.y * envelope),
+                               pack2(gf.z * envelope, gf.w * envelope));
             }
+            if (!kLast)
+            {
+                run.flush(targets, at.word(0, half));
+            }
+            __syncwarp();  // the stage's rows are this warp's own: its next writes come after
         }
-        if (!cores.run(64, work, image_b2t, 3))
+        sh.along[at.row(at.lane)] = sum_across(along, at.lane);
+        if (!cores.run_transposed(64, sh.work, sh.image_b2, 3))
         {
             break;
         }
         // ((Gf C) B2) * sigmoid(z1) into the work tile.
-#pragma unroll
+#pragma unroll 1
         for (int half = 0; half < 2; ++half)
         {
             float q[32];
@@ -544,17 +553,12 @@ __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
 #pragma unroll
                 for (int e = 0; e < 8; ++e)
                 {
-                    s[e] = q[8 * c + e] * sigmoid(z[8 * c + e] + bias1[32 * half + 8 * c + e]);
+                    s[e] = q[8 * c + e] * sigmoid(z[8 * c + e] + sh.bias1[32 * half + 8 * c + e]);
                 }
-                umma::store8(work, threadIdx.x, 4 * half + c, s);
+                umma::store8(sh.work, threadIdx.x, 4 * half + c, s);
             }
         }
-        if (gv4 != nullptr)
-        {
-            // this tile's run stage overwrote B1^T
-            copy_bytes(image_b1t, a.images + kB1T * umma::kImageBytes, umma::kImageBytes);
-        }
-        if (!cores.run(64, work, image_b1t, 4))
+        if (!cores.run_transposed(64, sh.work, sh.image_b1, 4))
         {
             break;
         }
@@ -568,22 +572,28 @@ __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
             umma::load32(cores.tmem + 64 + 32 * half, u);
             umma::wait_loads();
 #pragma unroll
-            for (int e = 0; e < 32; ++e)
+            for (int c = 0; c < 4; ++c)
             {
-                const int k = 32 * half + e;
-                const float offset = t - static_cast<float>(k);
-                const float g = k < a.gaussians ? __expf(-0.5f * offset * offset) : 0.0f;
-                through -= u[e] * g * offset;
+                if (32 * half + 8 * c < a.gaussians)
+                {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                    {
+                        const float offset = t - static_cast<float>(32 * half + 8 * c + e);
+                        through -= u[8 * c + e] * gaussian(offset) * offset;
+                    }
+                }
             }
         }
-        if (live)
+        if (ab.x >= 0)
         {
-            float total = slope * along + through / a.width;
+            const float slope = -0.5f * a.phase * sine;
+            float total = slope * sh.along[threadIdx.x] + through / a.width;
             if (!a.first)
             {
                 total += a.dedr[p];
             }
-            if (!a.last)
+            if (!kLast)
             {
                 a.dedr[p] = total;
             }
@@ -593,12 +603,14 @@ __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
                 const float ux = scale * g.x, uy = scale * g.y, uz = scale * g.z;
                 if (a.forces != nullptr)
                 {
-                    atomicAdd(a.forces + 3 * static_cast<std::int64_t>(ab.x), -ux);
-                    atomicAdd(a.forces + 3 * static_cast<std::int64_t>(ab.x) + 1, -uy);
-                    atomicAdd(a.forces + 3 * static_cast<std::int64_t>(ab.x) + 2, -uz);
-                    atomicAdd(a.forces + 3 * static_cast<std::int64_t>(ab.y), ux);
-                    atomicAdd(a.forces + 3 * static_cast<std::int64_t>(ab.y) + 1, uy);
-                    atomicAdd(a.forces + 3 * static_cast<std::int64_t>(ab.y) + 2, uz);
+                    float* fa = a.forces + 3 * static_cast<std::int64_t>(ab.x);
+                    float* fb = a.forces + 3 * static_cast<std::int64_t>(ab.y);
+                    atomicAdd(fa, -ux);
+                    atomicAdd(fa + 1, -uy);
+                    atomicAdd(fa + 2, -uz);
+                    atomicAdd(fb, ux);
+                    atomicAdd(fb + 1, uy);
+                    atomicAdd(fb + 2, uz);
                 }
                 w[0] -= static_cast<double>(ux) * g.x;
                 w[1] -= static_cast<double>(uy) * g.y;
@@ -609,7 +621,7 @@ __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
             }
         }
     }
-    if (a.last && a.virial != nullptr)
+    if (kLast && a.virial != nullptr)
     {
         __shared__ double sums[4][6];
 #pragma unroll
@@ -1077,16 +1089,19 @@ int nd_schnet_energy_force_virial(const nd_schnet_args* args, nd_stream_t stream
     ND_CUDA_TRY(configured.run([] {
         cudaError_t rc = cudaFuncSetAttribute(pair_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairForwardShared);
         auto then = [&rc](cudaError_t next) { rc = rc != cudaSuccess ? rc : next; };
-        then(cudaFuncSetAttribute(pair_reverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairReverseShared));
+        then(cudaFuncSetAttribute(pair_reverse_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairReverseShared));
+        then(cudaFuncSetAttribute(pair_reverse_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairReverseShared));
         then(cudaFuncSetAttribute(atom_forward_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAtomShared));
         then(cudaFuncSetAttribute(atom_forward_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAtomShared));
         then(cudaFuncSetAttribute(atom_reverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAtomShared));
         then(cudaFuncSetAttribute(pair_forward_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-        then(cudaFuncSetAttribute(pair_reverse_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        then(cudaFuncSetAttribute(pair_reverse_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        then(cudaFuncSetAttribute(pair_reverse_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
         return rc;
     }));
     const int forward_grid = pair_grid(reinterpret_cast<const void*>(pair_forward_kernel), kPairForwardShared, 64);
-    const int reverse_grid = std::min(kVirialSlots, pair_grid(reinterpret_cast<const void*>(pair_reverse_kernel), kPairReverseShared, 128));
+    const int reverse_grid = pair_grid(reinterpret_cast<const void*>(pair_reverse_kernel<false>), kPairReverseShared, 128);
+    const int last_grid = std::min(kVirialSlots, pair_grid(reinterpret_cast<const void*>(pair_reverse_kernel<true>), kPairReverseShared, 128));
 
     ND_CUDA_TRY(cudaMemsetAsync(counters, 0, 256, stream));
     if (s.forces != nullptr)
@@ -1188,15 +1203,21 @@ int nd_schnet_energy_force_virial(const nd_schnet_args* args, nd_stream_t stream
             pass.grad_v = b > 0 ? grad_v : nullptr;
             pass.dedr = dedr;
             pass.first = last ? 1 : 0;
-            pass.last = b == 0 ? 1 : 0;
             pass.forces = s.forces;
             pass.virial = virial_partials;
-            pair_reverse_kernel<<<reverse_grid, kTile, kPairReverseShared, stream>>>(pass);
+            if (b > 0)
+            {
+                pair_reverse_kernel<false><<<reverse_grid, kTile, kPairReverseShared, stream>>>(pass);
+            }
+            else
+            {
+                pair_reverse_kernel<true><<<last_grid, kTile, kPairReverseShared, stream>>>(pass);
+            }
             ND_LAUNCH_CHECK();
         }
     }
     finalize_kernel<<<1, 256, 0, stream>>>(energy_partials, atom_tiles, virial_partials,
-                                           reverse ? reverse_grid : 0, s.energy,
+                                           reverse ? last_grid : 0, s.energy,
                                            reverse ? s.virial : nullptr);
     ND_LAUNCH_CHECK();
     ND_CUDA_TRY(cudaMemcpyAsync(s.status, counters, 4 * sizeof(int), cudaMemcpyDeviceToDevice, stream));

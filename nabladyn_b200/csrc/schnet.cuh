@@ -103,11 +103,36 @@ __device__ __forceinline__ float approx_reciprocal(float x)
     return y;
 }
 
+constexpr float kLog2E = 1.44269504088896340736f;
+
+// The hardware exponential and logarithm of base two, denormals flushed (one instruction each;
+// without the flush the compiler adds scaling on both sides).
+__device__ __forceinline__ float exp2_approx(float x)
+{
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+__device__ __forceinline__ float log2_approx(float x)
+{
+    float y;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // ln(1 + e^x) - ln 2 and its derivative, in FP32 with the hardware exp and log; the results
-// feed BF16 operands.
+// feed BF16 operands. e^-|x| underflows to zero where its logarithm term is below an ulp.
 __device__ __forceinline__ float softplus_shifted(float x)
 {
-    return fmaxf(x, 0.0f) + __logf(1.0f + __expf(-fabsf(x))) - kLn2;
+    const float log2 = log2_approx(1.0f + exp2_approx(-fabsf(x) * kLog2E));
+    return fmaxf(x, 0.0f) + log2 * kLn2 - kLn2;
+}
+
+// The Gaussian exp(-u^2 / 2); below the smallest normal number it is zero.
+__device__ __forceinline__ float gaussian(float u)
+{
+    return exp2_approx(-0.5f * u * u * kLog2E);
 }
 
 // 1 / (1 + e^-x) = (1 + tanh(x / 2)) / 2, with the hardware tanh (one special-function op).
@@ -203,18 +228,41 @@ struct Cores
                          std::uint32_t column2, const unsigned char* tile2,
                          const unsigned char* image2, int step)
     {
+        return issue(
+            [&] {
+                umma::product(*slot + column, umma::smem_address(tile), umma::smem_address(image));
+                if (tile2 != nullptr)
+                {
+                    umma::product(*slot + column2, umma::smem_address(tile2),
+                                  umma::smem_address(image2));
+                }
+            },
+            step);
+    }
+
+    // D[column offset] = tile * image, the image read the other way.
+    __device__ bool run_transposed(std::uint32_t column, const unsigned char* tile,
+                                   const unsigned char* image, int step)
+    {
+        return issue(
+            [&] {
+                umma::product_transposed(*slot + column, umma::smem_address(tile),
+                                         umma::smem_address(image));
+            },
+            step);
+    }
+
+    // Issues products from one thread, after every thread's operand writes, and waits for them.
+    template <typename Products>
+    __device__ __forceinline__ bool issue(Products products, int step)
+    {
         umma::fence_operands();
         umma::fence_before_sync();
         __syncthreads();
         if (threadIdx.x == 0)
         {
             umma::fence_after_sync();
-            umma::product(*slot + column, umma::smem_address(tile), umma::smem_address(image));
-            if (tile2 != nullptr)
-            {
-                umma::product(*slot + column2, umma::smem_address(tile2),
-                              umma::smem_address(image2));
-            }
+            products();
             umma::commit(barrier);
         }
         const bool done = umma::barrier_wait(barrier, phase);
@@ -244,24 +292,116 @@ struct Cores
     }
 };
 
-// Gaussians g_k(r) = exp(-(r / D - k)^2 / 2), k < K, zero above, into this thread's row.
-__device__ __forceinline__ void store_basis(unsigned char* tile, float r_over_width, int gaussians,
-                                            bool live)
+// Gaussians g_k(r) = exp(-(r / D - k)^2 / 2) into this thread's row: every k of a word of eight
+// that starts below K (the weight image is zero in columns K and up), zero above.
+__device__ __forceinline__ void store_basis(unsigned char* tile, float r_over_width, int gaussians)
 {
 #pragma unroll
     for (int c = 0; c < 8; ++c)
     {
-        float values[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e)
+        float values[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (8 * c < gaussians)
         {
-            const int k = 8 * c + e;
-            const float u = r_over_width - static_cast<float>(k);
-            values[e] = (live && k < gaussians) ? __expf(-0.5f * u * u) : 0.0f;
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+            {
+                values[e] = gaussian(r_over_width - static_cast<float>(8 * c + e));
+            }
         }
         umma::store8(tile, threadIdx.x, c, values);
     }
 }
+
+// Feature lanes. A tile's products leave one pair per thread, but the gathers and scatters of
+// feature rows (128 or 256 bytes each) want a row per few lanes: a thread per row touches 32
+// lines per instruction, and those accesses, not the arithmetic, bound the pair kernels (75 %
+// of the load/store unit's wavefronts). So the half's 32 columns of a pair's FP32 filter go
+// through shared memory (put_run_part: 16 KB, chunks swizzled by row), and eight lanes take a
+// row of it, four features each, four rows of the warp's 32 at a time: a gathered half row is
+// one 64-byte segment, a scattered one a whole 128-byte line. A lane meets rows 4 i + group,
+// i = 0 .. 7, in the list's order, so the first atom's side is summed in registers along its
+// run and added once per run and half.
+constexpr int kLaneRows = 8;  // rows a lane meets per half tile
+
+struct FeatureLane
+{
+    int group;   // 0 .. 3
+    int lane;    // 0 .. 7: features 4 lane .. 4 lane + 3 of the half
+    int warp_row;
+
+    __device__ FeatureLane()
+        : group((threadIdx.x & 31) >> 3), lane(threadIdx.x & 7), warp_row(threadIdx.x & ~31u)
+    {
+    }
+
+    __device__ int row(int i) const { return warp_row + 4 * i + group; }
+
+    // This lane's word of a BF16 feature row's half, and of an FP32 one's.
+    __device__ std::int64_t word(int atom, int half) const
+    {
+        return 16 * static_cast<std::int64_t>(atom) + 8 * half + lane;
+    }
+};
+
+// Four features of a staged half row.
+__device__ __forceinline__ float4 staged4(const float* stage, int row, int lane)
+{
+    return reinterpret_cast<const float4*>(stage)[row * 8 + (lane ^ (row & 7))];
+}
+
+__device__ __forceinline__ float4 widen4(const uint2& word)
+{
+    return make_float4(__uint_as_float(word.x << 16), __uint_as_float(word.x & 0xFFFF0000u),
+                       __uint_as_float(word.y << 16), __uint_as_float(word.y & 0xFFFF0000u));
+}
+
+__device__ __forceinline__ float4 operator*(const float4& a, const float4& b)
+{
+    return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w);
+}
+
+__device__ __forceinline__ float4 operator*(const float4& a, float b)
+{
+    return make_float4(a.x * b, a.y * b, a.z * b, a.w * b);
+}
+
+__device__ __forceinline__ float4 operator+(const float4& a, const float4& b)
+{
+    return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
+
+__device__ __forceinline__ float sum4(const float4& a) { return (a.x + a.y) + (a.z + a.w); }
+
+// The first atom of a lane's run of rows and the sums kept for it.
+template <int kSums>
+struct RunSums
+{
+    int atom = -1;
+    float4 sums[kSums];
+
+    // Adds the sums to their rows (word: this lane's of atom 0's half row).
+    __device__ void flush(float4* const (&targets)[kSums], std::int64_t word)
+    {
+        if (atom >= 0)
+        {
+#pragma unroll
+            for (int s = 0; s < kSums; ++s)
+            {
+                atomicAdd(targets[s] + 16 * static_cast<std::int64_t>(atom) + word, sums[s]);
+            }
+        }
+    }
+
+    __device__ void start(int next)
+    {
+        atom = next;
+#pragma unroll
+        for (int s = 0; s < kSums; ++s)
+        {
+            sums[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+};
 
 // Run sums of first-atom rows. Every pair's first-atom vector (32 columns, [32 half,
 // 32 half + 32) of a [N][64] target) is staged in shared memory (16 KB: float4 chunks

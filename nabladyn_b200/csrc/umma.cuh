@@ -59,12 +59,13 @@ constexpr std::uint32_t kInstruction = (1u << 4) | (1u << 7) | (1u << 10) |
 
 // D (+)= A B^T for one K = 16 step; issued by one thread.
 __device__ __forceinline__ void mma(std::uint32_t tmem, std::uint64_t a, std::uint64_t b,
-                                    std::uint32_t accumulate)
+                                    std::uint32_t accumulate,
+                                    std::uint32_t instruction = kInstruction)
 {
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
         " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-        "l"(a), "l"(b), "r"(kInstruction), "r"(accumulate));
+        "l"(a), "l"(b), "r"(instruction), "r"(accumulate));
 }
 
 // D = A B^T over K = 64: four instructions; `a` and `b` are shared-memory byte addresses.
@@ -75,6 +76,34 @@ __device__ __forceinline__ void product(std::uint32_t tmem, std::uint32_t a, std
     {
         mma(tmem, matrix_descriptor(a + 256 * step), matrix_descriptor(b + 256 * step),
             step > 0 ? 1u : 0u);
+    }
+}
+
+// D = A B over K = 64 with B a weight image read the other way (its row index is the reduction
+// index), so one image serves a layer and its reverse. The same core matrices read MN-major:
+// 8 rows of the reduction index by 16 bytes of columns; the stride-dimension offset is the step
+// between 8-column groups (128 bytes) and the leading-dimension offset the step between 8-row
+// groups (1024 bytes); K = 16 takes two row groups (2048 bytes). PTX ISA, tcgen05 canonical
+// layouts without swizzle; bit 16 of the instruction descriptor marks B as MN-major.
+__device__ __forceinline__ std::uint64_t transposed_descriptor(std::uint32_t address)
+{
+    std::uint64_t descriptor = (address >> 4) & 0x3FFFu;
+    descriptor |= static_cast<std::uint64_t>(1024 >> 4) << 16;
+    descriptor |= static_cast<std::uint64_t>(128 >> 4) << 32;
+    descriptor |= static_cast<std::uint64_t>(1) << 46;
+    return descriptor;
+}
+
+constexpr std::uint32_t kTransposedB = kInstruction | (1u << 16);
+
+__device__ __forceinline__ void product_transposed(std::uint32_t tmem, std::uint32_t a,
+                                                   std::uint32_t b)
+{
+#pragma unroll
+    for (int step = 0; step < 4; ++step)
+    {
+        mma(tmem, matrix_descriptor(a + 256 * step), transposed_descriptor(b + 2048 * step),
+            step > 0 ? 1u : 0u, kTransposedB);
     }
 }
 
