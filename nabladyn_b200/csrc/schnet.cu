@@ -375,27 +375,27 @@ __global__ void __launch_bounds__(kTile, 6) pair_forward_kernel(PairPass a)
             stage_half(cores.tmem + 32 * half, sh.bias2 + 32 * half, envelope, sh.stage);
             __syncwarp();
             RunSums<1> run;
-            float4* const targets[1] = {m4};
-            float4 va = make_float4(0.f, 0.f, 0.f, 0.f);
+            run.start(sh.first[at.row(0)]);
+            float4* const targets[1] = {m4 + at.word(0, half)};
+            float4 va = widen4(__ldg(v + at.word(max(run.key, 0), half)));
 #pragma unroll
             for (int i = 0; i < kLaneRows; ++i)
             {
                 const int row = at.row(i);
                 const int first = sh.first[row];
-                if (first != run.atom)
+                if (first != run.key)
                 {
-                    run.flush(targets, at.word(0, half));
-                    run.start(first);
-                    va = widen4(__ldg(v + at.word(first < 0 ? 0 : first, half)));
+                    run.turn(first, targets);
+                    va = widen4(__ldg(v + at.word(max(first, 0), half)));
                 }
+                const float4 f = staged4(sh.stage, row, at.lane);
                 if (first >= 0)
                 {
-                    const float4 f = staged4(sh.stage, row, at.lane);
                     atomicAdd(m4 + at.word(sh.second[row], half), f * va);
-                    run.sums[0] = run.sums[0] + f * widen4(vb[i]);
                 }
+                run.sums[0] = run.sums[0] + f * widen4(vb[i]);
             }
-            run.flush(targets, at.word(0, half));
+            run.finish(targets, at.group);
             __syncwarp();  // the stage's rows are this warp's own: its next writes come after
         }
     }
@@ -492,21 +492,26 @@ __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
             stage_half(cores.tmem + 64 + 32 * half, sh.bias2 + 32 * half, 1.0f, sh.stage);
             __syncwarp();
             RunSums<1> run;
-            float4* const targets[1] = {gv4};
-            float4 va = make_float4(0.f, 0.f, 0.f, 0.f), ma = va;
+            run.start(sh.first[at.row(0)]);
+            float4* const targets[1] = {gv4 + at.word(0, half)};
+            float4 va = widen4(__ldg(v + at.word(max(run.key, 0), half)));
+            float4 ma = widen4(__ldg(gm + at.word(max(run.key, 0), half)));
 #pragma unroll
             for (int i = 0; i < kLaneRows; ++i)
             {
                 const int row = at.row(i);
                 const int first = sh.first[row];
-                if (first != run.atom)
+                if (first != run.key)
                 {
-                    if (!kLast)
+                    if (kLast)
                     {
-                        run.flush(targets, at.word(0, half));
+                        run.key = first;
                     }
-                    run.start(first);
-                    const std::int64_t word = at.word(first < 0 ? 0 : first, half);
+                    else
+                    {
+                        run.turn(first, targets);
+                    }
+                    const std::int64_t word = at.word(max(first, 0), half);
                     va = widen4(__ldg(v + word));
                     ma = widen4(__ldg(gm + word));
                 }
@@ -515,10 +520,13 @@ __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
                 const float4 right = widen4(vb[i]), right_gm = widen4(mb[i]);
                 const float4 gf = ma * right + right_gm * va;
                 along[i] += sum4(gf * raw);
-                if (!kLast && first >= 0)
+                if (!kLast)
                 {
                     const float4 scaled = raw * envelope;
-                    atomicAdd(gv4 + at.word(sh.second[row], half), scaled * ma);
+                    if (first >= 0)
+                    {
+                        atomicAdd(gv4 + at.word(sh.second[row], half), scaled * ma);
+                    }
                     run.sums[0] = run.sums[0] + scaled * right_gm;
                 }
                 *reinterpret_cast<uint2*>(sh.work +
@@ -528,7 +536,7 @@ __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
             }
             if (!kLast)
             {
-                run.flush(targets, at.word(0, half));
+                run.finish(targets, at.group);
             }
             __syncwarp();  // the stage's rows are this warp's own: its next writes come after
         }

@@ -320,7 +320,7 @@ __device__ __forceinline__ void store_basis(unsigned char* tile, float r_over_wi
 // row of it, four features each, four rows of the warp's 32 at a time: a gathered half row is
 // one 64-byte segment, a scattered one a whole 128-byte line. A lane meets rows 4 i + group,
 // i = 0 .. 7, in the list's order, so the first atom's side is summed in registers along its
-// run and added once per run and half.
+// run and added once per run, warp and half.
 constexpr int kLaneRows = 8;  // rows a lane meets per half tile
 
 struct FeatureLane
@@ -372,33 +372,82 @@ __device__ __forceinline__ float4 operator+(const float4& a, const float4& b)
 
 __device__ __forceinline__ float sum4(const float4& a) { return (a.x + a.y) + (a.z + a.w); }
 
-// The first atom of a lane's run of rows and the sums kept for it.
+// First-atom sums of a warp's 32 rows. A group sums its rows along each run; its first and last
+// runs, which the other groups share, wait for the end, where the four groups meet: so a run
+// costs one atomic per warp and column, and two calls differ only in the order of the warps'
+// atomics (a run inside one group's rows, shorter than eight rows, is added by that group).
 template <int kSums>
 struct RunSums
 {
-    int atom = -1;
-    float4 sums[kSums];
+    int key;       // the present run's first atom (-1: dead rows)
+    int head_key;  // the first run's, once it ended; kOpen before
+    float4 sums[kSums], head[kSums];
+    static constexpr int kOpen = -2;
 
-    // Adds the sums to their rows (word: this lane's of atom 0's half row).
-    __device__ void flush(float4* const (&targets)[kSums], std::int64_t word)
+    __device__ __forceinline__ void start(int first)
     {
-        if (atom >= 0)
-        {
-#pragma unroll
-            for (int s = 0; s < kSums; ++s)
-            {
-                atomicAdd(targets[s] + 16 * static_cast<std::int64_t>(atom) + word, sums[s]);
-            }
-        }
-    }
-
-    __device__ void start(int next)
-    {
-        atom = next;
+        key = first;
+        head_key = kOpen;
 #pragma unroll
         for (int s = 0; s < kSums; ++s)
         {
+            sums[s] = head[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+
+    // Ends the present run when `first` starts another one. `targets` point to this lane's word
+    // of atom 0's half row.
+    __device__ __forceinline__ void turn(int first, float4* const (&targets)[kSums])
+    {
+        const bool opening = head_key == kOpen;
+#pragma unroll
+        for (int s = 0; s < kSums; ++s)
+        {
+            if (opening)
+            {
+                head[s] = sums[s];
+            }
+            else if (key >= 0)
+            {
+                atomicAdd(targets[s] + 16 * static_cast<std::int64_t>(key), sums[s]);
+            }
             sums[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        head_key = opening ? key : head_key;
+        key = first;
+    }
+
+    __device__ __forceinline__ void finish(float4* const (&targets)[kSums], int group)
+    {
+        while (true)
+        {
+            const unsigned open = __ballot_sync(kFullMask, head_key >= 0 || key >= 0);
+            if (open == 0)
+            {
+                break;
+            }
+            const int atom =
+                __shfl_sync(kFullMask, head_key >= 0 ? head_key : key, __ffs(open) - 1);
+#pragma unroll
+            for (int s = 0; s < kSums; ++s)
+            {
+                const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+                float4 total = (head_key == atom ? head[s] : zero) + (key == atom ? sums[s] : zero);
+#pragma unroll
+                for (int offset = 8; offset < 32; offset *= 2)
+                {
+                    total.x += __shfl_xor_sync(kFullMask, total.x, offset);
+                    total.y += __shfl_xor_sync(kFullMask, total.y, offset);
+                    total.z += __shfl_xor_sync(kFullMask, total.z, offset);
+                    total.w += __shfl_xor_sync(kFullMask, total.w, offset);
+                }
+                if (group == 0)
+                {
+                    atomicAdd(targets[s] + 16 * static_cast<std::int64_t>(atom), total);
+                }
+            }
+            head_key = head_key == atom ? kOpen : head_key;
+            key = key == atom ? -1 : key;
         }
     }
 };
