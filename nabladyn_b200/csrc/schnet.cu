@@ -232,9 +232,16 @@ struct PairPass
 // product completed), in the reverse pass the FP32 filter's stage (the forward pass stages it
 // in the row tile, free by then), biases, the pairs' atoms and envelopes, barrier and
 // tensor-memory slot.
+//
+// The reverse pass's row tile has its 16-byte chunks 144 bytes and its eight-row groups 1,216
+// bytes apart: the eight lanes that write one row, four rows at a time, then spread over the
+// shared-memory banks.
 constexpr int kPairTail = 2 * 256 + 4 * kTile * 4 + 64;
+constexpr int kReverseChunk = 144, kReverseGroup = 8 * kReverseChunk + 64;
+constexpr int kReverseTileBytes = kTile / 8 * kReverseGroup;
 constexpr int kPairForwardShared = 2 * umma::kImageBytes + umma::kTileBytes + kPairTail;
-constexpr int kPairReverseShared = 2 * umma::kImageBytes + 2 * umma::kTileBytes + kPairTail;
+constexpr int kPairReverseShared =
+    2 * umma::kImageBytes + kReverseTileBytes + umma::kTileBytes + kPairTail;
 
 struct PairShared
 {
@@ -251,14 +258,13 @@ struct PairShared
     std::uint64_t* barrier;
     std::uint32_t* slot;
 
-    __device__ PairShared(unsigned char* shared, bool own_stage)
+    __device__ PairShared(unsigned char* shared, bool reverse)
     {
         image_b1 = shared;
         image_b2 = image_b1 + umma::kImageBytes;
         work = image_b2 + umma::kImageBytes;
-        unsigned char* after = work + umma::kTileBytes;
-        stage = reinterpret_cast<float*>(own_stage ? after : work);
-        bias1 = reinterpret_cast<float*>(own_stage ? after + umma::kTileBytes : after);
+        stage = reinterpret_cast<float*>(reverse ? work + kReverseTileBytes : work);
+        bias1 = stage + kTile * 32;
         bias2 = bias1 + kFeatures;
         first = reinterpret_cast<int*>(bias2 + kFeatures);
         second = first + kTile;
@@ -281,6 +287,7 @@ struct PairShared
 };
 
 // ssp(z + b1) of this thread's row, from tensor-memory columns 0-63, into the row tile.
+template <int kChunk = 128, int kGroup = 1024>
 __device__ __forceinline__ void store_softplus(std::uint32_t tmem, const float* bias1,
                                                unsigned char* tile)
 {
@@ -299,26 +306,8 @@ __device__ __forceinline__ void store_softplus(std::uint32_t tmem, const float* 
             {
                 s[e] = softplus_shifted(z[8 * c + e] + bias1[32 * half + 8 * c + e]);
             }
-            umma::store8(tile, threadIdx.x, 4 * half + c, s);
+            umma::store8<kChunk, kGroup>(tile, threadIdx.x, 4 * half + c, s);
         }
-    }
-}
-
-// A half (32 columns) of this thread's FP32 row, (value + bias) * scale, into the stage.
-__device__ __forceinline__ void stage_half(std::uint32_t tmem, const float* bias, float scale,
-                                           float* stage)
-{
-    float f[32];
-    umma::load32(tmem, f);
-    umma::wait_loads();
-#pragma unroll
-    for (int q = 0; q < 8; ++q)
-    {
-        put_run_part(stage, q,
-                     make_float4((f[4 * q] + bias[4 * q]) * scale,
-                                 (f[4 * q + 1] + bias[4 * q + 1]) * scale,
-                                 (f[4 * q + 2] + bias[4 * q + 2]) * scale,
-                                 (f[4 * q + 3] + bias[4 * q + 3]) * scale));
     }
 }
 
@@ -441,6 +430,25 @@ __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
     const auto* gm = reinterpret_cast<const uint2*>(a.grad_m);
     float4* const gv4 = reinterpret_cast<float4*>(a.grad_v);
     const FeatureLane at;
+    // D[64 + n] = the row tile times an image, read either way.
+    auto product = [&](std::uint32_t column, const unsigned char* image, bool transposed, int step) {
+        return cores.issue(
+            [&] {
+                const std::uint32_t tile = umma::smem_address(sh.work);
+                const std::uint32_t b = umma::smem_address(image);
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                {
+                    umma::mma(*sh.slot + column,
+                              umma::matrix_descriptor(tile + 2 * kReverseChunk * k, kReverseChunk,
+                                                      kReverseGroup),
+                              transposed ? umma::matrix_descriptor(b + 2048 * k, 1024, 128)
+                                         : umma::matrix_descriptor(b + 256 * k),
+                              k > 0 ? 1u : 0u, transposed ? umma::kTransposedB : umma::kInstruction);
+                }
+            },
+            step);
+    };
     double w[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // xx yy zz xy xz yz
 
     // Each tile's pair records are loaded one tile ahead (see pair_forward_kernel).
@@ -465,14 +473,14 @@ __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
         sh.second[threadIdx.x] = ab.y;
         sh.envelope[threadIdx.x] = 0.5f * (cosine + 1.0f);
         cores.tile_index = tile;
-        store_basis(sh.work, t, a.gaussians);
-        if (!cores.run(0, sh.work, sh.image_b1, 1))
+        store_basis<kReverseChunk, kReverseGroup>(sh.work, t, a.gaussians);
+        if (!product(0, sh.image_b1, false, 1))
         {
             break;
         }
         // ssp(z1) into the work tile; z1 - b1 stays in columns 0-63.
-        store_softplus(cores.tmem, sh.bias1, sh.work);
-        if (!cores.run(64, sh.work, sh.image_b2, 2))
+        store_softplus<kReverseChunk, kReverseGroup>(cores.tmem, sh.bias1, sh.work);
+        if (!product(64, sh.image_b2, false, 2))
         {
             break;
         }
@@ -529,8 +537,9 @@ __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
                     }
                     run.sums[0] = run.sums[0] + scaled * right_gm;
                 }
-                *reinterpret_cast<uint2*>(sh.work +
-                                          umma::image_offset(row, 32 * half + 4 * at.lane)) =
+                *reinterpret_cast<uint2*>(sh.work + (row >> 3) * kReverseGroup +
+                                          (4 * half + at.lane / 2) * kReverseChunk +
+                                          (row & 7) * 16 + (at.lane & 1) * 8) =
                     make_uint2(pack2(gf.x * envelope, gf.y * envelope),
                                pack2(gf.z * envelope, gf.w * envelope));
             }
@@ -541,7 +550,7 @@ __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
             __syncwarp();  // the stage's rows are this warp's own: its next writes come after
         }
         sh.along[at.row(at.lane)] = sum_across(along, at.lane);
-        if (!cores.run_transposed(64, sh.work, sh.image_b2, 3))
+        if (!product(64, sh.image_b2, true, 3))
         {
             break;
         }
@@ -563,10 +572,10 @@ __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
                 {
                     s[e] = q[8 * c + e] * sigmoid(z[8 * c + e] + sh.bias1[32 * half + 8 * c + e]);
                 }
-                umma::store8(sh.work, threadIdx.x, 4 * half + c, s);
+                umma::store8<kReverseChunk, kReverseGroup>(sh.work, threadIdx.x, 4 * half + c, s);
             }
         }
-        if (!cores.run_transposed(64, sh.work, sh.image_b1, 4))
+        if (!product(64, sh.image_b1, true, 4))
         {
             break;
         }

@@ -1,7 +1,7 @@
 // Pieces shared by the SchNet kernels (schnet.cu: E, F and W; schnet_tangent.cu: the
 // parameter gradient of a force and virial loss): sizes, the packed parameter block and the
 // workspace layouts, the activations, BF16 feature rows, the per-CTA tensor-core context,
-// the Gaussian basis and the run sums of first-atom rows.
+// the Gaussian basis, and the feature lanes that gather and scatter rows.
 
 #pragma once
 
@@ -169,10 +169,10 @@ __device__ __forceinline__ std::uint32_t pack2(float lo, float hi)
     return *reinterpret_cast<std::uint32_t*>(&pair);
 }
 
-// Shared-memory staging of weight images and bias vectors, by all 128 threads.
+// Shared-memory staging of weight images and bias vectors, by all threads.
 __device__ __forceinline__ void copy_bytes(unsigned char* to, const unsigned char* from, int bytes)
 {
-    for (int i = threadIdx.x * 16; i < bytes; i += kTile * 16)
+    for (int i = threadIdx.x * 16; i < bytes; i += blockDim.x * 16)
     {
         *reinterpret_cast<uint4*>(to + i) = __ldg(reinterpret_cast<const uint4*>(from + i));
     }
@@ -206,7 +206,7 @@ struct Cores
         umma::fence_before_sync();
         __syncthreads();
         umma::fence_after_sync();
-        tmem = *slot + ((32u * (threadIdx.x / 32)) << 16);
+        tmem = *slot + ((32u * (threadIdx.x / 32 % 4)) << 16);
     }
 
     int* counters;  // [4]: pairs, status bits, first stage that gave up, its tile
@@ -240,21 +240,16 @@ struct Cores
             step);
     }
 
-    // D[column offset] = tile * image, the image read the other way.
-    __device__ bool run_transposed(std::uint32_t column, const unsigned char* tile,
-                                   const unsigned char* image, int step)
-    {
-        return issue(
-            [&] {
-                umma::product_transposed(*slot + column, umma::smem_address(tile),
-                                         umma::smem_address(image));
-            },
-            step);
-    }
-
     // Issues products from one thread, after every thread's operand writes, and waits for them.
     template <typename Products>
     __device__ __forceinline__ bool issue(Products products, int step)
+    {
+        begin(products);
+        return finish(step);
+    }
+
+    template <typename Products>
+    __device__ __forceinline__ void begin(Products products)
     {
         umma::fence_operands();
         umma::fence_before_sync();
@@ -265,6 +260,11 @@ struct Cores
             products();
             umma::commit(barrier);
         }
+    }
+
+    // Waits for the products begun last.
+    __device__ __forceinline__ bool finish(int step)
+    {
         const bool done = umma::barrier_wait(barrier, phase);
         phase ^= 1u;
         const bool lost = __syncthreads_or(!done);
@@ -294,6 +294,7 @@ struct Cores
 
 // Gaussians g_k(r) = exp(-(r / D - k)^2 / 2) into this thread's row: every k of a word of eight
 // that starts below K (the weight image is zero in columns K and up), zero above.
+template <int kChunk = 128, int kGroup = 1024>
 __device__ __forceinline__ void store_basis(unsigned char* tile, float r_over_width, int gaussians)
 {
 #pragma unroll
@@ -308,7 +309,7 @@ __device__ __forceinline__ void store_basis(unsigned char* tile, float r_over_wi
                 values[e] = gaussian(r_over_width - static_cast<float>(8 * c + e));
             }
         }
-        umma::store8(tile, threadIdx.x, c, values);
+        umma::store8<kChunk, kGroup>(tile, threadIdx.x, c, values);
     }
 }
 
@@ -316,9 +317,9 @@ __device__ __forceinline__ void store_basis(unsigned char* tile, float r_over_wi
 // feature rows (128 or 256 bytes each) want a row per few lanes: a thread per row touches 32
 // lines per instruction, and those accesses, not the arithmetic, bound the pair kernels (75 %
 // of the load/store unit's wavefronts). So the half's 32 columns of a pair's FP32 filter go
-// through shared memory (put_run_part: 16 KB, chunks swizzled by row), and eight lanes take a
+// through shared memory (stage4: 16 KB, chunks swizzled by row), and eight lanes take a
 // row of it, four features each, four rows of the warp's 32 at a time: a gathered half row is
-// one 64-byte segment, a scattered one a whole 128-byte line. A lane meets rows 4 i + group,
+// one 64-byte segment, a scattered one a whole 128-byte line. A lane meets rows 8 group + i,
 // i = 0 .. 7, in the list's order, so the first atom's side is summed in registers along its
 // run and added once per run, warp and half.
 constexpr int kLaneRows = 8;  // rows a lane meets per half tile
@@ -334,7 +335,7 @@ struct FeatureLane
     {
     }
 
-    __device__ int row(int i) const { return warp_row + 4 * i + group; }
+    __device__ int row(int i) const { return warp_row + kLaneRows * group + i; }
 
     // This lane's word of a BF16 feature row's half, and of an FP32 one's.
     __device__ std::int64_t word(int atom, int half) const
@@ -372,11 +373,11 @@ __device__ __forceinline__ float4 operator+(const float4& a, const float4& b)
 
 __device__ __forceinline__ float sum4(const float4& a) { return (a.x + a.y) + (a.z + a.w); }
 
-// First-atom sums of a warp's 32 rows. A group sums its rows along each run; its first and last
-// runs, which the other groups share, wait for the end, where the four groups meet: so a run
-// costs one atomic per warp and column, and two calls differ only in the order of the warps'
-// atomics (a run inside one group's rows, shorter than eight rows, is added by that group).
-template <int kSums>
+// First-atom sums of a warp's rows. A group sums its rows along each run and adds the runs that
+// begin and end inside them; its first and last runs, which its neighbours may share, wait for
+// the end, where the groups meet: so a run costs one atomic per warp and column, and two calls
+// differ only in the order of the warps' atomics.
+template <int kSums, int kGroups = 4>
 struct RunSums
 {
     int key;       // the present run's first atom (-1: dead rows)
@@ -396,7 +397,7 @@ struct RunSums
     }
 
     // Ends the present run when `first` starts another one. `targets` point to this lane's word
-    // of atom 0's half row.
+    // of atom 0's row.
     __device__ __forceinline__ void turn(int first, float4* const (&targets)[kSums])
     {
         const bool opening = head_key == kOpen;
@@ -434,7 +435,7 @@ struct RunSums
                 const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
                 float4 total = (head_key == atom ? head[s] : zero) + (key == atom ? sums[s] : zero);
 #pragma unroll
-                for (int offset = 8; offset < 32; offset *= 2)
+                for (int offset = 32 / kGroups; offset < 32; offset *= 2)
                 {
                     total.x += __shfl_xor_sync(kFullMask, total.x, offset);
                     total.y += __shfl_xor_sync(kFullMask, total.y, offset);
@@ -452,57 +453,34 @@ struct RunSums
     }
 };
 
-// Run sums of first-atom rows. Every pair's first-atom vector (32 columns, [32 half,
-// 32 half + 32) of a [N][64] target) is staged in shared memory (16 KB: float4 chunks
-// swizzled by row against bank conflicts; thread t stages row t); the tile's pairs keep the
-// list's order, so a first atom's pairs are runs of rows: each warp sums its 32 rows column
-// by column and adds one atomic per run and column instead of one per pair. Dead rows carry
-// first = -1.
-
-// Stages chunk q (columns 4q .. 4q + 3 of the half) of this thread's row.
-__device__ __forceinline__ void put_run_part(float* stage, int q, float4 value)
+// Stages float4 `q` (columns 4 q .. 4 q + 3 of the half) of this thread's row.
+__device__ __forceinline__ void stage4(float* stage, int q, float4 value)
 {
     reinterpret_cast<float4*>(stage)[threadIdx.x * 8 + (q ^ (threadIdx.x & 7))] = value;
 }
 
-// Sums the staged rows over runs into `target`. Each warp sums the 32 rows its own threads
-// staged, so a warp barrier orders the staging; `block_barrier` ends with a block barrier,
-// for callers whose next writes to the stage's bytes come from other warps.
-__device__ __forceinline__ void sum_runs(const float* stage, const int* first, float* target,
-                                         int half, bool block_barrier)
+// A half (32 columns) of this thread's FP32 row, (value + bias) * scale, into the stage.
+__device__ __forceinline__ void stage_half(std::uint32_t tmem, const float* bias, float scale,
+                                           float* stage)
 {
-    __syncwarp();
-    const int column = threadIdx.x & 31;
-    const int begin = (threadIdx.x >> 5) * 32;
-    float sum = 0.0f;
-    for (int r = begin; r < begin + 32; ++r)
+    float f[32];
+    umma::load32(tmem, f);
+    umma::wait_loads();
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
     {
-        sum += stage[(r * 8 + ((column >> 2) ^ (r & 7))) * 4 + (column & 3)];
-        const int atom = first[r];
-        if (r == begin + 31 || first[r + 1] != atom)
-        {
-            if (atom >= 0)
-            {
-                atomicAdd(target + static_cast<std::int64_t>(atom) * kFeatures + 32 * half + column,
-                          sum);
-            }
-            sum = 0.0f;
-        }
-    }
-    if (block_barrier)
-    {
-        __syncthreads();
-    }
-    else
-    {
-        __syncwarp();
+        stage4(stage, q,
+               make_float4((f[4 * q] + bias[4 * q]) * scale,
+                           (f[4 * q + 1] + bias[4 * q + 1]) * scale,
+                           (f[4 * q + 2] + bias[4 * q + 2]) * scale,
+                           (f[4 * q + 3] + bias[4 * q + 3]) * scale));
     }
 }
 
 // Resident CTAs per SM times the SM count, for a persistent grid: the least of the register
 // file, shared memory (227 KB a CTA can use, 1 KB reserved per CTA) and tensor memory (512
 // columns) over one CTA's needs.
-int pair_grid(const void* kernel, int shared_bytes, int tmem_columns)
+int pair_grid(const void* kernel, int shared_bytes, int tmem_columns, int threads = kTile)
 {
     int sms = 148;
     multiprocessors(&sms);
@@ -510,7 +488,7 @@ int pair_grid(const void* kernel, int shared_bytes, int tmem_columns)
     cudaFuncAttributes attributes{};
     if (cudaFuncGetAttributes(&attributes, kernel) == cudaSuccess)
     {
-        const int registers = ((attributes.numRegs * 32 + 255) / 256) * 256 * (kTile / 32);
+        const int registers = ((attributes.numRegs * 32 + 255) / 256) * 256 * (threads / 32);
         const int by_registers = 65536 / std::max(1, registers);
         const int by_shared =
             (228 * 1024) / (shared_bytes + static_cast<int>(attributes.sharedSizeBytes) + 1024);

@@ -120,114 +120,80 @@ __device__ __forceinline__ PairTerms pair_terms(const TangentPass& a, const floa
     return t;
 }
 
-// Row p of per-pair array `kind`, or null for a dead row.
-__device__ __forceinline__ uint4* pair_row(const TangentPass& a, int kind, int p, bool live)
-{
-    return live ? a.rows + (static_cast<std::int64_t>(kind) * a.capacity + p) * 8 : nullptr;
-}
-
 // g_k = exp(-(t - k)^2 / 2) (zero for k >= K) and g_dot_k = g_k (t - k) scale, scale = -rdot / D,
-// into this thread's row of two tiles, and into HBM rows when given (there with g_63 = 1 when
-// K < 64).
+// into this thread's row of two tiles.
 __device__ __forceinline__ void store_basis_tangent(unsigned char* tile, unsigned char* tile_dot,
-                                                    float t, float scale, int gaussians, bool live,
-                                                    uint4* row, uint4* row_dot)
+                                                    float t, float scale, int gaussians)
 {
 #pragma unroll
     for (int c = 0; c < 8; ++c)
     {
-        float g[8];
-        float gd[8];
+        float g[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        float gd[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (8 * c < gaussians)  // the weight image is zero in columns K and up
+        {
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
-        {
-            const int k = 8 * c + e;
-            const float u = t - static_cast<float>(k);
-            g[e] = (live && k < gaussians) ? __expf(-0.5f * u * u) : 0.0f;
-            gd[e] = g[e] * u * scale;
-        }
-        const uint4 word = umma::pack8(g);
-        const uint4 word_dot = umma::pack8(gd);
-        *reinterpret_cast<uint4*>(tile + umma::image_offset(threadIdx.x, 8 * c)) = word;
-        *reinterpret_cast<uint4*>(tile_dot + umma::image_offset(threadIdx.x, 8 * c)) = word_dot;
-        if (row != nullptr)
-        {
-            // With K < 64 the HBM row's column 63 (a zero the products never use) holds 1, so
-            // the sum over pairs of z_bar^T g carries the bias gradient sum(z_bar) there.
-            if (c == 7 && gaussians < 64)
+            for (int e = 0; e < 8; ++e)
             {
-                g[7] = 1.0f;
-                row[c] = umma::pack8(g);
+                const float u = t - static_cast<float>(8 * c + e);
+                g[e] = gaussian(u);
+                gd[e] = g[e] * u * scale;
             }
-            else
-            {
-                row[c] = word;
-            }
-            row_dot[c] = word_dot;
         }
+        umma::store8(tile, threadIdx.x, c, g);
+        umma::store8(tile_dot, threadIdx.x, c, gd);
     }
 }
 
 // s = ssp(z + b1) and s_dot = sigmoid(z + b1) z_dot from tensor-memory columns 0-63 (z - b1) and
-// 64-127 (z_dot) into this thread's row of two tiles, and into HBM rows when given.
+// 64-127 (z_dot) into this thread's row of two tiles.
 __device__ __forceinline__ void store_activations(std::uint32_t tmem, const float* bias1,
-                                                  unsigned char* tile, unsigned char* tile_dot,
-                                                  uint4* row, uint4* row_dot)
+                                                  unsigned char* tile, unsigned char* tile_dot)
 {
-#pragma unroll
-    for (int half = 0; half < 2; ++half)
+#pragma unroll 1  // the unrolled kernel overflows the instruction cache
+    for (int part = 0; part < 4; ++part)
     {
-        float z[32];
-        float zd[32];
-        umma::load32(tmem + 32 * half, z);
-        umma::load32(tmem + 64 + 32 * half, zd);
+        float z[16], zd[16];
+        umma::load16(tmem + 16 * part, z);
+        umma::load16(tmem + 64 + 16 * part, zd);
         umma::wait_loads();
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+        for (int c = 0; c < 2; ++c)
         {
             float s[8];
             float sd[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e)
             {
-                const float x = z[8 * c + e] + bias1[32 * half + 8 * c + e];
+                const float x = z[8 * c + e] + bias1[16 * part + 8 * c + e];
                 s[e] = softplus_shifted(x);
                 sd[e] = sigmoid(x) * zd[8 * c + e];
             }
-            const int column = 4 * half + c;
-            const uint4 word = umma::pack8(s);
-            const uint4 word_dot = umma::pack8(sd);
-            *reinterpret_cast<uint4*>(tile + umma::image_offset(threadIdx.x, 8 * column)) = word;
-            *reinterpret_cast<uint4*>(tile_dot + umma::image_offset(threadIdx.x, 8 * column)) =
-                word_dot;
-            if (row != nullptr)
-            {
-                row[column] = word;
-                row_dot[column] = word_dot;
-            }
+            umma::store8(tile, threadIdx.x, 2 * part + c, s);
+            umma::store8(tile_dot, threadIdx.x, 2 * part + c, sd);
         }
     }
 }
 
-// Shared memory: weight images, two row tiles, (reverse) two 16 KB run stages, biases,
-// barrier and tensor-memory slot.
-constexpr int kTangentForwardShared = 2 * umma::kImageBytes + 2 * umma::kTileBytes + 2 * 256 + 64;
-constexpr int kTangentReverseShared = 3 * umma::kImageBytes + 4 * umma::kTileBytes + 2 * 256 + 64;
+constexpr int kTangentForwardShared =
+    2 * umma::kImageBytes + 2 * umma::kTileBytes + 2 * 256 + 2 * kTile * 4 + 64;
 
-__global__ void __launch_bounds__(kTile, 3) tangent_forward_kernel(TangentPass a)
+__global__ void __launch_bounds__(kTile, 4) tangent_forward_kernel(TangentPass a)
 {
     extern __shared__ __align__(1024) unsigned char shared[];
     unsigned char* image_b1 = shared;
     unsigned char* image_b2 = image_b1 + umma::kImageBytes;
     unsigned char* tile = image_b2 + umma::kImageBytes;
     unsigned char* tile_dot = tile + umma::kTileBytes;
-    // first-atom runs of m_dot, in a row tile once the products are done
-    float* stage_dot = reinterpret_cast<float*>(tile);
+    // f and f_dot, a half at a time, in the row tiles once the products are done
+    float* stage = reinterpret_cast<float*>(tile);
+    float* stage_dot = reinterpret_cast<float*>(tile_dot);
     float* bias1 = reinterpret_cast<float*>(tile_dot + umma::kTileBytes);
     float* bias2 = bias1 + kFeatures;
-    auto* barrier = reinterpret_cast<std::uint64_t*>(bias2 + kFeatures);
+    int* first = reinterpret_cast<int*>(bias2 + kFeatures);
+    int* second = first + kTile;
+    auto* barrier = reinterpret_cast<std::uint64_t*>(second + kTile);
     auto* slot = reinterpret_cast<std::uint32_t*>(barrier + 1);
-    __shared__ int tile_first[kTile];
     __shared__ float wbar[9];
 
     copy_bytes(image_b1, a.images + kB1 * umma::kImageBytes, umma::kImageBytes);
@@ -245,118 +211,134 @@ __global__ void __launch_bounds__(kTile, 3) tangent_forward_kernel(TangentPass a
     Cores cores;
     cores.open(barrier, slot, 128, a.counters, 5);
     const int count = *reinterpret_cast<volatile int*>(a.counters);
-    float4* md4 = reinterpret_cast<float4*>(a.m_dot);
+    const auto* v = reinterpret_cast<const uint2*>(a.v);
+    const auto* v_dot = reinterpret_cast<const uint2*>(a.v_dot);
+    float4* const md4 = reinterpret_cast<float4*>(a.m_dot);
+    const FeatureLane at;
 
     for (int index = blockIdx.x; index * kTile < count; index += gridDim.x)
     {
         const int p = index * kTile + threadIdx.x;
         const PairTerms t = pair_terms(a, wbar, p, count);
-        tile_first[threadIdx.x] = t.live ? t.ab.x : -1;
+        first[threadIdx.x] = t.live ? t.ab.x : -1;
+        second[threadIdx.x] = t.ab.y;
         cores.tile_index = index;
-        store_basis_tangent(tile, tile_dot, t.g.w / a.width, -t.rate / a.width, a.gaussians,
-                            t.live, nullptr, nullptr);
+        store_basis_tangent(tile, tile_dot, t.g.w / a.width, -t.rate / a.width, a.gaussians);
         if (!cores.run2(0, tile, image_b1, 64, tile_dot, image_b1, 1))
         {
             break;
         }
-        store_activations(cores.tmem, bias1, tile, tile_dot, nullptr, nullptr);
+        store_activations(cores.tmem, bias1, tile, tile_dot);
         if (!cores.run2(0, tile, image_b2, 64, tile_dot, image_b2, 2))
         {
             break;
         }
-#pragma unroll
+        // m_dot_a += f_dot v_b + f v_dot_b along the runs, m_dot_b += f_dot v_a + f v_dot_a.
+#pragma unroll 1
         for (int half = 0; half < 2; ++half)
         {
+            uint2 vb[kLaneRows], vdb[kLaneRows];
 #pragma unroll
-            for (int batch = 0; batch < 4; batch += kGatherBatch)
+            for (int i = 0; i < kLaneRows; ++i)
             {
-                // The batch's gathers first; dead rows read atom 0 and contribute zeros.
-                uint4 raw[kGatherBatch][4];
+                const std::int64_t word = at.word(second[at.row(i)], half);
+                vb[i] = __ldg(v + word);
+                vdb[i] = __ldg(v_dot + word);
+            }
+            {
+                float u[32], ud[32];
+                umma::load32(cores.tmem + 32 * half, u);
+                umma::load32(cores.tmem + 64 + 32 * half, ud);
+                umma::wait_loads();
+                const float* bias = bias2 + 32 * half;
 #pragma unroll
-                for (int i = 0; i < kGatherBatch; ++i)
+                for (int q = 0; q < 8; ++q)
                 {
-                    const int k = 32 * half + 8 * (batch + i);
-                    const std::int64_t ga = 8 * static_cast<std::int64_t>(t.ab.x) + k / 8;
-                    const std::int64_t gb = 8 * static_cast<std::int64_t>(t.ab.y) + k / 8;
-                    raw[i][0] = __ldg(a.v + ga);
-                    raw[i][1] = __ldg(a.v + gb);
-                    raw[i][2] = __ldg(a.v_dot + ga);
-                    raw[i][3] = __ldg(a.v_dot + gb);
-                }
+                    float f[4], fd[4];
 #pragma unroll
-                for (int i = 0; i < kGatherBatch; ++i)
-                {
-                    const int c = batch + i;
-                    const int k = 32 * half + 8 * c;
-                    float u[8];
-                    float ud[8];
-                    umma::load8(cores.tmem + k, u);
-                    umma::load8(cores.tmem + 64 + k, ud);
-                    umma::wait_loads();
-                    float va[8], vb[8], vda[8], vdb[8], f[8], fd[8];
-                    widen8(raw[i][0], va);
-                    widen8(raw[i][1], vb);
-                    widen8(raw[i][2], vda);
-                    widen8(raw[i][3], vdb);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
+                    for (int e = 0; e < 4; ++e)
                     {
-                        const float raw_filter = u[j] + bias2[k + j];
-                        f[j] = raw_filter * t.envelope;
-                        fd[j] = ud[j] * t.envelope + raw_filter * t.moving;
+                        const float raw_filter = u[4 * q + e] + bias[4 * q + e];
+                        f[e] = raw_filter * t.envelope;
+                        fd[e] = ud[4 * q + e] * t.envelope + raw_filter * t.moving;
                     }
-                    if (t.live)
-                    {
-                        const std::int64_t gb = 8 * static_cast<std::int64_t>(t.ab.y) + k / 8;
-#pragma unroll
-                        for (int h4 = 0; h4 < 2; ++h4)
-                        {
-                            const int o = 4 * h4;
-                            atomicAdd(md4 + 2 * gb + h4,
-                                      make_float4(fd[o] * va[o] + f[o] * vda[o],
-                                                  fd[o + 1] * va[o + 1] + f[o + 1] * vda[o + 1],
-                                                  fd[o + 2] * va[o + 2] + f[o + 2] * vda[o + 2],
-                                                  fd[o + 3] * va[o + 3] + f[o + 3] * vda[o + 3]));
-                        }
-                    }
-#pragma unroll
-                    for (int h4 = 0; h4 < 2; ++h4)
-                    {
-                        const int o = 4 * h4;
-                        put_run_part(stage_dot, 2 * c + h4,
-                                     make_float4(fd[o] * vb[o] + f[o] * vdb[o],
-                                                 fd[o + 1] * vb[o + 1] + f[o + 1] * vdb[o + 1],
-                                                 fd[o + 2] * vb[o + 2] + f[o + 2] * vdb[o + 2],
-                                                 fd[o + 3] * vb[o + 3] + f[o + 3] * vdb[o + 3]));
-                    }
+                    stage4(stage, q, make_float4(f[0], f[1], f[2], f[3]));
+                    stage4(stage_dot, q, make_float4(fd[0], fd[1], fd[2], fd[3]));
                 }
             }
-            sum_runs(stage_dot, tile_first, a.m_dot, half, half == 1);  // the next basis overwrites it
+            __syncwarp();
+            RunSums<1> run;
+            run.start(first[at.row(0)]);
+            float4* const targets[1] = {md4 + at.word(0, half)};
+            float4 va = widen4(__ldg(v + at.word(max(run.key, 0), half)));
+            float4 vda = widen4(__ldg(v_dot + at.word(max(run.key, 0), half)));
+#pragma unroll
+            for (int i = 0; i < kLaneRows; ++i)
+            {
+                const int row = at.row(i);
+                const int atom = first[row];
+                if (atom != run.key)
+                {
+                    run.turn(atom, targets);
+                    va = widen4(__ldg(v + at.word(max(atom, 0), half)));
+                    vda = widen4(__ldg(v_dot + at.word(max(atom, 0), half)));
+                }
+                const float4 f = staged4(stage, row, at.lane), fd = staged4(stage_dot, row, at.lane);
+                if (atom >= 0)
+                {
+                    atomicAdd(md4 + at.word(second[row], half), fd * va + f * vda);
+                }
+                run.sums[0] = run.sums[0] + (fd * widen4(vb[i]) + f * widen4(vdb[i]));
+            }
+            run.finish(targets, at.group);
+            __syncwarp();  // the stages' rows are this warp's own: its next writes come after
         }
     }
     cores.close(128);
 }
 
-__global__ void __launch_bounds__(kTile, 2) tangent_reverse_kernel(TangentPass a)
+// The reverse pass. A tile's steps form one long chain (four products with row-wise work between
+// them), so two CTAs share an SM (tensor memory holds no more: z, z_dot, u and u_dot are 256
+// columns) and each gives a tile 256 threads: thread t computes columns 32 (t / 128) .. + 31 of
+// row t % 128 in the row-wise steps. In the scatter, eight lanes take a row's 32 staged columns
+// (columns 16 step .. + 15 of both halves, step 0 and 1), four rows of the warp's 16 at a time.
+// The eight BF16 rows of a pair leave from the operand tiles in whole lines while the tensor
+// cores read them; with chunks 144 bytes and eight-row groups 1,184 bytes apart both that and
+// the lanes' writes of four rows spread over the shared-memory banks.
+constexpr int kReverseThreads = 256;
+constexpr int kRowChunk = 144, kRowGroup = 8 * kRowChunk + 32;  // of the row tiles
+constexpr int kRowTileBytes = kTile / 8 * kRowGroup;
+constexpr int kTangentReverseShared = 2 * umma::kImageBytes + 2 * kRowTileBytes +
+                                      2 * kTile * 32 * 4 + 2 * 256 + 6 * kTile * 4 + 128;
+
+__device__ __forceinline__ unsigned char* row_word(unsigned char* tile, int row, int c)
+{
+    return tile + (row >> 3) * kRowGroup + c * kRowChunk + (row & 7) * 16;
+}
+
+__global__ void __launch_bounds__(kReverseThreads, 2) tangent_reverse_kernel(TangentPass a)
 {
     extern __shared__ __align__(1024) unsigned char shared[];
     unsigned char* image_b1 = shared;
     unsigned char* image_b2 = image_b1 + umma::kImageBytes;
-    unsigned char* image_b2t = image_b2 + umma::kImageBytes;
-    unsigned char* tile = image_b2t + umma::kImageBytes;
-    unsigned char* tile_dot = tile + umma::kTileBytes;
-    float* stage = reinterpret_cast<float*>(tile_dot + umma::kTileBytes);  // v_bar runs, 16 KB
-    float* stage_dot = stage + kTile * 32;                                  // v_dot_bar runs
+    unsigned char* tile = image_b2 + umma::kImageBytes;
+    unsigned char* tile_dot = tile + kRowTileBytes;
+    float* stage = reinterpret_cast<float*>(tile_dot + kRowTileBytes);  // f
+    float* stage_dot = stage + kTile * 32;                              // f_dot
     float* bias1 = stage_dot + kTile * 32;
     float* bias2 = bias1 + kFeatures;
-    auto* barrier = reinterpret_cast<std::uint64_t*>(bias2 + kFeatures);
+    int* first = reinterpret_cast<int*>(bias2 + kFeatures);
+    int* second = first + kTile;
+    float* envelopes = reinterpret_cast<float*>(second + kTile);
+    float* movings = envelopes + kTile;
+    float* offsets = movings + kTile;  // r / D
+    float* scales = offsets + kTile;   // -rdot / D
+    float* wbar = scales + kTile;
+    auto* barrier = reinterpret_cast<std::uint64_t*>(wbar + 10);
     auto* slot = reinterpret_cast<std::uint32_t*>(barrier + 1);
-    __shared__ int tile_first[kTile];
-    __shared__ float wbar[9];
 
     copy_bytes(image_b1, a.images + kB1 * umma::kImageBytes, umma::kImageBytes);
     copy_bytes(image_b2, a.images + kB2 * umma::kImageBytes, umma::kImageBytes);
-    copy_bytes(image_b2t, a.images + kB2T * umma::kImageBytes, umma::kImageBytes);
     if (threadIdx.x < kFeatures)
     {
         bias1[threadIdx.x] = a.b1[threadIdx.x];
@@ -370,169 +352,251 @@ __global__ void __launch_bounds__(kTile, 2) tangent_reverse_kernel(TangentPass a
     // 192-255 u_dot, then s_dot_bar.
     Cores cores;
     cores.open(barrier, slot, 256, a.counters, 6);
+    const std::uint32_t tmem = *slot;
     const int count = *reinterpret_cast<volatile int*>(a.counters);
-    float4* vbar4 = reinterpret_cast<float4*>(a.v_bar);
-    float4* vdbar4 = reinterpret_cast<float4*>(a.v_dot_bar);
+    const auto* v = reinterpret_cast<const uint2*>(a.v);
+    const auto* v_dot = reinterpret_cast<const uint2*>(a.v_dot);
+    const auto* m_bar = reinterpret_cast<const uint2*>(a.m_bar);
+    const auto* m_dot_bar = reinterpret_cast<const uint2*>(a.m_dot_bar);
+    float4* const vbar4 = reinterpret_cast<float4*>(a.v_bar);
+    float4* const vdbar4 = reinterpret_cast<float4*>(a.v_dot_bar);
+    const int row = threadIdx.x % kTile, side = threadIdx.x / kTile;
+    // The scatter's rows: 16 of the 32 that this warp and the one of the other side staged.
+    const int lane = threadIdx.x % 8, group = threadIdx.x % 32 / 8;
+    const int lane_row = 32 * (threadIdx.x / 32 % 4) + 16 * side + 4 * group;
+
+    // Both streams' products of the tiles with an image (read the other way when transposed).
+    auto products = [&](std::uint32_t column, const unsigned char* image, bool transposed) {
+        const std::uint32_t b = umma::smem_address(image);
+#pragma unroll
+        for (int stream = 0; stream < 2; ++stream)
+        {
+            const std::uint32_t from = umma::smem_address(stream == 0 ? tile : tile_dot);
+#pragma unroll
+            for (int step = 0; step < 4; ++step)
+            {
+                umma::mma(tmem + column + 64 * stream,
+                          umma::matrix_descriptor(from + 2 * kRowChunk * step, kRowChunk, kRowGroup),
+                          transposed ? umma::matrix_descriptor(b + 2048 * step, 1024, 128)
+                                     : umma::matrix_descriptor(b + 256 * step),
+                          step > 0 ? 1u : 0u,
+                          transposed ? umma::kTransposedB : umma::kInstruction);
+            }
+        }
+    };
+    // The tiles' live rows to the per-pair arrays `kind` and `kind` + 1, eight lanes a row. The
+    // Gaussians' HBM row holds 1 in column 63 when K < 64 (a column the products never use).
+    auto copy_rows = [&](int kind, int index, bool ones) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+        {
+            const int r = (k * kReverseThreads + threadIdx.x) / 8, c = threadIdx.x % 8;
+            const int p = index * kTile + r;
+            if (p < count)
+            {
+                uint4 word = *reinterpret_cast<const uint4*>(row_word(tile, r, c));
+                if (ones && c == 7)
+                {
+                    word.w = (word.w & 0xFFFFu) | 0x3F800000u;
+                }
+                a.rows[(static_cast<std::int64_t>(kind) * a.capacity + p) * 8 + c] = word;
+                a.rows[(static_cast<std::int64_t>(kind + 1) * a.capacity + p) * 8 + c] =
+                    *reinterpret_cast<const uint4*>(row_word(tile_dot, r, c));
+            }
+        }
+    };
 
     for (int index = blockIdx.x; index * kTile < count; index += gridDim.x)
     {
-        const int p = index * kTile + threadIdx.x;
-        const PairTerms t = pair_terms(a, wbar, p, count);
-        tile_first[threadIdx.x] = t.live ? t.ab.x : -1;
         cores.tile_index = index;
-        store_basis_tangent(tile, tile_dot, t.g.w / a.width, -t.rate / a.width, a.gaussians,
-                            t.live, pair_row(a, kRowG, p, t.live), pair_row(a, kRowGDot, p, t.live));
-        if (!cores.run2(0, tile, image_b1, 64, tile_dot, image_b1, 1))
+        if (side == 0)
         {
-            break;
+            const PairTerms t = pair_terms(a, wbar, index * kTile + row, count);
+            first[row] = t.live ? t.ab.x : -1;
+            second[row] = t.ab.y;
+            envelopes[row] = t.envelope;
+            movings[row] = t.moving;
+            offsets[row] = t.g.w / a.width;
+            scales[row] = -t.rate / a.width;
         }
-        store_activations(cores.tmem, bias1, tile, tile_dot, pair_row(a, kRowS, p, t.live),
-                          pair_row(a, kRowSDot, p, t.live));
-        if (!cores.run2(128, tile, image_b2, 192, tile_dot, image_b2, 2))
+        __syncthreads();  // and the last tile's rows have left
         {
-            break;
-        }
-        uint4* row_ub = pair_row(a, kRowUBar, p, t.live);
-        uint4* row_udb = pair_row(a, kRowUDotBar, p, t.live);
-#pragma unroll
-        for (int half = 0; half < 2; ++half)
-        {
-#pragma unroll
-            for (int batch = 0; batch < 4; batch += kGatherBatch)
-            {
-                // The batch's gathers first (eight rows, kGatherBatch words each), so their
-                // latencies overlap; dead rows read atom 0 and contribute zeros.
-                uint4 raw[kGatherBatch][8];
-#pragma unroll
-                for (int i = 0; i < kGatherBatch; ++i)
-                {
-                    const int k = 32 * half + 8 * (batch + i);
-                    const std::int64_t ga = 8 * static_cast<std::int64_t>(t.ab.x) + k / 8;
-                    const std::int64_t gb = 8 * static_cast<std::int64_t>(t.ab.y) + k / 8;
-                    raw[i][0] = __ldg(a.v + ga);
-                    raw[i][1] = __ldg(a.v + gb);
-                    raw[i][2] = __ldg(a.v_dot + ga);
-                    raw[i][3] = __ldg(a.v_dot + gb);
-                    raw[i][4] = __ldg(a.m_bar + ga);
-                    raw[i][5] = __ldg(a.m_bar + gb);
-                    raw[i][6] = __ldg(a.m_dot_bar + ga);
-                    raw[i][7] = __ldg(a.m_dot_bar + gb);
-                }
-#pragma unroll
-                for (int i = 0; i < kGatherBatch; ++i)
-                {
-                    const int c = batch + i;
-                    const int k = 32 * half + 8 * c;
-                    float u[8];
-                    float ud[8];
-                    umma::load8(cores.tmem + 128 + k, u);
-                    umma::load8(cores.tmem + 192 + k, ud);
-                    umma::wait_loads();
-                    float va[8], vb[8], vda[8], vdb[8], ma[8], mb[8], mda[8], mdb[8];
-                    widen8(raw[i][0], va);
-                    widen8(raw[i][1], vb);
-                    widen8(raw[i][2], vda);
-                    widen8(raw[i][3], vdb);
-                    widen8(raw[i][4], ma);
-                    widen8(raw[i][5], mb);
-                    widen8(raw[i][6], mda);
-                    widen8(raw[i][7], mdb);
-                    float ub[8], udb[8], first[8], first_dot[8], to_second[8], to_second_dot[8];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                    {
-                        const float raw_filter = u[j] + bias2[k + j];
-                        const float f = raw_filter * t.envelope;
-                        const float fd = ud[j] * t.envelope + raw_filter * t.moving;
-                        const float fb = ma[j] * vb[j] + mb[j] * va[j] + mda[j] * vdb[j] +
-                                         mdb[j] * vda[j];
-                        const float fdb = mda[j] * vb[j] + mdb[j] * va[j];
-                        to_second[j] = f * ma[j] + fd * mda[j];
-                        to_second_dot[j] = f * mda[j];
-                        first[j] = f * mb[j] + fd * mdb[j];
-                        first_dot[j] = f * mdb[j];
-                        ub[j] = fb * t.envelope + fdb * t.moving;
-                        udb[j] = fdb * t.envelope;
-                    }
-                    if (t.live)
-                    {
-                        const std::int64_t gb = 8 * static_cast<std::int64_t>(t.ab.y) + k / 8;
-#pragma unroll
-                        for (int h4 = 0; h4 < 2; ++h4)
-                        {
-                            const int o = 4 * h4;
-                            atomicAdd(vbar4 + 2 * gb + h4,
-                                      make_float4(to_second[o], to_second[o + 1],
-                                                  to_second[o + 2], to_second[o + 3]));
-                            atomicAdd(vdbar4 + 2 * gb + h4,
-                                      make_float4(to_second_dot[o], to_second_dot[o + 1],
-                                                  to_second_dot[o + 2], to_second_dot[o + 3]));
-                        }
-                    }
-                    put_run_part(stage, 2 * c, make_float4(first[0], first[1], first[2], first[3]));
-                    put_run_part(stage, 2 * c + 1,
-                                 make_float4(first[4], first[5], first[6], first[7]));
-                    put_run_part(stage_dot, 2 * c,
-                                 make_float4(first_dot[0], first_dot[1], first_dot[2], first_dot[3]));
-                    put_run_part(stage_dot, 2 * c + 1,
-                                 make_float4(first_dot[4], first_dot[5], first_dot[6], first_dot[7]));
-                    const int column = 4 * half + c;
-                    const uint4 word = umma::pack8(ub);
-                    const uint4 word_dot = umma::pack8(udb);
-                    *reinterpret_cast<uint4*>(tile + umma::image_offset(threadIdx.x, 8 * column)) =
-                        word;
-                    *reinterpret_cast<uint4*>(tile_dot +
-                                              umma::image_offset(threadIdx.x, 8 * column)) =
-                        word_dot;
-                    if (row_ub != nullptr)
-                    {
-                        row_ub[column] = word;
-                        row_udb[column] = word_dot;
-                    }
-                }
-            }
-            // the stages are this kernel's own: only this warp writes their rows again
-            sum_runs(stage, tile_first, a.v_bar, half, false);
-            sum_runs(stage_dot, tile_first, a.v_dot_bar, half, false);
-        }
-        if (!cores.run2(128, tile, image_b2t, 192, tile_dot, image_b2t, 3))
-        {
-            break;
-        }
-        uint4* row_zb = pair_row(a, kRowZBar, p, t.live);
-        uint4* row_zdb = pair_row(a, kRowZDotBar, p, t.live);
-#pragma unroll
-        for (int half = 0; half < 2; ++half)
-        {
-            float sb[32];
-            float sdb[32];
-            float z[32];
-            float zd[32];
-            umma::load32(cores.tmem + 128 + 32 * half, sb);
-            umma::load32(cores.tmem + 192 + 32 * half, sdb);
-            umma::load32(cores.tmem + 32 * half, z);
-            umma::load32(cores.tmem + 64 + 32 * half, zd);
-            umma::wait_loads();
+            const float t = offsets[row], scale = scales[row];
 #pragma unroll
             for (int c = 0; c < 4; ++c)
             {
-                float zb[8];
-                float zdb[8];
+                const int k0 = 32 * side + 8 * c;
+                float g[8], gd[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                {
+                    const float u = t - static_cast<float>(k0 + e);
+                    g[e] = k0 + e < a.gaussians ? gaussian(u) : 0.0f;
+                    gd[e] = g[e] * u * scale;
+                }
+                *reinterpret_cast<uint4*>(row_word(tile, row, 4 * side + c)) = umma::pack8(g);
+                *reinterpret_cast<uint4*>(row_word(tile_dot, row, 4 * side + c)) = umma::pack8(gd);
+            }
+        }
+        cores.begin([&] { products(0, image_b1, false); });
+        copy_rows(kRowG, index, a.gaussians < 64);
+        if (!cores.finish(1))
+        {
+            break;
+        }
+        // s = ssp(z + b1) and s_dot = sigmoid(z + b1) z_dot.
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half)
+        {
+            float z[16], zd[16];
+            const int column = 32 * side + 16 * half;
+            umma::load16(cores.tmem + column, z);
+            umma::load16(cores.tmem + 64 + column, zd);
+            umma::wait_loads();
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+            {
+                float s[8], sd[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                {
+                    const float x = z[8 * c + e] + bias1[column + 8 * c + e];
+                    s[e] = softplus_shifted(x);
+                    sd[e] = sigmoid(x) * zd[8 * c + e];
+                }
+                *reinterpret_cast<uint4*>(row_word(tile, row, column / 8 + c)) = umma::pack8(s);
+                *reinterpret_cast<uint4*>(row_word(tile_dot, row, column / 8 + c)) = umma::pack8(sd);
+            }
+        }
+        cores.begin([&] { products(128, image_b2, false); });
+        copy_rows(kRowS, index, false);
+        if (!cores.finish(2))
+        {
+            break;
+        }
+#pragma unroll 1
+        for (int step = 0; step < 2; ++step)
+        {
+            // This lane's word of a feature row: columns 16 step + 4 lane of the first half, or
+            // of the second half for lanes 4 .. 7.
+            const int place = 8 * (lane / 4) + 4 * step + lane % 4;
+            uint2 vb[4], vdb[4], mb[4], mdb[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+            {
+                const std::int64_t word =
+                    16 * static_cast<std::int64_t>(second[lane_row + i]) + place;
+                vb[i] = __ldg(v + word);
+                vdb[i] = __ldg(v_dot + word);
+                mb[i] = __ldg(m_bar + word);
+                mdb[i] = __ldg(m_dot_bar + word);
+            }
+            {
+                float u[16], ud[16];
+                const int column = 32 * side + 16 * step;
+                umma::load16(cores.tmem + 128 + column, u);
+                umma::load16(cores.tmem + 192 + column, ud);
+                umma::wait_loads();
+                const float envelope = envelopes[row], moving = movings[row];
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                {
+                    float f[4], fd[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                    {
+                        const float raw_filter = u[4 * q + e] + bias2[column + 4 * q + e];
+                        f[e] = raw_filter * envelope;
+                        fd[e] = ud[4 * q + e] * envelope + raw_filter * moving;
+                    }
+                    const int at = row * 8 + ((4 * side + q) ^ (row & 7));
+                    reinterpret_cast<float4*>(stage)[at] = make_float4(f[0], f[1], f[2], f[3]);
+                    reinterpret_cast<float4*>(stage_dot)[at] = make_float4(fd[0], fd[1], fd[2], fd[3]);
+                }
+            }
+            umma::fence_before_sync();
+            __syncthreads();
+            RunSums<2> run;
+            run.start(first[lane_row]);
+            float4* const targets[2] = {vbar4 + place, vdbar4 + place};
+            float4 va, vda, ma, mda;
+            auto load_first = [&](int atom) {
+                const std::int64_t word = 16 * static_cast<std::int64_t>(max(atom, 0)) + place;
+                va = widen4(__ldg(v + word));
+                vda = widen4(__ldg(v_dot + word));
+                ma = widen4(__ldg(m_bar + word));
+                mda = widen4(__ldg(m_dot_bar + word));
+            };
+            load_first(run.key);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+            {
+                const int r = lane_row + i;
+                const int atom = first[r];
+                if (atom != run.key)
+                {
+                    run.turn(atom, targets);
+                    load_first(atom);
+                }
+                const float envelope = envelopes[r], moving = movings[r];
+                const float4 f = staged4(stage, r, lane), fd = staged4(stage_dot, r, lane);
+                const float4 right_v = widen4(vb[i]), right_vd = widen4(vdb[i]);
+                const float4 right_m = widen4(mb[i]), right_md = widen4(mdb[i]);
+                const float4 fb = ma * right_v + right_m * va + mda * right_vd + right_md * vda;
+                const float4 fdb = mda * right_v + right_md * va;
+                if (atom >= 0)
+                {
+                    const std::int64_t word = 16 * static_cast<std::int64_t>(second[r]) + place;
+                    atomicAdd(vbar4 + word, f * ma + fd * mda);
+                    atomicAdd(vdbar4 + word, f * mda);
+                }
+                run.sums[0] = run.sums[0] + (f * right_m + fd * right_md);
+                run.sums[1] = run.sums[1] + f * right_md;
+                const float4 ub = fb * envelope + fdb * moving, udb = fdb * envelope;
+                const int to = 8 * (place & 1);
+                *reinterpret_cast<uint2*>(row_word(tile, r, place / 2) + to) =
+                    make_uint2(pack2(ub.x, ub.y), pack2(ub.z, ub.w));
+                *reinterpret_cast<uint2*>(row_word(tile_dot, r, place / 2) + to) =
+                    make_uint2(pack2(udb.x, udb.y), pack2(udb.z, udb.w));
+            }
+            run.finish(targets, group);
+            __syncthreads();  // the stages are written again, or the tiles read
+        }
+        cores.begin([&] { products(128, image_b2, true); });
+        copy_rows(kRowUBar, index, false);
+        if (!cores.finish(3))
+        {
+            break;
+        }
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half)
+        {
+            float sb[16], sdb[16], z[16], zd[16];
+            const int column = 32 * side + 16 * half;
+            umma::load16(cores.tmem + 128 + column, sb);
+            umma::load16(cores.tmem + 192 + column, sdb);
+            umma::load16(cores.tmem + column, z);
+            umma::load16(cores.tmem + 64 + column, zd);
+            umma::wait_loads();
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+            {
+                float zb[8], zdb[8];
 #pragma unroll
                 for (int e = 0; e < 8; ++e)
                 {
                     const int i = 8 * c + e;
-                    const float sg = sigmoid(z[i] + bias1[32 * half + i]);
+                    const float sg = sigmoid(z[i] + bias1[column + i]);
                     zb[e] = sb[i] * sg + sdb[i] * zd[i] * sg * (1.0f - sg);
                     zdb[e] = sdb[i] * sg;
                 }
-                if (row_zb != nullptr)
-                {
-                    row_zb[4 * half + c] = umma::pack8(zb);
-                    row_zdb[4 * half + c] = umma::pack8(zdb);
-                }
+                *reinterpret_cast<uint4*>(row_word(tile, row, column / 8 + c)) = umma::pack8(zb);
+                *reinterpret_cast<uint4*>(row_word(tile_dot, row, column / 8 + c)) = umma::pack8(zdb);
             }
         }
+        umma::fence_before_sync();
+        __syncthreads();
+        copy_rows(kRowZBar, index, false);
     }
     cores.close(256);
 }
@@ -647,8 +711,8 @@ int nd_schnet_tangent(const nd_schnet_tangent_args* args, int32_t direction,
     }
     else
     {
-        const int grid = pair_grid(reinterpret_cast<const void*>(tangent_reverse_kernel), kTangentReverseShared, 256);
-        tangent_reverse_kernel<<<grid, kTile, kTangentReverseShared, stream>>>(pass);
+        const int grid = pair_grid(reinterpret_cast<const void*>(tangent_reverse_kernel), kTangentReverseShared, 256, kReverseThreads);
+        tangent_reverse_kernel<<<grid, kReverseThreads, kTangentReverseShared, stream>>>(pass);
         ND_LAUNCH_CHECK();
         zero_tail_kernel<<<std::min<std::int64_t>(1184, blocks_for(s.capacity * 8)), kThreads, 0, stream>>>(
             pass.rows, s.capacity, pass.counters);

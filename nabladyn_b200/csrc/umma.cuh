@@ -43,11 +43,13 @@ __device__ __forceinline__ std::uint32_t smem_address(const void* pointer)
 
 // Shared-memory matrix descriptor: start address, leading and stride byte offsets (all in
 // 16-byte units), the sm_100 descriptor version (bit 46) and no swizzle (bits 61-63 = 0).
-__device__ __forceinline__ std::uint64_t matrix_descriptor(std::uint32_t address)
+__device__ __forceinline__ std::uint64_t matrix_descriptor(std::uint32_t address,
+                                                           std::uint32_t leading = 128,
+                                                           std::uint32_t stride = 1024)
 {
     std::uint64_t descriptor = (address >> 4) & 0x3FFFu;
-    descriptor |= static_cast<std::uint64_t>(128 >> 4) << 16;
-    descriptor |= static_cast<std::uint64_t>(1024 >> 4) << 32;
+    descriptor |= static_cast<std::uint64_t>(leading >> 4) << 16;
+    descriptor |= static_cast<std::uint64_t>(stride >> 4) << 32;
     descriptor |= static_cast<std::uint64_t>(1) << 46;
     return descriptor;
 }
@@ -79,33 +81,14 @@ __device__ __forceinline__ void product(std::uint32_t tmem, std::uint32_t a, std
     }
 }
 
-// D = A B over K = 64 with B a weight image read the other way (its row index is the reduction
-// index), so one image serves a layer and its reverse. The same core matrices read MN-major:
-// 8 rows of the reduction index by 16 bytes of columns; the stride-dimension offset is the step
-// between 8-column groups (128 bytes) and the leading-dimension offset the step between 8-row
-// groups (1024 bytes); K = 16 takes two row groups (2048 bytes). PTX ISA, tcgen05 canonical
-// layouts without swizzle; bit 16 of the instruction descriptor marks B as MN-major.
-__device__ __forceinline__ std::uint64_t transposed_descriptor(std::uint32_t address)
-{
-    std::uint64_t descriptor = (address >> 4) & 0x3FFFu;
-    descriptor |= static_cast<std::uint64_t>(1024 >> 4) << 16;
-    descriptor |= static_cast<std::uint64_t>(128 >> 4) << 32;
-    descriptor |= static_cast<std::uint64_t>(1) << 46;
-    return descriptor;
-}
-
+// B as a weight image read the other way (its row index is the reduction index), so one image
+// serves a layer and its reverse: D = A B. The same core matrices read MN-major: 8 rows of the
+// reduction index by 16 bytes of columns; the stride-dimension offset is the step between
+// 8-column groups (128 bytes) and the leading-dimension offset the step between 8-row groups
+// (1024 bytes), so the descriptor is matrix_descriptor(b + 2048 * step, 1024, 128), K = 16
+// taking two row groups. PTX ISA, tcgen05 canonical layouts without swizzle; bit 16 of the
+// instruction descriptor marks B as MN-major.
 constexpr std::uint32_t kTransposedB = kInstruction | (1u << 16);
-
-__device__ __forceinline__ void product_transposed(std::uint32_t tmem, std::uint32_t a,
-                                                   std::uint32_t b)
-{
-#pragma unroll
-    for (int step = 0; step < 4; ++step)
-    {
-        mma(tmem, matrix_descriptor(a + 256 * step), transposed_descriptor(b + 2048 * step),
-            step > 0 ? 1u : 0u, kTransposedB);
-    }
-}
 
 // Arrive on `barrier` once every product this thread issued has completed.
 __device__ __forceinline__ void commit(std::uint64_t* barrier)
@@ -172,6 +155,25 @@ __device__ __forceinline__ void load32(std::uint32_t tmem, float (&out)[32])
         : "r"(tmem));
 #pragma unroll
     for (int i = 0; i < 32; ++i)
+    {
+        out[i] = __uint_as_float(r[i]);
+    }
+}
+
+// 16 consecutive 32-bit columns of this thread's lane (follow with wait_loads()).
+__device__ __forceinline__ void load16(std::uint32_t tmem, float (&out)[16])
+{
+    std::uint32_t r[16];
+    __syncwarp();
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
+        "%11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
+          "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(tmem));
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
     {
         out[i] = __uint_as_float(r[i]);
     }
@@ -259,10 +261,12 @@ __device__ __forceinline__ uint4 pack8(const float* v)
     return word;
 }
 
-// Stores 8 values as columns 8c .. 8c + 7 of `row` of a row tile.
+// Stores 8 values as columns 8c .. 8c + 7 of `row` of a row tile whose 16-byte chunks lie kChunk
+// and whose eight-row groups kGroup bytes apart.
+template <int kChunk = 128, int kGroup = 1024>
 __device__ __forceinline__ void store8(unsigned char* tile, int row, int c, const float* v)
 {
-    *reinterpret_cast<uint4*>(tile + image_offset(row, 8 * c)) = pack8(v);
+    *reinterpret_cast<uint4*>(tile + (row >> 3) * kGroup + c * kChunk + (row & 7) * 16) = pack8(v);
 }
 
 }  // namespace nd::umma
