@@ -188,10 +188,14 @@ __global__ void __launch_bounds__(kThreads) compact_write_kernel(
     }
 }
 
-// x = embedding[type], v0 = (embedding A0^T)[type].
-__global__ void embed_kernel(const std::int64_t* __restrict__ types, std::int64_t atoms,
-                             const float* __restrict__ table, const float* __restrict__ table_v,
-                             float* __restrict__ x, float* __restrict__ v)
+// x = embedding[type], v0 = (embedding A0^T)[type]; and zero in what the passes add to: every
+// block's messages (`m`, `blocks` buffers of `row` float4 each), Gv and the forces. One thread
+// per four features of an atom.
+__global__ void __launch_bounds__(kThreads) embed_kernel(
+    const std::int64_t* __restrict__ types, std::int64_t atoms, const float* __restrict__ table,
+    const float* __restrict__ table_v, float* __restrict__ x, float* __restrict__ v,
+    float4* __restrict__ m, int blocks, std::int64_t row, float4* __restrict__ grad_v,
+    float* __restrict__ forces)
 {
     const std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= atoms * 16)
@@ -204,6 +208,19 @@ __global__ void embed_kernel(const std::int64_t* __restrict__ types, std::int64_
     reinterpret_cast<float4*>(x)[i] = reinterpret_cast<const float4*>(table)[type * 16 + q];
     const float4 value = reinterpret_cast<const float4*>(table_v)[type * 16 + q];
     reinterpret_cast<uint2*>(v)[i] = make_uint2(pack2(value.x, value.y), pack2(value.z, value.w));
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int b = 0; b < blocks; ++b)
+    {
+        m[b * row + i] = zero;
+    }
+    if (grad_v != nullptr)
+    {
+        grad_v[i] = zero;
+    }
+    if (forces != nullptr && i < atoms * 3)
+    {
+        forces[i] = 0.0f;
+    }
 }
 
 struct PairPass
@@ -683,85 +700,171 @@ struct AtomPass
     float* v_next;         // forward: the next block's v in BF16 (null for the last block)
     const float* readout;  // forward, last block: R1, e1, R2, e2
     float* grad;           // forward, last block: writes dE/dx; reverse: reads, updates
-    const float* grad_v;   // reverse: Gv of the next block (null for the last block)
+    float* grad_v;         // reverse: Gv of the next block, read and set to zero (null for the
+                           // last block)
     float* grad_m;         // reverse: writes Gm in BF16
     double* energy;        // forward, last block: per-CTA partials
     int* counters;
 };
 
-constexpr int kAtomShared = 3 * umma::kImageBytes + umma::kTileBytes +
-                            (kHidden * kFeatures + 3 * kHidden) * 4 + 2 * 256 + 64;
+// The atom-wise layers: one CTA of 256 threads per 128 atoms, thread t computing columns
+// 32 (t / 128) .. + 31 of row t % 128. A small system has fewer tiles than SMs and one chain of
+// products per tile, so what counts is the chain's length: two threads per row halve its
+// row-wise part.
+constexpr int kAtomThreads = 256;
+constexpr int kHalf = kFeatures / 2;
+constexpr int kReadoutFloats = kHidden * kFeatures + 3 * kHidden;
+constexpr int kAtomShared =
+    3 * umma::kImageBytes + umma::kTileBytes + kReadoutFloats * 4 + 2 * 256 + 64;
+// The readout's exchange lies over the images and the tile, free by then: first the rows of x
+// (68 floats apart: a row's 16-byte words then start in different banks), later ssp(y) and
+// sigmoid(y) R2 of every hidden unit and row.
+constexpr int kExchangeRow = 68;
+static_assert(kTile * kExchangeRow * 4 <= 3 * umma::kImageBytes + umma::kTileBytes &&
+                  2 * kHidden * kTile * 4 <= 3 * umma::kImageBytes + umma::kTileBytes,
+              "the exchange fits");
 
-__device__ __forceinline__ void load_row(const float* source, std::int64_t row, bool live, float* out)
+struct AtomRow
 {
-    const float4* s4 = reinterpret_cast<const float4*>(source) + 16 * row;
-#pragma unroll
-    for (int q = 0; q < 16; ++q)
-    {
-        const float4 value = live ? s4[q] : make_float4(0.f, 0.f, 0.f, 0.f);
-        out[4 * q] = value.x;
-        out[4 * q + 1] = value.y;
-        out[4 * q + 2] = value.z;
-        out[4 * q + 3] = value.w;
-    }
-}
+    std::int64_t row;  // the atom
+    bool live;
+    int local;  // row of the tile
+    int side;   // columns 32 side .. 32 side + 31
 
-__device__ __forceinline__ void store_tile_row(unsigned char* tile, const float* values)
-{
-#pragma unroll
-    for (int c = 0; c < 8; ++c)
+    __device__ explicit AtomRow(std::int64_t atoms)
+        : local(threadIdx.x % kTile), side(threadIdx.x / kTile)
     {
-        umma::store8(tile, threadIdx.x, c, values + 8 * c);
+        row = static_cast<std::int64_t>(blockIdx.x) * kTile + local;
+        live = row < atoms;
     }
-}
 
-// The 64 accumulator columns of this thread's row.
-__device__ __forceinline__ void load_row_tmem(std::uint32_t tmem, float* out)
-{
-    float part[32];
-    umma::load32(tmem, part);
-    umma::wait_loads();
-#pragma unroll
-    for (int i = 0; i < 32; ++i)
+    __device__ __forceinline__ void load(const float* source, float (&out)[kHalf]) const
     {
-        out[i] = part[i];
-    }
-    umma::load32(tmem + 32, part);
-    umma::wait_loads();
+        const float4* s4 = reinterpret_cast<const float4*>(source) + 16 * row + 8 * side;
 #pragma unroll
-    for (int i = 0; i < 32; ++i)
-    {
-        out[32 + i] = part[i];
+        for (int q = 0; q < 8; ++q)
+        {
+            const float4 value = live ? s4[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+            out[4 * q] = value.x;
+            out[4 * q + 1] = value.y;
+            out[4 * q + 2] = value.z;
+            out[4 * q + 3] = value.w;
+        }
     }
-}
 
-__device__ __forceinline__ void store_row(float* target, std::int64_t row, const float* values)
-{
-    float4* t4 = reinterpret_cast<float4*>(target) + 16 * row;
-#pragma unroll
-    for (int q = 0; q < 16; ++q)
+    __device__ __forceinline__ void store(float* target, const float (&values)[kHalf]) const
     {
-        t4[q] = make_float4(values[4 * q], values[4 * q + 1], values[4 * q + 2], values[4 * q + 3]);
+        float4* t4 = reinterpret_cast<float4*>(target) + 16 * row + 8 * side;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+        {
+            if (live)
+            {
+                t4[q] = make_float4(values[4 * q], values[4 * q + 1], values[4 * q + 2],
+                                    values[4 * q + 3]);
+            }
+        }
     }
-}
 
-__device__ __forceinline__ void store_row_bf16(float* target, std::int64_t row, const float* values)
+    __device__ __forceinline__ void store_bf16(float* target, const float (&values)[kHalf]) const
+    {
+        uint4* t4 = reinterpret_cast<uint4*>(target) + 8 * row + 4 * side;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+        {
+            if (live)
+            {
+                t4[q] = umma::pack8(values + 8 * q);
+            }
+        }
+    }
+
+    __device__ __forceinline__ void store_tile(unsigned char* tile,
+                                               const float (&values)[kHalf]) const
+    {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+        {
+            umma::store8(tile, local, 4 * side + c, values + 8 * c);
+        }
+    }
+
+    // The accumulator's columns of this thread.
+    __device__ __forceinline__ void load_product(const Cores& cores, float (&out)[kHalf]) const
+    {
+        umma::load32(cores.tmem + 32 * side, out);
+        umma::wait_loads();
+    }
+};
+
+// e = ssp(x R1^T + e1) R2^T + e2 and dE/dx of the last block's x: each side computes half of
+// the hidden units from whole rows, then half of the gradient's columns from all of them (the
+// sums over features and over hidden units run in index order).
+__device__ __forceinline__ float readout_row(const AtomRow& at, const float* readout,
+                                             float* exchange, const float (&x)[kHalf],
+                                             float (&grad)[kHalf])
 {
-    uint4* t4 = reinterpret_cast<uint4*>(target) + 8 * row;
+    const float* r1 = readout;
+    const float* e1 = readout + kHidden * kFeatures;
+    const float* r2 = e1 + kHidden;
+    const float e2 = r2[kHidden];
 #pragma unroll
     for (int q = 0; q < 8; ++q)
     {
-        t4[q] = make_uint4(pack2(values[8 * q], values[8 * q + 1]),
-                           pack2(values[8 * q + 2], values[8 * q + 3]),
-                           pack2(values[8 * q + 4], values[8 * q + 5]),
-                           pack2(values[8 * q + 6], values[8 * q + 7]));
+        *reinterpret_cast<float4*>(exchange + at.local * kExchangeRow + 32 * at.side + 4 * q) =
+            make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
     }
+    __syncthreads();
+    float whole[kFeatures];
+#pragma unroll
+    for (int q = 0; q < 16; ++q)
+    {
+        const float4 value =
+            *reinterpret_cast<const float4*>(exchange + at.local * kExchangeRow + 4 * q);
+        whole[4 * q] = value.x;
+        whole[4 * q + 1] = value.y;
+        whole[4 * q + 2] = value.z;
+        whole[4 * q + 3] = value.w;
+    }
+    __syncthreads();
+    float* softplus = exchange;                   // [hidden][row]
+    float* slopes = exchange + kHidden * kTile;
+#pragma unroll 2
+    for (int j = kHidden / 2 * at.side; j < kHidden / 2 * (at.side + 1); ++j)
+    {
+        float y = e1[j];
+#pragma unroll
+        for (int k = 0; k < kFeatures; ++k)
+        {
+            y = fmaf(whole[k], r1[j * kFeatures + k], y);
+        }
+        softplus[j * kTile + at.local] = softplus_shifted(y);
+        slopes[j * kTile + at.local] = sigmoid(y) * r2[j];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kHalf; ++k)
+    {
+        grad[k] = 0.0f;
+    }
+    float e = e2;
+    for (int j = 0; j < kHidden; ++j)
+    {
+        e += softplus[j * kTile + at.local] * r2[j];
+        const float s = slopes[j * kTile + at.local];
+#pragma unroll
+        for (int k = 0; k < kHalf; ++k)
+        {
+            grad[k] = fmaf(s, r1[j * kFeatures + 32 * at.side + k], grad[k]);
+        }
+    }
+    return e;
 }
 
 // h = m D1^T + d1, x += ssp(h) D2^T + d2, then v' = x A'^T, or on the last block the readout:
 // e = ssp(x R1^T + e1) R2^T + e2 and dE/dx.
 template <bool kLast>
-__global__ void __launch_bounds__(kTile) atom_forward_kernel(AtomPass a)
+__global__ void __launch_bounds__(kAtomThreads) atom_forward_kernel(AtomPass a)
 {
     extern __shared__ __align__(1024) unsigned char shared[];
     unsigned char* image_d1 = shared;
@@ -769,11 +872,15 @@ __global__ void __launch_bounds__(kTile) atom_forward_kernel(AtomPass a)
     unsigned char* image_a = image_d2 + umma::kImageBytes;
     unsigned char* tile = image_a + umma::kImageBytes;
     float* readout = reinterpret_cast<float*>(tile + umma::kTileBytes);
-    float* bias1 = readout + kHidden * kFeatures + 3 * kHidden;
+    float* bias1 = readout + kReadoutFloats;
     float* bias2 = bias1 + kFeatures;
     auto* barrier = reinterpret_cast<std::uint64_t*>(bias2 + kFeatures);
     auto* slot = reinterpret_cast<std::uint32_t*>(barrier + 1);
 
+    const AtomRow at(a.atoms);
+    float values[kHalf], x[kHalf];
+    at.load(a.m, values);
+    at.load(a.x, x);
     copy_bytes(image_d1, a.images + kD1 * umma::kImageBytes, umma::kImageBytes);
     copy_bytes(image_d2, a.images + kD2 * umma::kImageBytes, umma::kImageBytes);
     if (!kLast)
@@ -782,7 +889,7 @@ __global__ void __launch_bounds__(kTile) atom_forward_kernel(AtomPass a)
     }
     else
     {
-        for (int i = threadIdx.x; i < kHidden * kFeatures + 3 * kHidden; i += kTile)
+        for (int i = threadIdx.x; i < kReadoutFloats; i += kAtomThreads)
         {
             readout[i] = a.readout[i];
         }
@@ -795,104 +902,57 @@ __global__ void __launch_bounds__(kTile) atom_forward_kernel(AtomPass a)
     Cores cores;
     cores.open(barrier, slot, 64, a.counters, 3);
     cores.tile_index = blockIdx.x;
-    const std::int64_t row = static_cast<std::int64_t>(blockIdx.x) * kTile + threadIdx.x;
-    const bool live = row < a.atoms;
     double energy = 0.0;
-    bool ok = true;
+    at.store_tile(tile, values);
+    bool ok = cores.run(0, tile, image_d1, 1);
+    if (ok)
     {
-        float values[kFeatures];
-        load_row(a.m, row, live, values);
-        store_tile_row(tile, values);
-        ok = cores.run(0, tile, image_d1, 1);
-        if (ok)
+        at.load_product(cores, values);
+#pragma unroll
+        for (int k = 0; k < kHalf; ++k)
         {
-            load_row_tmem(cores.tmem, values);
-#pragma unroll
-            for (int k = 0; k < kFeatures; ++k)
-            {
-                values[k] += bias1[k];
-            }
-            if (live)
-            {
-                store_row(a.h, row, values);
-            }
-#pragma unroll
-            for (int k = 0; k < kFeatures; ++k)
-            {
-                values[k] = softplus_shifted(values[k]);
-            }
-            store_tile_row(tile, values);
-            ok = cores.run(0, tile, image_d2, 2);
+            values[k] += bias1[32 * at.side + k];
         }
-        if (ok)
+        at.store(a.h, values);
+#pragma unroll
+        for (int k = 0; k < kHalf; ++k)
         {
-            float x[kFeatures];
-            load_row(a.x, row, live, x);
-            load_row_tmem(cores.tmem, values);
+            values[k] = softplus_shifted(values[k]);
+        }
+        at.store_tile(tile, values);
+        ok = cores.run(0, tile, image_d2, 2);
+    }
+    if (ok)
+    {
+        at.load_product(cores, values);
 #pragma unroll
-            for (int k = 0; k < kFeatures; ++k)
+        for (int k = 0; k < kHalf; ++k)
+        {
+            x[k] += values[k] + bias2[32 * at.side + k];
+        }
+        if (!kLast)
+        {
+            at.store(a.x, x);
+            at.store_tile(tile, x);
+            ok = cores.run(0, tile, image_a, 3);
+            if (ok)
             {
-                x[k] += values[k] + bias2[k];
+                at.load_product(cores, values);
+                at.store_bf16(a.v_next, values);
             }
-            if (!kLast)
-            {
-                if (live)
-                {
-                    store_row(a.x, row, x);
-                }
-                store_tile_row(tile, x);
-                ok = cores.run(0, tile, image_a, 3);
-                if (ok)
-                {
-                    load_row_tmem(cores.tmem, values);
-                    if (live)
-                    {
-                        store_row_bf16(a.v_next, row, values);
-                    }
-                }
-            }
-            else
-            {
-                const float* r1 = readout;
-                const float* e1 = readout + kHidden * kFeatures;
-                const float* r2 = e1 + kHidden;
-                const float e2 = r2[kHidden];
-                float grad[kFeatures];
-#pragma unroll
-                for (int k = 0; k < kFeatures; ++k)
-                {
-                    grad[k] = 0.0f;
-                }
-                float e = e2;
-                for (int j = 0; j < kHidden; ++j)
-                {
-                    float y = e1[j];
-#pragma unroll
-                    for (int k = 0; k < kFeatures; ++k)
-                    {
-                        y = fmaf(x[k], r1[j * kFeatures + k], y);
-                    }
-                    e += softplus_shifted(y) * r2[j];
-                    const float s = sigmoid(y) * r2[j];
-#pragma unroll
-                    for (int k = 0; k < kFeatures; ++k)
-                    {
-                        grad[k] = fmaf(s, r1[j * kFeatures + k], grad[k]);
-                    }
-                }
-                if (live)
-                {
-                    store_row(a.grad, row, grad);
-                    energy = e;
-                }
-            }
+        }
+        else
+        {
+            const float e = readout_row(at, readout, reinterpret_cast<float*>(shared), x, values);
+            at.store(a.grad, values);
+            energy = at.live && at.side == 0 ? e : 0.0;
         }
     }
     if (kLast)
     {
         __shared__ double sums[4];
         const double s = warp_sum(energy);
-        if ((threadIdx.x & 31) == 0)
+        if ((threadIdx.x & 31) == 0 && at.side == 0)
         {
             sums[threadIdx.x / 32] = s;
         }
@@ -905,9 +965,9 @@ __global__ void __launch_bounds__(kTile) atom_forward_kernel(AtomPass a)
     cores.close(64);
 }
 
-// Reverse of one block's atom-wise layers: G += Gv' A' (the next block's messages), then
-// Gh = (G D2) * sigmoid(h) and Gm = Gh D1.
-__global__ void __launch_bounds__(kTile) atom_reverse_kernel(AtomPass a)
+// Reverse of one block's atom-wise layers: G += Gv' A' (the next block's messages; Gv' goes
+// back to zero for this block's pair pass), then Gh = (G D2) * sigmoid(h) and Gm = Gh D1.
+__global__ void __launch_bounds__(kAtomThreads) atom_reverse_kernel(AtomPass a)
 {
     extern __shared__ __align__(1024) unsigned char shared[];
     unsigned char* image_d2t = shared;
@@ -917,9 +977,17 @@ __global__ void __launch_bounds__(kTile) atom_reverse_kernel(AtomPass a)
     auto* barrier = reinterpret_cast<std::uint64_t*>(tile + umma::kTileBytes);
     auto* slot = reinterpret_cast<std::uint32_t*>(barrier + 1);
 
+    const bool chained = a.grad_v != nullptr;
+    const AtomRow at(a.atoms);
+    float grad[kHalf], values[kHalf], h[kHalf];
+    at.load(a.grad, grad);
+    at.load(a.h, h);
+    if (chained)
+    {
+        at.load(a.grad_v, values);
+    }
     copy_bytes(image_d2t, a.images + kD2T * umma::kImageBytes, umma::kImageBytes);
     copy_bytes(image_d1t, a.images + kD1T * umma::kImageBytes, umma::kImageBytes);
-    const bool chained = a.grad_v != nullptr;
     if (chained)
     {
         copy_bytes(image_at, a.next_images + kAT * umma::kImageBytes, umma::kImageBytes);
@@ -927,110 +995,70 @@ __global__ void __launch_bounds__(kTile) atom_reverse_kernel(AtomPass a)
     Cores cores;
     cores.open(barrier, slot, 64, a.counters, 4);
     cores.tile_index = blockIdx.x;
-    const std::int64_t row = static_cast<std::int64_t>(blockIdx.x) * kTile + threadIdx.x;
-    const bool live = row < a.atoms;
     bool ok = true;
-    float grad[kFeatures];
-    float values[kFeatures];
-    load_row(a.grad, row, live, grad);
     if (chained)
     {
-        load_row(a.grad_v, row, live, values);
-        store_tile_row(tile, values);
+        at.store_tile(tile, values);
+        const float zeros[kHalf] = {};
+        at.store(a.grad_v, zeros);
         ok = cores.run(0, tile, image_at, 1);
         if (ok)
         {
-            load_row_tmem(cores.tmem, values);
+            at.load_product(cores, values);
 #pragma unroll
-            for (int k = 0; k < kFeatures; ++k)
+            for (int k = 0; k < kHalf; ++k)
             {
                 grad[k] += values[k];
             }
-            if (live)
-            {
-                store_row(a.grad, row, grad);
-            }
+            at.store(a.grad, grad);
         }
     }
     if (ok)
     {
-        store_tile_row(tile, grad);
+        at.store_tile(tile, grad);
         ok = cores.run(0, tile, image_d2t, 2);
     }
     if (ok)
     {
-        float h[kFeatures];
-        load_row(a.h, row, live, h);
-        load_row_tmem(cores.tmem, values);
+        at.load_product(cores, values);
 #pragma unroll
-        for (int k = 0; k < kFeatures; ++k)
+        for (int k = 0; k < kHalf; ++k)
         {
             values[k] *= sigmoid(h[k]);
         }
-        store_tile_row(tile, values);
+        at.store_tile(tile, values);
         ok = cores.run(0, tile, image_d1t, 3);
     }
     if (ok)
     {
-        load_row_tmem(cores.tmem, values);
-        if (live)
-        {
-            store_row_bf16(a.grad_m, row, values);
-        }
+        at.load_product(cores, values);
+        at.store_bf16(a.grad_m, values);
     }
     cores.close(64);
 }
 
-// E and W from the per-CTA partials in a fixed order; the status word out.
-__global__ void finalize_kernel(const double* __restrict__ energy_partials, int energy_count,
-                                const double* __restrict__ virial_partials, int virial_count,
-                                double* energy, double* virial)
+// E and W from the per-CTA partials in a fixed order: a warp per sum.
+constexpr int kFinalizeWarps = 10;
+
+__global__ void __launch_bounds__(kFinalizeWarps * 32) finalize_kernel(
+    const double* __restrict__ energy_partials, int energy_count,
+    const double* __restrict__ virial_partials, int virial_count, double* energy, double* virial)
 {
-    __shared__ double sums[10][8];
     const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x / 32;
-    double e = 0.0;
-    for (int i = threadIdx.x; i < energy_count; i += blockDim.x)
+    const int sum = threadIdx.x / 32;  // 0: E, 1 + c: component c of W
+    const double* from = sum == 0 ? energy_partials : virial_partials + (sum - 1);
+    const int count = sum == 0 ? energy_count : virial_count, stride = sum == 0 ? 1 : 9;
+    double value = 0.0;
+#pragma unroll 8
+    for (int i = lane; i < count; i += 32)
     {
-        e += energy_partials[i];
+        value += from[static_cast<std::int64_t>(stride) * i];
     }
-    e = warp_sum(e);
-    if (lane == 0)
+    value = warp_sum(value);
+    double* to = sum == 0 ? energy : (virial != nullptr ? virial + (sum - 1) : nullptr);
+    if (lane == 0 && to != nullptr)
     {
-        sums[0][warp] = e;
-    }
-    for (int c = 0; c < 9; ++c)
-    {
-        double s = 0.0;
-        for (int i = threadIdx.x; i < virial_count; i += blockDim.x)
-        {
-            s += virial_partials[9 * i + c];
-        }
-        s = warp_sum(s);
-        if (lane == 0)
-        {
-            sums[1 + c][warp] = s;
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < 10)
-    {
-        double total = 0.0;
-        for (int w = 0; w < 8; ++w)
-        {
-            total += sums[threadIdx.x][w];
-        }
-        if (threadIdx.x == 0)
-        {
-            if (energy != nullptr)
-            {
-                energy[0] = total;
-            }
-        }
-        else if (virial != nullptr)
-        {
-            virial[threadIdx.x - 1] = total;
-        }
+        *to = value;
     }
 }
 
@@ -1121,10 +1149,6 @@ int nd_schnet_energy_force_virial(const nd_schnet_args* args, nd_stream_t stream
     const int last_grid = std::min(kVirialSlots, pair_grid(reinterpret_cast<const void*>(pair_reverse_kernel<true>), kPairReverseShared, 128));
 
     ND_CUDA_TRY(cudaMemsetAsync(counters, 0, 256, stream));
-    if (s.forces != nullptr)
-    {
-        ND_CUDA_TRY(cudaMemsetAsync(s.forces, 0, s.num_atoms * 3 * sizeof(float), stream));
-    }
     if (s.num_columns > 0)
     {
         const unsigned column_blocks = blocks_for(s.num_columns);
@@ -1145,7 +1169,9 @@ int nd_schnet_energy_force_virial(const nd_schnet_args* args, nd_stream_t stream
     }
     embed_kernel<<<blocks_for(s.num_atoms * 16), kThreads, 0, stream>>>(
         s.atom_types, s.num_atoms, reinterpret_cast<const float*>(weights + wl.tables),
-        reinterpret_cast<const float*>(weights + wl.tables + s.num_types * kFeatures * 4), x, v(0));
+        reinterpret_cast<const float*>(weights + wl.tables + s.num_types * kFeatures * 4), x, v(0),
+        reinterpret_cast<float4*>(m(0)), s.interactions, row_bytes / 16,
+        reverse ? reinterpret_cast<float4*>(grad_v) : nullptr, s.forces);
     ND_LAUNCH_CHECK();
 
     PairPass pass{};
@@ -1159,7 +1185,6 @@ int nd_schnet_energy_force_virial(const nd_schnet_args* args, nd_stream_t stream
     for (int b = 0; b < s.interactions; ++b)
     {
         const bool last = b == s.interactions - 1;
-        ND_CUDA_TRY(cudaMemsetAsync(m(b), 0, s.num_atoms * kFeatures * 4, stream));
         pass.images = block_images(b);
         pass.b1 = block_vector(b, 0);
         pass.b2 = block_vector(b, 1);
@@ -1183,17 +1208,16 @@ int nd_schnet_energy_force_virial(const nd_schnet_args* args, nd_stream_t stream
         atoms.counters = counters;
         if (last)
         {
-            atom_forward_kernel<true><<<atom_tiles, kTile, kAtomShared, stream>>>(atoms);
+            atom_forward_kernel<true><<<atom_tiles, kAtomThreads, kAtomShared, stream>>>(atoms);
         }
         else
         {
-            atom_forward_kernel<false><<<atom_tiles, kTile, kAtomShared, stream>>>(atoms);
+            atom_forward_kernel<false><<<atom_tiles, kAtomThreads, kAtomShared, stream>>>(atoms);
         }
         ND_LAUNCH_CHECK();
     }
     if (reverse)
     {
-        ND_CUDA_TRY(cudaMemsetAsync(virial_partials, 0, kVirialSlots * 9 * sizeof(double), stream));
         for (int b = s.interactions - 1; b >= 0; --b)
         {
             const bool last = b == s.interactions - 1;
@@ -1206,12 +1230,8 @@ int nd_schnet_energy_force_virial(const nd_schnet_args* args, nd_stream_t stream
             atoms.grad_v = last ? nullptr : grad_v;
             atoms.grad_m = grad_m;
             atoms.counters = counters;
-            atom_reverse_kernel<<<atom_tiles, kTile, kAtomShared, stream>>>(atoms);
+            atom_reverse_kernel<<<atom_tiles, kAtomThreads, kAtomShared, stream>>>(atoms);
             ND_LAUNCH_CHECK();
-            if (b > 0)
-            {
-                ND_CUDA_TRY(cudaMemsetAsync(grad_v, 0, s.num_atoms * kFeatures * 4, stream));
-            }
             pass.images = block_images(b);
             pass.b1 = block_vector(b, 0);
             pass.b2 = block_vector(b, 1);
@@ -1233,7 +1253,7 @@ int nd_schnet_energy_force_virial(const nd_schnet_args* args, nd_stream_t stream
             ND_LAUNCH_CHECK();
         }
     }
-    finalize_kernel<<<1, 256, 0, stream>>>(energy_partials, atom_tiles, virial_partials,
+    finalize_kernel<<<1, kFinalizeWarps * 32, 0, stream>>>(energy_partials, atom_tiles, virial_partials,
                                            reverse ? last_grid : 0, s.energy,
                                            reverse ? s.virial : nullptr);
     ND_LAUNCH_CHECK();
