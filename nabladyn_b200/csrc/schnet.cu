@@ -273,7 +273,6 @@ struct PairShared
     float* envelope;  // reverse
     float* along;     // reverse
     std::uint64_t* barrier;
-    std::uint32_t* slot;
 
     __device__ PairShared(unsigned char* shared, bool reverse)
     {
@@ -288,13 +287,10 @@ struct PairShared
         envelope = reinterpret_cast<float*>(second + kTile);
         along = envelope + kTile;
         barrier = reinterpret_cast<std::uint64_t*>(along + kTile);
-        slot = reinterpret_cast<std::uint32_t*>(barrier + 1);
     }
 
-    __device__ void load(const PairPass& a)
+    __device__ void load_biases(const PairPass& a)
     {
-        copy_bytes(image_b1, a.images + kB1 * umma::kImageBytes, umma::kImageBytes);
-        copy_bytes(image_b2, a.images + kB2 * umma::kImageBytes, umma::kImageBytes);
         if (threadIdx.x < kFeatures)
         {
             bias1[threadIdx.x] = a.b1[threadIdx.x];
@@ -332,9 +328,11 @@ __global__ void __launch_bounds__(kTile, 6) pair_forward_kernel(PairPass a)
 {
     extern __shared__ __align__(1024) unsigned char shared[];
     PairShared sh(shared, false);
-    sh.load(a);
+    sh.load_biases(a);
     Cores cores;
-    cores.open(sh.barrier, sh.slot, 64, a.counters, 1);
+    cores.open(sh.barrier, 64, a.counters, 1,
+               {{sh.image_b1, a.images + kB1 * umma::kImageBytes},
+                {sh.image_b2, a.images + kB2 * umma::kImageBytes}});
     const int count = *reinterpret_cast<volatile int*>(a.counters);
     const auto* v = reinterpret_cast<const uint2*>(a.v);
     float4* const m4 = reinterpret_cast<float4*>(a.m);
@@ -438,10 +436,12 @@ __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
 {
     extern __shared__ __align__(1024) unsigned char shared[];
     PairShared sh(shared, true);
-    sh.load(a);
+    sh.load_biases(a);
     // Columns 0-63 keep z1 - b1 for the whole tile; 64-127 take the other products in turn.
     Cores cores;
-    cores.open(sh.barrier, sh.slot, 128, a.counters, 2);
+    cores.open(sh.barrier, 128, a.counters, 2,
+               {{sh.image_b1, a.images + kB1 * umma::kImageBytes},
+                {sh.image_b2, a.images + kB2 * umma::kImageBytes}});
     const int count = *reinterpret_cast<volatile int*>(a.counters);
     const auto* v = reinterpret_cast<const uint2*>(a.v);
     const auto* gm = reinterpret_cast<const uint2*>(a.grad_m);
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
                 {
-                    umma::mma(*sh.slot + column,
+                    umma::mma(*cores.slot + column,
                               umma::matrix_descriptor(tile + 2 * kReverseChunk * k, kReverseChunk,
                                                       kReverseGroup),
                               transposed ? umma::matrix_descriptor(b + 2048 * k, 1024, 128)
@@ -875,19 +875,12 @@ __global__ void __launch_bounds__(kAtomThreads) atom_forward_kernel(AtomPass a)
     float* bias1 = readout + kReadoutFloats;
     float* bias2 = bias1 + kFeatures;
     auto* barrier = reinterpret_cast<std::uint64_t*>(bias2 + kFeatures);
-    auto* slot = reinterpret_cast<std::uint32_t*>(barrier + 1);
 
     const AtomRow at(a.atoms);
     float values[kHalf], x[kHalf];
     at.load(a.m, values);
     at.load(a.x, x);
-    copy_bytes(image_d1, a.images + kD1 * umma::kImageBytes, umma::kImageBytes);
-    copy_bytes(image_d2, a.images + kD2 * umma::kImageBytes, umma::kImageBytes);
-    if (!kLast)
-    {
-        copy_bytes(image_a, a.next_images + kA * umma::kImageBytes, umma::kImageBytes);
-    }
-    else
+    if (kLast)
     {
         for (int i = threadIdx.x; i < kReadoutFloats; i += kAtomThreads)
         {
@@ -900,7 +893,17 @@ __global__ void __launch_bounds__(kAtomThreads) atom_forward_kernel(AtomPass a)
         bias2[threadIdx.x] = a.d2[threadIdx.x];
     }
     Cores cores;
-    cores.open(barrier, slot, 64, a.counters, 3);
+    const ImageCopy d1{image_d1, a.images + kD1 * umma::kImageBytes};
+    const ImageCopy d2{image_d2, a.images + kD2 * umma::kImageBytes};
+    if constexpr (kLast)
+    {
+        cores.open(barrier, 64, a.counters, 3, {d1, d2});
+    }
+    else
+    {
+        cores.open(barrier, 64, a.counters, 3,
+                   {d1, d2, {image_a, a.next_images + kA * umma::kImageBytes}});
+    }
     cores.tile_index = blockIdx.x;
     double energy = 0.0;
     at.store_tile(tile, values);
@@ -975,7 +978,6 @@ __global__ void __launch_bounds__(kAtomThreads) atom_reverse_kernel(AtomPass a)
     unsigned char* image_at = image_d1t + umma::kImageBytes;
     unsigned char* tile = image_at + umma::kImageBytes;
     auto* barrier = reinterpret_cast<std::uint64_t*>(tile + umma::kTileBytes);
-    auto* slot = reinterpret_cast<std::uint32_t*>(barrier + 1);
 
     const bool chained = a.grad_v != nullptr;
     const AtomRow at(a.atoms);
@@ -986,14 +988,18 @@ __global__ void __launch_bounds__(kAtomThreads) atom_reverse_kernel(AtomPass a)
     {
         at.load(a.grad_v, values);
     }
-    copy_bytes(image_d2t, a.images + kD2T * umma::kImageBytes, umma::kImageBytes);
-    copy_bytes(image_d1t, a.images + kD1T * umma::kImageBytes, umma::kImageBytes);
+    Cores cores;
+    const ImageCopy d2t{image_d2t, a.images + kD2T * umma::kImageBytes};
+    const ImageCopy d1t{image_d1t, a.images + kD1T * umma::kImageBytes};
     if (chained)
     {
-        copy_bytes(image_at, a.next_images + kAT * umma::kImageBytes, umma::kImageBytes);
+        cores.open(barrier, 64, a.counters, 4,
+                   {d2t, d1t, {image_at, a.next_images + kAT * umma::kImageBytes}});
     }
-    Cores cores;
-    cores.open(barrier, slot, 64, a.counters, 4);
+    else
+    {
+        cores.open(barrier, 64, a.counters, 4, {d2t, d1t});
+    }
     cores.tile_index = blockIdx.x;
     bool ok = true;
     if (chained)

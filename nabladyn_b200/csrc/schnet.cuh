@@ -169,35 +169,45 @@ __device__ __forceinline__ std::uint32_t pack2(float lo, float hi)
     return *reinterpret_cast<std::uint32_t*>(&pair);
 }
 
-// Shared-memory staging of weight images and bias vectors, by all threads.
-__device__ __forceinline__ void copy_bytes(unsigned char* to, const unsigned char* from, int bytes)
+// One weight image of a CTA: where it goes in shared memory and where it comes from.
+struct ImageCopy
 {
-    for (int i = threadIdx.x * 16; i < bytes; i += blockDim.x * 16)
-    {
-        *reinterpret_cast<uint4*>(to + i) = __ldg(reinterpret_cast<const uint4*>(from + i));
-    }
-}
+    unsigned char* to;
+    const unsigned char* from;
+};
 
-// The per-CTA tensor-core context: tensor memory, the completion barrier and its phase.
+// The per-CTA tensor-core context: tensor memory, the completion barrier and its phase, and the
+// weight images, which copies of the bulk engine bring in behind whatever precedes the first
+// product.
 struct Cores
 {
-    std::uint64_t* barrier;
+    std::uint64_t* barrier;  // [3]: products; the slot; the images' copies
     std::uint32_t* slot;
     std::uint32_t tmem;  // this warp's lanes, column 0
     unsigned phase;
+    bool images_pending;  // thread 0: the first product waits for the images
 
-    __device__ void open(std::uint64_t* barrier_, std::uint32_t* slot_, std::uint32_t columns,
-                         int* counters_, int stage_)
+    template <int kImages>
+    __device__ void open(std::uint64_t* barrier_, std::uint32_t columns, int* counters_,
+                         int stage_, const ImageCopy (&images)[kImages])
     {
         barrier = barrier_;
-        slot = slot_;
+        slot = reinterpret_cast<std::uint32_t*>(barrier + 1);
         phase = 0;
         counters = counters_;
         stage = stage_;
         tile_index = -1;
+        images_pending = true;
         if (threadIdx.x == 0)
         {
             umma::barrier_init(barrier);
+            umma::barrier_init(barrier + 2);
+            umma::expect_bytes(barrier + 2, kImages * umma::kImageBytes);
+#pragma unroll
+            for (int k = 0; k < kImages; ++k)
+            {
+                umma::bulk_load(images[k].to, images[k].from, umma::kImageBytes, barrier + 2);
+            }
         }
         if (threadIdx.x < 32)
         {
@@ -257,6 +267,11 @@ struct Cores
         if (threadIdx.x == 0)
         {
             umma::fence_after_sync();
+            if (images_pending && !umma::barrier_wait(barrier + 2, 0))
+            {
+                atomicOr(counters + 1, kProductLost);
+            }
+            images_pending = false;
             products();
             umma::commit(barrier);
         }
@@ -282,6 +297,10 @@ struct Cores
 
     __device__ void close(std::uint32_t columns)
     {
+        if (threadIdx.x == 0 && images_pending)
+        {
+            umma::barrier_wait(barrier + 2, 0);  // no product ran: the copies may be in flight
+        }
         umma::fence_before_sync();
         __syncthreads();
         if (threadIdx.x < 32)

@@ -193,11 +193,8 @@ __global__ void __launch_bounds__(kTile, 4) tangent_forward_kernel(TangentPass a
     int* first = reinterpret_cast<int*>(bias2 + kFeatures);
     int* second = first + kTile;
     auto* barrier = reinterpret_cast<std::uint64_t*>(second + kTile);
-    auto* slot = reinterpret_cast<std::uint32_t*>(barrier + 1);
     __shared__ float wbar[9];
 
-    copy_bytes(image_b1, a.images + kB1 * umma::kImageBytes, umma::kImageBytes);
-    copy_bytes(image_b2, a.images + kB2 * umma::kImageBytes, umma::kImageBytes);
     if (threadIdx.x < kFeatures)
     {
         bias1[threadIdx.x] = a.b1[threadIdx.x];
@@ -209,7 +206,9 @@ __global__ void __launch_bounds__(kTile, 4) tangent_forward_kernel(TangentPass a
     }
     // Columns 0-63: z, then u; 64-127: z_dot, then u_dot.
     Cores cores;
-    cores.open(barrier, slot, 128, a.counters, 5);
+    cores.open(barrier, 128, a.counters, 5,
+               {{image_b1, a.images + kB1 * umma::kImageBytes},
+                {image_b2, a.images + kB2 * umma::kImageBytes}});
     const int count = *reinterpret_cast<volatile int*>(a.counters);
     const auto* v = reinterpret_cast<const uint2*>(a.v);
     const auto* v_dot = reinterpret_cast<const uint2*>(a.v_dot);
@@ -335,10 +334,7 @@ __global__ void __launch_bounds__(kReverseThreads, 2) tangent_reverse_kernel(Tan
     float* scales = offsets + kTile;   // -rdot / D
     float* wbar = scales + kTile;
     auto* barrier = reinterpret_cast<std::uint64_t*>(wbar + 10);
-    auto* slot = reinterpret_cast<std::uint32_t*>(barrier + 1);
 
-    copy_bytes(image_b1, a.images + kB1 * umma::kImageBytes, umma::kImageBytes);
-    copy_bytes(image_b2, a.images + kB2 * umma::kImageBytes, umma::kImageBytes);
     if (threadIdx.x < kFeatures)
     {
         bias1[threadIdx.x] = a.b1[threadIdx.x];
@@ -351,8 +347,10 @@ __global__ void __launch_bounds__(kReverseThreads, 2) tangent_reverse_kernel(Tan
     // Columns 0-63 keep z - b1 and 64-127 z_dot for the whole tile; 128-191 take u, then s_bar;
     // 192-255 u_dot, then s_dot_bar.
     Cores cores;
-    cores.open(barrier, slot, 256, a.counters, 6);
-    const std::uint32_t tmem = *slot;
+    cores.open(barrier, 256, a.counters, 6,
+               {{image_b1, a.images + kB1 * umma::kImageBytes},
+                {image_b2, a.images + kB2 * umma::kImageBytes}});
+    const std::uint32_t tmem = *cores.slot;
     const int count = *reinterpret_cast<volatile int*>(a.counters);
     const auto* v = reinterpret_cast<const uint2*>(a.v);
     const auto* v_dot = reinterpret_cast<const uint2*>(a.v_dot);

@@ -27,6 +27,7 @@ constexpr int kCols = 64;           // N and K of every product
 constexpr int kImageBytes = 64 * 64 * 2;   // one 64 x 64 BF16 weight image
 constexpr int kTileBytes = 128 * 64 * 2;   // one 128 x 64 BF16 row tile
 constexpr int kWaitLimit = 1 << 22;        // mbarrier polls before a product counts as lost
+constexpr int kFreePolls = 64;             // polls before the clock is read
 constexpr std::uint64_t kWaitNanoseconds = 500000000;  // and at most 0.5 s of waiting
 
 // Byte offset of element (row, k) in an operand image.
@@ -228,9 +229,18 @@ __device__ __forceinline__ std::uint64_t nanoseconds()
 }
 
 // Waits for `phase` of the barrier, at most kWaitLimit polls and kWaitNanoseconds (a poll
-// may suspend the thread for a while); false when it gave up.
+// may suspend the thread for a while); false when it gave up. The clock is read only once the
+// first polls have failed: reading it takes longer than most products.
 __device__ __forceinline__ bool barrier_wait(std::uint64_t* barrier, unsigned phase)
 {
+#pragma unroll 1
+    for (int poll = 0; poll < kFreePolls; ++poll)
+    {
+        if (barrier_test(barrier, phase))
+        {
+            return true;
+        }
+    }
     const std::uint64_t start = nanoseconds();
     for (int poll = 0; poll < kWaitLimit; ++poll)
     {
@@ -244,6 +254,27 @@ __device__ __forceinline__ bool barrier_wait(std::uint64_t* barrier, unsigned ph
         }
     }
     return false;
+}
+
+// Adds one arrival and `bytes` of expected copies to the barrier's phase, and a copy from
+// global to shared memory that counts on it (16-byte aligned addresses and sizes, this GPU's
+// memory, this CTA only).
+__device__ __forceinline__ void expect_bytes(std::uint64_t* barrier, std::uint32_t bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
+                     smem_address(barrier)),
+                 "r"(bytes)
+                 : "memory");
+}
+
+__device__ __forceinline__ void bulk_load(void* to, const void* from, std::uint32_t bytes,
+                                          std::uint64_t* barrier)
+{
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
+            "r"(smem_address(to)),
+        "l"(from), "r"(bytes), "r"(smem_address(barrier))
+        : "memory");
 }
 
 // Eight floats as eight BF16 (round to nearest even) in one 16-byte word.
