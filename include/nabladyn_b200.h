@@ -216,6 +216,32 @@ int nd_wrap(int dtype, const void* positions, const void* cells, int64_t frames,
  * double backward). */
 int nd_lj_batch_parameter_backward(const nd_lj_batch_args* args, nd_stream_t stream);
 
+/* The training loss of a batch, L = sum_c w_c t_c with t_c = sum_f k_f mean_i ((X - Y) / s_c)^2
+ * (src/nabladyn/training/_loss.py:105-125), and its gradient in the predictions X: the forward
+ * call writes the slopes dt_c/dX where `gradients` is given, the backward call takes them as
+ * `predicted` and writes dL/dX. Predictions, labels, coefficients, outputs and incoming
+ * gradients are values of `dtype`. */
+typedef struct nd_loss_args {
+    int dtype;
+    int32_t channels;             /* 1 to 3 */
+    int64_t frames;               /* F */
+    const void* predicted[3];     /* [F, sizes] each */
+    const void* labels[3];
+    int64_t sizes[3];             /* components per frame */
+    double weights[3];
+    double scales[3];
+    const void* coefficients;     /* k [F]; NULL: 1/F */
+    double* scratch;              /* forward: [4] */
+    void* total;                  /* forward: [1] L */
+    void* terms[3];               /* forward: [1] t_c each */
+    const void* total_grad;       /* backward: [1] or NULL (zero) */
+    const void* term_grads[3];    /* backward: [1] each or NULL (zero) */
+    void* gradients[3];           /* [F, sizes] each, or NULL where not wanted */
+} nd_loss_args;
+
+int nd_loss_forward(const nd_loss_args* args, nd_stream_t stream);
+int nd_loss_backward(const nd_loss_args* args, nd_stream_t stream);
+
 /* ------------------------------------------------------------------------------------------
  * The MD engine: velocity-Verlet (NVE) and Nose-Hoover chain (NVT) steps of a Lennard-Jones
  * system with the neighbor rebuild decided on the GPU.

@@ -114,6 +114,26 @@ class LJBatchArgs(ctypes.Structure):
     ]
 
 
+class LossArgs(ctypes.Structure):
+    _fields_ = [
+        ("dtype", ctypes.c_int),
+        ("channels", ctypes.c_int32),
+        ("frames", ctypes.c_int64),
+        ("predicted", ctypes.c_void_p * 3),
+        ("labels", ctypes.c_void_p * 3),
+        ("sizes", ctypes.c_int64 * 3),
+        ("weights", ctypes.c_double * 3),
+        ("scales", ctypes.c_double * 3),
+        ("coefficients", ctypes.c_void_p),
+        ("scratch", ctypes.c_void_p),
+        ("total", ctypes.c_void_p),
+        ("terms", ctypes.c_void_p * 3),
+        ("total_grad", ctypes.c_void_p),
+        ("term_grads", ctypes.c_void_p * 3),
+        ("gradients", ctypes.c_void_p * 3),
+    ]
+
+
 class MDSystem(ctypes.Structure):
     _fields_ = [
         ("dtype", ctypes.c_int),
@@ -319,6 +339,8 @@ _SIGNATURES = {
                      ctypes.c_void_p],
     "nd_lj_frames_parameter_backward": [ctypes.POINTER(LJBatchArgs), ctypes.c_void_p,
                                         ctypes.c_void_p],
+    "nd_loss_forward": [ctypes.POINTER(LossArgs), ctypes.c_void_p],
+    "nd_loss_backward": [ctypes.POINTER(LossArgs), ctypes.c_void_p],
     "nd_wrap": [ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64,
                 ctypes.c_void_p, ctypes.c_void_p],
     "nd_md_import": [

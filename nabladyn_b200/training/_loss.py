@@ -1,12 +1,19 @@
 """The supervised loss: scaled errors of predicted energies, forces and virials.
 
-The same scales and loss as src/nabladyn/training/_loss.py:26-46 and :105-125.
+The same scales and loss as src/nabladyn/training/_loss.py:26-46 and :105-125. On a GPU the
+loss of plain tensors and its first derivatives take one kernel each (nd_loss_forward,
+nd_loss_backward); anything else, such as a functorch transform, tensor weights or a second
+derivative, is computed by the torch operations that define it.
 """
 
+import ctypes
 from collections.abc import Mapping
 
 import torch
 from torch import Tensor
+from torch.autograd import forward_ad
+
+from .._native import LossArgs, call, dtype_code, on_device, ptr, stream_handle
 
 CHANNELS = ("energy", "forces", "virial")
 
@@ -36,12 +43,131 @@ def loss(predicted: Mapping[str, Tensor], labels: Mapping[str, Tensor],
     A channel's term is each frame's mean of ((X - X*) / s_X)^2 over its components, times the
     frame's coefficient [B] (1/B when ``coefficients`` is None), summed over the frames.
     """
+    if _one_kernel(predicted, labels, weights, scales, coefficients):
+        names = tuple(predicted)
+        total, *terms = _Loss.apply(
+            tuple(float(weights[name]) for name in names),
+            tuple(float(scales[name]) for name in names), coefficients,
+            *(labels[name] for name in names), *(predicted[name] for name in names))
+        return total, dict(zip(names, terms))
+    return _defined(predicted, labels, weights, scales, coefficients)
+
+
+def _defined(predicted, labels, weights, scales, coefficients):
+    """The loss by torch operations."""
     terms = {}
     for name, value in predicted.items():
         squares = ((value - labels[name]) / scales[name]).square()
         per_frame = squares.reshape(squares.shape[0], -1).mean(dim=1)
         terms[name] = per_frame.mean() if coefficients is None else (coefficients * per_frame).sum()
     return sum(weights[name] * term for name, term in terms.items()), terms
+
+
+def _one_kernel(predicted, labels, weights, scales, coefficients) -> bool:
+    """Whether the loss is one of plain CUDA tensors with number weights and scales, outside
+    every functorch transform, forward-mode level and trace."""
+    if (not 1 <= len(predicted) <= 3 or torch._C._are_functorch_transforms_active()
+            or forward_ad._current_level >= 0 or torch.compiler.is_compiling()
+            or torch.jit.is_tracing()):
+        return False
+    first = next(iter(predicted.values()))
+    if (not isinstance(first, Tensor) or not first.is_cuda or first.ndim == 0
+            or first.dtype not in (torch.float32, torch.float64) or first.shape[0] == 0):
+        return False
+    frames = first.shape[0]
+
+    def plain(x, shape) -> bool:
+        return (type(x) in (Tensor, torch.nn.Parameter) and x.layout is torch.strided
+                and x.dtype == first.dtype and x.device == first.device and x.shape == shape)
+
+    for name, value in predicted.items():
+        label, weight, scale = labels[name], weights[name], scales[name]
+        if (not isinstance(weight, (int, float)) or not isinstance(scale, (int, float))
+                or not isinstance(label, Tensor) or label.requires_grad or not plain(value, label.shape)
+                or not plain(label, value.shape) or value.ndim == 0 or value.shape[0] != frames
+                or value.numel() == 0):
+            return False
+    return coefficients is None or (isinstance(coefficients, Tensor)
+                                    and not coefficients.requires_grad
+                                    and plain(coefficients, (frames,)))
+
+
+class _Loss(torch.autograd.Function):
+    """(L, t_c for every channel) of predictions, differentiable in the predictions.
+
+    The forward keeps the terms' slopes dt_c/dX, so the backward needs neither predictions nor
+    labels; those are saved for a second derivative alone.
+    """
+
+    @staticmethod
+    def forward(ctx, weights, scales, coefficients, *tensors):
+        count = len(weights)
+        labels, predicted = tensors[:count], tensors[count:]
+        like = predicted[0]
+        total, *terms = (torch.empty((), dtype=like.dtype, device=like.device)
+                         for _ in range(1 + count))
+        wanted = ctx.needs_input_grad[3 + count:]
+        slopes = [torch.empty(value.shape, dtype=like.dtype, device=like.device) if want else None
+                  for value, want in zip(predicted, wanted)]
+        scratch = torch.empty(4, dtype=torch.float64, device=like.device)
+        kept = [value.contiguous() for value in (*predicted, *labels)]  # until the launch
+        shares = None if coefficients is None else coefficients.contiguous()
+        args = _loss_args(weights, kept[:count])
+        args.coefficients, args.scratch, args.total = ptr(shares), ptr(scratch), ptr(total)
+        for c, term in enumerate(terms):
+            args.labels[c], args.scales[c] = ptr(kept[count + c]), scales[c]
+            args.terms[c], args.gradients[c] = ptr(term), ptr(slopes[c])
+        with on_device(like.device):
+            call("nd_loss_forward", ctypes.byref(args), stream_handle(like.device))
+        ctx.weights, ctx.scales, ctx.slopes = weights, scales, slopes
+        ctx.has_coefficients = coefficients is not None
+        if any(wanted):
+            ctx.save_for_backward(*((coefficients,) if ctx.has_coefficients else ()), *tensors)
+        return total, *terms
+
+    @staticmethod
+    def backward(ctx, total_grad, *term_grads):
+        count = len(ctx.weights)
+        if torch.is_grad_enabled():  # a graph of this backward is asked for
+            gradients = _defined_backward(ctx, total_grad, term_grads)
+        else:
+            slopes = ctx.slopes
+            gradients = [None if slope is None else torch.empty_like(slope) for slope in slopes]
+            like = next(slope for slope in slopes if slope is not None)
+            args = _loss_args(ctx.weights, [like if s is None else s for s in slopes])
+            args.total_grad = ptr(total_grad)
+            for c, gradient in enumerate(gradients):
+                args.term_grads[c], args.gradients[c] = ptr(term_grads[c]), ptr(gradient)
+            with on_device(like.device):
+                call("nd_loss_backward", ctypes.byref(args), stream_handle(like.device))
+        return (None, None, None, *(None,) * count, *gradients)
+
+
+def _defined_backward(ctx, total_grad, term_grads):
+    """The first derivatives by torch operations, differentiable themselves."""
+    saved, count = ctx.saved_tensors, len(ctx.weights)
+    coefficients, saved = (saved[0], saved[1:]) if ctx.has_coefficients else (None, saved)
+    gradients = []
+    for c, (label, value) in enumerate(zip(saved[:count], saved[count:])):
+        if ctx.slopes[c] is None:
+            gradients.append(None)
+            continue
+        frames, size = value.shape[0], value.numel() // value.shape[0]
+        share = value.new_full((frames,), 1.0 / frames) if coefficients is None else coefficients
+        share = share.reshape(frames, *(1,) * (value.ndim - 1))
+        factor = total_grad * ctx.weights[c] + term_grads[c]
+        gradients.append(factor * share * 2.0 * (value - label) / (size * ctx.scales[c] ** 2))
+    return gradients
+
+
+def _loss_args(weights, channels) -> LossArgs:
+    """The arguments of one tensor [F, ...] per channel."""
+    args = LossArgs(dtype=dtype_code(channels[0].dtype), channels=len(weights),
+                    frames=channels[0].shape[0])
+    for c, value in enumerate(channels):
+        args.predicted[c], args.sizes[c] = ptr(value), value.numel() // value.shape[0]
+        args.weights[c] = weights[c]
+    return args
 
 
 __all__ = ("CHANNELS", "scales", "loss")
