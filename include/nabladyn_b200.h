@@ -94,6 +94,17 @@ int nd_neighbors_count_first_frame(int dtype, const void* positions, const void*
                                    int64_t num_atoms, double radius,
                                    const nd_neighbor_buffers* buffers, nd_stream_t stream);
 
+/* The starting values of a new list, before nd_neighbors_count_first_frame: the frame wrapped
+ * into [0, L) into reuse->reference_positions (positions may lie anywhere), the cell, the grid
+ * (`dims` bins per axis, host values, of width L / n), its limits, zero bin counts, total,
+ * status and reuse words, no rebuild asked for and one made. `non_finite` [1] becomes 1 when a
+ * coordinate is not finite, else 0. The buffers' pairs, scratch and per-atom arrays are not
+ * touched and may be NULL. */
+int nd_neighbors_start(int dtype, const void* positions, const void* cell, int64_t num_atoms,
+                       const int32_t* dims, const nd_reuse_buffers* reuse,
+                       const nd_neighbor_buffers* buffers, int32_t* non_finite,
+                       nd_stream_t stream);
+
 /* fill_first_frame(positions, cell, radius, <15 buffers>)
  * (src/nabladyn/neighbors/csrc/runtime/entry_points.cu:354-399): the pairs, into the capacity
  * the host chose, then the total, the overflow check and the padding. */

@@ -314,6 +314,11 @@ class Integrator(ctypes.Structure):
 _SIGNATURES = {
     "nd_abi_version": [],
     "nd_neighbors_scan_temp_bytes": [ctypes.c_int64, c_int64_p],
+    "nd_neighbors_start": [
+        ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p,
+        ctypes.POINTER(ReuseBuffers), ctypes.POINTER(NeighborBuffers), ctypes.c_void_p,
+        ctypes.c_void_p,
+    ],
     "nd_neighbors_count_first_frame": [
         ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_double,
         ctypes.POINTER(NeighborBuffers), ctypes.c_void_p,

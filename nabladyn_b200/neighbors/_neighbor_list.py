@@ -8,13 +8,14 @@ grid rule, inner lists, and the exceptions with their messages. The device work 
 kernels in libnabladyn_b200.so), so the same buffers in the same order cross that boundary.
 
 How this class keeps them is its own: one ``_DeviceList`` owns every tensor of a list (the 15
-schema buffers and the update's 6), built from a size plan; the pair count of a first frame is
+schema buffers and the update's 6), given their starting values by one kernel; the pair count of a first frame is
 read as one (offset, count) pair of the last atom instead of a sum over all atoms; the status
 word is decoded by one function shared with the MD engines.
 """
 
 from __future__ import annotations
 
+import ctypes
 import math
 from numbers import Real
 
@@ -22,7 +23,8 @@ import torch
 from torch import Tensor
 
 from .. import space
-from .._native import INVALID_CELL, NON_FINITE, OVERFLOW, neighbor_ops
+from .._native import (INVALID_CELL, NON_FINITE, OVERFLOW, NeighborBuffers, ReuseBuffers, call,
+                       dtype_code, neighbor_ops, on_device, ptr, stream_handle)
 from ._pairs import NeighborPairs
 
 _INT32_MAX = 2**31 - 1
@@ -103,40 +105,58 @@ def _validate_frame(positions: Tensor, cell: Tensor) -> None:
 
 
 class _DeviceList:
-    """Every device tensor of one list, created from its size plan.
+    """Every device tensor of one list, created for its first frame.
 
-    ``build_args()`` and ``update_args()`` give them in the schemas' orders. The pairs start as
-    [2, 1] and are replaced once the first frame is counted; all-pairs lists (a first grid of
-    at most three bins per axis) carry an N x ceil(N / 32) word matrix, others an empty one.
+    ``build_args()`` and ``update_args()`` give them in the schemas' orders. One kernel wraps the
+    frame into ``reference_positions`` and writes the starting values (nd_neighbors_start); its
+    verdict on the coordinates lands in ``non_finite``. The pairs start as [2, 1] and are
+    replaced once the first frame is counted; all-pairs lists (a first grid of at most three
+    bins per axis) carry an N x ceil(N / 32) word matrix, others an empty one.
     """
 
-    def __init__(self, num_atoms: int, dims: list[int], lengths: list[float], scan_bytes: int,
-                 dtype: torch.dtype, device: torch.device):
+    def __init__(self, positions: Tensor, cell: Tensor, dims: list[int], scan_bytes: int):
+        num_atoms, dtype, device = positions.shape[0], positions.dtype, positions.device
         ints = {"dtype": torch.int32, "device": device}
+        floats = {"dtype": dtype, "device": device}
         bins = math.prod(dims)
         words = num_atoms * ((num_atoms + 31) // 32) if max(dims) <= 3 else 0
-        self.tensors: dict[str, Tensor] = {
-            "dims": torch.tensor(dims, **ints),
-            "widths": torch.tensor([length / count for length, count in zip(lengths, dims)],
-                                   dtype=dtype, device=device),
+        t = self.tensors = {
+            "dims": torch.empty(3, **ints),
+            "widths": torch.empty(3, **floats),
             "atom_bin": torch.empty(num_atoms, **ints),
-            "bin_counts": torch.zeros(bins + 1, **ints),
+            "bin_counts": torch.empty(bins + 1, **ints),
             "bin_offsets": torch.empty(bins + 1, **ints),
             "unordered_ids": torch.empty(num_atoms, **ints),
             "sorted_ids": torch.empty(num_atoms, **ints),
-            "sorted_positions": torch.empty((num_atoms, 3), dtype=dtype, device=device),
+            "sorted_positions": torch.empty((num_atoms, 3), **floats),
             "scan_temp": torch.empty(scan_bytes, dtype=torch.uint8, device=device),
             "pair_counts": torch.empty(num_atoms, **ints),
             "pair_offsets": torch.empty(num_atoms, **ints),
-            "pair_total": torch.zeros(1, **ints),
-            "status": torch.zeros(2, **ints),
+            "pair_total": torch.empty(1, **ints),
+            "status": torch.empty(2, **ints),
             "pairs": torch.empty((2, 1), **ints),
-            "bits": torch.zeros(words, **ints),
-            "limits": torch.tensor(dims, **ints),
-            "reuse": torch.zeros(4, dtype=dtype, device=device),
-            "rebuild": torch.zeros(1, **ints),
-            "rebuild_count": torch.ones(1, **ints),
+            "bits": torch.empty(words, **ints),
+            "limits": torch.empty(3, **ints),
+            "reuse": torch.empty(4, **floats),
+            "rebuild": torch.empty(1, **ints),
+            "rebuild_count": torch.empty(1, **ints),
+            "reference_positions": torch.empty((num_atoms, 3), **floats),
+            "reference_cell": torch.empty(3, **floats),
         }
+        self.non_finite = torch.empty(1, **ints)
+        positions, cell = positions.detach().contiguous(), cell.detach().contiguous()
+        buffers = NeighborBuffers(
+            dims=ptr(t["dims"]), widths=ptr(t["widths"]), bin_counts=ptr(t["bin_counts"]),
+            num_bin_slots=bins + 1, pair_total=ptr(t["pair_total"]), status=ptr(t["status"]))
+        reuse = ReuseBuffers(
+            reference_positions=ptr(t["reference_positions"]),
+            reference_cell=ptr(t["reference_cell"]), limits=ptr(t["limits"]),
+            reuse=ptr(t["reuse"]), rebuild=ptr(t["rebuild"]),
+            rebuild_count=ptr(t["rebuild_count"]))
+        with on_device(device):
+            call("nd_neighbors_start", dtype_code(dtype), ptr(positions), ptr(cell), num_atoms,
+                 (ctypes.c_int32 * 3)(*dims), reuse, buffers, ptr(self.non_finite),
+                 stream_handle(device))
 
     def __getitem__(self, name: str) -> Tensor:
         return self.tensors[name]
@@ -194,21 +214,23 @@ class NeighborList:
         _validate_frame(positions, cell)
         lengths = [float(length) for length in cell.tolist()]
         check_cell_lengths(lengths, self._cutoff)
-        if not bool(torch.isfinite(positions).all()):
-            raise ValueError("positions must be finite")
         dims = grid(lengths, self.radius, positions.dtype)
         if math.prod(dims) >= _INT32_MAX:
+            if not bool(torch.isfinite(positions).all()):
+                raise ValueError("positions must be finite")
             raise ValueError("the grid must have fewer than 2**31 - 1 bins")
         ops = neighbor_ops()
         n = positions.shape[0]
-        scan_bytes = max(ops.scan_temp_bytes(positions, math.prod(dims) + 1),
-                         ops.scan_temp_bytes(positions, n))
-        device = _DeviceList(n, dims, lengths, scan_bytes, positions.dtype, positions.device)
-        frame = space.wrapped_only(positions, cell)
-        box = cell.detach().contiguous()
+        scan_bytes = ops.scan_temp_bytes(positions, max(math.prod(dims) + 1, n))
+        device = _DeviceList(positions, cell, dims, scan_bytes)
+        frame, box = device["reference_positions"], device["reference_cell"]
         ops.count_first_frame(frame, box, self.radius, *device.build_args())
-        # The pairs of the frame: the last atom's offset plus its count.
-        offset, last = torch.stack([device["pair_offsets"][-1], device["pair_counts"][-1]]).tolist()
+        # The pairs of the frame: the last atom's offset plus its count. A non-finite coordinate
+        # was counted in some bin; its frame is refused here, with the one read of the count.
+        offset, last, bad = torch.cat([device["pair_offsets"][-1:], device["pair_counts"][-1:],
+                                       device.non_finite]).tolist()
+        if bad:
+            raise ValueError("positions must be finite")
         count = offset + last
         capacity = max(8, math.ceil(self._capacity_multiplier * count))
         if capacity > _INT32_MAX:
@@ -219,8 +241,6 @@ class NeighborList:
         device.tensors["pairs"] = torch.empty((2, capacity), dtype=torch.int32,
                                               device=positions.device)
         ops.fill_first_frame(frame, box, self.radius, *device.build_args())
-        device.tensors["reference_positions"] = frame.clone()
-        device.tensors["reference_cell"] = box.clone()
         self._device = device
         # The list stays failed until its inner lists are built from the same frame.
         self._failure = "an inner list was not allocated"

@@ -47,3 +47,40 @@ def test_dense_and_short_grids_match_the_oracle(cuda, dtype, lengths, radius, ba
     listed.update(x, cell)
     assert listed._rebuild_count == 3
     np.testing.assert_array_equal(listed.tensors().index.cpu().numpy(), index)
+
+
+def test_a_frame_of_non_finite_coordinates_is_refused(cuda):
+    """Every coordinate NaN or infinite, so that all atoms would share a bin: refused, and the
+    list stays usable for the next frame."""
+    listed = NeighborList(1.0, skin=0.1)
+    cell = torch.full((3,), 20.0, device=cuda)
+    bad = torch.full((150000, 3), float("nan"), device=cuda)
+    bad[::2] = float("inf")
+    with pytest.raises(ValueError, match="positions must be finite"):
+        listed.allocate(bad, cell)
+    with pytest.raises(RuntimeError, match="allocate"):
+        listed.tensors()
+    one = 20.0 * torch.rand((1000, 3), device=cuda)
+    one[77, 1] = -float("inf")
+    with pytest.raises(ValueError, match="positions must be finite"):
+        listed.allocate(one, cell)
+    one[77, 1] = 3.0
+    listed.allocate(one, cell)
+    assert listed.num_pairs > 0
+
+
+@pytest.mark.parametrize("dtype", (torch.float32, torch.float64))
+def test_first_frame_starts_the_list(cuda, dtype):
+    """Strided positions far outside the cell: the reference frame is the wrapped one, and an
+    update with the same frame reuses its pairs."""
+    generator = torch.Generator().manual_seed(5)
+    wide = 60.0 * torch.randn((900, 3), generator=generator, dtype=torch.float64)
+    x = torch.stack([wide, wide], dim=-1).to(dtype).to(cuda)[..., 0]
+    cell = torch.tensor([9.0, 5.1, 4.7], dtype=dtype, device=cuda)
+    listed = NeighborList(1.0, skin=0.1)
+    listed.allocate(x, cell)
+    held = listed._device_tensors()
+    assert torch.equal(held["reference_positions"], space.wrap(x, cell)[0])
+    assert torch.equal(held["reference_cell"], cell) and held["limits"].tolist() == [8, 4, 4]
+    listed.update(x, cell)
+    assert listed._rebuild_count == 1
