@@ -422,6 +422,12 @@ int nd_md_graph_destroy(void* graph);
 int nd_serve_run(const nd_replica_pool* pool, const int32_t* slots, const int32_t* budgets,
                  int32_t count, int32_t mode, nd_stream_t stream);
 
+/* nd_serve_run with `team` CTAs (1, 2, 4 or 8: one thread-block cluster) per replica, of which a
+ * replica of N atoms uses at most N / 1024. A replica's results do not depend on the team. */
+int nd_serve_run_teams(const nd_replica_pool* pool, const int32_t* slots,
+                       const int32_t* budgets, int32_t count, int32_t mode, int32_t team,
+                       nd_stream_t stream);
+
 /* ---- SchNet (src/nabladyn/potential/_schnet/_potential.py:45-208) ---------------------------
  * E, F and W of a SchNet model with 64 features and 2..64 Gaussians over a [2, C] pair list,
  * float32 positions, BF16 tcgen05 tensor cores with FP32 accumulation for every 64 x 64 product,

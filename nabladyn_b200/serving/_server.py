@@ -14,10 +14,12 @@ Each request is an independent one-type Lennard-Jones NVT simulation (the refere
   hands back their frame and frees their room, so requests that arrived meanwhile are
   admitted in the next round;
 * pipelines the rounds: the next round is on the device while the host reads the last one's
-  slot table, harvests and admits, so the device does not wait for the host between rounds.
+  slot table, harvests and admits, so the device does not wait for the host between rounds;
+* gives each replica one CTA, or a cluster of up to eight where it would else outlast the rest
+  (a few requests, or the largest of many).
 
-Replicas never interact on the device: each is advanced by its own CTA, so a replica's result
-does not depend on which others share its rounds.
+Replicas never interact on the device, and a replica's sums are taken in an order of its own,
+so its result does not depend on which others share its rounds or on its number of CTAs.
 """
 
 from __future__ import annotations
@@ -97,6 +99,10 @@ class _Active:
     units: int
     admitted: float
     steps_left: int = field(default=0)
+
+    def work(self) -> int:
+        """Atom-steps left, the admission's forces counted as one step."""
+        return (self.steps_left + 1) * self.request.positions.shape[0]
 
 
 @dataclass
@@ -179,6 +185,7 @@ class ReplicaServer:
         self._pinned: dict[str, list] = {}  # _upload's areas
         self._pinned_turn: dict[str, int] = {}
         self._free_slots = list(range(self.max_slots - 1, -1, -1))
+        self.multiprocessors = torch.cuda.get_device_properties(dev).multi_processor_count
 
     # -- room ----------------------------------------------------------------------------
 
@@ -331,8 +338,20 @@ class ReplicaServer:
                              np.frombuffer(bytes(records), dtype=np.uint8).reshape(-1, size))
         self.table.view(self.max_slots, size).index_copy_(0, slots, table)
 
+    def _team(self, active, work: int) -> int:
+        """CTAs per replica for a lane's ``active`` replicas while all lanes hold ``work``
+        atom-steps: the least power of two that lets the longest of them finish no later than
+        the work spread over every SM would, as far as the lane's teams have SMs side by side.
+        A replica's result does not depend on it."""
+        longest = max((entry.work() for entry in active), default=0)
+        room = self.multiprocessors // max(1, len(active))
+        team = 1
+        while team < 8 and 2 * team <= room and longest * self.multiprocessors > team * work:
+            team *= 2
+        return team
+
     def _launch(self, slots: list[int], budgets: list[int] | None, mode: int,
-                lane: str = "") -> None:
+                lane: str = "", team: int = 1) -> None:
         if not slots:
             return
         slot_tensor = self._upload(f"launch_slots_{mode}{lane}",
@@ -341,9 +360,9 @@ class ReplicaServer:
                                       np.asarray(budgets, dtype=np.int32))
                          if budgets is not None else None)
         with torch.cuda.device(self.device):
-            call("nd_serve_run", self.pool, slot_tensor.data_ptr(),
+            call("nd_serve_run_teams", self.pool, slot_tensor.data_ptr(),
                  budget_tensor.data_ptr() if budget_tensor is not None else None,
-                 len(slots), mode, stream_handle(self.device))
+                 len(slots), mode, team, stream_handle(self.device))
 
     @staticmethod
     def _int_field(raw: np.ndarray, name: str) -> np.ndarray:
@@ -484,16 +503,19 @@ class ReplicaServer:
                 lane.active[slot] = _Active(request, slot, offset, units, now,
                                             int(request.steps))
             progressed = False
+            work = sum(entry.work() for lane in lanes for entry in lane.active.values())
             for lane in lanes:
                 with torch.cuda.stream(lane.stream):
                     batch = placing[lane.name]
                     self._place(batch, lane.name)
-                    self._launch([slot for _, slot, _ in batch], None, 0, lane.name)
+                    team = self._team(lane.active.values(), work)
+                    self._launch([slot for _, slot, _ in batch], None, 0, lane.name, team)
                     if lane.active and len(lane.rounds) < 2:
                         launched = [(slot, lane.active[slot]) for slot in lane.active]
                         budgets = [lane.budget(entry, self.round_atom_steps)
                                    for _, entry in launched]
-                        self._launch([slot for slot, _ in launched], budgets, 1, lane.name)
+                        self._launch([slot for slot, _ in launched], budgets, 1, lane.name,
+                                     team)
                         lane.rounds.append((launched, *self._table_copy(lane)))
                         progressed = True
             # While the rounds run: the next admissions' host work, then the finished rounds.
