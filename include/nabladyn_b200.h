@@ -428,6 +428,20 @@ int nd_serve_run_teams(const nd_replica_pool* pool, const int32_t* slots,
                        const int32_t* budgets, int32_t count, int32_t mode, int32_t team,
                        nd_stream_t stream);
 
+/* The device part of `count` admissions: record k (its offsets set; the kinetic energy of its
+ * thermostat block is computed here) into slot slots[k], and its frame, num_atoms rows from
+ * starts[k] of the float64 positions [atoms, 3], velocities [atoms, 3] and masses [atoms], into
+ * its room in the pool, the center of mass's velocity removed. Device pointers. */
+int nd_serve_admit(const nd_replica_pool* pool, const nd_replica* records, const int32_t* slots,
+                   const int64_t* starts, const double* positions, const double* velocities,
+                   const double* masses, int32_t count, nd_stream_t stream);
+
+/* The frames of `count` finished replicas as their records describe them, replica k from row
+ * starts[k] on: wrapped positions, velocities with the pending chain factor applied, images. */
+int nd_serve_harvest(const nd_replica_pool* pool, const nd_replica* records,
+                     const int64_t* starts, int32_t count, float* positions, float* velocities,
+                     int64_t* images, nd_stream_t stream);
+
 /* ---- SchNet (src/nabladyn/potential/_schnet/_potential.py:45-208) ---------------------------
  * E, F and W of a SchNet model with 64 features and 2..64 Gaussians over a [2, C] pair list,
  * float32 positions, BF16 tcgen05 tensor cores with FP32 accumulation for every 64 x 64 product,

@@ -378,6 +378,13 @@ _SIGNATURES = {
         ctypes.POINTER(ReplicaPool), ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int32,
         ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p,
     ],
+    "nd_serve_admit": [
+        ctypes.POINTER(ReplicaPool), *[ctypes.c_void_p] * 6, ctypes.c_int32, ctypes.c_void_p,
+    ],
+    "nd_serve_harvest": [
+        ctypes.POINTER(ReplicaPool), ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int32,
+        ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
+    ],
     "nd_schnet_energy_force_virial": [ctypes.POINTER(SchNetArgs), ctypes.c_void_p],
     "nd_schnet_tangent": [ctypes.POINTER(SchNetTangentArgs), ctypes.c_int32, ctypes.c_void_p],
     "nd_schnet_atoms": [ctypes.POINTER(SchNetAtomArgs), ctypes.c_int32, ctypes.c_int32,

@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <cstddef>
 #include <cstdint>
 
 #include "common.cuh"
@@ -902,6 +903,146 @@ __global__ void __launch_bounds__(kServeThreads, 1) serve_kernel(ServePool p, co
     }
 }
 
+// Frames of newly admitted replicas into the pool, a CTA per replica: float32 positions and
+// masses, velocities with the center of mass taken out in float64 before the rounding, zero
+// forces and images, and the slot's record with the kinetic energy of the rounded velocities.
+// Bound by the 56 B read per atom (twice: the second pass hits L2). It replaces the conversion
+// on the host, 95 ms of one core for 512 replicas (1.5 million atoms) before the first launch;
+// the host now copies the arrays as they are, and this kernel takes 0.1 ms a batch.
+__global__ void __launch_bounds__(kServeThreads)
+    admit_kernel(ServePool p, const nd_replica* records, const int* slots,
+                 const std::int64_t* starts, const double* positions, const double* velocities,
+                 const double* masses)
+{
+    __shared__ double warp_sums[kServeWarps];
+    const nd_replica* record = records + blockIdx.x;
+    const int n = record->num_atoms;
+    const std::int64_t a0 = record->atom_offset, first = starts[blockIdx.x];
+    const double* x = positions + 3 * first;
+    const double* v = velocities + 3 * first;
+    const double* m = masses + first;
+    double momentum[3] = {0, 0, 0}, total = 0;
+    for (int i = threadIdx.x; i < n; i += kServeThreads)
+    {
+        const double mass = m[i];
+        total += mass;
+        for (int a = 0; a < 3; ++a)
+        {
+            momentum[a] += mass * v[3 * i + a];
+        }
+    }
+    total = block_sum(total, warp_sums);
+    for (int a = 0; a < 3; ++a)
+    {
+        momentum[a] = block_sum(momentum[a], warp_sums) / total;  // the center's velocity
+    }
+    double kinetic = 0;
+    for (int i = threadIdx.x; i < n; i += kServeThreads)
+    {
+        const std::int64_t atom = a0 + i;
+        Pos4<float> position;
+        position.x = static_cast<float>(x[3 * i]);
+        position.y = static_cast<float>(x[3 * i + 1]);
+        position.z = static_cast<float>(x[3 * i + 2]);
+        position.w = 0.0f;
+        p.pos[atom] = position;
+        double squared = 0;
+        for (int a = 0; a < 3; ++a)
+        {
+            const float rounded = static_cast<float>(v[3 * i + a] - momentum[a]);
+            squared += double(rounded) * rounded;
+            p.vel[3 * atom + a] = rounded;
+            p.force[3 * atom + a] = 0.0f;
+            p.images[3 * atom + a] = 0;
+        }
+        kinetic += m[i] * squared;
+        const float mass = static_cast<float>(m[i]);
+        p.mass[atom] = mass;
+        p.inv_mass[atom] = 1.0f / mass;
+    }
+    kinetic = 0.5 * block_sum(kinetic, warp_sums);
+    constexpr int kWords = sizeof(nd_replica) / sizeof(std::uint64_t);
+    constexpr int kKineticWord =
+        offsetof(nd_replica, thermostat) / sizeof(std::uint64_t) + kKineticA;
+    static_assert(sizeof(nd_replica) % sizeof(std::uint64_t) == 0 && kWords <= kServeThreads,
+                  "a thread copies a word of the record");
+    if (threadIdx.x < kWords)
+    {
+        const std::uint64_t word = reinterpret_cast<const std::uint64_t*>(record)[threadIdx.x];
+        reinterpret_cast<std::uint64_t*>(p.replicas + slots[blockIdx.x])[threadIdx.x] =
+            threadIdx.x == kKineticWord
+                ? static_cast<std::uint64_t>(__double_as_longlong(kinetic))
+                : word;
+    }
+}
+
+// Frames of finished replicas, a CTA per replica, from row starts[k] on: the positions wrapped
+// with every product rounded by itself (as wrap_separately), the images with those crossings,
+// the velocities with the pending chain factor applied. One pass where about twenty elementwise
+// launches read three uploaded per-atom arrays (harvests of 512 replicas: 70 -> 15 ms of the
+// host's time).
+__global__ void __launch_bounds__(kServeThreads)
+    harvest_kernel(ServePool p, const nd_replica* records, const std::int64_t* starts,
+                   float* positions, float* velocities, std::int64_t* images)
+{
+    const nd_replica* record = records + blockIdx.x;
+    const int n = record->num_atoms;
+    const std::int64_t a0 = record->atom_offset, first = starts[blockIdx.x];
+    const float scale = static_cast<float>(record->thermostat[kPendingScale]);
+    const float cell[3] = {record->cell[0], record->cell[1], record->cell[2]};
+    for (int i = threadIdx.x; i < n; i += kServeThreads)
+    {
+        const Pos4<float> position = p.pos[a0 + i];
+        const float x[3] = {position.x, position.y, position.z};
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+        {
+            float crossings = floorf(x[a] / cell[a]);
+            float wrapped = x[a] - __fmul_rn(crossings, cell[a]);
+            if (wrapped < 0.0f)
+            {
+                wrapped += cell[a];
+                crossings -= 1.0f;
+            }
+            if (wrapped >= cell[a])
+            {
+                wrapped -= cell[a];
+                crossings += 1.0f;
+            }
+            const std::int64_t from = 3 * (a0 + i) + a, to = 3 * (first + i) + a;
+            positions[to] = wrapped;
+            velocities[to] = p.vel[from] * scale;
+            images[to] = p.images[from] + static_cast<long long>(crossings);
+        }
+    }
+}
+
+bool pool_of(const nd_replica_pool* pool, ServePool& p)
+{
+    if (!(pool->replicas && pool->positions && pool->velocities && pool->forces &&
+          pool->masses && pool->inverse_masses && pool->images && pool->reference_positions &&
+          pool->neighbors && pool->neighbor_counts && pool->sorted && pool->scratch &&
+          pool->cell_starts && pool->ordered_positions))
+    {
+        return false;
+    }
+    p.replicas = pool->replicas;
+    p.pos = static_cast<Pos4<float>*>(pool->positions);
+    p.vel = static_cast<float*>(pool->velocities);
+    p.force = static_cast<float*>(pool->forces);
+    p.mass = static_cast<float*>(pool->masses);
+    p.inv_mass = static_cast<float*>(pool->inverse_masses);
+    p.images = reinterpret_cast<long long*>(pool->images);
+    p.ref_pos = static_cast<Pos4<float>*>(pool->reference_positions);
+    p.nbr = pool->neighbors;
+    p.nbr_count = pool->neighbor_counts;
+    p.sorted = pool->sorted;
+    p.scratch = pool->scratch;
+    p.cell_start = pool->cell_starts;
+    p.ordered = static_cast<Pos4<float>*>(pool->ordered_positions);
+    return true;
+}
+
 }  // namespace nd
 
 extern "C" int nd_serve_run(const nd_replica_pool* pool, const int32_t* slots,
@@ -920,31 +1061,12 @@ extern "C" int nd_serve_run_teams(const nd_replica_pool* pool, const int32_t* sl
     ND_REQUIRE(pool != nullptr && slots != nullptr, "the pool or the slot list is null");
     ND_REQUIRE(mode == 0 || (mode == 1 && budgets != nullptr), "mode is 0 (admit) or 1 (run)");
     ND_REQUIRE(count >= 0 && count <= 1 << 20, "count out of range");
-    ND_REQUIRE(pool->replicas && pool->positions && pool->velocities && pool->forces &&
-                   pool->masses && pool->inverse_masses && pool->images &&
-                   pool->reference_positions && pool->neighbors && pool->neighbor_counts &&
-                   pool->sorted && pool->scratch && pool->cell_starts &&
-                   pool->ordered_positions,
-               "a pool buffer is null");
+    nd::ServePool p;
+    ND_REQUIRE(nd::pool_of(pool, p), "a pool buffer is null");
     if (count == 0)
     {
         return ND_OK;
     }
-    nd::ServePool p;
-    p.replicas = pool->replicas;
-    p.pos = static_cast<nd::Pos4<float>*>(pool->positions);
-    p.vel = static_cast<float*>(pool->velocities);
-    p.force = static_cast<float*>(pool->forces);
-    p.mass = static_cast<float*>(pool->masses);
-    p.inv_mass = static_cast<float*>(pool->inverse_masses);
-    p.images = reinterpret_cast<long long*>(pool->images);
-    p.ref_pos = static_cast<nd::Pos4<float>*>(pool->reference_positions);
-    p.nbr = pool->neighbors;
-    p.nbr_count = pool->neighbor_counts;
-    p.sorted = pool->sorted;
-    p.scratch = pool->scratch;
-    p.cell_start = pool->cell_starts;
-    p.ordered = static_cast<nd::Pos4<float>*>(pool->ordered_positions);
     cudaLaunchConfig_t config{};
     config.gridDim = dim3(static_cast<unsigned>(count) * static_cast<unsigned>(team));
     config.blockDim = dim3(nd::kServeThreads);
@@ -957,5 +1079,46 @@ extern "C" int nd_serve_run_teams(const nd_replica_pool* pool, const int32_t* sl
     config.numAttrs = team > 1 ? 1 : 0;
     ND_CUDA_TRY(cudaLaunchKernelEx(&config, nd::serve_kernel, p, slots, budgets,
                                    static_cast<int>(mode), static_cast<int>(team)));
+    return ND_OK;
+}
+
+extern "C" int nd_serve_admit(const nd_replica_pool* pool, const nd_replica* records,
+                              const int32_t* slots, const int64_t* starts,
+                              const double* positions, const double* velocities,
+                              const double* masses, int32_t count, nd_stream_t stream)
+{
+    ND_REQUIRE(pool != nullptr, "the pool is null");
+    ND_REQUIRE(count >= 0 && count <= 1 << 20, "count out of range");
+    nd::ServePool p;
+    ND_REQUIRE(nd::pool_of(pool, p), "a pool buffer is null");
+    if (count == 0)
+    {
+        return ND_OK;
+    }
+    ND_REQUIRE(records && slots && starts && positions && velocities && masses,
+               "an admission buffer is null");
+    nd::admit_kernel<<<count, nd::kServeThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+        p, records, slots, starts, positions, velocities, masses);
+    ND_CUDA_TRY(cudaGetLastError());
+    return ND_OK;
+}
+
+extern "C" int nd_serve_harvest(const nd_replica_pool* pool, const nd_replica* records,
+                                const int64_t* starts, int32_t count, float* positions,
+                                float* velocities, int64_t* images, nd_stream_t stream)
+{
+    ND_REQUIRE(pool != nullptr, "the pool is null");
+    ND_REQUIRE(count >= 0 && count <= 1 << 20, "count out of range");
+    nd::ServePool p;
+    ND_REQUIRE(nd::pool_of(pool, p), "a pool buffer is null");
+    if (count == 0)
+    {
+        return ND_OK;
+    }
+    ND_REQUIRE(records && starts && positions && velocities && images,
+               "a harvest buffer is null");
+    nd::harvest_kernel<<<count, nd::kServeThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+        p, records, starts, positions, velocities, images);
+    ND_CUDA_TRY(cudaGetLastError());
     return ND_OK;
 }

@@ -5,8 +5,8 @@ Each request is an independent one-type Lennard-Jones NVT simulation (the refere
 
 * admits a request when a slot and room in the HBM budget are free (first fit over the pool's
   atom ranges), uploads its frame and has the replica kernel build its list and first forces;
-  the host work of an admission (the slot record, the frame in pinned memory) is done ahead,
-  while the device runs the previous round, and the upload itself needs no host sync;
+  an admission's host work is the slot record and a copy of the frame into pinned memory,
+  without a host sync, and a kernel converts the frames into the pool;
 * every round launches the replica kernel once over all active slots, each slot with a budget
   of steps inversely proportional to its size, so a round costs about the same on every SM and
   small replicas are not held back by large ones;
@@ -108,10 +108,12 @@ class _Active:
 @dataclass
 class _Staged:
     """A request made ready on the host while the device runs a round: its slot record (all
-    but the offsets) and its frame in pinned memory, uploaded without a host sync."""
+    but the offsets and the kinetic energy) and its frame as float64 arrays."""
 
     record: Replica
-    frame: torch.Tensor  # [n, 9] float32: x, y, z, 0, vx, vy, vz, m, 1/m
+    positions: np.ndarray
+    velocities: np.ndarray
+    masses: np.ndarray
 
 
 @dataclass
@@ -136,13 +138,35 @@ class _Lane:
         return max(1, min(entry.steps_left, steps))
 
 
+def _layout(*parts) -> tuple[dict, int]:
+    """Where each (name, dtype, count) lies in one block, every part on a 256-byte boundary
+    (name -> first byte, bytes, dtype), and the block's bytes."""
+    where, at = {}, 0
+    for name, dtype, count in parts:
+        nbytes = np.dtype(dtype).itemsize * count
+        where[name] = (at, nbytes, dtype)
+        at += -(-nbytes // 256) * 256
+    return where, at
+
+
+def _views(block: torch.Tensor, parts: dict) -> dict:
+    """The parts of a host block as arrays."""
+    raw = block.numpy()
+    return {name: raw[at:at + nbytes].view(dtype) for name, (at, nbytes, dtype) in parts.items()}
+
+
+def _addresses(block: torch.Tensor, parts: dict) -> dict:
+    """The addresses of the parts of a device block."""
+    return {name: block.data_ptr() + part[0] for name, part in parts.items()}
+
+
 class ReplicaServer:
     """Resident replicas in one device pool, advanced in rounds by the replica kernel.
 
     ``budget_bytes`` bounds the pool (about 0.5 kB per atom); ``max_slots`` bounds the replicas
     resident at once; ``round_atom_steps`` is the work a slot gets per round, in atom-steps;
-    ``stage_ahead`` is how many arrived requests the host makes ready (slot record, frame in
-    pinned memory) while a round runs on the device (0: each at its admission).
+    ``stage_ahead`` is how many arrived requests the host makes ready (slot record, frame as
+    float64 arrays) while a round runs on the device (0: each at its admission).
     ``large_atoms``: replicas of at least this many atoms run in rounds of their own, on a
     second stream, ``large_round_steps`` steps a round (None: one stream for all).
     """
@@ -182,8 +206,9 @@ class ReplicaServer:
             setattr(pool, name, tensor.data_ptr())
         self.pool = pool
         self._free_units = [(0, n // _ALIGN)]  # (first unit, units), sorted, merged
-        self._pinned: dict[str, list] = {}  # _upload's areas
+        self._pinned: dict[str, list] = {}  # _area's areas
         self._pinned_turn: dict[str, int] = {}
+        self._landing: torch.Tensor | None = None  # pinned, for harvested frames
         self._free_slots = list(range(self.max_slots - 1, -1, -1))
         self.multiprocessors = torch.cuda.get_device_properties(dev).multi_processor_count
 
@@ -215,9 +240,8 @@ class ReplicaServer:
 
     # -- admission -----------------------------------------------------------------------
 
-    def _describe(self, request: ReplicaRequest, slot: int,
-                  offset: int) -> tuple[Replica, np.ndarray]:
-        """The slot record of a request and its float32 velocities, center of mass removed."""
+    def _describe(self, request: ReplicaRequest) -> Replica:
+        """The slot record of a request, without its offsets and its kinetic energy."""
         n = int(request.positions.shape[0])
         if not 2 <= n <= 65535:
             raise ValueError("a replica holds 2 to 65535 atoms")
@@ -233,9 +257,6 @@ class ReplicaServer:
         eps = float(np.finfo(np.float32).eps)
         allowance = radius - float(request.cutoff) - 32 * eps * max(lengths)
         record = Replica()
-        record.atom_offset = offset
-        record.list_offset = offset * _WIDTH
-        record.cell_offset = slot * (_MAX_CELLS + 1)
         record.num_atoms = n
         record.width = _WIDTH
         for a in range(3):
@@ -249,15 +270,9 @@ class ReplicaServer:
         record.sigma = request.sigma
         record.epsilon = request.epsilon
         record.steps_left = int(request.steps)
-        masses = np.asarray(request.masses, dtype=np.float64)
-        velocities = np.asarray(request.velocities, dtype=np.float64)
-        velocities = velocities - (masses[:, None] * velocities).sum(axis=0) / masses.sum()
-        velocities32 = velocities.astype(np.float32)
-        kinetic = 0.5 * float((masses[:, None] * velocities32.astype(np.float64) ** 2).sum())
         kT = BOLTZMANN * float(request.temperature)
         degrees = 3 * n - 3
         base = kT * float(request.thermostat_timescale) ** 2
-        record.thermostat[_KINETIC_A] = kinetic
         record.thermostat[_PENDING] = 1.0
         record.thermostat[_CHAIN_MASS] = degrees * base
         record.thermostat[_CHAIN_MASS + 1] = base
@@ -265,78 +280,85 @@ class ReplicaServer:
         record.thermostat[_KT] = kT
         record.thermostat[_DEGREES] = degrees
         record.thermostat[_TIMESTEP] = request.timestep
-        return record, velocities32
+        return record
 
     def _stage(self, request: ReplicaRequest) -> _Staged:
-        """The host part of an admission: the record and the frame (uploaded by _place)."""
-        record, velocities32 = self._describe(request, 0, 0)
-        n = record.num_atoms
-        frame = torch.empty((n, 9), dtype=torch.float32)
-        masses = np.asarray(request.masses, dtype=np.float32)
-        host = frame.numpy()
-        host[:, :3] = np.asarray(request.positions, dtype=np.float32)
-        host[:, 3] = 0.0
-        host[:, 4:7] = velocities32
-        host[:, 7] = masses
-        host[:, 8] = 1.0 / masses
-        return _Staged(record, frame)
+        """The host part of an admission (uploaded by _place)."""
+        record = self._describe(request)
+        masses = np.asarray(request.masses, dtype=np.float64)
+        if masses.ndim == 0:
+            raise IndexError("masses are one value per atom")
+        return _Staged(record, np.asarray(request.positions, dtype=np.float64),
+                       np.asarray(request.velocities, dtype=np.float64), masses)
 
-    def _upload(self, name: str, values: np.ndarray) -> torch.Tensor:
-        """A host array on the device without a host sync, on the current stream: through one
-        of two pinned areas kept per `name` and grown as needed (a copy from pageable memory
-        would wait for the round running on the stream, and a new pinned block per call costs
-        more than the copy). An area is reused after the copy made from it two calls before,
-        which an earlier round's completion has already finished in the serve loop."""
-        values = np.ascontiguousarray(values)
+    def _area(self, name: str, nbytes: int) -> torch.Tensor:
+        """`nbytes` of pinned memory to write a copy's source into: one of two areas kept per
+        `name` and grown as needed (a copy from pageable memory would wait for the round running
+        on the stream, and a new pinned block per call costs more than the copy). An area is
+        reused after the copy made from it two calls before, which an earlier round's completion
+        has already finished in the serve loop."""
         areas = self._pinned.setdefault(name, [[None, None], [None, None]])
         turn = self._pinned_turn[name] = self._pinned_turn.get(name, 1) ^ 1
         area, copied = areas[turn]
         if copied is not None:
             copied.synchronize()
-        if area is None or area.numel() < values.nbytes:
-            grown = max(values.nbytes, 2 * (area.numel() if area is not None else 0), 1 << 16)
-            area = torch.empty(grown, dtype=torch.uint8, pin_memory=True)
-        host = area[:values.nbytes]
-        host.numpy()[:] = values.reshape(-1).view(np.uint8)
+        if area is None or area.numel() < nbytes:
+            grown = max(nbytes, 2 * (area.numel() if area is not None else 0), 1 << 16)
+            area = areas[turn][0] = torch.empty(grown, dtype=torch.uint8, pin_memory=True)
+        return area[:nbytes]
+
+    def _send(self, name: str, host: torch.Tensor) -> torch.Tensor:
+        """The area taken last from `name`, on the device without a host sync, on the current
+        stream."""
         device = host.to(self.device, non_blocking=True)
         copied = torch.cuda.Event()
         copied.record(torch.cuda.current_stream(self.device))
-        areas[turn] = [area, copied]
+        self._pinned[name][self._pinned_turn[name]][1] = copied
+        return device
+
+    def _upload(self, name: str, values: np.ndarray) -> torch.Tensor:
+        """A host array on the device without a host sync, on the current stream."""
+        values = np.ascontiguousarray(values)
+        host = self._area(name, values.nbytes)
+        host.numpy()[:] = values.reshape(-1).view(np.uint8)
         dtype = torch.from_numpy(np.empty(0, dtype=values.dtype)).dtype
-        return device.view(dtype).reshape(values.shape)
+        return self._send(name, host).view(dtype).reshape(values.shape)
 
     def _place(self, batch: list[tuple[_Staged, int, int]], lane: str = "") -> None:
-        """The device part of admissions, for a batch at once: the frames' pinned rows copied
-        into one device block and scattered into the pool, the slot records written with their
-        offsets; no host sync."""
+        """The device part of admissions, for a batch at once: the records and the float64
+        frames in one pinned area, one copy and one kernel that converts them into the pool;
+        no host sync."""
         if not batch:
             return
-        size = ctypes.sizeof(Replica)
-        records = bytearray()
-        destination = []
-        for staged, slot, offset in batch:
+        size, count = ctypes.sizeof(Replica), len(batch)
+        atoms = sum(staged.record.num_atoms for staged, _, _ in batch)
+        parts, nbytes = _layout(
+            ("records", np.uint8, size * count), ("starts", np.int64, count),
+            ("slots", np.int32, count), ("positions", np.float64, 3 * atoms),
+            ("velocities", np.float64, 3 * atoms), ("masses", np.float64, atoms))
+        host = self._area("admit" + lane, nbytes)
+        part = _views(host, parts)
+        positions = part["positions"].reshape(-1, 3)
+        velocities = part["velocities"].reshape(-1, 3)
+        begin = 0
+        for k, (staged, slot, offset) in enumerate(batch):
             record = staged.record
-            n = record.num_atoms
             record.atom_offset = offset
             record.list_offset = offset * _WIDTH
             record.cell_offset = slot * (_MAX_CELLS + 1)
-            records += ctypes.string_at(ctypes.addressof(record), size)
-            destination.append(np.arange(offset, offset + n, dtype=np.int64))
-        frames = np.concatenate([staged.frame.numpy() for staged, _, _ in batch])
-        rows = self._upload("frames" + lane, frames)
-        index = self._upload("rows" + lane, np.concatenate(destination))
-        b = self.buffers
-        b["positions"].index_copy_(0, index, rows[:, :4])
-        b["velocities"].index_copy_(0, index, rows[:, 4:7])
-        b["forces"].index_fill_(0, index, 0.0)
-        b["masses"].index_copy_(0, index, rows[:, 7])
-        b["inverse_masses"].index_copy_(0, index, rows[:, 8])
-        b["images"].index_fill_(0, index, 0)
-        slots = self._upload("slots" + lane,
-                             np.array([slot for _, slot, _ in batch], dtype=np.int64))
-        table = self._upload("records" + lane,
-                             np.frombuffer(bytes(records), dtype=np.uint8).reshape(-1, size))
-        self.table.view(self.max_slots, size).index_copy_(0, slots, table)
+            part["records"][size * k:size * (k + 1)] = np.frombuffer(record, dtype=np.uint8)
+            end = begin + record.num_atoms
+            part["starts"][k], part["slots"][k] = begin, slot
+            positions[begin:end] = staged.positions
+            velocities[begin:end] = staged.velocities
+            part["masses"][begin:end] = staged.masses
+            begin = end
+        block = self._send("admit" + lane, host)
+        at = _addresses(block, parts)
+        with torch.cuda.device(self.device):
+            call("nd_serve_admit", self.pool, at["records"], at["slots"], at["starts"],
+                 at["positions"], at["velocities"], at["masses"], count,
+                 stream_handle(self.device))
 
     def _team(self, active, work: int) -> int:
         """CTAs per replica for a lane's ``active`` replicas while all lanes hold ``work``
@@ -378,38 +400,40 @@ class ReplicaServer:
         (first unit, units, slot)."""
         if not done:
             return []
-        rows, cells, scales, sizes = [], [], [], []
-        for active, raw in done:
-            record = Replica.from_buffer_copy(raw.tobytes())
-            n, offset = record.num_atoms, active.offset
-            rows.append(np.arange(offset, offset + n, dtype=np.int64))
-            cells.append(np.broadcast_to(np.asarray(record.cell, dtype=np.float32), (n, 3)))
-            scales.append(np.full(n, np.float32(record.thermostat[_PENDING]), dtype=np.float32))
-            sizes.append((record, n))
-        index = self._upload("harvest_rows", np.concatenate(rows))
-        cell = self._upload("harvest_cells", np.concatenate(cells))
-        scale = self._upload("harvest_scales", np.concatenate(scales))
-        unwrapped = self.buffers["positions"][index, :3]
-        crossings = torch.floor(unwrapped / cell)
-        wrapped = unwrapped - crossings * cell
-        below = wrapped < 0
-        wrapped = torch.where(below, wrapped + cell, wrapped)
-        crossings = torch.where(below, crossings - 1, crossings)
-        above = wrapped >= cell
-        wrapped = torch.where(above, wrapped - cell, wrapped)
-        crossings = torch.where(above, crossings + 1, crossings)
-        velocities = self.buffers["velocities"][index] * scale[:, None]
-        images = self.buffers["images"][index] + crossings.to(torch.int64)
-        frame = torch.cat([wrapped, velocities], dim=1).cpu().numpy()
-        images = images.cpu().numpy()
+        size, count = ctypes.sizeof(Replica), len(done)
+        records = [Replica.from_buffer_copy(raw.tobytes()) for _, raw in done]
+        atoms = sum(record.num_atoms for record in records)
+        parts, nbytes = _layout(("records", np.uint8, size * count), ("starts", np.int64, count))
+        host = self._area("harvest", nbytes)
+        part = _views(host, parts)
+        part["records"][:] = np.concatenate([raw for _, raw in done])
+        part["starts"][:] = np.cumsum([0] + [record.num_atoms for record in records[:-1]])
+        block = self._send("harvest", host)
+        given = _addresses(block, parts)
+        parts, nbytes = _layout(
+            ("positions", np.float32, 3 * atoms), ("velocities", np.float32, 3 * atoms),
+            ("images", np.int64, 3 * atoms))
+        out = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+        at = _addresses(out, parts)
+        with torch.cuda.device(self.device):
+            call("nd_serve_harvest", self.pool, given["records"], given["starts"], count,
+                 at["positions"], at["velocities"], at["images"], stream_handle(self.device))
+        if self._landing is None or self._landing.numel() < nbytes:
+            grown = max(nbytes, 2 * (self._landing.numel() if self._landing is not None else 0))
+            self._landing = torch.empty(grown, dtype=torch.uint8, pin_memory=True)
+        self._landing[:nbytes].copy_(out, non_blocking=True)
+        torch.cuda.current_stream(self.device).synchronize()
+        frame = {name: values.reshape(-1, 3)
+                 for name, values in _views(self._landing, parts).items()}
         results, begin = [], 0
-        for (active, _), (record, n) in zip(done, sizes):
+        for (active, _), record in zip(done, records):
+            n = record.num_atoms
             end = begin + n
             results.append(ReplicaResult(
                 name=active.request.name,
-                positions=frame[begin:end, :3].copy(),
-                velocities=frame[begin:end, 3:].copy(),
-                images=images[begin:end].copy(),
+                positions=frame["positions"][begin:end].copy(),
+                velocities=frame["velocities"][begin:end].copy(),
+                images=frame["images"][begin:end].copy(),
                 energy=float(record.energy),
                 status=int(record.status),
                 rebuilds=int(record.rebuild_count),
@@ -495,18 +519,22 @@ class ReplicaServer:
                 pending.popleft()
                 slot = self._free_slots.pop()
                 offset = first * _ALIGN
-                ready = staged.pop(id(request)) if id(request) in staged else self._stage(request)
                 lane = lane_of(request)
-                placing[lane.name].append((ready, slot, offset))
-                # The pinned frame may go once its copy is queued: the host allocator keeps
-                # the block until the copy has run.
+                placing[lane.name].append((request, slot, offset))
                 lane.active[slot] = _Active(request, slot, offset, units, now,
                                             int(request.steps))
             progressed = False
-            work = sum(entry.work() for lane in lanes for entry in lane.active.values())
-            for lane in lanes:
+            work = None
+            # The large replicas first: their rounds run while the small ones are made ready.
+            for lane in reversed(lanes):
                 with torch.cuda.stream(lane.stream):
-                    batch = placing[lane.name]
+                    if not (placing[lane.name] or lane.active and len(lane.rounds) < 2):
+                        continue
+                    if work is None:
+                        work = sum(entry.work() for other in lanes
+                                   for entry in other.active.values())
+                    batch = [(staged.pop(id(request), None) or self._stage(request), slot,
+                              offset) for request, slot, offset in placing[lane.name]]
                     self._place(batch, lane.name)
                     team = self._team(lane.active.values(), work)
                     self._launch([slot for _, slot, _ in batch], None, 0, lane.name, team)
