@@ -210,7 +210,6 @@ class ReplicaServer:
         self._pinned_turn: dict[str, int] = {}
         self._landing: torch.Tensor | None = None  # pinned, for harvested frames
         self._free_slots = list(range(self.max_slots - 1, -1, -1))
-        self.multiprocessors = torch.cuda.get_device_properties(dev).multi_processor_count
 
     # -- room ----------------------------------------------------------------------------
 
@@ -366,9 +365,10 @@ class ReplicaServer:
         the work spread over every SM would, as far as the lane's teams have SMs side by side.
         A replica's result does not depend on it."""
         longest = max((entry.work() for entry in active), default=0)
-        room = self.multiprocessors // max(1, len(active))
+        sms = torch.cuda.get_device_properties(self.device).multi_processor_count
+        room = sms // max(1, len(active))
         team = 1
-        while team < 8 and 2 * team <= room and longest * self.multiprocessors > team * work:
+        while team < 8 and 2 * team <= room and longest * sms > team * work:
             team *= 2
         return team
 
