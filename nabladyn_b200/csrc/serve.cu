@@ -30,7 +30,7 @@ namespace nd {
 constexpr int kServeThreads = 512;
 constexpr int kServeWarps = kServeThreads / kWarp;
 constexpr int kServeMaxCells = 4096;
-constexpr int kServeTeam = 8;         // CTAs a replica gets at most (a portable cluster)
+constexpr int kServeTeam = 8;          // CTAs a replica gets at most (a portable cluster)
 constexpr int kServeTeamAtoms = 1024;  // atoms for each of them: two rows per thread
 
 struct ServePool
@@ -179,42 +179,6 @@ __device__ void block_scan_cells(int* counts, int cells, int* warp_totals)
     __syncthreads();
 }
 
-// Adds to `list` the atoms k = begin .. end - 1 closer to `me` (atom i) than the list radius
-// under the minimum image, in k order (the all-pairs path of a replica with fewer than three
-// cells along an axis). Four candidates at a time, loaded before any is tested.
-__device__ __forceinline__ void scan_candidates(const ReplicaScalars& r, const Pos4<float>& me,
-                                                int i, int begin, int end,
-                                                const Pos4<float>* pos, ListWriter& list)
-{
-    constexpr int kGroup = 4;
-    for (int k = begin; k < end; k += kGroup)
-    {
-        int j[kGroup];
-        Pos4<float> p[kGroup];
-#pragma unroll
-        for (int u = 0; u < kGroup; ++u)
-        {
-            j[u] = k + u < end ? k + u : -1;
-        }
-#pragma unroll
-        for (int u = 0; u < kGroup; ++u)
-        {
-            p[u] = j[u] >= 0 ? pos[j[u]] : me;
-        }
-#pragma unroll
-        for (int u = 0; u < kGroup; ++u)
-        {
-            const float d2 = squared_norm(min_image(me.x, p[u].x, r.cell[0]),
-                                          min_image(me.y, p[u].y, r.cell[1]),
-                                          min_image(me.z, p[u].z, r.cell[2]));
-            if (j[u] >= 0 && j[u] != i && d2 < r.radius_squared)
-            {
-                list.add(j[u]);
-            }
-        }
-    }
-}
-
 // The image of one stencil cell along an axis: the cell index h + d wrapped into [0, dims),
 // and which side of the displacement takes the period. Past the upper face the center moves
 // (center - L), past the lower face the candidate does (candidate - L): the two forms the
@@ -245,40 +209,136 @@ __device__ __forceinline__ AxisImage axis_image(int h, int d, int dims, float le
     return a;
 }
 
-// Adds to `list` the candidates of one stencil cell, k = begin .. end - 1 of the cell-ordered
-// copy (x, y, z, and the atom's index in w), that lie closer than the list radius to the
-// center (cell-order row `self`), in k order: one 16-B load per candidate, no index lookup
-// and no per-candidate image choice. Eight candidates at a time, all loaded before any is
-// tested; their hits are kept as bits and appended lowest first (one append loop per group
-// instead of a branch per candidate; groups of 4 and 16 measured slower).
-__device__ __forceinline__ void scan_cell(const ReplicaScalars& r, float cx, float cy, float cz,
-                                          float sx, float sy, float sz, int self,
-                                          const Pos4<float>* ordered, int begin,
-                                          int end, StagedListWriter& list)
+// A row's chunks (see ListWriter), staged in a ring of 16 entries per lane in shared memory:
+// a hit is one predicated 2-byte store, without a branch, and after every eight candidates one
+// drain moves a full chunk to global memory. Entry e of a warp's lane lies at [e % 16][lane].
+struct RingListWriter
 {
-    constexpr int kGroup = 8;
+    uint4* chunks;
+    std::uint16_t* ring;  // this lane's entry 0
+    int width;
+    int row;
+    int count;
+    int drained;  // entries in global memory, or dropped beyond the width: a multiple of 8
+
+    __device__ __forceinline__ RingListWriter(std::uint16_t* list, std::uint16_t* ring_,
+                                              int width_, int row_)
+        : chunks(reinterpret_cast<uint4*>(list)), ring(ring_), width(width_), row(row_), count(0),
+          drained(0)
+    {
+    }
+
+    __device__ __forceinline__ void add(bool hit, int index)
+    {
+        if (hit)
+        {
+            ring[(count & 15) * kWarp] = static_cast<std::uint16_t>(index);
+            ++count;
+        }
+    }
+
+    // After at most eight adds.
+    __device__ __forceinline__ void drain()
+    {
+        if (count - drained >= kChunk)
+        {
+            store();
+        }
+    }
+
+    __device__ __forceinline__ void store()
+    {
+        if (drained < width)
+        {
+            const std::uint16_t* from = ring + (drained & 15) * kWarp;
+            unsigned packed[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+            {
+                packed[k] = from[2 * k * kWarp] |
+                            static_cast<unsigned>(from[(2 * k + 1) * kWarp]) << 16;
+            }
+            chunks[chunk_index(row, drained / kChunk, width)] =
+                make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        }
+        drained += kChunk;
+    }
+
+    // Stores a partial last chunk, its unused slots set to `pad`.
+    __device__ __forceinline__ void finish(unsigned pad)
+    {
+        if (count > drained)
+        {
+            for (int e = count; e < drained + kChunk; ++e)
+            {
+                ring[(e & 15) * kWarp] = static_cast<std::uint16_t>(pad);
+            }
+            store();
+        }
+    }
+};
+
+// Adds to `list` the candidates k = begin .. end - 1 of the cell-ordered copy (x, y, z, and the
+// atom's index in w) that lie closer than the list radius to the center (cell-order row
+// `self`), in k order: one 16-B load per candidate, no index lookup and no per-candidate image
+// choice. With kImaged the center and the candidates are moved by the cell's image (center at
+// cx, candidates by -sx). Eight candidates at a time, all loaded before any is tested.
+// Issue and the hits' divergence bound the scan. An append loop over each group's hit bits ran as
+// often as the warp's fullest lane had hits (4-5 times for 1.1 hits on average) and fetched every
+// index from memory: 148 replicas of 12,000 atoms, 60 steps with 7.5 rebuilds, 62.8 -> 55.4 ms.
+template <bool kImaged>
+__device__ __forceinline__ void scan_run(const ReplicaScalars& r, float cx, float cy, float cz,
+                                         float sx, float sy, float sz, int self,
+                                         const Pos4<float>* ordered, int begin, int end,
+                                         RingListWriter& list)
+{
+    constexpr int kGroup = kChunk;
     for (int k = begin; k < end; k += kGroup)
     {
         Pos4<float> p[kGroup];
 #pragma unroll
         for (int u = 0; u < kGroup; ++u)
         {
-            p[u] = k + u < end ? ordered[k + u] : far_atom<float>();
+            p[u] = ordered[min(k + u, end - 1)];
         }
-        unsigned hits = 0;
 #pragma unroll
         for (int u = 0; u < kGroup; ++u)
         {
-            const float d2 = squared_norm(cx - (p[u].x - sx), cy - (p[u].y - sy),
-                                          cz - (p[u].z - sz));
-            hits |= static_cast<unsigned>(k + u != self && d2 < r.radius_squared) << u;
+            const float d2 = kImaged ? squared_norm(cx - (p[u].x - sx), cy - (p[u].y - sy),
+                                                    cz - (p[u].z - sz))
+                                     : squared_norm(cx - p[u].x, cy - p[u].y, cz - p[u].z);
+            list.add(k + u < end && k + u != self && d2 < r.radius_squared,
+                     __float_as_int(p[u].w));
         }
-        while (hits != 0)
+        list.drain();
+    }
+}
+
+// Adds to `list` the atoms k < n closer to `me` (atom `self`) than the list radius under the
+// minimum image, in k order: the path of a replica with fewer than three cells along an axis
+// (592 replicas of 500 atoms, 60 steps with 4.7 rebuilds: 7.8 -> 6.4 ms with the ring in place
+// of chunks packed in registers by a branch per hit).
+__device__ __forceinline__ void scan_all(const ReplicaScalars& r, const Pos4<float>& me, int self,
+                                         const Pos4<float>* pos, RingListWriter& list)
+{
+    constexpr int kGroup = kChunk;
+    for (int k = 0; k < r.n; k += kGroup)
+    {
+        Pos4<float> p[kGroup];
+#pragma unroll
+        for (int u = 0; u < kGroup; ++u)
         {
-            const int u = __ffs(hits) - 1;
-            hits &= hits - 1;
-            list.add(static_cast<unsigned>(reinterpret_cast<const int*>(ordered + k + u)[3]));
+            p[u] = pos[min(k + u, r.n - 1)];
         }
+#pragma unroll
+        for (int u = 0; u < kGroup; ++u)
+        {
+            const float d2 = squared_norm(min_image(me.x, p[u].x, r.cell[0]),
+                                          min_image(me.y, p[u].y, r.cell[1]),
+                                          min_image(me.z, p[u].z, r.cell[2]));
+            list.add(k + u < r.n && k + u != self && d2 < r.radius_squared, k + u);
+        }
+        list.drain();
     }
 }
 
@@ -387,12 +447,13 @@ __device__ void rebuild_replica(const Team& team, const ReplicaScalars& r, Pos4<
     // scanned with its image, so the entries are those of a scan of every candidate with its
     // own minimum image. nbr_count[row] holds the count in its low 16 bits and the direct
     // entries in its high 16 bits (a count is at most N - 1 < 2^16).
-    // A row's entries go through 16 bytes of shared memory per thread, a chunk at a time to
-    // global memory (the staged writer measured 14 % faster than packing them in registers).
-    __shared__ __align__(16) std::uint16_t lane_slots[kServeThreads][kChunk];
+    // The three cells of a stencil row are adjacent in the cell order, so those without an image
+    // along x are one run of candidates.
+    __shared__ std::uint16_t rings[kServeWarps][2 * kChunk][kWarp];
     for (int row = team.first(); row < n; row += team.stride())
     {
-        StagedListWriter list(nbr, lane_slots[threadIdx.x], r.width, row);
+        RingListWriter list(nbr, &rings[threadIdx.x / kWarp][0][threadIdx.x % kWarp], r.width,
+                            row);
         int direct = 0;
         if (grid)
         {
@@ -400,6 +461,7 @@ __device__ void rebuild_replica(const Team& team, const ReplicaScalars& r, Pos4<
             const int hx = axis_bin(me.x, r.widths[0], r.dims[0]);
             const int hy = axis_bin(me.y, r.widths[1], r.dims[1]);
             const int hz = axis_bin(me.z, r.widths[2], r.dims[2]);
+            const int low = max(hx - 1, 0), high = min(hx + 1, r.dims[0] - 1);
             for (int pass = 0; pass < 2; ++pass)
             {
                 for (int dz = -1; dz <= 1; ++dz)
@@ -410,19 +472,32 @@ __device__ void rebuild_replica(const Team& team, const ReplicaScalars& r, Pos4<
                     {
                         const AxisImage iy = axis_image(hy, dy, r.dims[1], r.cell[1]);
                         const float cy = me.y - iy.center_shift;
-                        for (int dx = -1; dx <= 1; ++dx)
+                        const bool imaged = hy + dy != iy.cell || hz + dz != iz.cell;
+                        const int* first = counts + r.dims[0] * (iy.cell + r.dims[1] * iz.cell);
+                        if (pass == 0)
                         {
-                            const AxisImage ix = axis_image(hx, dx, r.dims[0], r.cell[0]);
-                            const bool imaged = hx + dx != ix.cell || hy + dy != iy.cell ||
-                                                hz + dz != iz.cell;
-                            if (imaged != (pass == 1))
+                            if (!imaged)
                             {
-                                continue;
+                                scan_run<false>(r, me.x, cy, cz, 0.0f, 0.0f, 0.0f, row, ordered,
+                                                first[low], first[high + 1], list);
                             }
-                            const int c = ix.cell + r.dims[0] * (iy.cell + r.dims[1] * iz.cell);
-                            scan_cell(r, me.x - ix.center_shift, cy, cz, ix.candidate_shift,
-                                      iy.candidate_shift, iz.candidate_shift, row, ordered,
-                                      counts[c], counts[c + 1], list);
+                            continue;
+                        }
+                        // Past the lower face, between the faces, past the upper face.
+                        for (int side = -1; side <= 1; ++side)
+                        {
+                            const bool there = side < 0    ? hx == 0
+                                               : side == 0 ? imaged
+                                                           : hx == r.dims[0] - 1;
+                            if (there)
+                            {
+                                const int from = side < 0 ? r.dims[0] - 1 : side == 0 ? low : 0;
+                                const int to = side < 0 ? r.dims[0] : side == 0 ? high + 1 : 1;
+                                scan_run<true>(r, side > 0 ? me.x - r.cell[0] : me.x, cy, cz,
+                                               side < 0 ? r.cell[0] : 0.0f, iy.candidate_shift,
+                                               iz.candidate_shift, row, ordered, first[from],
+                                               first[to], list);
+                            }
                         }
                     }
                 }
@@ -431,15 +506,12 @@ __device__ void rebuild_replica(const Team& team, const ReplicaScalars& r, Pos4<
                     direct = list.count;
                 }
             }
-            list.finish(0xffffu);
         }
         else
         {
-            ListWriter all(nbr, r.width, row, 0xffffu);
-            scan_candidates(r, pos[row], row, 0, n, pos, all);
-            all.finish();
-            list.count = all.count;
+            scan_all(r, pos[row], row, pos, list);
         }
+        list.finish(0xffffu);
         nbr_count[row] = list.count | (direct << 16);
         if (list.count > r.width)
         {
@@ -650,7 +722,7 @@ __device__ double sum_units(const double* values, int units, double* warp_sums)
 // closes it from the same sums; a step costs two cluster barriers, a rebuild three more. Every
 // branch around a barrier is decided from values that all CTAs read after the same barrier.
 // 512 replicas of 64 to 16,384 atoms, 100 steps each: 192 ms on the GPU with one CTA each,
-// 118 ms with the teams the server picks.
+// 118 ms with the teams the server picks (103 ms with the candidate scan as it is now).
 __global__ void __launch_bounds__(kServeThreads, 1) serve_kernel(ServePool p, const int* slots,
                                                               const int* budgets, int mode,
                                                               int team_ctas)
