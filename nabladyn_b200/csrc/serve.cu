@@ -722,7 +722,7 @@ __device__ double sum_units(const double* values, int units, double* warp_sums)
 // closes it from the same sums; a step costs two cluster barriers, a rebuild three more. Every
 // branch around a barrier is decided from values that all CTAs read after the same barrier.
 // 512 replicas of 64 to 16,384 atoms, 100 steps each: 192 ms on the GPU with one CTA each,
-// 118 ms with the teams the server picks (103 ms with the candidate scan as it is now).
+// 118 ms with the teams the server picks (98 ms with the candidate scan as it is now).
 __global__ void __launch_bounds__(kServeThreads, 1) serve_kernel(ServePool p, const int* slots,
                                                               const int* budgets, int mode,
                                                               int team_ctas)

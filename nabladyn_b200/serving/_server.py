@@ -38,6 +38,7 @@ from ..neighbors._neighbor_list import check_cell_lengths, grid
 from ..units import BOLTZMANN
 
 _ALIGN = 32          # atoms per allocation unit (one warp of list chunks)
+_BATCH = 1 << 18     # atoms of frames copied at once (a replica's, if it has more)
 _MAX_CELLS = 4096    # kServeMaxCells in serve.cu
 _WIDTH = 192         # list slots per atom: room for ~1.5x the mean count at 22 atoms/nm^3
 _BYTES_PER_ATOM = 16 + 12 + 12 + 4 + 4 + 24 + 16 + 2 * _WIDTH + 4 + 4 + 4 + 16
@@ -147,6 +148,20 @@ def _layout(*parts) -> tuple[dict, int]:
         where[name] = (at, nbytes, dtype)
         at += -(-nbytes // 256) * 256
     return where, at
+
+
+def _batches(items: list, atoms) -> list[list]:
+    """The items in order, in batches of at most _BATCH atoms by ``atoms(item)``: the pinned
+    areas stay small (pinning 100 MB takes 30-90 ms) and copies overlap the host's next batch."""
+    batches, room = [], 0
+    for item in items:
+        n = atoms(item)
+        if not batches or n > room:
+            batches.append([])
+            room = _BATCH
+        batches[-1].append(item)
+        room -= n
+    return batches
 
 
 def _views(block: torch.Tensor, parts: dict) -> dict:
@@ -327,8 +342,6 @@ class ReplicaServer:
         """The device part of admissions, for a batch at once: the records and the float64
         frames in one pinned area, one copy and one kernel that converts them into the pool;
         no host sync."""
-        if not batch:
-            return
         size, count = ctypes.sizeof(Replica), len(batch)
         atoms = sum(staged.record.num_atoms for staged, _, _ in batch)
         parts, nbytes = _layout(
@@ -398,8 +411,6 @@ class ReplicaServer:
         applied to the velocities, images with the last crossings): computed on the device for
         all of them together and read back in one copy; their room and slots go to `freed` as
         (first unit, units, slot)."""
-        if not done:
-            return []
         size, count = ctypes.sizeof(Replica), len(done)
         records = [Replica.from_buffer_copy(raw.tobytes()) for _, raw in done]
         atoms = sum(record.num_atoms for record in records)
@@ -535,7 +546,8 @@ class ReplicaServer:
                                    for entry in other.active.values())
                     batch = [(staged.pop(id(request), None) or self._stage(request), slot,
                               offset) for request, slot, offset in placing[lane.name]]
-                    self._place(batch, lane.name)
+                    for part in _batches(batch, lambda entry: entry[0].record.num_atoms):
+                        self._place(part, lane.name)
                     team = self._team(lane.active.values(), work)
                     self._launch([slot for _, slot, _ in batch], None, 0, lane.name, team)
                     if lane.active and len(lane.rounds) < 2:
@@ -616,6 +628,7 @@ class ReplicaServer:
         # stream after this round.
         side.wait_event(event)
         with torch.cuda.stream(side):
-            return self._harvest(done, now, freed)
+            return [result for part in _batches(done, lambda entry: entry[0].units * _ALIGN)
+                    for result in self._harvest(part, now, freed)]
 
 __all__ = ("ReplicaRequest", "ReplicaResult", "ReplicaServer")
