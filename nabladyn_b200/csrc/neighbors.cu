@@ -413,9 +413,36 @@ __device__ __forceinline__ int next_hit(unsigned& hits)
     return j;
 }
 
+// Pads the columns from the total on, by `threads` threads: column k holds the self-pair
+// (k mod N, k mod N), spreading their zero gradients over the atoms; the threads start at the
+// total and step together, so each takes one remainder and the stores are whole lines.
+__device__ __forceinline__ void pad_columns(index_t total, index_t num_atoms, index_t capacity,
+                                            index_t* __restrict__ pairs, unsigned thread,
+                                            unsigned threads)
+{
+    if (total >= capacity)
+    {
+        return;
+    }
+    const unsigned n = static_cast<unsigned>(num_atoms);
+    const unsigned end = static_cast<unsigned>(capacity);
+    const unsigned step = threads % n;
+    unsigned column = static_cast<unsigned>(total) + thread;  // below 2^32: the grid is bounded
+    unsigned atom = column % n;
+    for (; column < end; column += threads)
+    {
+        pairs[column] = static_cast<index_t>(atom);
+        pairs[static_cast<std::int64_t>(capacity) + column] = static_cast<index_t>(atom);
+        atom += step;
+        atom -= atom >= n ? n : 0u;
+    }
+}
+
 // Counts (kFill false) or writes (kFill true) the pairs of one home bin. The fill of an update
 // also stores the frame it was built from: each CTA its home atoms' positions, the first the
-// cell and the rebuild count.
+// cell and the rebuild count. The fill's first `pad_ctas` CTAs write the padding columns instead:
+// those stores are bound by memory and the fill by instruction issue, so one hides the other
+// (1,048,576 atoms, update: fill 519 us and padding after it 73 us, together 537 us).
 //
 // The candidates, home bin first, are staged kHoodSlots at a time (once, in all but very dense
 // bins) and tested against the bin's atoms 32 at a time.
@@ -436,14 +463,22 @@ __global__ void __launch_bounds__(kThreadCount) hood_pairs_kernel(
     T* __restrict__ reference_cell,
     index_t* __restrict__ rebuild_count,
     const index_t* __restrict__ rebuild,
-    const index_t* __restrict__ status
+    const index_t* __restrict__ status,
+    index_t num_atoms,
+    int pad_ctas
 )
 {
     if (!rebuilding(rebuild, status))
     {
         return;
     }
-    const index_t home = static_cast<index_t>(blockIdx.x);
+    if (kFill && static_cast<int>(blockIdx.x) < pad_ctas)
+    {
+        pad_columns(pair_offsets[num_atoms - 1] + pair_counts[num_atoms - 1], num_atoms, capacity,
+                    pairs, blockIdx.x * kThreadCount + threadIdx.x, pad_ctas * kThreadCount);
+        return;
+    }
+    const index_t home = static_cast<index_t>(blockIdx.x) - (kFill ? pad_ctas : 0);
     const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
     const index_t begin = bin_offsets[home];
     const int homes = bin_offsets[home + 1] - begin;
@@ -814,12 +849,10 @@ __global__ void row_fill_kernel(
 // ---------------------------------------------------------------------------------------
 // Total, overflow and padding, in one launch over the capacity.
 
-// Every thread derives the total from the last count and offset. Column k at or past the
-// total holds the self-pair (k mod N, k mod N), spreading their zero gradients over the atoms;
-// the threads start at the total and step by the grid, so each takes one remainder and the
-// stores are whole lines. The first thread stores the total and, above the capacity, the
-// overflow bit and the pairs needed; with an overflow there is no padding column, so the gate's
-// read of the status cannot race.
+// Every thread derives the total from the last count and offset. The first thread stores the
+// total and, above the capacity, the overflow bit and the pairs needed; with an overflow there is
+// no padding column, so the gate's read of the status cannot race. A list whose fill has padded
+// already (`pad` zero) needs the first thread only.
 __global__ void total_and_pad_kernel(
     const index_t* __restrict__ pair_counts,
     const index_t* __restrict__ pair_offsets,
@@ -828,7 +861,8 @@ __global__ void total_and_pad_kernel(
     index_t* __restrict__ pair_total,
     index_t* __restrict__ pairs,
     index_t* __restrict__ status,
-    const index_t* __restrict__ rebuild
+    const index_t* __restrict__ rebuild,
+    int pad
 )
 {
     if (!rebuilding(rebuild, status))
@@ -846,25 +880,19 @@ __global__ void total_and_pad_kernel(
             status[1] = total > status[1] ? total : status[1];
         }
     }
-    if (total >= capacity)
+    if (pad)
     {
-        return;
-    }
-    const unsigned n = static_cast<unsigned>(num_atoms);
-    const unsigned end = static_cast<unsigned>(capacity);
-    const unsigned stride = gridDim.x * blockDim.x, step = stride % n;
-    unsigned column = static_cast<unsigned>(total) + thread;  // below 2^32: the grid is bounded
-    unsigned atom = column % n;
-    for (; column < end; column += stride)
-    {
-        pairs[column] = static_cast<index_t>(atom);
-        pairs[static_cast<std::int64_t>(capacity) + column] = static_cast<index_t>(atom);
-        atom += step;
-        atom -= atom >= n ? n : 0u;
+        pad_columns(total, num_atoms, capacity, pairs, thread, gridDim.x * blockDim.x);
     }
 }
 
 constexpr std::int64_t kPadBlocks = 148 * 8;  // every SM full; more columns take more steps
+
+// The fill's CTAs that pad: few, because each takes a slot from the fill, and one more per 2^21
+// columns of capacity, so that a roomy list's padding does not outlast the fill (1,048,576 atoms,
+// fill and padding: 24 CTAs 537 us, 48 CTAs 539 us, 148 CTAs 583 us, a launch of its own 592 us).
+constexpr std::int64_t kPadCtas = 37;
+constexpr std::int64_t kPadColumns = 1 << 21;
 
 // ---------------------------------------------------------------------------------------
 // The update's gate (the rule of src/nabladyn/neighbors/csrc/update/update.cuh:13-20).
@@ -1094,18 +1122,22 @@ int launch_grid(const T* positions, std::int64_t n, const List& list, cudaStream
 }
 
 template <typename T, bool kFill>
-void launch_hood(const T* cell, double radius, const List& list, const Commit<T>& commit,
-                 cudaStream_t stream)
+void launch_hood(const T* cell, std::int64_t n, double radius, const List& list,
+                 const Commit<T>& commit, cudaStream_t stream)
 {
     const nd_neighbor_buffers& b = *list.b;
     const T r = static_cast<T>(radius);
     const std::int64_t bins = b.num_bin_slots - 1;
+    const std::int64_t most = std::min<std::int64_t>(blocks_for(b.capacity), kPadBlocks);
+    const std::int64_t pad =
+        kFill ? std::min(most, std::max(kPadCtas, b.capacity / kPadColumns)) : 0;
     auto launch = [&](auto kernel, int threads) {
-        kernel<<<static_cast<unsigned>(bins), threads, 0, stream>>>(
+        kernel<<<static_cast<unsigned>(bins + pad), threads, 0, stream>>>(
             static_cast<const T*>(b.sorted_positions), b.sorted_ids, b.bin_offsets, b.dims, cell,
             r * r, b.pair_counts, b.pair_offsets, static_cast<index_t>(b.capacity), b.pairs,
             commit.positions, commit.reference_positions, commit.reference_cell,
-            commit.rebuild_count, list.rebuild, b.status);
+            commit.rebuild_count, list.rebuild, b.status, static_cast<index_t>(n),
+            static_cast<int>(pad));
     };
     if (bins <= kHoodFewBins)
     {
@@ -1137,7 +1169,7 @@ int launch_count(const T* positions, const T* cell, std::int64_t n, double radiu
     }
     else
     {
-        launch_hood<T, false>(cell, radius, list, Commit<T>{}, stream);
+        launch_hood<T, false>(cell, n, radius, list, Commit<T>{}, stream);
     }
     ND_LAUNCH_CHECK();
     ND_CUDA_TRY(scan_exclusive(b.pair_counts, b.pair_offsets, n, b.scan_temp, list.rebuild,
@@ -1161,14 +1193,15 @@ int launch_fill(const T* cell, std::int64_t n, double radius, const List& list,
     }
     else
     {
-        launch_hood<T, true>(cell, radius, list, commit, stream);
+        launch_hood<T, true>(cell, n, radius, list, commit, stream);
     }
     ND_LAUNCH_CHECK();
-    const auto pad_blocks = static_cast<unsigned>(
-        std::min<std::int64_t>(blocks_for(b.capacity), kPadBlocks));
-    total_and_pad_kernel<<<pad_blocks, kThreads, 0, stream>>>(
+    const bool pad = list.all_pairs();  // the grid's fill has padded
+    const std::int64_t pad_blocks =
+        pad ? std::min<std::int64_t>(blocks_for(b.capacity), kPadBlocks) : 1;
+    total_and_pad_kernel<<<static_cast<unsigned>(pad_blocks), kThreads, 0, stream>>>(
         b.pair_counts, b.pair_offsets, num_atoms, capacity, b.pair_total, b.pairs, b.status,
-        list.rebuild);
+        list.rebuild, pad);
     ND_LAUNCH_CHECK();
     return ND_OK;
 }

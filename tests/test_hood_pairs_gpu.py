@@ -84,3 +84,22 @@ def test_first_frame_starts_the_list(cuda, dtype):
     assert torch.equal(held["reference_cell"], cell) and held["limits"].tolist() == [8, 4, 4]
     listed.update(x, cell)
     assert listed._rebuild_count == 1
+
+
+@pytest.mark.parametrize("multiplier", (1.0, 1.3, 40.0))
+@pytest.mark.parametrize("atoms", (1300, 40001))
+def test_columns_past_the_total_are_self_pairs(cuda, atoms, multiplier):
+    """The padding that some CTAs of the fill write: column k holds (k mod N, k mod N), after a
+    tight, an ordinary and a roomy capacity (the largest takes more padding CTAs), and after an
+    update that rebuilds."""
+    rng = np.random.default_rng(atoms)
+    side = (atoms / 14.0) ** (1 / 3)
+    cell = torch.full((3,), side, device=cuda)
+    x = torch.tensor(rng.uniform(0, side, (atoms, 3)), dtype=torch.float32, device=cuda)
+    listed = NeighborList(1.0, skin=0.0, capacity_multiplier=multiplier)
+    listed.allocate(x, cell)
+    for _ in range(2):
+        index = listed.tensors().index.cpu().numpy()
+        columns = np.arange(listed.num_pairs, index.shape[1])
+        np.testing.assert_array_equal(index[:, listed.num_pairs:], [columns % atoms] * 2)
+        listed.update(x + 0.3, cell)
