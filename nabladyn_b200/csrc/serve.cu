@@ -796,10 +796,13 @@ __global__ void __launch_bounds__(kServeThreads, 1) serve_kernel(ServePool p, co
     const bool grid = r.dims[0] >= 3 && r.dims[1] >= 3 && r.dims[2] >= 3;
     const index_t* order = grid ? sorted : nullptr;
     // The sums of every 32 rows: in the cell counts' shared memory when one CTA owns the replica
-    // and they fit, else in the rebuild's scratch array (both idle outside a rebuild).
+    // and they fit, else in the rebuild's scratch array (both idle outside a rebuild), from its
+    // first 8-byte boundary on: a replica's room may begin at any atom.
     const int units = (r.n + kWarp - 1) / kWarp;
     const bool in_shared = team.size == 1 && 2 * units * sizeof(double) <= sizeof(counts);
-    double* kinetic_sums = reinterpret_cast<double*>(in_shared ? counts : scratch);
+    auto* aligned = reinterpret_cast<double*>(
+        (reinterpret_cast<std::uintptr_t>(scratch) + 7u) & ~std::uintptr_t{7});
+    double* kinetic_sums = in_shared ? reinterpret_cast<double*>(counts) : aligned;
     double* energy_sums = kinetic_sums + units;
     // The team's status bits from every CTA's slot.
     auto told = [&](const int* slots_by_rank) {

@@ -7,7 +7,7 @@ the team, so nothing is left to a tolerance."""
 import numpy as np
 import pytest
 
-from nabladyn_b200.serving import ReplicaRequest, ReplicaServer
+from nabladyn_b200.serving import ReplicaRequest, ReplicaServer, _server
 
 pytestmark = pytest.mark.gpu
 
@@ -44,3 +44,24 @@ def test_every_team_gives_the_same_bits(cuda, monkeypatch, cells, atoms):
         np.testing.assert_array_equal(other.velocities, one.velocities)
         np.testing.assert_array_equal(other.images, one.images)
         assert (other.energy, other.rebuilds, other.status) == (one.energy, one.rebuilds, 0)
+
+
+@pytest.mark.parametrize("team", (1, 2, 8))
+def test_a_room_that_begins_at_an_odd_atom(cuda, monkeypatch, team):
+    """The per-32-row sums of a team lie in per-atom memory: a replica whose room begins at atom
+    33 (and one of 33,000 atoms, whose sums a single CTA keeps there as well) gives the bits it
+    gives at atom 0."""
+    monkeypatch.setattr(ReplicaServer, "_team", lambda self, active, work: team)
+    atoms = 33000 if team == 1 else 4000
+    first = lattice_request((5, 5, 5), 20, 3, seed=1)
+    request = lattice_request((21, 21, 21) if team == 1 else (10, 10, 10), atoms, 12, seed=2)
+    alone = ReplicaServer(device=cuda, budget_bytes=64 << 20, max_slots=2)
+    expected = alone.serve([request], realtime=False)[0]
+    monkeypatch.setattr(_server, "_ALIGN", 33)
+    server = ReplicaServer(device=cuda, budget_bytes=64 << 20, max_slots=2, large_atoms=None)
+    results = {r.num_atoms: r for r in server.serve([first, request], realtime=False)}
+    got = results[atoms]
+    assert got.status == expected.status == 0 and got.steps == 12
+    np.testing.assert_array_equal(got.positions, expected.positions)
+    np.testing.assert_array_equal(got.velocities, expected.velocities)
+    assert got.energy == expected.energy
