@@ -296,7 +296,11 @@ __global__ void __launch_bounds__(kTile, 4) tangent_forward_kernel(TangentPass a
     cores.close(128);
 }
 
-// The reverse pass. A tile's steps form one long chain (four products with row-wise work between
+// The reverse pass. 32,768 beads, 1.19 million pairs: 1,200 -> 608 us (the forward pass 520 ->
+// 228 us), bound by the latency of a tile's steps and the shared-memory passes (59 % of the
+// wavefronts), then by the 1.3 GB of rows it writes (28 % of the DRAM's peak).
+//
+// A tile's steps form one long chain (four products with row-wise work between
 // them), so two CTAs share an SM (tensor memory holds no more: z, z_dot, u and u_dot are 256
 // columns) and each gives a tile 256 threads: thread t computes columns 32 (t / 128) .. + 31 of
 // row t % 128 in the row-wise steps. In the scatter, eight lanes take a row's 32 staged columns
