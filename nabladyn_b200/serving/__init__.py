@@ -2,7 +2,8 @@
 
 ``ReplicaServer`` keeps replicas resident in one device pool, admits requests as slots and HBM
 budget free up, advances every active replica by a per-replica budget of NVT steps in one
-launch of the replica kernel (nd_serve_run: one CTA per replica, whole steps inside the CTA),
+launch of the replica kernel (nd_serve_run_teams: a CTA or a cluster per replica, whole steps
+inside it),
 and hands back each finished replica's frame with its latency.
 """
 
