@@ -912,7 +912,8 @@ int lj_pairs(const nd_lj_pairs_args* a, cudaStream_t stream)
 // slots it is bound by the float64 arithmetic: the row's constants are worked out once per
 // block, and a thread keeps its rows' sums to itself (in registers for one row, else in its own
 // column of shared memory), since float64 atomics on a few shared words serialise the block
-// (64 frames of 4,096 atoms, two types, float32: 778 -> 118 us).
+// (64 frames of 4,096 atoms, two types, float32: 778 -> 99 us; gathering the force gradients before
+// the cutoff test, or six blocks per SM at 40 registers, gave 100).
 
 // One type-pair row's float64 constants.
 struct RowGradients
@@ -1012,10 +1013,19 @@ __global__ void __launch_bounds__(kLJThreads) lj_parameter_backward_kernel(Backw
     const index_t* firsts = f.pairs;
     const index_t* seconds = f.pairs + f.capacity;
     const unsigned stride = gridDim.x * kLJThreads;
-    for (unsigned column = blockIdx.x * kLJThreads + threadIdx.x; column < capacity;
-         column += stride)
+    // A column's atoms are read one column ahead: its gathers then wait for one load, not two.
+    unsigned column = blockIdx.x * kLJThreads + threadIdx.x;
+    index_t next_i = column < capacity ? firsts[column] : 0;
+    index_t next_j = column < capacity ? seconds[column] : 0;
+    while (column < capacity)
     {
-        const index_t i = firsts[column], j = seconds[column];
+        const index_t i = next_i, j = next_j;
+        column += stride;
+        if (column < capacity)
+        {
+            next_i = firsts[column];
+            next_j = seconds[column];
+        }
         if (!counts(i, j, f.num_atoms))
         {
             continue;
@@ -1084,28 +1094,31 @@ __global__ void __launch_bounds__(kLJThreads) lj_parameter_backward_kernel(Backw
     }
 }
 
+// As many blocks as the GPU holds at once: with eight per SM, of which five fit, the second wave
+// left two SMs in five idle (64 frames of 4,096 atoms: 118 us, in one wave 99).
 template <typename T, bool kPacked>
 int launch_backward(const BackwardPass<T>& pass, std::int64_t frames, cudaStream_t stream)
 {
+    const bool types = pass.frames.num_types > 1;
+    const int rows = pass.frames.num_types * (pass.frames.num_types + 1) / 2;
+    const std::size_t bytes = types ? 2 * rows * kLJThreads * sizeof(double) : 0;
+    auto* kernel = types ? lj_parameter_backward_kernel<T, kPacked, true>
+                         : lj_parameter_backward_kernel<T, kPacked, false>;
+    if (types)
+    {
+        static DeviceGrant grant;
+        ND_CUDA_TRY(grant.allow(lj_parameter_backward_kernel<T, kPacked, true>, bytes));
+    }
+    int resident = 1;
+    ND_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, kLJThreads, bytes));
     unsigned blocks = 1;
-    const int counted = frame_blocks<kLJThreads>(pass.frames.capacity, frames, 8, &blocks);
+    const int counted =
+        frame_blocks<kLJThreads>(pass.frames.capacity, frames, std::max(1, resident), &blocks);
     if (counted != ND_OK)
     {
         return counted;
     }
-    const dim3 grid(blocks, static_cast<unsigned>(frames));
-    if (pass.frames.num_types == 1)
-    {
-        lj_parameter_backward_kernel<T, kPacked, false><<<grid, kLJThreads, 0, stream>>>(pass);
-    }
-    else
-    {
-        const int rows = pass.frames.num_types * (pass.frames.num_types + 1) / 2;
-        const std::size_t bytes = 2 * rows * kLJThreads * sizeof(double);
-        static DeviceGrant grant;
-        ND_CUDA_TRY(grant.allow(lj_parameter_backward_kernel<T, kPacked, true>, bytes));
-        lj_parameter_backward_kernel<T, kPacked, true><<<grid, kLJThreads, bytes, stream>>>(pass);
-    }
+    kernel<<<dim3(blocks, static_cast<unsigned>(frames)), kLJThreads, bytes, stream>>>(pass);
     ND_LAUNCH_CHECK();
     return ND_OK;
 }
