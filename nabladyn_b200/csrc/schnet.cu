@@ -1054,6 +1054,10 @@ __global__ void __launch_bounds__(kAtomThreads) atom_reverse_kernel(AtomPass a)
 
 // E and W from the per-CTA partials in a fixed order: a warp per sum.
 constexpr int kFinalizeWarps = 10;
+// Partials a lane loads before it adds any: all of its own when the last pass runs 592 CTAs (four
+// per SM). Loaded as they are added they were a chain of round trips to L2: 7.5 -> 2.5 us, at the
+// end of an evaluation whose every launch waits for the one before.
+constexpr int kFinalizeLoads = 19;
 
 __global__ void __launch_bounds__(kFinalizeWarps * 32) finalize_kernel(
     const double* __restrict__ energy_partials, int energy_count,
@@ -1064,10 +1068,20 @@ __global__ void __launch_bounds__(kFinalizeWarps * 32) finalize_kernel(
     const double* from = sum == 0 ? energy_partials : virial_partials + (sum - 1);
     const int count = sum == 0 ? energy_count : virial_count, stride = sum == 0 ? 1 : 9;
     double value = 0.0;
-#pragma unroll 8
-    for (int i = lane; i < count; i += 32)
+    for (int base = lane; base < count; base += 32 * kFinalizeLoads)
     {
-        value += from[static_cast<std::int64_t>(stride) * i];
+        double part[kFinalizeLoads];
+#pragma unroll
+        for (int k = 0; k < kFinalizeLoads; ++k)
+        {
+            const int i = base + 32 * k;
+            part[k] = i < count ? from[static_cast<std::int64_t>(stride) * i] : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < kFinalizeLoads; ++k)
+        {
+            value += part[k];
+        }
     }
     value = warp_sum(value);
     double* to = sum == 0 ? energy : (virial != nullptr ? virial + (sum - 1) : nullptr);
