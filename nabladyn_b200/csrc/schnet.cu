@@ -21,7 +21,8 @@
 // forward, and its reverse) run in persistent CTAs that keep their weight images in shared
 // memory; the atom-wise products in one CTA per 128 atoms. Everything else is FP32, the
 // energy and virial sums FP64 in a fixed order. The feature rows the pair kernels gather
-// (v and Gm) are stored in BF16; messages, their reverse and forces are summed in FP32.
+// (v and Gm) are stored in BF16; messages, their reverse and forces are summed in FP32, in an
+// order that is fixed up to the atomics (add_runs in schnet.cuh).
 
 #include "schnet.cuh"
 
@@ -254,14 +255,14 @@ struct PairPass
 // shared-memory passes between products and the atomics, in a chain of dependent steps per tile;
 // the tensor pipe is busy 8 % of the time. A row's features are gathered and scattered by eight
 // lanes, 16 bytes each, so a warp's load covers four whole rows; with a thread per row each load
-// touched 32. 32,768 beads, 1.19 million pairs: forward 269 -> 136 us, reverse 533 -> 250 us,
-// the E/F/W call 2,210 -> 1,290 us. Unrolled over the two column halves the kernels overflow the
+// touched 32. 32,768 beads, 1.19 million pairs: forward 269 -> 157 us, reverse 533 -> 300 us (the
+// last pass 241), the E/F/W call 2,210 -> 1,510 us. Unrolled over the two column halves the kernels overflow the
 // instruction cache, so those loops stay rolled.
 //
 // The reverse pass's row tile has its 16-byte chunks 144 bytes and its eight-row groups 1,216
 // bytes apart: the eight lanes that write one row, four rows at a time, then spread over the
 // shared-memory banks.
-constexpr int kPairTail = 2 * 256 + 4 * kTile * 4 + 64;
+constexpr int kPairTail = 2 * 256 + 3 * kTile * 4 + 64;
 constexpr int kReverseChunk = 144, kReverseGroup = 8 * kReverseChunk + 64;
 constexpr int kReverseTileBytes = kTile / 8 * kReverseGroup;
 constexpr int kPairForwardShared = 2 * umma::kImageBytes + umma::kTileBytes + kPairTail;
@@ -279,7 +280,6 @@ struct PairShared
     int* first;       // -1: a dead row
     int* second;
     float* envelope;  // reverse
-    float* along;     // reverse
     std::uint64_t* barrier;
 
     __device__ PairShared(unsigned char* shared, bool reverse)
@@ -293,8 +293,7 @@ struct PairShared
         first = reinterpret_cast<int*>(bias2 + kFeatures);
         second = first + kTile;
         envelope = reinterpret_cast<float*>(second + kTile);
-        along = envelope + kTile;
-        barrier = reinterpret_cast<std::uint64_t*>(along + kTile);
+        barrier = reinterpret_cast<std::uint64_t*>(envelope + kTile);
     }
 
     __device__ void load_biases(const PairPass& a)
@@ -386,18 +385,16 @@ __global__ void __launch_bounds__(kTile, 6) pair_forward_kernel(PairPass a)
             }
             stage_half(cores.tmem + 32 * half, sh.bias2 + 32 * half, envelope, sh.stage);
             __syncwarp();
-            RunSums<1> run;
-            run.start(sh.first[at.row(0)]);
-            float4* const targets[1] = {m4 + at.word(0, half)};
-            float4 va = widen4(__ldg(v + at.word(max(run.key, 0), half)));
+            int key = sh.first[at.row(0)];
+            float4 va = widen4(__ldg(v + at.word(max(key, 0), half)));
 #pragma unroll
             for (int i = 0; i < kLaneRows; ++i)
             {
                 const int row = at.row(i);
                 const int first = sh.first[row];
-                if (first != run.key)
+                if (first != key)
                 {
-                    run.turn(first, targets);
+                    key = first;
                     va = widen4(__ldg(v + at.word(max(first, 0), half)));
                 }
                 const float4 f = staged4(sh.stage, row, at.lane);
@@ -405,37 +402,14 @@ __global__ void __launch_bounds__(kTile, 6) pair_forward_kernel(PairPass a)
                 {
                     atomicAdd(m4 + at.word(sh.second[row], half), f * va);
                 }
-                run.sums[0] = run.sums[0] + f * widen4(vb[i]);
+                restage4(sh.stage, row, at.lane, f * widen4(vb[i]));
             }
-            run.finish(targets, at.group);
+            __syncwarp();
+            add_runs(sh.stage, sh.first, at.warp_row, a.m + 32 * half + (threadIdx.x & 31));
             __syncwarp();  // the stage's rows are this warp's own: its next writes come after
         }
     }
     cores.close(64);
-}
-
-// Eight values per lane, summed over the eight lanes of each group: lane l returns the sum of
-// value l.
-__device__ __forceinline__ float sum_across(const float (&values)[8], int lane)
-{
-    float four[4], two[2];
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-    {
-        const float keep = (lane & 4) ? values[k + 4] : values[k];
-        const float give = (lane & 4) ? values[k] : values[k + 4];
-        four[k] = keep + __shfl_xor_sync(kFullMask, give, 4);
-    }
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-    {
-        const float keep = (lane & 2) ? four[k + 2] : four[k];
-        const float give = (lane & 2) ? four[k] : four[k + 2];
-        two[k] = keep + __shfl_xor_sync(kFullMask, give, 2);
-    }
-    const float keep = (lane & 1) ? two[1] : two[0];
-    const float give = (lane & 1) ? two[0] : two[1];
-    return keep + __shfl_xor_sync(kFullMask, give, 1);
 }
 
 // kLast: the last pass (block 0) has no Gv to scatter and applies forces and virial.
@@ -510,7 +484,7 @@ __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
             break;
         }
         // f_raw, Gf = Gm_a v_b + Gm_b v_a, Gf . f_raw, Gv, and Gf C into the work tile.
-        float along[kLaneRows] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        float along = 0.0f;
 #pragma unroll 1
         for (int half = 0; half < 2; ++half)
         {
@@ -524,26 +498,18 @@ __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
             }
             stage_half(cores.tmem + 64 + 32 * half, sh.bias2 + 32 * half, 1.0f, sh.stage);
             __syncwarp();
-            RunSums<1> run;
-            run.start(sh.first[at.row(0)]);
-            float4* const targets[1] = {gv4 + at.word(0, half)};
-            float4 va = widen4(__ldg(v + at.word(max(run.key, 0), half)));
-            float4 ma = widen4(__ldg(gm + at.word(max(run.key, 0), half)));
+            int key = sh.first[at.row(0)];
+            float4 va = widen4(__ldg(v + at.word(max(key, 0), half)));
+            float4 ma = widen4(__ldg(gm + at.word(max(key, 0), half)));
+            float4 to_first[kLaneRows];
 #pragma unroll
             for (int i = 0; i < kLaneRows; ++i)
             {
                 const int row = at.row(i);
                 const int first = sh.first[row];
-                if (first != run.key)
+                if (first != key)
                 {
-                    if (kLast)
-                    {
-                        run.key = first;
-                    }
-                    else
-                    {
-                        run.turn(first, targets);
-                    }
+                    key = first;
                     const std::int64_t word = at.word(max(first, 0), half);
                     va = widen4(__ldg(v + word));
                     ma = widen4(__ldg(gm + word));
@@ -551,8 +517,8 @@ __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
                 const float envelope = sh.envelope[row];
                 const float4 raw = staged4(sh.stage, row, at.lane);
                 const float4 right = widen4(vb[i]), right_gm = widen4(mb[i]);
-                const float4 gf = ma * right + right_gm * va;
-                along[i] += sum4(gf * raw);
+                const float4 gf = fma4(ma, right, right_gm * va);
+                restage4(sh.stage, row, at.lane, gf);
                 if (!kLast)
                 {
                     const float4 scaled = raw * envelope;
@@ -560,7 +526,7 @@ __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
                     {
                         atomicAdd(gv4 + at.word(sh.second[row], half), scaled * ma);
                     }
-                    run.sums[0] = run.sums[0] + scaled * right_gm;
+                    to_first[i] = scaled * right_gm;
                 }
                 *reinterpret_cast<uint2*>(sh.work + (row >> 3) * kReverseGroup +
                                           (4 * half + at.lane / 2) * kReverseChunk +
@@ -568,13 +534,39 @@ __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
                     make_uint2(pack2(gf.x * envelope, gf.y * envelope),
                                pack2(gf.z * envelope, gf.w * envelope));
             }
+            __syncwarp();
+            // Gf . f_raw of this thread's own row, in column order.
+#pragma unroll
+            for (int part = 0; part < 2; ++part)
+            {
+                float raw[16];
+                umma::load16(cores.tmem + 64 + 32 * half + 16 * part, raw);
+                umma::wait_loads();
+                const float* bias = sh.bias2 + 32 * half + 16 * part;
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                {
+                    const float4 gf = staged4(sh.stage, threadIdx.x, 4 * part + q);
+                    along = fmaf(gf.x, raw[4 * q] + bias[4 * q], along);
+                    along = fmaf(gf.y, raw[4 * q + 1] + bias[4 * q + 1], along);
+                    along = fmaf(gf.z, raw[4 * q + 2] + bias[4 * q + 2], along);
+                    along = fmaf(gf.w, raw[4 * q + 3] + bias[4 * q + 3], along);
+                }
+            }
+            __syncwarp();
             if (!kLast)
             {
-                run.finish(targets, at.group);
+#pragma unroll
+                for (int i = 0; i < kLaneRows; ++i)
+                {
+                    restage4(sh.stage, at.row(i), at.lane, to_first[i]);
+                }
+                __syncwarp();
+                add_runs(sh.stage, sh.first, at.warp_row,
+                         a.grad_v + 32 * half + (threadIdx.x & 31));
+                __syncwarp();  // the stage's rows are this warp's own: its next writes come after
             }
-            __syncwarp();  // the stage's rows are this warp's own: its next writes come after
         }
-        sh.along[at.row(at.lane)] = sum_across(along, at.lane);
         if (!product(64, sh.image_b2, true, 3))
         {
             break;
@@ -622,7 +614,7 @@ __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
                     for (int e = 0; e < 8; ++e)
                     {
                         const float offset = t - static_cast<float>(32 * half + 8 * c + e);
-                        through -= u[8 * c + e] * gaussian(offset) * offset;
+                        through -= u[8 * c + e] * gaussian_flushed(offset) * offset;
                     }
                 }
             }
@@ -630,7 +622,7 @@ __global__ void __launch_bounds__(kTile, 4) pair_reverse_kernel(PairPass a)
         if (ab.x >= 0)
         {
             const float slope = -0.5f * a.phase * sine;
-            float total = slope * sh.along[threadIdx.x] + through / a.width;
+            float total = slope * along + through / a.width;
             if (!a.first)
             {
                 total += a.dedr[p];

@@ -129,8 +129,12 @@ __device__ __forceinline__ float softplus_shifted(float x)
     return fmaxf(x, 0.0f) + log2 * kLn2 - kLn2;
 }
 
-// The Gaussian exp(-u^2 / 2); below the smallest normal number it is zero.
-__device__ __forceinline__ float gaussian(float u)
+// The Gaussian exp(-u^2 / 2). As an operand of the tensor cores it keeps denormal results: their
+// sums can lose the last bit to a product that lies below it. Where FP32 arithmetic weights it, a
+// value below the smallest normal number changes nothing and is zero (three operations fewer).
+__device__ __forceinline__ float gaussian(float u) { return __expf(-0.5f * u * u); }
+
+__device__ __forceinline__ float gaussian_flushed(float u)
 {
     return exp2_approx(-0.5f * u * u * kLog2E);
 }
@@ -339,8 +343,8 @@ __device__ __forceinline__ void store_basis(unsigned char* tile, float r_over_wi
 // through shared memory (stage4: 16 KB, chunks swizzled by row), and eight lanes take a
 // row of it, four features each, four rows of the warp's 32 at a time: a gathered half row is
 // one 64-byte segment, a scattered one a whole 128-byte line. A lane meets rows 8 group + i,
-// i = 0 .. 7, in the list's order, so the first atom's side is summed in registers along its
-// run and added once per run, warp and half.
+// i = 0 .. 7, and leaves the first atoms' side in the stage, where add_runs sums it along the
+// runs, one atomic per run, warp and column.
 constexpr int kLaneRows = 8;  // rows a lane meets per half tile
 
 struct FeatureLane
@@ -385,92 +389,76 @@ __device__ __forceinline__ float4 operator*(const float4& a, float b)
     return make_float4(a.x * b, a.y * b, a.z * b, a.w * b);
 }
 
-__device__ __forceinline__ float4 operator+(const float4& a, const float4& b)
+// a b + c, rounded once: which product of a sum of two is rounded by itself is written out, since
+// a compiler chooses differently from one kernel to the next.
+__device__ __forceinline__ float4 fma4(const float4& a, const float4& b, const float4& c)
 {
-    return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+    return make_float4(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y), fmaf(a.z, b.z, c.z),
+                       fmaf(a.w, b.w, c.w));
 }
 
-__device__ __forceinline__ float sum4(const float4& a) { return (a.x + a.y) + (a.z + a.w); }
-
-// First-atom sums of a warp's rows. A group sums its rows along each run and adds the runs that
-// begin and end inside them; its first and last runs, which its neighbours may share, wait for
-// the end, where the groups meet: so a run costs one atomic per warp and column, and two calls
-// differ only in the order of the warps' atomics.
-template <int kSums, int kGroups = 4>
-struct RunSums
+// Replaces four features of a staged half row.
+__device__ __forceinline__ void restage4(float* stage, int row, int lane, float4 value)
 {
-    int key;       // the present run's first atom (-1: dead rows)
-    int head_key;  // the first run's, once it ended; kOpen before
-    float4 sums[kSums], head[kSums];
-    static constexpr int kOpen = -2;
+    reinterpret_cast<float4*>(stage)[row * 8 + (lane ^ (row & 7))] = value;
+}
 
-    __device__ __forceinline__ void start(int first)
-    {
-        key = first;
-        head_key = kOpen;
-#pragma unroll
-        for (int s = 0; s < kSums; ++s)
+// First-atom sums of a warp's 32 staged half rows from `begin` on, a lane per column: each run of
+// one first atom (`first`; -1: dead rows) is summed row by row from zero and added once, to
+// `target` (this lane's column of atom 0's row) moved to the run's atom. The order is part of the
+// result: the sums feed BF16 operands, where an FP32 sum's last bit can turn a rounding. Sums
+// kept in the feature lanes' registers, their row groups joined by shuffles, cost no pass through
+// shared memory (32,768 beads: forward 129 us, reverse 242, the E/F/W call 1,287) but add the rows
+// in another order; with this pass 157, 300 and 1,510. An atomic per column is faster here than
+// one per four columns after shuffles (reverse 300 and 320 us).
+__device__ __forceinline__ void add_runs(const float* stage, const int* first, int begin,
+                                         float* target)
+{
+    constexpr int kAhead = 8;  // rows read before any is added
+    const int lane = threadIdx.x & 31;
+    const int atom = first[begin + lane];
+    const int after = __shfl_down_sync(kFullMask, atom, 1);
+    const unsigned ends = __ballot_sync(kFullMask, lane == 31 || after != atom);
+    const float* rows = stage + begin * 32;
+    float sum = 0.0f;
+    auto add = [&](int r) {
+        const int run = first[begin + r];
+        if (run >= 0)
         {
-            sums[s] = head[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+            atomicAdd(target + static_cast<std::int64_t>(run) * kFeatures, sum);
+        }
+        sum = 0.0f;
+    };
+#pragma unroll 1
+    for (int r0 = 0; r0 < 32; r0 += kAhead)
+    {
+        float part[kAhead];
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k)
+        {
+            part[k] = rows[(r0 + k) * 32 + (lane ^ (4 * k))];  // chunk (lane / 4) ^ (row % 8)
+        }
+        const unsigned inside = ends >> r0 & ((1u << kAhead) - 1u);
+        if (inside == 0)
+        {
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k)
+            {
+                sum += part[k];
+            }
+            continue;
+        }
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k)
+        {
+            sum += part[k];
+            if (inside & (1u << k))
+            {
+                add(r0 + k);
+            }
         }
     }
-
-    // Ends the present run when `first` starts another one. `targets` point to this lane's word
-    // of atom 0's row.
-    __device__ __forceinline__ void turn(int first, float4* const (&targets)[kSums])
-    {
-        const bool opening = head_key == kOpen;
-#pragma unroll
-        for (int s = 0; s < kSums; ++s)
-        {
-            if (opening)
-            {
-                head[s] = sums[s];
-            }
-            else if (key >= 0)
-            {
-                atomicAdd(targets[s] + 16 * static_cast<std::int64_t>(key), sums[s]);
-            }
-            sums[s] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        head_key = opening ? key : head_key;
-        key = first;
-    }
-
-    __device__ __forceinline__ void finish(float4* const (&targets)[kSums], int group)
-    {
-        while (true)
-        {
-            const unsigned open = __ballot_sync(kFullMask, head_key >= 0 || key >= 0);
-            if (open == 0)
-            {
-                break;
-            }
-            const int atom =
-                __shfl_sync(kFullMask, head_key >= 0 ? head_key : key, __ffs(open) - 1);
-#pragma unroll
-            for (int s = 0; s < kSums; ++s)
-            {
-                const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-                float4 total = (head_key == atom ? head[s] : zero) + (key == atom ? sums[s] : zero);
-#pragma unroll
-                for (int offset = 32 / kGroups; offset < 32; offset *= 2)
-                {
-                    total.x += __shfl_xor_sync(kFullMask, total.x, offset);
-                    total.y += __shfl_xor_sync(kFullMask, total.y, offset);
-                    total.z += __shfl_xor_sync(kFullMask, total.z, offset);
-                    total.w += __shfl_xor_sync(kFullMask, total.w, offset);
-                }
-                if (group == 0)
-                {
-                    atomicAdd(targets[s] + 16 * static_cast<std::int64_t>(atom), total);
-                }
-            }
-            head_key = head_key == atom ? kOpen : head_key;
-            key = key == atom ? -1 : key;
-        }
-    }
-};
+}
 
 // Stages float4 `q` (columns 4 q .. 4 q + 3 of the half) of this thread's row.
 __device__ __forceinline__ void stage4(float* stage, int q, float4 value)

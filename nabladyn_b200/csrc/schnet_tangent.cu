@@ -259,45 +259,44 @@ __global__ void __launch_bounds__(kTile, 4) tangent_forward_kernel(TangentPass a
                     {
                         const float raw_filter = u[4 * q + e] + bias[4 * q + e];
                         f[e] = raw_filter * t.envelope;
-                        fd[e] = ud[4 * q + e] * t.envelope + raw_filter * t.moving;
+                        fd[e] = fmaf(raw_filter, t.moving, ud[4 * q + e] * t.envelope);
                     }
                     stage4(stage, q, make_float4(f[0], f[1], f[2], f[3]));
                     stage4(stage_dot, q, make_float4(fd[0], fd[1], fd[2], fd[3]));
                 }
             }
             __syncwarp();
-            RunSums<1> run;
-            run.start(first[at.row(0)]);
-            float4* const targets[1] = {md4 + at.word(0, half)};
-            float4 va = widen4(__ldg(v + at.word(max(run.key, 0), half)));
-            float4 vda = widen4(__ldg(v_dot + at.word(max(run.key, 0), half)));
+            int key = first[at.row(0)];
+            float4 va = widen4(__ldg(v + at.word(max(key, 0), half)));
+            float4 vda = widen4(__ldg(v_dot + at.word(max(key, 0), half)));
 #pragma unroll
             for (int i = 0; i < kLaneRows; ++i)
             {
                 const int row = at.row(i);
                 const int atom = first[row];
-                if (atom != run.key)
+                if (atom != key)
                 {
-                    run.turn(atom, targets);
+                    key = atom;
                     va = widen4(__ldg(v + at.word(max(atom, 0), half)));
                     vda = widen4(__ldg(v_dot + at.word(max(atom, 0), half)));
                 }
                 const float4 f = staged4(stage, row, at.lane), fd = staged4(stage_dot, row, at.lane);
                 if (atom >= 0)
                 {
-                    atomicAdd(md4 + at.word(second[row], half), fd * va + f * vda);
+                    atomicAdd(md4 + at.word(second[row], half), fma4(fd, va, f * vda));
                 }
-                run.sums[0] = run.sums[0] + (fd * widen4(vb[i]) + f * widen4(vdb[i]));
+                restage4(stage, row, at.lane, fma4(fd, widen4(vb[i]), f * widen4(vdb[i])));
             }
-            run.finish(targets, at.group);
+            __syncwarp();
+            add_runs(stage, first, at.warp_row, a.m_dot + 32 * half + (threadIdx.x & 31));
             __syncwarp();  // the stages' rows are this warp's own: its next writes come after
         }
     }
     cores.close(128);
 }
 
-// The reverse pass. 32,768 beads, 1.19 million pairs: 1,200 -> 608 us (the forward pass 520 ->
-// 228 us), bound by the latency of a tile's steps and the shared-memory passes (59 % of the
+// The reverse pass. 32,768 beads, 1.19 million pairs: 1,200 -> 615 us (the forward pass 520 ->
+// 253 us), bound by the latency of a tile's steps and the shared-memory passes (59 % of the
 // wavefronts), then by the 1.3 GB of rows it writes (28 % of the DRAM's peak).
 //
 // A tile's steps form one long chain (four products with row-wise work between
@@ -364,8 +363,8 @@ __global__ void __launch_bounds__(kReverseThreads, 2) tangent_reverse_kernel(Tan
     float4* const vdbar4 = reinterpret_cast<float4*>(a.v_dot_bar);
     const int row = threadIdx.x % kTile, side = threadIdx.x / kTile;
     // The scatter's rows: 16 of the 32 that this warp and the one of the other side staged.
-    const int lane = threadIdx.x % 8, group = threadIdx.x % 32 / 8;
-    const int lane_row = 32 * (threadIdx.x / 32 % 4) + 16 * side + 4 * group;
+    const int lane = threadIdx.x % 8;
+    const int lane_row = 32 * (threadIdx.x / 32 % 4) + 16 * side + 4 * (threadIdx.x % 32 / 8);
 
     // Both streams' products of the tiles with an image (read the other way when transposed).
     auto products = [&](std::uint32_t column, const unsigned char* image, bool transposed) {
@@ -509,7 +508,7 @@ __global__ void __launch_bounds__(kReverseThreads, 2) tangent_reverse_kernel(Tan
                     {
                         const float raw_filter = u[4 * q + e] + bias2[column + 4 * q + e];
                         f[e] = raw_filter * envelope;
-                        fd[e] = ud[4 * q + e] * envelope + raw_filter * moving;
+                        fd[e] = fmaf(ud[4 * q + e], envelope, raw_filter * moving);
                     }
                     const int at = row * 8 + ((4 * side + q) ^ (row & 7));
                     reinterpret_cast<float4*>(stage)[at] = make_float4(f[0], f[1], f[2], f[3]);
@@ -518,9 +517,7 @@ __global__ void __launch_bounds__(kReverseThreads, 2) tangent_reverse_kernel(Tan
             }
             umma::fence_before_sync();
             __syncthreads();
-            RunSums<2> run;
-            run.start(first[lane_row]);
-            float4* const targets[2] = {vbar4 + place, vdbar4 + place};
+            int key = first[lane_row];
             float4 va, vda, ma, mda;
             auto load_first = [&](int atom) {
                 const std::int64_t word = 16 * static_cast<std::int64_t>(max(atom, 0)) + place;
@@ -529,39 +526,44 @@ __global__ void __launch_bounds__(kReverseThreads, 2) tangent_reverse_kernel(Tan
                 ma = widen4(__ldg(m_bar + word));
                 mda = widen4(__ldg(m_dot_bar + word));
             };
-            load_first(run.key);
+            load_first(key);
 #pragma unroll
             for (int i = 0; i < 4; ++i)
             {
                 const int r = lane_row + i;
                 const int atom = first[r];
-                if (atom != run.key)
+                if (atom != key)
                 {
-                    run.turn(atom, targets);
+                    key = atom;
                     load_first(atom);
                 }
                 const float envelope = envelopes[r], moving = movings[r];
                 const float4 f = staged4(stage, r, lane), fd = staged4(stage_dot, r, lane);
                 const float4 right_v = widen4(vb[i]), right_vd = widen4(vdb[i]);
                 const float4 right_m = widen4(mb[i]), right_md = widen4(mdb[i]);
-                const float4 fb = ma * right_v + right_m * va + mda * right_vd + right_md * vda;
-                const float4 fdb = mda * right_v + right_md * va;
+                const float4 fb = fma4(right_md, vda, fma4(mda, right_vd, fma4(ma, right_v, right_m * va)));
+                const float4 fdb = fma4(mda, right_v, right_md * va);
                 if (atom >= 0)
                 {
                     const std::int64_t word = 16 * static_cast<std::int64_t>(second[r]) + place;
-                    atomicAdd(vbar4 + word, f * ma + fd * mda);
+                    atomicAdd(vbar4 + word, fma4(f, ma, fd * mda));
                     atomicAdd(vdbar4 + word, f * mda);
                 }
-                run.sums[0] = run.sums[0] + (f * right_m + fd * right_md);
-                run.sums[1] = run.sums[1] + f * right_md;
-                const float4 ub = fb * envelope + fdb * moving, udb = fdb * envelope;
+                restage4(stage, r, lane, fma4(f, right_m, fd * right_md));
+                restage4(stage_dot, r, lane, f * right_md);
+                const float4 udb = fdb * envelope;
+                const float4 ub = fma4(fb, make_float4(envelope, envelope, envelope, envelope), fdb * moving);
                 const int to = 8 * (place & 1);
                 *reinterpret_cast<uint2*>(row_word(tile, r, place / 2) + to) =
                     make_uint2(pack2(ub.x, ub.y), pack2(ub.z, ub.w));
                 *reinterpret_cast<uint2*>(row_word(tile_dot, r, place / 2) + to) =
                     make_uint2(pack2(udb.x, udb.y), pack2(udb.z, udb.w));
             }
-            run.finish(targets, group);
+            __syncthreads();
+            // A warp sums 32 rows of one of the two stages: v_bar's or v_dot_bar's.
+            add_runs(side == 0 ? stage : stage_dot, first, 32 * (threadIdx.x / 32 % 4),
+                     (side == 0 ? a.v_bar : a.v_dot_bar) + 16 * step +
+                         32 * (threadIdx.x % 32 / 16) + threadIdx.x % 16);
             __syncthreads();  // the stages are written again, or the tiles read
         }
         cores.begin([&] { products(128, image_b2, true); });
