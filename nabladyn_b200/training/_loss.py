@@ -2,8 +2,8 @@
 
 The same scales and loss as src/nabladyn/training/_loss.py:26-46 and :105-125. On a GPU the
 loss of plain tensors and its first derivatives take one kernel each (nd_loss_forward,
-nd_loss_backward); anything else, such as a functorch transform, tensor weights or a second
-derivative, is computed by the torch operations that define it.
+nd_loss_backward); anything else, such as a functorch transform, tensor weights, batched
+gradients or a second derivative, is computed by torch operations.
 """
 
 import ctypes
@@ -45,11 +45,11 @@ def loss(predicted: Mapping[str, Tensor], labels: Mapping[str, Tensor],
     """
     if _one_kernel(predicted, labels, weights, scales, coefficients):
         names = tuple(predicted)
-        total, *terms = _Loss.apply(
+        total, *rest = _Loss.apply(
             tuple(float(weights[name]) for name in names),
             tuple(float(scales[name]) for name in names), coefficients,
             *(labels[name] for name in names), *(predicted[name] for name in names))
-        return total, dict(zip(names, terms))
+        return total, dict(zip(names, rest))
     return _defined(predicted, labels, weights, scales, coefficients)
 
 
@@ -63,12 +63,19 @@ def _defined(predicted, labels, weights, scales, coefficients):
     return sum(weights[name] * term for name, term in terms.items()), terms
 
 
+def _plain_context() -> bool:
+    """Whether nothing watches or transforms torch operations: no functorch transform,
+    forward-mode level, trace or dispatch mode, which see the operations of a formula and would
+    not see a kernel."""
+    return not (torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0
+                or torch.compiler.is_compiling() or torch.jit.is_tracing()
+                or torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack())
+
+
 def _one_kernel(predicted, labels, weights, scales, coefficients) -> bool:
-    """Whether the loss is one of plain CUDA tensors with number weights and scales, outside
-    every functorch transform, forward-mode level and trace."""
-    if (not 1 <= len(predicted) <= 3 or torch._C._are_functorch_transforms_active()
-            or forward_ad._current_level >= 0 or torch.compiler.is_compiling()
-            or torch.jit.is_tracing()):
+    """Whether the loss is one of plain CUDA tensors with number weights and scales, and nothing
+    watches its operations."""
+    if not 1 <= len(predicted) <= 3 or not _plain_context():
         return False
     first = next(iter(predicted.values()))
     if (not isinstance(first, Tensor) or not first.is_cuda or first.ndim == 0
@@ -93,10 +100,13 @@ def _one_kernel(predicted, labels, weights, scales, coefficients) -> bool:
 
 
 class _Loss(torch.autograd.Function):
-    """(L, t_c for every channel) of predictions, differentiable in the predictions.
+    """(L, t_c for every channel, their slopes dt_c/dX) of predictions, differentiable in the
+    predictions to any order.
 
-    The forward keeps the terms' slopes dt_c/dX, so the backward needs neither predictions nor
-    labels; those are saved for a second derivative alone.
+    The slopes are outputs, and all that is saved: the first derivative scales them and the second
+    differentiates them through this node again (dt_c/dX is linear in X), so nothing of the
+    predictions and labels is kept, a caller may overwrite them before the backward, and saved
+    tensors are released and hooked like those of any other operation.
     """
 
     @staticmethod
@@ -119,19 +129,22 @@ class _Loss(torch.autograd.Function):
             args.terms[c], args.gradients[c] = ptr(term), ptr(slopes[c])
         with on_device(like.device):
             call("nd_loss_forward", ctypes.byref(args), stream_handle(like.device))
-        ctx.weights, ctx.scales, ctx.slopes = weights, scales, slopes
-        ctx.has_coefficients = coefficients is not None
-        if any(wanted):
-            ctx.save_for_backward(*((coefficients,) if ctx.has_coefficients else ()), *tensors)
-        return total, *terms
+        ctx.weights, ctx.scales = weights, scales
+        ctx.set_materialize_grads(False)
+        ctx.save_for_backward(coefficients, *slopes)
+        return total, *terms, *slopes
 
     @staticmethod
-    def backward(ctx, total_grad, *term_grads):
+    def backward(ctx, total_grad, *rest):
         count = len(ctx.weights)
-        if torch.is_grad_enabled():  # a graph of this backward is asked for
-            gradients = _defined_backward(ctx, total_grad, term_grads)
+        term_grads, slope_grads = rest[:count], rest[count:]
+        coefficients, *slopes = ctx.saved_tensors
+        given = [g for g in (total_grad, *term_grads) if g is not None]
+        if (torch.is_grad_enabled() or any(g is not None for g in slope_grads)
+                or not _plain_context() or not all(_addressable(g, slopes) for g in given)):
+            gradients = [_gradient(ctx, c, slope, coefficients, total_grad, term_grads[c],
+                                   slope_grads[c]) for c, slope in enumerate(slopes)]
         else:
-            slopes = ctx.slopes
             gradients = [None if slope is None else torch.empty_like(slope) for slope in slopes]
             like = next(slope for slope in slopes if slope is not None)
             args = _loss_args(ctx.weights, [like if s is None else s for s in slopes])
@@ -143,21 +156,30 @@ class _Loss(torch.autograd.Function):
         return (None, None, None, *(None,) * count, *gradients)
 
 
-def _defined_backward(ctx, total_grad, term_grads):
-    """The first derivatives by torch operations, differentiable themselves."""
-    saved, count = ctx.saved_tensors, len(ctx.weights)
-    coefficients, saved = (saved[0], saved[1:]) if ctx.has_coefficients else (None, saved)
-    gradients = []
-    for c, (label, value) in enumerate(zip(saved[:count], saved[count:])):
-        if ctx.slopes[c] is None:
-            gradients.append(None)
-            continue
-        frames, size = value.shape[0], value.numel() // value.shape[0]
-        share = value.new_full((frames,), 1.0 / frames) if coefficients is None else coefficients
-        share = share.reshape(frames, *(1,) * (value.ndim - 1))
-        factor = total_grad * ctx.weights[c] + term_grads[c]
-        gradients.append(factor * share * 2.0 * (value - label) / (size * ctx.scales[c] ** 2))
-    return gradients
+def _addressable(gradient: Tensor, slopes) -> bool:
+    """Whether an incoming gradient is one number of the slopes' dtype in memory (a batched one,
+    of a vectorised Jacobian, has no storage)."""
+    like = next((slope for slope in slopes if slope is not None), None)
+    return (like is not None and type(gradient) is Tensor and torch._C._has_storage(gradient)
+            and gradient.layout is torch.strided and gradient.ndim == 0
+            and gradient.dtype == like.dtype and gradient.device == like.device)
+
+
+def _gradient(ctx, c, slope, coefficients, total_grad, term_grad, slope_grad):
+    """dL/dX of channel c by torch operations, differentiable themselves."""
+    if slope is None:
+        return None
+    parts = []
+    if total_grad is not None:
+        parts.append(total_grad * ctx.weights[c] * slope)
+    if term_grad is not None:
+        parts.append(term_grad * slope)
+    if slope_grad is not None:  # dt_c/dX = 2 k_f (X - Y) / (n s_c^2)
+        frames = slope.shape[0]
+        factor = 2.0 / (slope.numel() // frames * ctx.scales[c] ** 2)
+        parts.append(slope_grad * (factor / frames) if coefficients is None else
+                     slope_grad * (factor * coefficients.reshape(frames, *(1,) * (slope.ndim - 1))))
+    return sum(parts) if parts else None
 
 
 def _loss_args(weights, channels) -> LossArgs:
