@@ -296,9 +296,29 @@ class ReplicaServer:
         record.thermostat[_TIMESTEP] = request.timestep
         return record
 
-    def _stage(self, request: ReplicaRequest) -> _Staged:
-        """The host part of an admission (uploaded by _place)."""
+    def _checked(self, request: ReplicaRequest) -> Replica:
+        """The record of a request whose arrays an admission can take as well: numbers that fill
+        [n, 3] and [n]. Nothing of them is kept."""
         record = self._describe(request)
+        n = record.num_atoms
+        for name, shape in (("positions", (n, 3)), ("velocities", (n, 3)), ("masses", (n,))):
+            value = getattr(request, name)
+            if not (isinstance(value, np.ndarray) and value.dtype.kind in "biuf"):
+                value = np.asarray(value, dtype=np.float64)
+            given = value.shape
+            if given == shape:
+                continue
+            if name == "masses" and given == ():
+                raise IndexError("masses are one value per atom")
+            while len(given) > len(shape) and given[0] == 1:
+                given = given[1:]
+            if np.broadcast_shapes(given, shape) != shape:
+                raise ValueError(f"{name} of shape {value.shape} do not fill {shape}")
+        return record
+
+    def _stage(self, request: ReplicaRequest, record: Replica | None = None) -> _Staged:
+        """The host part of an admission (uploaded by _place)."""
+        record = self._describe(request) if record is None else record
         masses = np.asarray(request.masses, dtype=np.float64)
         if masses.ndim == 0:
             raise IndexError("masses are one value per atom")
@@ -485,19 +505,40 @@ class ReplicaServer:
         A slot keeps its replica in every round launched before the host learns that it
         finished; the kernel clamps each budget to the steps left, so such a replica runs no
         further step, and its slot and room are reused only once those rounds have run.
+
+        Every request is checked before any is launched; after an error no stream runs over the
+        pool any more, and the server holds no room or slot of the call.
         """
         pending = deque(sorted(requests, key=lambda r: r.arrival))
         for request in pending:
             n = request.positions.shape[0]
             if -(-n // _ALIGN) > self.capacity // _ALIGN:
                 raise ValueError(f"a replica of {n} atoms exceeds the server's budget")
+        # Every request is checked before anything is launched for one (10 us each).
+        records = {id(request): self._checked(request) for request in pending}
+        free = list(self._free_units), list(self._free_slots)
         lanes = [_Lane("", torch.cuda.current_stream(self.device), None)]
         if self.large_atoms is not None:
             lanes.append(_Lane("_large", torch.cuda.Stream(self.device), self.large_round_steps))
-        results: list[ReplicaResult] = []
-        staged: dict[int, _Staged] = {}  # by id(request): host work done ahead of admission
         # High priority: the harvest's few small kernels go ahead of the rounds' waiting CTAs.
         side = torch.cuda.Stream(self.device, priority=-1)
+        try:
+            return self._serve(pending, records, lanes, side, realtime)
+        except BaseException:
+            # Nothing may run over the pool, or hold room in it, once the caller has the error.
+            try:
+                for stream in (*(lane.stream for lane in lanes), side):
+                    stream.synchronize()
+            finally:
+                self._free_units, self._free_slots = free
+            raise
+
+    def _serve(self, pending: "deque[ReplicaRequest]", records: dict[int, Replica],
+               lanes: "list[_Lane]", side: torch.cuda.Stream,
+               realtime: bool) -> list[ReplicaResult]:
+        """The loop of ``serve`` over checked requests in the order of their arrivals."""
+        results: list[ReplicaResult] = []
+        staged: dict[int, _Staged] = {}  # by id(request): host work done ahead of admission
         start = time.perf_counter()
 
         def lane_of(request: ReplicaRequest) -> _Lane:
@@ -510,7 +551,7 @@ class ReplicaServer:
                 if realtime and request.arrival > now:
                     break
                 if id(request) not in staged:
-                    staged[id(request)] = self._stage(request)
+                    staged[id(request)] = self._stage(request, records[id(request)])
 
         while pending or any(lane.active or lane.rounds for lane in lanes):
             for lane in lanes:  # room and slots whose last rounds have run
@@ -544,8 +585,9 @@ class ReplicaServer:
                     if work is None:
                         work = sum(entry.work() for other in lanes
                                    for entry in other.active.values())
-                    batch = [(staged.pop(id(request), None) or self._stage(request), slot,
-                              offset) for request, slot, offset in placing[lane.name]]
+                    batch = [(staged.pop(id(request), None) or
+                              self._stage(request, records[id(request)]), slot, offset)
+                             for request, slot, offset in placing[lane.name]]
                     for part in _batches(batch, lambda entry: entry[0].record.num_atoms):
                         self._place(part, lane.name)
                     team = self._team(lane.active.values(), work)
