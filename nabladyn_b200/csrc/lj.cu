@@ -601,6 +601,9 @@ lj_frames_kernel(FramesPass<T> a)
         {
             continue;
         }
+        // E and W of the four columns, summed by themselves: the running sums then take a quarter
+        // of the terms.
+        T four_e = 0, four_xx = 0, four_yy = 0, four_zz = 0, four_xy = 0, four_xz = 0, four_yz = 0;
 #pragma unroll
         for (int k = 0; k < kLaneColumns; ++k)
         {
@@ -626,17 +629,17 @@ lj_frames_kernel(FramesPass<T> a)
                 const T inv_r2 = reciprocal(r2);
                 const T q = c.s2 * inv_r2;
                 const T p6 = q * q * q;
-                energy += c.eps4 * (p6 * p6 - p6) - c.shift;
+                four_e += c.eps4 * (p6 * p6 - p6) - c.shift;
                 const T fs = c.eps24 * (T(2) * p6 * p6 - p6) * inv_r2;
                 px = fs * dx;
                 py = fs * dy;
                 pz = fs * dz;
-                wxx += px * dx;
-                wyy += py * dy;
-                wzz += pz * dz;
-                wxy += px * dy;
-                wxz += px * dz;
-                wyz += py * dz;
+                four_xx += px * dx;
+                four_yy += py * dy;
+                four_zz += pz * dz;
+                four_xy += px * dy;
+                four_xz += px * dz;
+                four_yz += py * dz;
                 add_force<T, kPacked>(a, second[k], -px, -py, -pz);
             }
             const int at = kWarp * k + lane;
@@ -645,6 +648,13 @@ lj_frames_kernel(FramesPass<T> a)
             stage.z[at] = pz;
             stage.key[at] = hit ? first[k] : -1;
         }
+        energy += four_e;
+        wxx += four_xx;
+        wyy += four_yy;
+        wzz += four_zz;
+        wxy += four_xy;
+        wxz += four_xz;
+        wyz += four_yz;
         __syncwarp();
         // The first atoms' side: the lane's four consecutive columns, summed while the atom
         // stays the same.
