@@ -431,8 +431,10 @@ struct RowConstants
     T s2, eps4, eps24, shift;
 };
 
-// 1 / x: a hardware estimate and one Newton step in float32 (within an ulp of the rounded
-// quotient), the division in float64.
+// 1 / x. In float32 a hardware estimate and one Newton step: for normal results the bits of the
+// rounded quotient (every mantissa, exponents 2^-125 to 2^125), in two operations after the
+// estimate where the division takes about eight and a branch (1,048,576 atoms, the kernel: 414
+// and 446 us). In float64 the division.
 __device__ __forceinline__ float reciprocal(float x)
 {
     float y;
@@ -959,18 +961,6 @@ __device__ __forceinline__ PackedAtom<T> gather_gradient(const BackwardPass<T>& 
     }
 }
 
-// 1 / x in float64. A float32 x starts from the hardware estimate (23 bits), doubled twice.
-__device__ __forceinline__ double reciprocal64(float x)
-{
-    float estimate;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(estimate) : "f"(x));
-    double y = estimate;
-    const double d = x;
-    y = fma(y, fma(-d, y, 1.0), y);
-    return fma(y, fma(-d, y, 1.0), y);
-}
-__device__ __forceinline__ double reciprocal64(double x) { return 1.0 / x; }
-
 template <typename T, bool kPacked, bool kTypes>
 __global__ void __launch_bounds__(kLJThreads) lj_parameter_backward_kernel(BackwardPass<T> a)
 {
@@ -1054,7 +1044,7 @@ __global__ void __launch_bounds__(kLJThreads) lj_parameter_backward_kernel(Backw
         const int row =
             kTypes ? pair_row(word_type(left.w), word_type(right.w), f.num_types) : 0;
         const RowGradients c = rows[row];
-        const double inv_r2 = reciprocal64(r2);
+        const double inv_r2 = 1.0 / static_cast<double>(r2);
         const double q = c.s2 * inv_r2;
         const double p6 = q * q * q;
         const double x = tx, y = ty, z = tz;
