@@ -232,6 +232,7 @@ int nd_lj_batch_parameter_backward(const nd_lj_batch_args* args, nd_stream_t str
  * call writes the slopes dt_c/dX where `gradients` is given, the backward call takes them as
  * `predicted` and writes dL/dX. Predictions, labels, coefficients, outputs and incoming
  * gradients are values of `dtype`. */
+#define ND_LOSS_PARTIALS 3553
 typedef struct nd_loss_args {
     int dtype;
     int32_t channels;             /* 1 to 3 */
@@ -242,7 +243,7 @@ typedef struct nd_loss_args {
     double weights[3];
     double scales[3];
     const void* coefficients;     /* k [F]; NULL: 1/F */
-    double* scratch;              /* forward: [4] */
+    double* partials;             /* forward: [ND_LOSS_PARTIALS], any values */
     void* total;                  /* forward: [1] L */
     void* terms[3];               /* forward: [1] t_c each */
     const void* total_grad;       /* backward: [1] or NULL (zero) */

@@ -114,6 +114,9 @@ class LJBatchArgs(ctypes.Structure):
     ]
 
 
+LOSS_PARTIALS = 3553  # ND_LOSS_PARTIALS
+
+
 class LossArgs(ctypes.Structure):
     _fields_ = [
         ("dtype", ctypes.c_int),
@@ -125,7 +128,7 @@ class LossArgs(ctypes.Structure):
         ("weights", ctypes.c_double * 3),
         ("scales", ctypes.c_double * 3),
         ("coefficients", ctypes.c_void_p),
-        ("scratch", ctypes.c_void_p),
+        ("partials", ctypes.c_void_p),
         ("total", ctypes.c_void_p),
         ("terms", ctypes.c_void_p * 3),
         ("total_grad", ctypes.c_void_p),

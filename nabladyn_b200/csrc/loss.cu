@@ -23,6 +23,8 @@ namespace {
 
 constexpr int kChannels = 3;
 constexpr std::int64_t kLossItems = 8;  // elements per thread the grid aims at
+constexpr int kLossBlocks = 148 * 8;    // per channel, at most
+static_assert(ND_LOSS_PARTIALS >= kChannels * kLossBlocks + 1, "a sum per block and the count");
 
 template <typename T>
 struct LossPass
@@ -35,7 +37,7 @@ struct LossPass
     std::int64_t frames;
     const T* coefficients;         // null: 1/F
     int channels;
-    double* sums;                  // [kChannels], then the count of finished blocks
+    double* partials;              // forward: [channels][blocks], then the count of finished blocks
     T* total;
     T* terms[kChannels];
     const T* total_grad;           // backward: null means zero
@@ -66,40 +68,61 @@ __global__ void __launch_bounds__(kThreads) loss_forward_kernel(LossPass<T> a)
             slopes[i] = static_cast<T>(share * frame) * error / scale;  // 2 k (X - Y) / (s^2 n)
         }
     }
-    __shared__ double partial[kThreads / kWarp];
-    sum = warp_sum(sum);
-    if (threadIdx.x % kWarp == 0)
+    __shared__ double warp_sums[kThreads / kWarp];
+    __shared__ bool last;
+    // One block sum per block, in a fixed order; thread 0 gets it.
+    auto block_sum = [&](double value) {
+        value = warp_sum(value);
+        if (threadIdx.x % kWarp == 0)
+        {
+            warp_sums[threadIdx.x / kWarp] = value;
+        }
+        __syncthreads();
+        double all = 0.0;
+        for (int w = 0; w < kThreads / kWarp && threadIdx.x == 0; ++w)
+        {
+            all += warp_sums[w];
+        }
+        __syncthreads();
+        return all;
+    };
+    sum = block_sum(sum);
+    if (threadIdx.x == 0)
     {
-        partial[threadIdx.x / kWarp] = sum;
+        a.partials[c * gridDim.x + blockIdx.x] = sum;
+        __threadfence();
+        auto* finished = reinterpret_cast<unsigned*>(a.partials + a.channels * gridDim.x);
+        last = atomicAdd(finished, 1u) == gridDim.x * gridDim.y - 1;
     }
     __syncthreads();
-    if (threadIdx.x != 0)
+    if (!last)
     {
         return;
     }
-    for (int w = 1; w < kThreads / kWarp; ++w)
-    {
-        sum += partial[w];
-    }
-    atomicAdd(a.sums + c, sum);
-    __threadfence();
-    auto* finished = reinterpret_cast<unsigned*>(a.sums + kChannels);
-    if (atomicAdd(finished, 1u) != gridDim.x * gridDim.y - 1)
-    {
-        return;
-    }
-    // The last block: every sum is complete.
+    // The last block to finish: every block's sum is there. They are added in the blocks' order,
+    // whichever block this is, so a loss has the same bits each time.
     __threadfence();
     double total = 0.0;
     for (int k = 0; k < a.channels; ++k)
     {
-        const double all = *reinterpret_cast<volatile double*>(a.sums + k);
-        const double term = all / static_cast<double>(a.size[k]) /
-                            (a.coefficients != nullptr ? 1.0 : static_cast<double>(a.frames));
-        *a.terms[k] = static_cast<T>(term);
-        total += a.weight[k] * term;
+        double part = 0.0;
+        for (unsigned i = threadIdx.x; i < gridDim.x; i += kThreads)
+        {
+            part += *reinterpret_cast<volatile double*>(a.partials + k * gridDim.x + i);
+        }
+        part = block_sum(part);
+        if (threadIdx.x == 0)
+        {
+            const double term = part / static_cast<double>(a.size[k]) /
+                                (a.coefficients != nullptr ? 1.0 : static_cast<double>(a.frames));
+            *a.terms[k] = static_cast<T>(term);
+            total += a.weight[k] * term;
+        }
     }
-    *a.total = static_cast<T>(total);
+    if (threadIdx.x == 0)
+    {
+        *a.total = static_cast<T>(total);
+    }
 }
 
 // dL/dX = (w_c dL + dt_c) slope, the slopes in `predicted`.
@@ -141,7 +164,7 @@ LossPass<T> loss_pass(const nd_loss_args& s)
     a.frames = s.frames;
     a.coefficients = static_cast<const T*>(s.coefficients);
     a.channels = s.channels;
-    a.sums = s.scratch;
+    a.partials = s.partials;
     a.total = static_cast<T*>(s.total);
     a.total_grad = static_cast<const T*>(s.total_grad);
     return a;
@@ -173,7 +196,7 @@ dim3 loss_grid(const nd_loss_args& s)
         most = std::max(most, s.sizes[c] * s.frames);
     }
     const std::int64_t blocks = (most + kThreads * kLossItems - 1) / (kThreads * kLossItems);
-    return dim3(static_cast<unsigned>(std::min<std::int64_t>(blocks, 148 * 8)),
+    return dim3(static_cast<unsigned>(std::min<std::int64_t>(blocks, kLossBlocks)),
                 static_cast<unsigned>(s.channels));
 }
 
@@ -190,20 +213,22 @@ int nd_loss_forward(const nd_loss_args* args, nd_stream_t stream_handle)
     {
         return rc;
     }
-    ND_REQUIRE(args->total && args->scratch, "an output is null");
+    ND_REQUIRE(args->total && args->partials, "an output is null");
     for (int c = 0; c < args->channels; ++c)
     {
         ND_REQUIRE(args->terms[c], "an output is null");
     }
     auto stream = static_cast<cudaStream_t>(stream_handle);
-    ND_CUDA_TRY(cudaMemsetAsync(args->scratch, 0, (kChannels + 1) * sizeof(double), stream));
+    const dim3 grid = loss_grid(*args);
+    ND_CUDA_TRY(cudaMemsetAsync(args->partials + static_cast<std::int64_t>(grid.x) * grid.y, 0,
+                                sizeof(double), stream));
     if (args->dtype == ND_FLOAT32)
     {
-        loss_forward_kernel<float><<<loss_grid(*args), kThreads, 0, stream>>>(loss_pass<float>(*args));
+        loss_forward_kernel<float><<<grid, kThreads, 0, stream>>>(loss_pass<float>(*args));
     }
     else
     {
-        loss_forward_kernel<double><<<loss_grid(*args), kThreads, 0, stream>>>(loss_pass<double>(*args));
+        loss_forward_kernel<double><<<grid, kThreads, 0, stream>>>(loss_pass<double>(*args));
     }
     ND_LAUNCH_CHECK();
     return ND_OK;

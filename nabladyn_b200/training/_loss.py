@@ -13,7 +13,7 @@ import torch
 from torch import Tensor
 from torch.autograd import forward_ad
 
-from .._native import LossArgs, call, dtype_code, on_device, ptr, stream_handle
+from .._native import LOSS_PARTIALS, LossArgs, call, dtype_code, on_device, ptr, stream_handle
 
 CHANNELS = ("energy", "forces", "virial")
 
@@ -119,11 +119,11 @@ class _Loss(torch.autograd.Function):
         wanted = ctx.needs_input_grad[3 + count:]
         slopes = [torch.empty(value.shape, dtype=like.dtype, device=like.device) if want else None
                   for value, want in zip(predicted, wanted)]
-        scratch = torch.empty(4, dtype=torch.float64, device=like.device)
+        partials = torch.empty(LOSS_PARTIALS, dtype=torch.float64, device=like.device)
         kept = [value.contiguous() for value in (*predicted, *labels)]  # until the launch
         shares = None if coefficients is None else coefficients.contiguous()
         args = _loss_args(weights, kept[:count])
-        args.coefficients, args.scratch, args.total = ptr(shares), ptr(scratch), ptr(total)
+        args.coefficients, args.partials, args.total = ptr(shares), ptr(partials), ptr(total)
         for c, term in enumerate(terms):
             args.labels[c], args.scales[c] = ptr(kept[count + c]), scales[c]
             args.terms[c], args.gradients[c] = ptr(term), ptr(slopes[c])
