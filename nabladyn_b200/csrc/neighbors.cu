@@ -184,10 +184,23 @@ __global__ void order_bins_kernel(
 constexpr int kHoodThreads = 128;
 constexpr int kHoodFewThreads = 256;
 constexpr std::int64_t kHoodFewBins = 2 * 148;
+// Where bins outnumber atoms most are empty, and a CTA that finds so costs what the bin's pairs
+// would: a CTA then takes up to 32 bins (kManyCtas of them keep the GPU full; 100,000 atoms among
+// 27 million bins, update: 31.8 ms with a bin per CTA, 3.4 ms). In a gas also the bins with atoms
+// hold few, so a warp takes one by itself (0.7 atoms a bin, float64: 952 us, 586; 2.9 atoms a bin:
+// 461, 349). By the columns, because a droplet in a large box has as many empty bins but full ones
+// too, which want four warps (100,000 atoms of a liquid among 46,000 bins: 227 us, with a warp per
+// bin 690).
+constexpr std::int64_t kManyCtas = 148 * 32;
+constexpr std::int64_t kGasBins = 4;      // a bin for at most four atoms
+constexpr std::int64_t kGasColumns = 12;  // columns per atom at most
 constexpr int kHoodBins = 27;      // the home bin and its stencil, at most
-constexpr int kHoodSlots = 512;    // candidates staged at once (a liquid needs about 410)
-constexpr int kHoodWords = kHoodSlots / kWarp;
-constexpr int kHoodEntries = 3072;  // pairs of 32 centers staged at once (a liquid: 2,000)
+// Candidates staged at once (a liquid needs about 410), and pairs of 32 centers (2,000); few for
+// the one-warp CTAs of sparse bins, of which an SM then holds 32.
+constexpr int kHoodSlots = 512;
+constexpr int kHoodEntries = 3072;
+constexpr int kSparseSlots = 128;
+constexpr int kSparseEntries = 512;
 
 // The part of a home bin's stencil that holds candidates: the home bin (its atoms after the
 // center) and each stencil bin that comes later in bin order (all its atoms). With three or
@@ -364,14 +377,18 @@ __device__ __forceinline__ void shift_in_hits(float x0, float y0, float z0, floa
 
 // The hits of a lane's two centers among the 32 staged candidates from slot `base`: bit 31 - j
 // for candidate base + j, so the first candidate is the highest bit (one instruction finds it).
+// Of the warp's last words the first `groups` groups of eight candidates are tested.
+constexpr int kHoodGroup = 8;
+
 template <typename T, int kImages>
 __device__ __forceinline__ void hit_words(
     const Slot<T>* __restrict__ staged, const unsigned char* __restrict__ ahead, int base,
-    const CenterPair<T>& c, T lx, T ly, T lz, T radius_squared, unsigned& hits0, unsigned& hits1)
+    int groups, const CenterPair<T>& c, T lx, T ly, T lz, T radius_squared, unsigned& hits0,
+    unsigned& hits1)
 {
     hits0 = hits1 = 0;
 #pragma unroll 8
-    for (int j = 0; j < kWarp; ++j)
+    for (int j = 0; j < kHoodGroup * groups; ++j)
     {
         const Slot<T> p = staged[base + j];
         if (kImages == kMinimum)
@@ -396,6 +413,8 @@ __device__ __forceinline__ void hit_words(
             shift_in_hits(c.x0, c.y0, c.z0, c.x1, c.y1, c.z1, p, radius_squared, hits0, hits1);
         }
     }
+    hits0 <<= kWarp - kHoodGroup * groups;
+    hits1 <<= kWarp - kHoodGroup * groups;
 }
 
 // Bits of a word from slot `first` on whose candidates come after center `h` (slots and
@@ -442,15 +461,13 @@ __device__ __forceinline__ void pad_columns(index_t total, index_t num_atoms, in
 }
 
 // Counts (kFill false) or writes (kFill true) the pairs of one home bin. The fill of an update
-// also stores the frame it was built from: each CTA its home atoms' positions, the first the
-// cell and the rebuild count. The fill's first `pad_ctas` CTAs write the padding columns instead:
-// those stores are bound by memory and the fill by instruction issue, so one hides the other
-// (1,048,576 atoms, update: fill 519 us and padding after it 73 us, together 537 us).
+// also stores the frame it was built from, each CTA its home atoms' positions.
 //
 // The candidates, home bin first, are staged kHoodSlots at a time (once, in all but very dense
 // bins) and tested against the bin's atoms 32 at a time.
 template <typename T, bool kFill, int kThreadCount>
-__global__ void __launch_bounds__(kThreadCount) hood_pairs_kernel(
+__device__ __forceinline__ void hood_bin(
+    index_t home,
     const T* __restrict__ sorted_positions,
     const index_t* __restrict__ sorted_ids,
     const index_t* __restrict__ bin_offsets,
@@ -462,26 +479,12 @@ __global__ void __launch_bounds__(kThreadCount) hood_pairs_kernel(
     index_t capacity,
     index_t* __restrict__ pairs,
     const T* __restrict__ positions,
-    T* __restrict__ reference_positions,
-    T* __restrict__ reference_cell,
-    index_t* __restrict__ rebuild_count,
-    const index_t* __restrict__ rebuild,
-    const index_t* __restrict__ status,
-    index_t num_atoms,
-    int pad_ctas
+    T* __restrict__ reference_positions
 )
 {
-    if (!rebuilding(rebuild, status))
-    {
-        return;
-    }
-    if (kFill && static_cast<int>(blockIdx.x) < pad_ctas)
-    {
-        pad_columns(pair_offsets[num_atoms - 1] + pair_counts[num_atoms - 1], num_atoms, capacity,
-                    pairs, blockIdx.x * kThreadCount + threadIdx.x, pad_ctas * kThreadCount);
-        return;
-    }
-    const index_t home = static_cast<index_t>(blockIdx.x) - (kFill ? pad_ctas : 0);
+    constexpr bool kSparse = kThreadCount == kWarp;
+    constexpr int kSlots = kSparse ? kSparseSlots : kHoodSlots, kWords = kSlots / kWarp;
+    constexpr int kEntries = kSparse ? kSparseEntries : kHoodEntries;
     const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
     const index_t begin = bin_offsets[home];
     const int homes = bin_offsets[home + 1] - begin;
@@ -492,24 +495,16 @@ __global__ void __launch_bounds__(kThreadCount) hood_pairs_kernel(
             const std::int64_t id = sorted_ids[begin + k / 3];
             reference_positions[3 * id + k % 3] = positions[3 * id + k % 3];
         }
-        if (home == 0 && threadIdx.x < 3)
-        {
-            reference_cell[threadIdx.x] = cell[threadIdx.x];
-        }
-        if (home == 0 && threadIdx.x == 0)
-        {
-            ++rebuild_count[0];
-        }
     }
     if (homes == 0)
     {
         return;  // the whole CTA
     }
     __shared__ Hood hood;
-    __shared__ Slot<T> staged[kHoodSlots];
-    __shared__ unsigned char ahead[kHoodSlots];
-    __shared__ unsigned words[kFill ? kHoodWords : 1][kWarp + 1];  // one center apart: no conflicts
-    __shared__ std::uint16_t entries[kFill ? kHoodEntries : 1];    // center << 9 | slot
+    __shared__ Slot<T> staged[kSlots];
+    __shared__ unsigned char ahead[kSlots];
+    __shared__ unsigned words[kFill ? kWords : 1][kWarp + 1];  // one center apart: no conflicts
+    __shared__ std::uint16_t entries[kFill ? kEntries : 1];    // center << 9 | slot
     __shared__ int cursors[kWarp];                                 // fill: each center's next column
     __shared__ int warp_counts[kThreadCount / kWarp][kWarp];
     const T lx = cell[0], ly = cell[1], lz = cell[2];
@@ -521,7 +516,7 @@ __global__ void __launch_bounds__(kThreadCount) hood_pairs_kernel(
     __syncthreads();
     const int images = !fixed ? kMinimum : (hood.any_ahead ? kAhead : kPlain);
     const int total = hood.total;
-    const bool once = total <= kHoodSlots;
+    const bool once = total <= kSlots;
     const int half = lane / 16, q = lane % 16;
     for (int group = 0; group < homes; group += kWarp)
     {
@@ -547,10 +542,10 @@ __global__ void __launch_bounds__(kThreadCount) hood_pairs_kernel(
                 cursors[threadIdx.x] = pair_offsets[begin + group + threadIdx.x];
             }
         }
-        const bool packed = kFill && once && region_size <= kHoodEntries;
-        for (int chunk = 0; chunk < total; chunk += kHoodSlots)
+        const bool packed = kFill && once && region_size <= kEntries;
+        for (int chunk = 0; chunk < total; chunk += kSlots)
         {
-            const int size = total - chunk < kHoodSlots ? total - chunk : kHoodSlots;
+            const int size = total - chunk < kSlots ? total - chunk : kSlots;
             if (group == 0 || !once)
             {
                 __syncthreads();  // the last chunk's readers are done
@@ -577,21 +572,25 @@ __global__ void __launch_bounds__(kThreadCount) hood_pairs_kernel(
             const int used = (size + kWarp - 1) / kWarp;
             for (int pair = warp; 2 * pair < used; pair += kThreadCount / kWarp)
             {
-                const int w = 2 * pair + half;  // at most kHoodWords - 1
+                const int w = 2 * pair + half;  // at most kWords - 1
+                // Of a sparse bin's few candidates the groups there are; a liquid's words are full.
+                const int left = size - 2 * kWarp * pair;  // of the first half's word on
+                const int groups = kSparse ? min(kWarp, left + kHoodGroup - 1) / kHoodGroup
+                                           : kWarp / kHoodGroup;
                 unsigned hits0, hits1;
                 if (images == kPlain)
                 {
-                    hit_words<T, kPlain>(staged, ahead, kWarp * w, c, lx, ly, lz, radius_squared,
-                                         hits0, hits1);
+                    hit_words<T, kPlain>(staged, ahead, kWarp * w, groups, c, lx, ly, lz,
+                                         radius_squared, hits0, hits1);
                 }
                 else if (images == kAhead)
                 {
-                    hit_words<T, kAhead>(staged, ahead, kWarp * w, c, lx, ly, lz, radius_squared,
-                                         hits0, hits1);
+                    hit_words<T, kAhead>(staged, ahead, kWarp * w, groups, c, lx, ly, lz,
+                                         radius_squared, hits0, hits1);
                 }
                 else
                 {
-                    hit_words<T, kMinimum>(staged, ahead, kWarp * w, c, lx, ly, lz,
+                    hit_words<T, kMinimum>(staged, ahead, kWarp * w, groups, c, lx, ly, lz,
                                            radius_squared, hits0, hits1);
                 }
                 const int slot = chunk + kWarp * w;
@@ -639,7 +638,7 @@ __global__ void __launch_bounds__(kThreadCount) hood_pairs_kernel(
                     while (hits != 0)
                     {
                         const int j = next_hit(hits);
-                        if (static_cast<unsigned>(at) < static_cast<unsigned>(kHoodEntries))
+                        if (static_cast<unsigned>(at) < static_cast<unsigned>(kEntries))
                         {
                             entries[at] = static_cast<std::uint16_t>(tag + j);
                         }
@@ -700,6 +699,76 @@ __global__ void __launch_bounds__(kThreadCount) hood_pairs_kernel(
             }
         }
         __syncthreads();  // the next group's cursors, words and counts
+    }
+}
+
+// A home bin per CTA, or with kMany up to 32 bins, of which it takes those with atoms. An
+// update's fill stores the cell and the rebuild count in its first bin's CTA. The fill's first
+// `pad_ctas` CTAs write the padding columns instead: those stores are bound by memory and the fill
+// by instruction issue, so one hides the other (1,048,576 atoms, update: fill 519 us and padding
+// after it 73 us, together 537 us).
+template <typename T, bool kFill, int kThreadCount, bool kMany>
+__global__ void __launch_bounds__(kThreadCount) hood_pairs_kernel(
+    const T* __restrict__ sorted_positions,
+    const index_t* __restrict__ sorted_ids,
+    const index_t* __restrict__ bin_offsets,
+    const index_t* __restrict__ dims,
+    const T* __restrict__ cell,
+    T radius_squared,
+    index_t* __restrict__ pair_counts,
+    const index_t* __restrict__ pair_offsets,
+    index_t capacity,
+    index_t* __restrict__ pairs,
+    const T* __restrict__ positions,
+    T* __restrict__ reference_positions,
+    T* __restrict__ reference_cell,
+    index_t* __restrict__ rebuild_count,
+    const index_t* __restrict__ rebuild,
+    const index_t* __restrict__ status,
+    index_t num_atoms,
+    int pad_ctas,
+    index_t num_bins
+)
+{
+    if (!rebuilding(rebuild, status))
+    {
+        return;
+    }
+    if (kFill && static_cast<int>(blockIdx.x) < pad_ctas)
+    {
+        pad_columns(pair_offsets[num_atoms - 1] + pair_counts[num_atoms - 1], num_atoms, capacity,
+                    pairs, blockIdx.x * kThreadCount + threadIdx.x, pad_ctas * kThreadCount);
+        return;
+    }
+    const index_t cta = static_cast<index_t>(blockIdx.x) - (kFill ? pad_ctas : 0);
+    if (kFill && reference_positions != nullptr && cta == 0)
+    {
+        if (threadIdx.x < 3)
+        {
+            reference_cell[threadIdx.x] = cell[threadIdx.x];
+        }
+        if (threadIdx.x == 0)
+        {
+            ++rebuild_count[0];
+        }
+    }
+    if (!kMany)
+    {
+        hood_bin<T, kFill, kThreadCount>(cta, sorted_positions, sorted_ids, bin_offsets, dims, cell,
+                                         radius_squared, pair_counts, pair_offsets, capacity,
+                                         pairs, positions, reference_positions);
+        return;
+    }
+    // A CTA's bins lie `ctas` apart, so the bins of a droplet go to many CTAs.
+    const std::int64_t ctas = gridDim.x - (kFill ? pad_ctas : 0);
+    const std::int64_t mine = cta + ctas * static_cast<std::int64_t>(threadIdx.x % kWarp);
+    const bool some = mine < num_bins && bin_offsets[mine] != bin_offsets[mine + 1];
+    for (unsigned bins = __ballot_sync(kFullMask, some); bins != 0; bins &= bins - 1)
+    {
+        const auto home = static_cast<index_t>(cta + ctas * (__ffs(static_cast<int>(bins)) - 1));
+        hood_bin<T, kFill, kThreadCount>(home, sorted_positions, sorted_ids, bin_offsets, dims,
+                                         cell, radius_squared, pair_counts, pair_offsets, capacity,
+                                         pairs, positions, reference_positions);
     }
 }
 
@@ -1136,21 +1205,37 @@ void launch_hood(const T* cell, std::int64_t n, double radius, const List& list,
     const std::int64_t most = std::min<std::int64_t>(blocks_for(b.capacity), kPadBlocks);
     const std::int64_t pad =
         kFill ? std::min(most, std::max(kPadCtas, b.capacity / kPadColumns)) : 0;
+    // A list that has its pairs says by its columns whether its atoms are a gas; a first count
+    // does not know, and may be of a droplet in a large box.
+    const bool gas = b.capacity > 1 && b.capacity <= kGasColumns * n && kGasBins * bins > n;
+    const std::int64_t per_cta =
+        gas || bins > n
+            ? std::min<std::int64_t>(kWarp, std::max<std::int64_t>(1, bins / kManyCtas))
+            : 1;
+    const std::int64_t ctas = (bins + per_cta - 1) / per_cta;
     auto launch = [&](auto kernel, int threads) {
-        kernel<<<static_cast<unsigned>(bins + pad), threads, 0, stream>>>(
+        kernel<<<static_cast<unsigned>(ctas + pad), threads, 0, stream>>>(
             static_cast<const T*>(b.sorted_positions), b.sorted_ids, b.bin_offsets, b.dims, cell,
             r * r, b.pair_counts, b.pair_offsets, static_cast<index_t>(b.capacity), b.pairs,
             commit.positions, commit.reference_positions, commit.reference_cell,
             commit.rebuild_count, list.rebuild, b.status, static_cast<index_t>(n),
-            static_cast<int>(pad));
+            static_cast<int>(pad), static_cast<index_t>(bins));
     };
-    if (bins <= kHoodFewBins)
+    if (gas)
     {
-        launch(hood_pairs_kernel<T, kFill, kHoodFewThreads>, kHoodFewThreads);
+        launch(hood_pairs_kernel<T, kFill, kWarp, true>, kWarp);
+    }
+    else if (per_cta > 1)
+    {
+        launch(hood_pairs_kernel<T, kFill, kHoodThreads, true>, kHoodThreads);
+    }
+    else if (bins <= kHoodFewBins)
+    {
+        launch(hood_pairs_kernel<T, kFill, kHoodFewThreads, false>, kHoodFewThreads);
     }
     else
     {
-        launch(hood_pairs_kernel<T, kFill, kHoodThreads>, kHoodThreads);
+        launch(hood_pairs_kernel<T, kFill, kHoodThreads, false>, kHoodThreads);
     }
 }
 
