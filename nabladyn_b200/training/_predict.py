@@ -86,14 +86,17 @@ def predict(model: LennardJones, parameters: Mapping[str, Tensor], positions: Te
     unknown = set(channels) - set(CHANNELS)
     if not channels or unknown:
         raise ValueError(f"channels must be a nonempty subsequence of {CHANNELS}")
+    if cells.shape != (positions.shape[0], 3) or cells.device != positions.device:
+        raise ValueError(f"cells must be a [{positions.shape[0]}, 3] tensor on {positions.device}")
+    dtype = torch.promote_types(positions.dtype, cells.dtype)
+    positions, cells = positions.detach().to(dtype), cells.detach().to(dtype)
     sigma = parameters.get("sigma", model.sigma)
     epsilon = parameters.get("epsilon", model.epsilon)
     stack = stacks[-1]
     if stack.dtype != torch.int32:
         stack = stack.to(torch.int32)
     energy, forces, virial = _BatchLJ.apply(
-        sigma, epsilon, positions.detach().contiguous(), cells.detach().contiguous(),
-        stack.contiguous(),
+        sigma, epsilon, positions.contiguous(), cells.contiguous(), stack.contiguous(),
         model._kernel_types, model.num_types, model.cutoff,
     )
     values = {"energy": energy, "forces": forces, "virial": virial}
