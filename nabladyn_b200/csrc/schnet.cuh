@@ -21,13 +21,13 @@ constexpr int kHidden = 32;      // the readout's hidden layer, features / 2
 constexpr int kTile = 128;       // rows per tensor-core tile = threads per CTA
 constexpr int kImagesPerBlock = 10;
 constexpr float kLn2 = 0.693147180559945309f;
-constexpr int kGatherBatch = 2;  // feature words (8 features) a pair kernel gathers before use
 
 // Status bits of the SchNet status word.
 constexpr int kBadPair = 1;       // a pair index outside [0, N)
 constexpr int kProductLost = 16;  // a tensor-core product did not complete in time
 
-// Weight images of one block, in this order.
+// Weight images of one block, in this order. The two transposes of the filter layers are part of the
+// block's layout only: the reverse passes read the layers' own images the other way.
 enum Image : int
 {
     kB1 = 0,   // filter1.weight [64 out][K in, zero-padded to 64]
@@ -96,13 +96,6 @@ struct Workspace
     }
 };
 
-__device__ __forceinline__ float approx_reciprocal(float x)
-{
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 constexpr float kLog2E = 1.44269504088896340736f;
 
 // The hardware exponential and logarithm of base two, denormals flushed (one instruction each;
@@ -145,26 +138,6 @@ __device__ __forceinline__ float sigmoid(float x)
     float t;
     asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.5f * x));
     return fmaf(0.5f, t, 0.5f);
-}
-
-// Feature rows that the pair kernels gather (v = x A^T and Gm) are kept in BF16: 128 B per
-// row, read 16 bytes at a time. Eight consecutive features (the word at group = 8 row +
-// feature / 8), widened to floats.
-__device__ __forceinline__ void widen8(const uint4& word, float (&out)[8])
-{
-    const std::uint32_t w[4] = {word.x, word.y, word.z, word.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-    {
-        out[2 * i] = __uint_as_float(w[i] << 16);
-        out[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-    }
-}
-
-__device__ __forceinline__ void load8(const uint4* __restrict__ rows, std::int64_t group,
-                                      float (&out)[8])
-{
-    widen8(__ldg(rows + group), out);
 }
 
 __device__ __forceinline__ std::uint32_t pack2(float lo, float hi)
@@ -336,7 +309,8 @@ __device__ __forceinline__ void store_basis(unsigned char* tile, float r_over_wi
     }
 }
 
-// Feature lanes. A tile's products leave one pair per thread, but the gathers and scatters of
+// Feature lanes. The feature rows that the pair kernels gather (v = x A^T and Gm) are kept in BF16,
+// 128 bytes a row. A tile's products leave one pair per thread, but the gathers and scatters of
 // feature rows (128 or 256 bytes each) want a row per few lanes: a thread per row touches 32
 // lines per instruction, and those accesses, not the arithmetic, bound the pair kernels (75 %
 // of the load/store unit's wavefronts). So the half's 32 columns of a pair's FP32 filter go
