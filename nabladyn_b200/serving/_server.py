@@ -296,13 +296,17 @@ class ReplicaServer:
         record.thermostat[_TIMESTEP] = request.timestep
         return record
 
-    def _checked(self, request: ReplicaRequest) -> Replica:
-        """The record of a request whose arrays an admission can take as well: numbers that fill
-        [n, 3] and [n]. Nothing of them is kept."""
-        record = self._describe(request)
-        n = record.num_atoms
-        for name, shape in (("positions", (n, 3)), ("velocities", (n, 3)), ("masses", (n,))):
-            value = getattr(request, name)
+    @staticmethod
+    def _check(request: ReplicaRequest) -> None:
+        """Raises where an admission would: the atom count, the cell, and arrays that are not
+        numbers filling [n, 3] and [n]."""
+        n = request.positions.shape[0]
+        if not 2 <= n <= 65535:
+            raise ValueError("a replica holds 2 to 65535 atoms")
+        check_cell_lengths([float(x) for x in request.cell], request.cutoff)
+        for name, value, shape in (("positions", request.positions, (n, 3)),
+                                   ("velocities", request.velocities, (n, 3)),
+                                   ("masses", request.masses, (n,))):
             if not (isinstance(value, np.ndarray) and value.dtype.kind in "biuf"):
                 value = np.asarray(value, dtype=np.float64)
             given = value.shape
@@ -314,11 +318,10 @@ class ReplicaServer:
                 given = given[1:]
             if np.broadcast_shapes(given, shape) != shape:
                 raise ValueError(f"{name} of shape {value.shape} do not fill {shape}")
-        return record
 
-    def _stage(self, request: ReplicaRequest, record: Replica | None = None) -> _Staged:
+    def _stage(self, request: ReplicaRequest) -> _Staged:
         """The host part of an admission (uploaded by _place)."""
-        record = self._describe(request) if record is None else record
+        record = self._describe(request)
         masses = np.asarray(request.masses, dtype=np.float64)
         if masses.ndim == 0:
             raise IndexError("masses are one value per atom")
@@ -514,8 +517,7 @@ class ReplicaServer:
             n = request.positions.shape[0]
             if -(-n // _ALIGN) > self.capacity // _ALIGN:
                 raise ValueError(f"a replica of {n} atoms exceeds the server's budget")
-        # Every request is checked before anything is launched for one (10 us each).
-        records = {id(request): self._checked(request) for request in pending}
+            self._check(request)  # before anything is launched for another one (3 us each)
         free = list(self._free_units), list(self._free_slots)
         lanes = [_Lane("", torch.cuda.current_stream(self.device), None)]
         if self.large_atoms is not None:
@@ -523,7 +525,7 @@ class ReplicaServer:
         # High priority: the harvest's few small kernels go ahead of the rounds' waiting CTAs.
         side = torch.cuda.Stream(self.device, priority=-1)
         try:
-            return self._serve(pending, records, lanes, side, realtime)
+            return self._serve(pending, lanes, side, realtime)
         except BaseException:
             # Nothing may run over the pool, or hold room in it, once the caller has the error.
             try:
@@ -533,9 +535,8 @@ class ReplicaServer:
                 self._free_units, self._free_slots = free
             raise
 
-    def _serve(self, pending: "deque[ReplicaRequest]", records: dict[int, Replica],
-               lanes: "list[_Lane]", side: torch.cuda.Stream,
-               realtime: bool) -> list[ReplicaResult]:
+    def _serve(self, pending: "deque[ReplicaRequest]", lanes: "list[_Lane]",
+               side: torch.cuda.Stream, realtime: bool) -> list[ReplicaResult]:
         """The loop of ``serve`` over checked requests in the order of their arrivals."""
         results: list[ReplicaResult] = []
         staged: dict[int, _Staged] = {}  # by id(request): host work done ahead of admission
@@ -551,7 +552,7 @@ class ReplicaServer:
                 if realtime and request.arrival > now:
                     break
                 if id(request) not in staged:
-                    staged[id(request)] = self._stage(request, records[id(request)])
+                    staged[id(request)] = self._stage(request)
 
         while pending or any(lane.active or lane.rounds for lane in lanes):
             for lane in lanes:  # room and slots whose last rounds have run
@@ -585,9 +586,8 @@ class ReplicaServer:
                     if work is None:
                         work = sum(entry.work() for other in lanes
                                    for entry in other.active.values())
-                    batch = [(staged.pop(id(request), None) or
-                              self._stage(request, records[id(request)]), slot, offset)
-                             for request, slot, offset in placing[lane.name]]
+                    batch = [(staged.pop(id(request), None) or self._stage(request), slot,
+                              offset) for request, slot, offset in placing[lane.name]]
                     for part in _batches(batch, lambda entry: entry[0].record.num_atoms):
                         self._place(part, lane.name)
                     team = self._team(lane.active.values(), work)

@@ -74,7 +74,8 @@ def test_what_an_admission_takes_is_accepted(server):
     for given in ({"masses": np.full(1, 39.948)}, {"velocities": np.zeros(3)},
                   {"velocities": np.zeros((1, 64, 3), dtype=np.float32)},
                   {"positions": torch.zeros(64, 3)}, {"masses": [39] * 64}):
-        assert server._checked(request(64, **given)).num_atoms == 64
+        server._check(request(64, **given))
+        assert server._stage(request(64, **given)).record.num_atoms == 64
 
 
 def test_a_failed_launch_leaves_nothing_running_and_nothing_taken(server, monkeypatch):
