@@ -275,11 +275,11 @@ __global__ void __launch_bounds__(kLJThreads) lj_pairs_kernel(
 //     lanes that end on the same first atom meet in a segmented warp sum, and a first atom
 //     costs two or three atomics instead of one per column. An index in any other order gives
 //     the same sums with more atomics.
-// Measured, float32, the whole call: 1,048,576 atoms (64 million columns) 1,765 -> 432 us, of
-// which packing and wide atomics 587, a column per lane in the gathers and atomics 525, 16-byte
-// reads of the staged forces and padding skipped 432; 27,000 atoms of two types 165 -> 47 us; 512
-// atoms in float64 150 -> 47 us. At the largest the L1 pipe is busy 76 % of the time (gathers and
-// atomics of lines that are random in memory) and issue 62 %.
+// Measured, float32, the whole call: 1,048,576 atoms (64 million columns) 1,765 -> 428 us, 415 of it
+// this kernel; step by step 587 with packing and wide atomics, 525 with a column per lane in the
+// gathers and atomics, 432 with 16-byte reads of the staged forces and padding skipped. 27,000
+// atoms of two types 165 -> 47 us; 512 atoms in float64 150 -> 47 us. At the largest the L1 pipe
+// is busy 79 % of the time (gathers and atomics of lines that are random in memory), issue 67 %.
 
 // Blocks an SM holds: the registers of four columns in flight, 80 (float32) or 124 (float64).
 template <typename T>
@@ -924,7 +924,7 @@ int lj_pairs(const nd_lj_pairs_args* a, cudaStream_t stream)
 // slots it is bound by the float64 arithmetic: the row's constants are worked out once per
 // block, and a thread keeps its rows' sums to itself (in registers for one row, else in its own
 // column of shared memory), since float64 atomics on a few shared words serialise the block
-// (64 frames of 4,096 atoms, two types, float32: 778 -> 99 us; gathering the force gradients before
+// (64 frames of 4,096 atoms, two types, float32: 778 -> 98 us; gathering the force gradients before
 // the cutoff test, or six blocks per SM at 40 registers, gave 100).
 
 // One type-pair row's float64 constants.

@@ -174,9 +174,10 @@ __global__ void order_bins_kernel(
 // appended by a thread of their own: a center's words find their columns by a 16-lane scan.
 // A bin's columns are one contiguous range, so entries go to shared memory first and leave in
 // whole lines. 1,048,576 atoms, float32, the whole update: 1,710 us with a warp per home bin and
-// appends by the centers' lanes, 952 us so (count 216, fill 519: issue 72 and 78 % busy). A warp
-// per center with a lane per candidate (ranks by popcounts) took 575 us for the fill, ten or
-// twelve CTAs per SM (48 or 40 registers, spilling) 545 and 528 us.
+// appends by the centers' lanes, 903 us so (count 216, fill with the padding 537: issue 73 and
+// 78 % busy). Without the padding the fill took 519; a warp per center with a lane per candidate
+// (ranks by popcounts) took 575, ten or twelve CTAs per SM (48 or 40 registers, spilling) 545 and
+// 528 us.
 
 // Threads per CTA: four warps share a bin's words where the bins fill the GPU (7 CTAs per SM);
 // with at most two bins per SM eight warps shorten the one wave there is (64 bins of a

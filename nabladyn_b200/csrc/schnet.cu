@@ -251,9 +251,9 @@ struct PairPass
 // in the row tile, free by then), biases, the pairs' atoms and envelopes, barrier and
 // tensor-memory slot.
 //
-// What bounds the pair passes is the special-function unit (47 % busy forward, 40 % reverse), the
-// shared-memory passes between products and the atomics, in a chain of dependent steps per tile;
-// the tensor pipe is busy 8 % of the time. A row's features are gathered and scattered by eight
+// What bounds the pair passes are the shared-memory passes between products (65 % of the load/store
+// wavefronts forward, 54 % reverse), the special-function unit (36 %, 31-40 %) and the atomics, in
+// a chain of dependent steps per tile; the tensor pipe is busy 6-8 % of the time. A row's features are gathered and scattered by eight
 // lanes, 16 bytes each, so a warp's load covers four whole rows; with a thread per row each load
 // touched 32. 32,768 beads, 1.19 million pairs: forward 269 -> 157 us, reverse 533 -> 300 us (the
 // last pass 241), the E/F/W call 2,210 -> 1,510 us. Unrolled over the two column halves the kernels overflow the

@@ -296,8 +296,8 @@ __global__ void __launch_bounds__(kTile, 4) tangent_forward_kernel(TangentPass a
 }
 
 // The reverse pass. 32,768 beads, 1.19 million pairs: 1,200 -> 615 us (the forward pass 520 ->
-// 253 us), bound by the latency of a tile's steps and the shared-memory passes (59 % of the
-// wavefronts), then by the 1.3 GB of rows it writes (28 % of the DRAM's peak).
+// 253 us), bound by the latency of a tile's steps and the shared-memory passes (61 % of the
+// wavefronts), then by the 1.3 GB of rows it writes (27 % of the DRAM's peak).
 //
 // A tile's steps form one long chain (four products with row-wise work between
 // them), so two CTAs share an SM (tensor memory holds no more: z, z_dot, u and u_dot are 256
