@@ -12,6 +12,8 @@ from collections.abc import Mapping
 import torch
 from torch import Tensor
 from torch.autograd import forward_ad
+from torch.overrides import _get_current_function_mode_stack
+from torch.utils._device import DeviceContext
 
 from .._native import LOSS_PARTIALS, LossArgs, call, dtype_code, on_device, ptr, stream_handle
 
@@ -65,11 +67,14 @@ def _defined(predicted, labels, weights, scales, coefficients):
 
 def _plain_context() -> bool:
     """Whether nothing watches or transforms torch operations: no functorch transform,
-    forward-mode level, trace or dispatch mode, which see the operations of a formula and would
-    not see a kernel."""
+    forward-mode level, trace, dispatch or function mode, which see the operations of a formula
+    and would not see a kernel. (A default device is a function mode that watches nothing.)"""
     return not (torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0
                 or torch.compiler.is_compiling() or torch.jit.is_tracing()
-                or torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack())
+                or torch._C._len_torch_dispatch_stack()
+                or (torch._C._len_torch_function_stack()
+                    and any(not isinstance(mode, DeviceContext)
+                            for mode in _get_current_function_mode_stack())))
 
 
 def _one_kernel(predicted, labels, weights, scales, coefficients) -> bool:

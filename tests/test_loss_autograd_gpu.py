@@ -142,3 +142,9 @@ def test_a_dispatch_mode_sees_the_operations(case):
         training.loss({k: v.detach() for k, v in predicted.items()}, labels, WEIGHTS, SCALES,
                       coefficients)
     assert any("sub" in name for name in Names.seen) and any("mean" in n for n in Names.seen)
+
+
+def test_a_default_device_keeps_the_kernel(case):
+    with torch.device("cuda"):
+        total, _ = kernel(case)  # asserts the kernel's node
+    torch.testing.assert_close(total, defined(case)[0], **CLOSE)
