@@ -259,6 +259,7 @@ __global__ void __launch_bounds__(kTile, 4) tangent_forward_kernel(TangentPass a
                     {
                         const float raw_filter = u[4 * q + e] + bias[4 * q + e];
                         f[e] = raw_filter * t.envelope;
+                        // The reverse pass fuses the other product; each as it always has.
                         fd[e] = fmaf(raw_filter, t.moving, ud[4 * q + e] * t.envelope);
                     }
                     stage4(stage, q, make_float4(f[0], f[1], f[2], f[3]));
